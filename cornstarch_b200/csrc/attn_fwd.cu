@@ -21,6 +21,8 @@
 //
 // Replaces the Triton kernels of the reference: cornstarch/kernel/bitfield_attention.py:215-523 (forward,
 // split-KV partials :1279-1436, compressed mask :104-156) and cornstarch/kernel/attention.py:56-345.
+#include <stdlib.h>
+
 #include "host.h"
 #include "kv_segments.h"
 #include "mask.cuh"
@@ -41,7 +43,7 @@ struct AttnFwdParams {
   const int64_t* k_bits;
   const int* q_pos;
   const int* k_pos;
-  const int8_t* cls;
+  const int8_t* cls;  // [B][nQ][nK], or null: index_tile_class decides
   __nv_bfloat16* O;
   long o_stride_b, o_stride_s;  // elements; head stride is D
   float* lse;                   // [B][Hq][Sq]
@@ -56,6 +58,12 @@ struct AttnFwdParams {
   float inv_scale;
   SegInfo seg;
 };
+
+// Class of a tile from the map, or (no map) from the indices.
+__device__ __forceinline__ int8_t tile_class(const AttnFwdParams& p, int b, int qi, int kj) {
+  if (p.cls == nullptr) return static_cast<int8_t>(index_tile_class(p.mask_mode, qi, kj, p.Sq, p.Sk));
+  return p.cls[((long)b * p.nQ + qi) * p.nK + kj];
+}
 
 // ---------------------------------------------------------------------------------------------
 // Tile classification: cls[b][qi][kj] = 0 (no pair allowed) / 2 (every pair allowed) / 1 (mixed).
@@ -207,8 +215,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int q0 = qi * AT_BM;
   {
     // this query tile's row of the class map, read once (every role walks it)
-    const int8_t* cls_g = p.cls + ((long)b * p.nQ + qi) * p.nK;
-    for (int j = threadIdx.x; j < p.nK; j += blockDim.x) cls_s[j] = cls_g[j];
+    for (int j = threadIdx.x; j < p.nK; j += blockDim.x) cls_s[j] = tile_class(p, b, qi, j);
   }
   const int8_t* cls_row = cls_s;
 
@@ -359,6 +366,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (p.q_bits) qb = p.q_bits[(long)b * p.Sq + q];
       if (p.q_pos) qpos = p.q_pos[(long)b * p.Sq + q];
     }
+    const QueryRule rule = make_query_rule(p.mask_mode, row_valid, qb, qpos);
     float m_used = -INFINITY, l_sum = 0.f;
     uint32_t it = 0, n_partial = 0;
     bool ok = true;
@@ -386,8 +394,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           if (half == 0) {
             const int k = j * AT_BN + r;
             const bool kv = k < p.Sk;
-            kb_s[buf * 128 + r] = (kv && p.k_bits) ? p.k_bits[(long)b * p.Sk + k] : 0;
-            kp_s[buf * 128 + r] = kv ? (p.k_pos ? p.k_pos[(long)b * p.Sk + k] : k) : -1;
+            const int kp = kv ? (p.k_pos ? p.k_pos[(long)b * p.Sk + k] : k) : -1;  // negative: a key that does not exist
+            kb_s[buf * 128 + r] = mask_key_bits(p.mask_mode, kp >= 0, (kv && p.k_bits) ? p.k_bits[(long)b * p.Sk + k] : 0);
+            kp_s[buf * 128 + r] = kp;
           }
           mbar_arrive(kb_full);
           if (!at_wait(kb_full, n_partial & 1, abort_flag)) {
@@ -425,11 +434,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            const int kpos = kp[i];
-            const bool allow = row_valid && kpos >= 0 && mask_allowed(p.mask_mode, qb, kb[i], qpos, kpos);
-            s[i] = allow ? s[i] : -INFINITY;
-          }
+          for (int i = 0; i < 64; ++i) s[i] = rule_allows(rule, kb[i], kp[i]) ? s[i] : -INFINITY;
         }
       }
       float mx0 = s[0], mx1 = s[1], mx2 = s[2], mx3 = s[3];
@@ -569,6 +574,8 @@ static int make_qkv_tmap(CUtensorMap* tm, const void* base, int D, int H, int S,
 
 }  // namespace csb
 
+#include "attn_fwd_pair.cuh"
+
 using namespace csb;
 
 // cls: int8 [B][nQ][nK] with nQ = ceil(Sq/bm), nK = ceil(Sk/bn).  row_work (optional, int32 [B][nQ],
@@ -596,11 +603,45 @@ struct CsbAttnExtras {
   long bias_sb, bias_sh, bias_sq;  // element strides (0 = broadcast)
 };
 
+// Two query tiles per thread block (attn_fwd_pair_kernel) or one (attn_fwd_kernel).  A block of the first kind takes 1.3
+// times as long for a key tile and does twice the work, so it wins where the GPU is full: 8192 tokens causal, 32 / 8 heads of
+// 128: 501 against 776 us; 4 x 729 tokens, 16 heads of 72, full: 39 against 57 us.  With fewer blocks than SMs the longest
+// chain of key tiles decides and one tile per block wins (1500 tokens, 8 heads: 23 against 32 us), except for one or two key
+// tiles, where the smaller set-up of the paired kernel does (64 tokens, 32 heads: 6.7 against 8.2 us).  In between, one tile
+// per block needs a second round: always dearer under a full mask (2 x 729 tokens: 18 against 29 us); under masks with a
+// causal part the late blocks are short, and only short chains gain (1024 tokens, 32 heads: 23 against 26 us; 3000 tokens, 8
+// heads: 53 against 38 us).
+static bool use_pairs(const AttnFwdParams& p, int n_seg, bool peers) {
+  if (n_seg != 1 || peers || p.seg.pull_ctas > 0 || p.mask_mode == MASK_DENSE || p.bias != nullptr) return false;
+  const long heads = (long)p.Hq * p.B;
+  if (p.nQ * heads <= sm_count()) return p.nK <= 2;
+  if ((p.nQ + 1) / 2 * heads >= sm_count() || p.mask_mode == MASK_FULL) return true;
+  return p.nK <= 12;
+}
+
+template <int NCH>
+static int launch_fwd_pair_n(const CUtensorMap& tq, const KvMaps& kvm, const AttnFwdParams& p, cudaStream_t s) {
+  auto kfn = attn_fwd_pair_kernel<NCH>;
+  static bool set = false;
+  if (!set) {
+    if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<NCH>::DYN_BYTES) != cudaSuccess) return launch_result();
+    set = true;
+  }
+  const long n_blocks = (long)((p.nQ + 1) / 2) * p.Hq * p.B;
+  if (n_blocks > 0x7fffffffL) return CSB_ERR_TOO_LARGE;
+  kfn<<<(unsigned)n_blocks, PAIR_THREADS, PairSmem<NCH>::DYN_BYTES, s>>>(tq, kvm.k[0], kvm.v[0], p);
+  return launch_result();
+}
+static int launch_fwd_pair(const CUtensorMap& tq, const KvMaps& kvm, const AttnFwdParams& p, cudaStream_t s) {
+  return p.D <= 64 ? launch_fwd_pair_n<1>(tq, kvm, p, s) : launch_fwd_pair_n<2>(tq, kvm, p, s);
+}
+
 static int attn_fwd_seg_impl(const void* q, const CsbKvSegments* kv, void* out, float* lse, int B, int Sq, int Sk, int Hq,
                              int Hk, int D, long q_stride_s, long q_stride_b, long o_stride_s, long o_stride_b, float scale,
                              int mask_mode, const long* q_bits, const long* k_bits, const int* q_pos, const int* k_pos,
                              const signed char* cls, int* status, void* stream, const CsbAttnExtras* ex) {
   if (D % 8 || D > 128 || D < 16 || Hq % Hk) return CSB_ERR_BAD_ARG;
+  if (cls == nullptr && !(mask_mode == MASK_FULL || (mask_mode == MASK_CAUSAL && q_pos == nullptr && k_pos == nullptr))) return CSB_ERR_BAD_ARG;
   if (mask_mode == MASK_DENSE && (ex == nullptr || ex->dmask == nullptr)) return CSB_ERR_BAD_ARG;
   if (kv == nullptr || kv->n_seg < 1 || kv->n_seg > CSB_MAX_SEG) return CSB_ERR_BAD_ARG;
   if ((Sk + AT_BN - 1) / AT_BN > AttnSmem<2>::MAX_NK) return CSB_ERR_TOO_LARGE;
@@ -646,6 +687,7 @@ static int attn_fwd_seg_impl(const void* q, const CsbKvSegments* kv, void* out, 
     if ((r = make_qkv_tmap(&kvm.v[i], vb, D, Hk, kv->rows[g], B, kv->v_stride_s[g], kv->v_stride_b[g]))) return r;
   }
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (use_pairs(p, kv->n_seg, kv->ready_flags != nullptr)) return launch_fwd_pair(tq, kvm, p, s);
   const long n_blocks = (long)p.nQ * Hq * B + p.seg.pull_ctas;
   if (n_blocks > 0x7fffffffL) return CSB_ERR_TOO_LARGE;
   dim3 grid((unsigned)n_blocks);

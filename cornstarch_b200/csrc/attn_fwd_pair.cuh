@@ -1,0 +1,390 @@
+// Attention forward with two 128-row query tiles per thread block (included by attn_fwd.cu).
+//
+// The two tiles ("streams") of a block are neighbours of one head and share every K / V tile that is loaded.  Each stream
+// has its own softmax group of four warps, ONE thread per query row, its own S buffer and its own accumulator in tensor
+// memory (2 x 128 columns of S, 2 x 128 of O).  The MMA warp alternates between the streams:
+//
+//     S0(0) S1(0) | P0V(0) S0(1)  P1V(0) S1(1) | P0V(1) S0(2)  P1V(1) S1(2) | ...
+//
+// so that one group computes exponentials while the tensor core works for the other, and the two softmax warps of a
+// scheduler are in different phases of a tile.  (With one tile per block both warps of a scheduler load, take maxima and
+// store at the same time; the special-function unit and the tensor core then idle in turns.)  One thread per row takes the
+// maximum with three-input instructions and scales and sums in packed pairs; nothing is exchanged between threads.
+// Measured (B200, 32 / 8 heads of 128): 8192 tokens causal 788 -> 495 us (1110 TFLOP/s), full 1329 -> 928 us (1185 TFLOP/s).
+//
+// Hand-overs per stream and tile: s_full (MMA -> softmax) and p_full (softmax -> MMA), strictly alternating, so no parity
+// wait can be two phases behind.  S(next) of a stream is issued after P V of its current tile, whose operand P lives in
+// the columns that S(next) overwrites; s_full of the next tile therefore also says that P V has retired, which is what
+// the lazy rescale of O needs.
+#pragma once
+
+namespace csb {
+
+// Three warpgroups: TMA, MMA and two spare warps; the softmax warps of stream 0; those of stream 1.  The block is launched
+// with 168 registers a thread; the first group hands 80 of them on (88 + 208 + 208 = 3 x 168).
+constexpr int PAIR_THREADS = 384;
+
+template <int NCH>
+struct PairSmem {
+  static constexpr int TILE_BYTES = NCH * CHUNK_BYTES;
+  static constexpr int Q_OFF = 0;                          // two query tiles
+  static constexpr int K_OFF = Q_OFF + 2 * TILE_BYTES;     // two stages
+  static constexpr int V_OFF = K_OFF + 2 * TILE_BYTES;     // two stages
+  static constexpr int META_OFF = V_OFF + 2 * TILE_BYTES;  // per softmax warp: key bits int64[128], key positions int[128]
+  static constexpr int META_WARP = 128 * 12;
+  static constexpr int CLS_OFF = META_OFF + 8 * META_WARP;  // tile classes of both streams
+  static constexpr int MAX_NK = AttnSmem<NCH>::MAX_NK;
+  static constexpr int BAR_OFF = CLS_OFF + 2 * MAX_NK;
+  static constexpr int NBAR = 16;
+  static constexpr int TOTAL = BAR_OFF + NBAR * 8 + 16;
+  static constexpr int DYN_BYTES = TOTAL + 1024;
+};
+
+// Which of the 128 keys of tile j this query row may attend to, as four words of 32 bits (tiles of class 1 only).
+// kb_w / kp_w: this warp's staging area for the keys' bits and positions.
+__device__ __forceinline__ void tile_mask_words(const AttnFwdParams& p, int b, int j, int q, bool row_valid, const QueryRule& rule,
+                                                int lane, int64_t* kb_w, int* kp_w, uint32_t (&w)[4]) {
+  const int k0 = j * AT_BN;
+  const bool by_index = p.mask_mode == MASK_FULL || (p.mask_mode == MASK_CAUSAL && p.q_pos == nullptr && p.k_pos == nullptr);
+  if (by_index) {
+    int n = p.Sk - k0;  // keys of the tile that exist
+    if (p.mask_mode == MASK_CAUSAL) n = min(n, q - k0 + 1);
+    if (!row_valid) n = 0;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int m = n - 32 * g;
+      w[g] = m >= 32 ? 0xffffffffu : (m <= 0 ? 0u : (1u << m) - 1u);
+    }
+    return;
+  }
+  __syncwarp();  // the previous tile's readers are done with the staging area
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = k0 + i * 32 + lane;
+    const bool kv = k < p.Sk;
+    const int kp = kv ? (p.k_pos ? p.k_pos[(long)b * p.Sk + k] : k) : -1;  // a negative position marks a key that does not exist
+    kb_w[i * 32 + lane] = mask_key_bits(p.mask_mode, kp >= 0, (kv && p.k_bits) ? p.k_bits[(long)b * p.Sk + k] : 0);
+    kp_w[i * 32 + lane] = kp;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    uint32_t m = 0;
+#pragma unroll 8
+    for (int i = 0; i < 32; ++i) m |= (rule_allows(rule, kb_w[g * 32 + i], kp_w[g * 32 + i]) ? 1u : 0u) << i;
+    w[g] = m;
+  }
+}
+
+template <int NCH>
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
+attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                     const __grid_constant__ CUtensorMap tm_v, const AttnFwdParams p) {
+  using L = PairSmem<NCH>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
+  uint64_t* q_full = bars;        // [2] per stream
+  uint64_t* k_full = bars + 2;    // [2] per stage
+  uint64_t* k_empty = bars + 4;   // [2]
+  uint64_t* v_full = bars + 6;    // [2]
+  uint64_t* v_empty = bars + 8;   // [2]
+  uint64_t* s_full = bars + 10;   // [2] per stream
+  uint64_t* p_full = bars + 12;   // [2] per stream, 128 arrivals
+  uint64_t* o_full = bars + 14;   // [2] per stream: its last P V has retired
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBAR);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int8_t* cls_s = reinterpret_cast<int8_t*>(smem + L::CLS_OFF);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // heaviest (last) query tiles first, over all heads and batch entries, as in attn_fwd_kernel
+  const int n_hb = p.Hq * p.B;
+  const int n_pairs = (p.nQ + 1) >> 1;
+  const int hb = blockIdx.x % n_hb;
+  const int qp0 = (n_pairs - 1 - (int)blockIdx.x / n_hb) * 2;  // first query tile of the pair
+  const int h = hb % p.Hq, b = hb / p.Hq;
+  const int hk = h / (p.Hq / p.Hk);
+  const int n_streams = qp0 + 1 < p.nQ ? 2 : 1;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    for (int j = threadIdx.x; j < p.nK; j += blockDim.x)
+      cls_s[s * L::MAX_NK + j] = s < n_streams ? tile_class(p, b, qp0 + s, j) : int8_t(0);
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 12; ++i) mbar_init(&bars[i], 1);
+    mbar_init(&p_full[0], 128);
+    mbar_init(&p_full[1], 128);
+    mbar_init(&o_full[0], 1);
+    mbar_init(&o_full[1], 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_S = tmem_base;        // stream s: columns [128 s, +128); P over the first 64 of them
+  const uint32_t tmem_O = tmem_base + 256;  // stream s: columns [128 s, +dk16)
+  const int8_t* cls0 = cls_s;
+  const int8_t* cls1 = cls_s + L::MAX_NK;
+  // next key tile at or after t that either stream needs
+  auto next_tile = [&](int t) -> int {
+    while (t < p.nK && (cls0[t] | cls1[t]) == 0) ++t;
+    return t;
+  };
+
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(&tm_k);
+      tma_prefetch_desc(&tm_v);
+      for (int s = 0; s < n_streams; ++s) {
+        mbar_expect_tx(&q_full[s], L::TILE_BYTES);
+#pragma unroll
+        for (int c = 0; c < NCH; ++c)
+          tma_load_4d(smem + L::Q_OFF + s * L::TILE_BYTES + c * CHUNK_BYTES, &tm_q, &q_full[s], c * 64, h, (qp0 + s) * AT_BM, b);
+      }
+      uint32_t it = 0;
+      for (int t = next_tile(0); t < p.nK; t = next_tile(t + 1), ++it) {
+        const int st = it & 1;
+        const uint32_t ph = (it >> 1) & 1;
+        if (!at_wait(&k_empty[st], ph ^ 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
+        mbar_expect_tx(&k_full[st], L::TILE_BYTES);
+#pragma unroll
+        for (int c = 0; c < NCH; ++c)
+          tma_load_4d(smem + L::K_OFF + st * L::TILE_BYTES + c * CHUNK_BYTES, &tm_k, &k_full[st], c * 64, hk, t * AT_BN, b);
+        if (!at_wait(&v_empty[st], ph ^ 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
+        mbar_expect_tx(&v_full[st], L::TILE_BYTES);
+#pragma unroll
+        for (int c = 0; c < NCH; ++c)
+          tma_load_4d(smem + L::V_OFF + st * L::TILE_BYTES + c * CHUNK_BYTES, &tm_v, &v_full[st], c * 64, hk, t * AT_BN, b);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer (whole warp in step, see umma_f16_w)
+    const uint32_t idesc_s = make_idesc_bf16(AT_BM, AT_BN, 0, 0);
+    const uint32_t idesc_o = make_idesc_bf16(AT_BM, p.dk16, 0, 1);
+    const int ksteps_s = p.dk16 / 16;
+    int last[2] = {-1, -1};  // last key tile of each stream
+    for (int t = 0; t < p.nK; ++t) {
+      if (cls0[t] != 0) last[0] = t;
+      if (cls1[t] != 0) last[1] = t;
+    }
+    bool ok = true;
+    auto fail = [&](int code) {
+      atomicCAS(p.status, 0, code);
+      *abort_flag = 1;
+      ok = false;
+    };
+    // S_s = Q_s K^T with the K tile of ring position it
+    auto issue_s = [&](int s, uint32_t it) {
+      const uint64_t q_desc = make_desc_kmajor_sw128(smem_u32(smem + L::Q_OFF + s * L::TILE_BYTES));
+      const uint64_t k_desc = make_desc_kmajor_sw128(smem_u32(smem + L::K_OFF + (it & 1) * L::TILE_BYTES));
+      for (int kk = 0; kk < ksteps_s; ++kk) {
+        const uint64_t off = static_cast<uint64_t>(((kk >> 2) * CHUNK_BYTES + (kk & 3) * 32) >> 4);
+        umma_f16_w(tmem_S + s * 128, q_desc + off, k_desc + off, idesc_s, kk > 0 ? 1u : 0u);
+      }
+      umma_commit_w(&s_full[s]);
+    };
+    uint32_t done[2] = {0, 0};  // tiles of each stream whose P V was issued
+    int t = next_tile(0);
+    if (t < p.nK) {
+      for (int s = 0; s < n_streams && ok; ++s)
+        if (!at_wait(&q_full[s], 0, abort_flag)) fail(ST_TIMEOUT_FULL);
+      if (ok && !at_wait(&k_full[0], 0, abort_flag)) fail(ST_TIMEOUT_FULL);
+      if (ok) {
+        tc_fence_after();
+        if (cls0[t] != 0) issue_s(0, 0);
+        if (cls1[t] != 0) issue_s(1, 0);
+        umma_commit_w(&k_empty[0]);
+      }
+    }
+    for (uint32_t it = 0; ok && t < p.nK; ++it) {
+      const int tn = next_tile(t + 1);
+      const int st = it & 1;
+      if (!at_wait(&v_full[st], (it >> 1) & 1, abort_flag)) { fail(ST_TIMEOUT_FULL); break; }
+      if (tn < p.nK && !at_wait(&k_full[st ^ 1], ((it + 1) >> 1) & 1, abort_flag)) { fail(ST_TIMEOUT_FULL); break; }
+      tc_fence_after();
+      const uint64_t v_desc = make_desc_mnmajor_sw128(smem_u32(smem + L::V_OFF + st * L::TILE_BYTES), CHUNK_BYTES);
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int8_t* cl = s == 0 ? cls0 : cls1;
+        if (cl[t] != 0) {
+          if (!at_wait(&p_full[s], done[s] & 1, abort_flag)) { fail(ST_TIMEOUT_MISC); break; }
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < AT_BN / 16; ++kk)
+            umma_f16_ts_w(tmem_O + s * 128, tmem_S + s * 128 + kk * 8, v_desc + static_cast<uint64_t>((kk * 2048) >> 4), idesc_o,
+                          (done[s] > 0 || kk > 0) ? 1u : 0u);
+          ++done[s];
+          if (t == last[s]) umma_commit_w(&o_full[s]);
+        }
+        if (tn < p.nK && cl[tn] != 0) issue_s(s, it + 1);
+      }
+      if (!ok) break;
+      umma_commit_w(&v_empty[st]);
+      if (tn < p.nK) umma_commit_w(&k_empty[st ^ 1]);
+      t = tn;
+    }
+    __syncwarp();
+  }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    // ------------------------------------------------------------------ softmax / epilogue: one thread per query row
+    const int s_id = (warp - 4) >> 2;   // stream
+    const int quarter = warp & 3;       // TMEM lane quarter this warp may touch
+    const int r = quarter * 32 + lane;  // row inside the tile == TMEM lane
+    const int q = (qp0 + s_id) * AT_BM + r;
+    const bool row_valid = q < p.Sq;
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t t_S = tmem_S + s_id * 128 + lane_addr;
+    const uint32_t t_O = tmem_O + s_id * 128 + lane_addr;
+    const int8_t* cls_row = s_id == 0 ? cls0 : cls1;
+    int64_t* kb_w = reinterpret_cast<int64_t*>(smem + L::META_OFF + (warp - 4) * L::META_WARP);
+    int* kp_w = reinterpret_cast<int*>(kb_w + 128);
+    int64_t qb = 0;
+    int qpos = q;
+    if (row_valid) {
+      if (p.q_bits) qb = p.q_bits[(long)b * p.Sq + q];
+      if (p.q_pos) qpos = p.q_pos[(long)b * p.Sq + q];
+    }
+    const QueryRule rule = make_query_rule(p.mask_mode, row_valid, qb, qpos);
+    float m_used = -INFINITY, l_sum = 0.f;
+    uint32_t it = 0;
+    bool ok = true;
+    const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    for (int j = 0; j < p.nK; ++j) {
+      const int c = cls_row[j];
+      if (c == 0) continue;
+      uint32_t w[4] = {0u, 0u, 0u, 0u};
+      if (c == 1) tile_mask_words(p, b, j, q, row_valid, rule, lane, kb_w, kp_w, w);  // while S is being computed
+      if (!at_wait(&s_full[s_id], it & 1, abort_flag)) {
+        if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_FULL);
+        *abort_flag = 1;
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      uint32_t v[4][32];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) tmem_ld_32x32(t_S + g * 32, v[g]);
+      tmem_ld_wait();
+      if (c == 1) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[g][i] = ((w[g] >> i) & 1u) ? v[g][i] : 0xff800000u;  // -inf
+      }
+      float mx[4];
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        mx[g] = max3(__uint_as_float(v[g][0]), __uint_as_float(v[g][1]), __uint_as_float(v[g][2]));
+#pragma unroll
+        for (int i = 3; i + 1 < 32; i += 2) mx[g] = max3(mx[g], __uint_as_float(v[g][i]), __uint_as_float(v[g][i + 1]));
+        mx[g] = fmaxf(mx[g], __uint_as_float(v[g][31]));
+      }
+      const float m_new = fmaxf(max3(mx[0], mx[1], mx[2]), fmaxf(mx[3], m_used));
+      const bool need = (m_new - m_used) * p.scale_log2 > 8.f;  // also true when m_used is -inf and m_new is finite
+      if (it > 0 && __any_sync(0xffffffffu, need)) {
+        // rare (lazy rescale); s_full of this tile says that the previous P V of this stream has retired
+        float alpha = 1.f;
+        if (need) alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * p.scale_log2);
+#pragma unroll 1
+        for (int cc = 0; cc < 4 * NCH; ++cc) {
+          uint32_t o[16];
+          tmem_ld_32x16(t_O + cc * 16, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st_32x16(t_O + cc * 16, o);
+        }
+        l_sum *= alpha;
+      }
+      if (need) m_used = m_new;
+      const float m_eff = (m_used == -INFINITY) ? 0.f : m_used * p.scale_log2;
+      const uint64_t negm2 = pack_f32x2(-m_eff, -m_eff);
+      uint64_t ls[2] = {0ull, 0ull};
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const uint64_t x2 = pack_u32x2(v[g][2 * i], v[g][2 * i + 1]);
+          float y0, y1;
+          unpack_f32x2(fma_f32x2(x2, scale2, negm2), y0, y1);
+          const float e0 = fast_exp2(y0), e1 = fast_exp2(y1);
+          ls[i & 1] = add_f32x2(ls[i & 1], pack_f32x2(e0, e1));
+          pk[i] = pack_bf16x2(e0, e1);
+        }
+        tmem_st_32x16(t_S + g * 16, pk);  // P over the first 64 columns of this stream's S (all of S is in registers)
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&p_full[s_id]);
+      {
+        float a0, a1;
+        unpack_f32x2(add_f32x2(ls[0], ls[1]), a0, a1);
+        l_sum += a0 + a1;
+      }
+      ++it;
+    }
+    // ---- epilogue
+    if (ok && it > 0 && !at_wait(&o_full[s_id], 0, abort_flag)) {
+      if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_MISC);
+      *abort_flag = 1;
+      ok = false;
+    }
+    if (ok && s_id < n_streams) {
+      tc_fence_after();
+      const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
+      __nv_bfloat16* o_row = p.O + (long)b * p.o_stride_b + (long)q * p.o_stride_s + (long)h * p.D;
+#pragma unroll
+      for (int cc = 0; cc < 2 * NCH; ++cc) {
+        uint32_t o[32];
+        if (it > 0) {
+          tmem_ld_32x32(t_O + cc * 32, o);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = 0u;
+        }
+        if (row_valid) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            const int col = cc * 32 + g * 8;
+            if (col + 8 <= p.D) {
+              float f[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) f[i] = it > 0 ? __uint_as_float(o[g * 8 + i]) * inv : 0.f;
+              uint4 u;
+              u.x = pack_bf16x2(f[0], f[1]);
+              u.y = pack_bf16x2(f[2], f[3]);
+              u.z = pack_bf16x2(f[4], f[5]);
+              u.w = pack_bf16x2(f[6], f[7]);
+              *reinterpret_cast<uint4*>(o_row + col) = u;
+            }
+          }
+        }
+      }
+      if (row_valid)
+        p.lse[((long)b * p.Hq + h) * p.Sq + q] = l_sum > 0.f ? m_used * p.scale + logf(l_sum) : -INFINITY;
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+}  // namespace csb

@@ -30,4 +30,56 @@ __host__ __device__ __forceinline__ bool mask_allowed(int mode, int64_t qb, int6
   return (mode == MASK_BITFIELD_PREFIX_CAUSAL) && (kpos < qpos);
 }
 
+// The same predicate without branches, for loops over the pairs of a partial tile (the branches above diverge between the
+// rows of a warp and cost tens of cycles per pair).  A query row becomes a rule, a key its bits and position:
+//     allowed = (kpos <= lim  and  (am & kb) != 0)  or  kb == qe
+//   text query      am = its bits,  lim = its position,                 qe = never
+//   modality query  am = all bits,  lim = position - 1 (prefix) / none, qe = its bits
+//   causal / full   am = all bits,  lim = its position / all,           qe = never   (every existing key has kb = 1)
+//   padding, rows that do not exist: lim = none, qe = never.   Keys that do not exist and padding keys: kb = 0.
+struct QueryRule {
+  int64_t am, qe;
+  int lim;
+};
+constexpr int64_t MASK_NEVER = int64_t(1) << 62;  // not a value of 62-bit key bits
+__host__ __device__ __forceinline__ QueryRule make_query_rule(int mode, bool exists, int64_t qb, int qpos) {
+  constexpr int NONE = -2147483647 - 1;
+  QueryRule r{BITFIELD_LOW62, MASK_NEVER, NONE};
+  if (!exists) return r;
+  if (mode == MASK_CAUSAL) {
+    r.lim = qpos;
+  } else if (mode == MASK_FULL || mode == MASK_DENSE) {
+    r.lim = 2147483647;
+  } else {
+    qb &= BITFIELD_LOW62;
+    if (qb & 1) {
+      r.am = qb;
+      r.lim = qpos;
+    } else if (qb != 0) {
+      r.qe = qb;
+      if (mode == MASK_BITFIELD_PREFIX_CAUSAL) r.lim = qpos - 1;
+    }
+  }
+  return r;
+}
+__host__ __device__ __forceinline__ int64_t mask_key_bits(int mode, bool exists, int64_t kb) {
+  if (!exists) return 0;
+  return (mode == MASK_BITFIELD || mode == MASK_BITFIELD_PREFIX_CAUSAL) ? (kb & BITFIELD_LOW62) : 1;
+}
+__host__ __device__ __forceinline__ bool rule_allows(const QueryRule& r, int64_t kb, int kpos) {
+  return ((kpos <= r.lim) & ((r.am & kb) != 0)) | (kb == r.qe);
+}
+
+// Class of the 128 x 128 tile (query tile qi, key tile kj) of a mask that depends on the token indices alone (MASK_FULL, or
+// MASK_CAUSAL without explicit positions): 0 = no allowed pair, 2 = every pair of an existing query row and all 128 keys
+// allowed, 1 = anything else.  What csb_mask_classify stores for these masks, without its launch and its map.
+__host__ __device__ __forceinline__ int index_tile_class(int mode, int qi, int kj, int Sq, int Sk) {
+  const int q0 = qi * 128, k0 = kj * 128;
+  const int q1 = q0 + 128 < Sq ? q0 + 127 : Sq - 1;
+  const bool whole = k0 + 128 <= Sk;
+  if (mode != MASK_CAUSAL) return whole ? 2 : 1;
+  if (k0 > q1) return 0;
+  return whole && k0 + 127 <= q0 ? 2 : 1;
+}
+
 }  // namespace csb
