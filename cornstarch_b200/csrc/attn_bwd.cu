@@ -15,9 +15,9 @@
 // handled by the same CTA.  dQ^T tiles are staged in shared memory as [q][d] rows and added into an fp32
 // accumulator by TMA reduce-add (one 32x32 block per warp), then converted to bf16 by a final pass.
 //
-// Warp roles (576 threads by default): warp 0 = TMA producer (K/V once, Q/dO ring of 3 stages), warp 1 = MMA
-// issuer, warps 2..17 = 512 compute threads (or 2..9 = 256).  Thread (r, group) owns KV row r (TMEM lane r) and 16
-// (32) of the 64 query columns of S^T / dP^T, and head-dim row r of dQ^T.  The pipeline keeps S^T one
+// Warp roles (768 threads by default): warp 0 = TMA producer (K/V once, Q/dO ring of 3 stages), warp 1 = MMA
+// issuer, warps 4..7 = dQ^T drain, warps 8..23 = 512 compute threads (or 8..15 = 256).  Thread (r, group) owns KV row r (TMEM lane r) and 16
+// (32) of the 64 query columns of S^T / dP^T; a drain thread moves head-dim row r of dQ^T.  The pipeline keeps S^T one
 // iteration ahead: while the compute warps turn S^T(i), dP^T(i) into P^T, dS^T, the tensor core
 // already holds S^T(i+1); dP^T(i+1) is issued as soon as dP^T(i) has been read, before the
 // dV/dK/dQ^T MMAs of iteration i, so the next exponentials overlap those MMAs.  Per-tile query
@@ -46,7 +46,7 @@ struct AttnBwdParams {
   const int64_t* k_bits;
   const int* q_pos;
   const int* k_pos;
-  const int8_t* cls;  // [B][nQ128][nK]
+  const int8_t* cls;  // [B][nQ128][nK], or null: index_tile_class decides
   const float* lse;   // [B][Hq][Sq]
   const float* delta; // [B][Hq][Sq]
   float* dq_acc;      // [B][Sq][Hq][D] fp32, zeroed by the caller
@@ -72,8 +72,8 @@ struct BwdSmem {
   static constexpr int DO_OFF = Q_OFF + QSTAGES * 2 * Q_CHUNK;
   static constexpr int DST_OFF = DO_OFF + QSTAGES * 2 * Q_CHUNK;  // dS^T [128 kv][64 q] bf16
   static constexpr int DQ_OFF = DST_OFF + KV_CHUNK;           // dQ staging: 8 warps x [32 q][32 d] fp32 (row-major, 4 KB each)
-  static constexpr int META_OFF = DQ_OFF + 8 * 4096;          // three buffers of: lse2[64] f32, delta*scale[64] f32, qpos[64] i32, qbits[64] i64
-  static constexpr int META_STAGE = 64 * 4 * 3 + 64 * 8;
+  static constexpr int META_OFF = DQ_OFF + 8 * 4096;          // three buffers of: -lse2[64] f32, -delta*scale[64] f32, and the mask rules lim[64] i32, am[64] i64, qe[64] i64
+  static constexpr int META_STAGE = 64 * 4 * 3 + 2 * 64 * 8;
   static constexpr int LIST_OFF = META_OFF + 3 * META_STAGE;  // valid 64-row query tiles of this key block: int16 index, int8 class
   static constexpr int MAX_TILES = 1024;                      // sequences up to 65536 tokens
   static constexpr int BAR_OFF = LIST_OFF + MAX_TILES * 4;
@@ -86,9 +86,13 @@ struct BwdSmem {
 template <int NCW>
 struct BwdCfg {
   static constexpr int COMPUTE_THREADS = NCW * 32;
-  static constexpr int THREADS = 64 + COMPUTE_THREADS;
+  static constexpr int DRAIN_THREADS = 128;  // four warps that only move dQ^T out (one per TMEM lane quarter)
+  static constexpr int THREADS = 128 + DRAIN_THREADS + COMPUTE_THREADS;
+  // Registers a thread after the split (warpgroups of 128 threads: TMA + MMA + two spare warps, drain, compute): with 16
+  // compute warps 80 + 48 + 4 x 88 = 6 x 80, with 8 compute warps 80 + 48 + 2 x 192 = 4 x 128 (what the launch allocates).
+  static constexpr int COMPUTE_REGS = NCW == 16 ? 88 : 192;
   static constexpr int GROUPS = NCW / 4;       // column groups
-  static constexpr int COLS = BW_BQ / GROUPS;  // query columns of S^T / dP^T / dQ^T per thread: 32 or 16
+  static constexpr int COLS = BW_BQ / GROUPS;  // query columns of S^T / dP^T per thread: 32 or 16
 };
 
 __device__ __forceinline__ bool bw_wait(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
@@ -198,7 +202,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     mbar_init(pds_full, CFG::COMPUTE_THREADS);
     mbar_init(pds_empty, 1);
     mbar_init(dq_full, 1);
-    mbar_init(dq_free, CFG::COMPUTE_THREADS);
+    mbar_init(dq_free, CFG::DRAIN_THREADS);
     mbar_init(dp_read, CFG::COMPUTE_THREADS);
     *abort_flag = 0;
     mbar_fence_init();
@@ -208,7 +212,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     int n = 0;
     for (int base = 0; base < p.nQ64 && n < L::MAX_TILES; base += 32) {
       const int i = base + lane;
-      const int8_t c = (i < p.nQ64) ? p.cls[((long)b * p.nQ128 + (i >> 1)) * p.nK + kj] : int8_t(0);
+      int8_t c = 0;
+      if (i < p.nQ64)
+        c = p.cls != nullptr ? p.cls[((long)b * p.nQ128 + (i >> 1)) * p.nK + kj]
+                             : static_cast<int8_t>(index_tile_class(p.mask_mode, i >> 1, kj, p.Sq, p.Sk));
       const uint32_t m = __ballot_sync(0xffffffffu, c != 0);
       const int pos = n + __popc(m & ((1u << lane) - 1u));
       if (c != 0 && pos < L::MAX_TILES) {
@@ -246,6 +253,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tmem_dV = tmem_base + 256;
   const uint32_t tmem_dK = tmem_base + 384;
 
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -359,9 +368,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
     }
     __syncwarp();
-  } else {
+  }
+  } else if (warp >= 8) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CFG::COMPUTE_REGS));
     // ------------------------------------------------------------------ compute threads (NCW warps)
-    const int cw = warp - 2;
+    const int cw = warp - 8;
     const int quarter = warp & 3;       // TMEM lane quarter this warp may touch
     const int half = cw >> 2;           // which group of COLS query columns (of 64) this warp handles
     const int r = quarter * 32 + lane;  // KV row in the tile == TMEM lane; also head-dim row of dQ^T
@@ -370,14 +381,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int kidx = k0 + r;
     const int krow = row0 + r;  // row inside the segment
     const bool k_valid = krow < p.seg.rows[sg];
-    const int64_t kb = (k_valid && p.k_bits) ? p.k_bits[(long)b * p.Sk + kidx] : 0;
+    const int64_t kb = mask_key_bits(p.mask_mode, k_valid, (k_valid && p.k_bits) ? p.k_bits[(long)b * p.Sk + kidx] : 0);
     const int kpos = k_valid ? (p.k_pos ? p.k_pos[(long)b * p.Sk + kidx] : kidx) : -1;
     const float LOG2E = 1.4426950408889634f;
+    const uint64_t scale_log2_2 = pack_f32x2(p.scale_log2, p.scale_log2), scale_2 = pack_f32x2(p.scale, p.scale);
+    const bool by_index = p.mask_mode == MASK_FULL || (p.mask_mode == MASK_CAUSAL && p.q_pos == nullptr && p.k_pos == nullptr);
     // the 64 threads with half == 0 and r < 64 stage the metadata of query row (tile * 64 + r)
     const bool stager = (half == 0) && (r < 64);
 
     float pf_lse = 0.f, pf_delta = 0.f;
-    int pf_qpos = -1;
+    int pf_qpos = 0;
+    bool pf_exists = false;
     int64_t pf_qbits = 0;
     auto prefetch_meta = [&](int it) {
       if (!stager || it >= n_iter) return;
@@ -385,42 +399,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int q = tile_idx[it % n_valid] * BW_BQ + r;
       const bool qv = q < p.Sq;
       const long idx = ((long)b * p.Hq + h) * p.Sq + q;
-      pf_lse = qv ? p.lse[idx] * LOG2E : INFINITY;
-      pf_delta = qv ? p.delta[idx] * p.scale : 0.f;
-      pf_qpos = qv ? (p.q_pos ? p.q_pos[(long)b * p.Sq + q] : q) : -1;
+      pf_lse = qv ? -(p.lse[idx] * LOG2E) : -INFINITY;  // negated: the two uses below are one packed FMA each
+      pf_delta = qv ? -(p.delta[idx] * p.scale) : 0.f;
+      pf_qpos = qv ? (p.q_pos ? p.q_pos[(long)b * p.Sq + q] : q) : 0;
+      pf_exists = qv && pf_qpos >= 0;
       pf_qbits = (qv && p.q_bits) ? p.q_bits[(long)b * p.Sq + q] : 0;
     };
 
     bool ok = true;
-    auto drain_dq = [&](int pit) -> bool {
-      if (!bw_wait(dq_full, pit & 1, abort_flag)) {
-        if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_FULL);
-        *abort_flag = 1;
-        return false;
-      }
-      tc_fence_after();
-      const int ph = hk * group + pit / n_valid;
-      const int pi = tile_idx[pit % n_valid];
-      uint32_t v[COLS];
-      tmem_ld_cols<COLS>(tmem_dQT + col0 + lane_addr, v);
-      tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(dq_free);
-      // this warp's [32 d][COLS q] block -> shared memory as [q][d] rows of 128 B -> one TMA reduce-add into dq_acc
-      if (lane == 0) tma_store_wait_read<0>();  // the previous block has left the staging buffer
-      __syncwarp();
-      float* stage = reinterpret_cast<float*>(smem + L::DQ_OFF + cw * (COLS * 128));
-#pragma unroll
-      for (int c = 0; c < COLS; ++c) stage[c * 32 + lane] = __uint_as_float(v[c]);
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0 && quarter * 32 < p.D) {
-        tma_reduce_add_4d(&tm_dq, stage, quarter * 32, ph, pi * BW_BQ + col0, b);  // box: 32 d x COLS q
-        tma_store_commit();
-      }
-      return true;
-    };
-
     // Query metadata of iteration it lives in buffer it % 3.  The stagers write the metadata of iteration it + 1 right
     // after they hold S^T / dP^T of iteration it in registers and BEFORE they arrive on dp_read(it); the MMA warp issues
     // dP^T(it + 1) only after dp_read(it) is complete, so sdp_full(it + 1) also tells every thread that the metadata is
@@ -431,8 +417,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       float* m = reinterpret_cast<float*>(smem + L::META_OFF + (it % 3) * L::META_STAGE);
       m[r] = pf_lse;
       m[64 + r] = pf_delta;
-      reinterpret_cast<int*>(m + 128)[r] = pf_qpos;
-      reinterpret_cast<int64_t*>(m + 192)[r] = pf_qbits;
+      const QueryRule rule = make_query_rule(p.mask_mode, pf_exists, pf_qbits, pf_qpos);
+      reinterpret_cast<int*>(m + 128)[r] = rule.lim;
+      reinterpret_cast<int64_t*>(m + 192)[r] = rule.am;
+      reinterpret_cast<int64_t*>(m + 320)[r] = rule.qe;
     };
     prefetch_meta(0);
     stage_meta(0);
@@ -443,8 +431,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int c = tile_cls[it % n_valid];
       float* m_lse = reinterpret_cast<float*>(smem + L::META_OFF + (it % 3) * L::META_STAGE);
       float* m_delta = m_lse + 64;
-      int* m_qpos = reinterpret_cast<int*>(m_delta + 64);
-      int64_t* m_qbits = reinterpret_cast<int64_t*>(m_qpos + 64);
+      const int* m_lim = reinterpret_cast<const int*>(m_lse + 128);
+      const int64_t* m_am = reinterpret_cast<const int64_t*>(m_lse + 192);
+      const int64_t* m_qe = reinterpret_cast<const int64_t*>(m_lse + 320);
       if (!bw_wait(sdp_full, it & 1, abort_flag)) {
         if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
@@ -473,35 +462,42 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
       for (int x4 = 0; x4 < COLS / 4; ++x4) {
         const float4 l4 = *reinterpret_cast<const float4*>(m_lse + col0 + x4 * 4);
-        const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
-#pragma unroll
-        for (int y = 0; y < 4; ++y)
-          pv[x4 * 4 + y] = fast_exp2(fmaf(__uint_as_float(sv[x4 * 4 + y]), p.scale_log2, -ls[y]));
+        float y0, y1, y2, y3;
+        unpack_f32x2(fma_f32x2(pack_u32x2(sv[x4 * 4], sv[x4 * 4 + 1]), scale_log2_2, pack_f32x2(l4.x, l4.y)), y0, y1);
+        unpack_f32x2(fma_f32x2(pack_u32x2(sv[x4 * 4 + 2], sv[x4 * 4 + 3]), scale_log2_2, pack_f32x2(l4.z, l4.w)), y2, y3);
+        pv[x4 * 4] = fast_exp2(y0);
+        pv[x4 * 4 + 1] = fast_exp2(y1);
+        pv[x4 * 4 + 2] = fast_exp2(y2);
+        pv[x4 * 4 + 3] = fast_exp2(y3);
       }
       if (c == 1) {
         if (p.mask_mode == MASK_DENSE) {
           const uint8_t* mcol = p.dmask + (long)b * p.dm_sb + kidx;
 #pragma unroll
           for (int x = 0; x < COLS; ++x) {
-            const bool allow = k_valid && m_qpos[col0 + x] >= 0 && __ldg(mcol + (long)(q_base + x) * p.dm_sq) != 0;
+            const bool allow = k_valid && m_lim[col0 + x] >= 0 && __ldg(mcol + (long)(q_base + x) * p.dm_sq) != 0;
             pv[x] = allow ? pv[x] : 0.f;
           }
+        } else if (by_index) {
+          // token indices alone decide (queries beyond Sq already have P = 0 through their statistics)
+          const int first = !k_valid ? COLS : (p.mask_mode == MASK_CAUSAL ? kidx - q_base : 0);
+#pragma unroll
+          for (int x = 0; x < COLS; ++x) pv[x] = x >= first ? pv[x] : 0.f;
         } else {
 #pragma unroll
           for (int x = 0; x < COLS; ++x) {
             const int col = col0 + x;
-            const bool allow = k_valid && m_qpos[col] >= 0 && mask_allowed(p.mask_mode, m_qbits[col], kb, m_qpos[col], kpos);
-            pv[x] = allow ? pv[x] : 0.f;
+            pv[x] = rule_allows(QueryRule{m_am[col], m_qe[col], m_lim[col]}, kb, kpos) ? pv[x] : 0.f;
           }
         }
       }
 #pragma unroll
       for (int x4 = 0; x4 < COLS / 4; ++x4) {
         const float4 d4 = *reinterpret_cast<const float4*>(m_delta + col0 + x4 * 4);
-        const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
-#pragma unroll
-        for (int y = 0; y < 4; ++y)
-          ds[x4 * 4 + y] = pv[x4 * 4 + y] * fmaf(__uint_as_float(dv[x4 * 4 + y]), p.scale, -dl[y]);
+        const uint64_t t0 = fma_f32x2(pack_u32x2(dv[x4 * 4], dv[x4 * 4 + 1]), scale_2, pack_f32x2(d4.x, d4.y));
+        const uint64_t t1 = fma_f32x2(pack_u32x2(dv[x4 * 4 + 2], dv[x4 * 4 + 3]), scale_2, pack_f32x2(d4.z, d4.w));
+        unpack_f32x2(mul_f32x2(pack_f32x2(pv[x4 * 4], pv[x4 * 4 + 1]), t0), ds[x4 * 4], ds[x4 * 4 + 1]);
+        unpack_f32x2(mul_f32x2(pack_f32x2(pv[x4 * 4 + 2], pv[x4 * 4 + 3]), t1), ds[x4 * 4 + 2], ds[x4 * 4 + 3]);
       }
       if (it > 0) {
         if (!bw_wait(pds_empty, (it - 1) & 1, abort_flag)) {
@@ -532,13 +528,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       fence_proxy_async_smem();
       tc_fence_before();
       mbar_arrive(pds_full);
-      // drain dQ^T of the previous iteration while the MMAs of this one run
-      if (it > 0) ok = drain_dq(it - 1);
     }
-    if (ok && n_iter > 0) ok = drain_dq(n_iter - 1);
-    if (lane == 0) tma_store_wait<0>();  // every reduce-add of this warp has completed
-    __syncwarp();
-    // ---- epilogue: dV and dK tiles (every MMA has retired once the last dQ^T was seen);
+    // ---- epilogue: dV and dK tiles (every MMA has retired once the last dS^T was consumed);
+    if (ok && n_iter > 0 && !bw_wait(pds_empty, (n_iter - 1) & 1, abort_flag)) {
+      if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_MISC);
+      *abort_flag = 1;
+      ok = false;
+    }
     //      the warps of a lane quarter split the head-dim columns
     if (ok && peer_ready) {
       tc_fence_after();
@@ -576,6 +572,45 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
       }
     }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    // ------------------------------------------------------------------ dQ^T drain: TMEM -> smem [q][d] rows -> reduce-add
+    // Warps of their own, so that the compute warps go straight from dS^T(it) to S^T(it + 1): with the drain in their loop
+    // the next exponentials waited for the tensor-memory loads and staging stores of an iteration that was long over.
+    const int quarter = warp & 3;
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    float* stage = reinterpret_cast<float*>(smem + L::DQ_OFF + quarter * (BW_BQ * 128));
+    for (int it = 0; it < n_iter; ++it) {
+      if (!bw_wait(dq_full, it & 1, abort_flag)) {
+        if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_FULL);
+        *abort_flag = 1;
+        break;
+      }
+      tc_fence_after();
+      if (lane == 0) tma_store_wait_read<0>();  // the previous block has left the staging buffer
+      __syncwarp();
+      // this warp's [32 d][64 q] block -> shared memory as [q][d] rows of 128 B -> one TMA reduce-add into dq_acc
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        uint32_t v[32];
+        tmem_ld_32x32(tmem_dQT + g * 32 + lane_addr, v);
+        tmem_ld_wait();
+        if (g == 1) {
+          tc_fence_before();
+          mbar_arrive(dq_free);
+        }
+#pragma unroll
+        for (int c = 0; c < 32; ++c) stage[(g * 32 + c) * 32 + lane] = __uint_as_float(v[c]);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0 && quarter * 32 < p.D) {
+        tma_reduce_add_4d(&tm_dq, stage, quarter * 32, hk * group + it / n_valid, tile_idx[it % n_valid] * BW_BQ, b);  // box: 32 d x 64 q
+        tma_store_commit();
+      }
+    }
+    if (lane == 0) tma_store_wait<0>();  // every reduce-add of this warp has completed
+    __syncwarp();
   }
 
   tc_fence_before();
@@ -616,6 +651,7 @@ static int attn_bwd_seg_impl(const void* q, const CsbKvSegments* kv, const void*
                              int mask_mode, const long* q_bits, const long* k_bits, const int* q_pos, const int* k_pos,
                              const signed char* cls, int* status, void* stream, const CsbAttnExtras* ex) {
   if (D % 8 || D > 128 || D < 16 || Hq % Hk) return CSB_ERR_BAD_ARG;
+  if (cls == nullptr && !(mask_mode == MASK_FULL || (mask_mode == MASK_CAUSAL && q_pos == nullptr && k_pos == nullptr))) return CSB_ERR_BAD_ARG;
   if (mask_mode == MASK_DENSE && (ex == nullptr || ex->dmask == nullptr)) return CSB_ERR_BAD_ARG;
   if (kv == nullptr || kv->n_seg < 1 || kv->n_seg > CSB_MAX_SEG) return CSB_ERR_BAD_ARG;
   if ((Sq + BW_BQ - 1) / BW_BQ > BwdSmem::MAX_TILES) return CSB_ERR_TOO_LARGE;
@@ -676,10 +712,10 @@ static int attn_bwd_seg_impl(const void* q, const CsbKvSegments* kv, const void*
   }();
   CUtensorMap tdq;
   {
-    // dq_acc is dense fp32 [B][Sq][Hq][D]; a block is 32 head-dim elements (128 B) x 32 or 16 query rows
+    // dq_acc is dense fp32 [B][Sq][Hq][D]; a block is 32 head-dim elements (128 B) x 64 query rows
     uint64_t dims[4] = {(uint64_t)D, (uint64_t)Hq, (uint64_t)Sq, (uint64_t)B};
     uint64_t strides[3] = {(uint64_t)D * 4, (uint64_t)Hq * D * 4, (uint64_t)Sq * Hq * D * 4};
-    uint32_t box[4] = {32, 1, (uint32_t)(wide ? BwdCfg<16>::COLS : BwdCfg<8>::COLS), 1};
+    uint32_t box[4] = {32, 1, (uint32_t)BW_BQ, 1};
     if ((r = make_tmap_nd_f32(&tdq, dq_acc, 4, dims, strides, box))) return r;
   }
   static bool attr = false;
