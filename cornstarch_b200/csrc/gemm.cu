@@ -92,12 +92,16 @@ __host__ __device__ __forceinline__ int ar_owner(int m_blk, int num_m, int world
 // CG = CTAs per MMA (tcgen05 cta_group): 1 = every thread block computes its own 128 x BN tile; 2 = a cluster of two
 // thread blocks computes one 256 x BN tile: each block stages its own 128 rows of A and HALF of the B tile (BN / 2
 // rows), the leader block issues the MMAs, which read both blocks' shared memory and write both blocks' tensor memory.
-template <int BN, int CG = 1>
+// An MN-major B tile is loaded in boxes 64 columns wide: with BN = 192 a block of a pair stages 128 columns for the 96 it
+// needs (the MMA reads the first 96).
+template <int BN, int CG = 1, bool B_MN = false>
 struct SmemLayout {
+  static constexpr int B_ROWS = B_MN ? (BN / CG + 63) / 64 * 64 : BN / CG;
   static constexpr int A_BYTES = BM * BK * 2;
-  static constexpr int B_BYTES = (BN / CG) * BK * 2;
+  static constexpr int B_BYTES = B_ROWS * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (CG == 2) ? 6 : ((BN == 256) ? 4 : 6);
+  static constexpr int STAGES = (CG == 2) ? (BN == 128 ? 8 : 6) : ((BN == 256) ? 4 : 6);
+  static constexpr uint32_t TMEM_COLS = 2 * BN > 256 ? 512 : 256;  // two accumulators; allocations are powers of two
   static constexpr int EPI_OFFSET = STAGES * STAGE_BYTES;  // two 16 KB output slabs (128 rows x 128 B, swizzled)
   static constexpr int EPI_SLAB_BYTES = 128 * 128;
   static constexpr int BAR_OFFSET = EPI_OFFSET + 2 * EPI_SLAB_BYTES;
@@ -405,7 +409,7 @@ template <int BN, bool A_MN, bool B_MN, int CG>
 __global__ void __launch_bounds__(192, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ EpiMaps epi_maps, const GemmParams p) {
-  using L = SmemLayout<BN, CG>;
+  using L = SmemLayout<BN, CG, B_MN>;
   constexpr int BNH = BN / CG;  // rows of B this thread block stages
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -457,10 +461,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
   if (warp == 1) {
     if constexpr (CG == 2) {
-      tmem_alloc_2cta(tmem_addr_slot, 2 * BN);  // the same warp of both blocks: the columns are allocated in both
+      tmem_alloc_2cta(tmem_addr_slot, L::TMEM_COLS);  // the same warp of both blocks: the columns are allocated in both
       tmem_relinquish_2cta();
     } else {
-      tmem_alloc(tmem_addr_slot, 2 * BN);
+      tmem_alloc(tmem_addr_slot, L::TMEM_COLS);
       tmem_relinquish();
     }
   }
@@ -528,7 +532,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           }
           if constexpr (B_MN) {
 #pragma unroll
-            for (int j = 0; j < BNH / 64; ++j)
+            for (int j = 0; j < L::B_ROWS / 64; ++j)
               tma_load_2d_to<CG>(sb + j * (64 * BK * 2), map_b, full_addr_s, n_row0 + j * 64, kb * BK);
           } else {
             tma_load_2d_to<CG>(sb, map_b, full_addr_s, kb * BK, n_row0);
@@ -802,8 +806,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   else __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    if constexpr (CG == 2) tmem_dealloc_2cta(tmem_base, 2 * BN);
-    else tmem_dealloc(tmem_base, 2 * BN);
+    if constexpr (CG == 2) tmem_dealloc_2cta(tmem_base, L::TMEM_COLS);
+    else tmem_dealloc(tmem_base, L::TMEM_COLS);
   }
 }
 
@@ -822,7 +826,7 @@ static int launch_gemm(const void* A, const void* B, const GemmParams& p, int ld
   else
     r = make_tmap_2d_bf16(&tb, B, p.N, p.K, ldb, BK, BN / CG);
   if (r) return r;
-  using L = SmemLayout<BN, CG>;
+  using L = SmemLayout<BN, CG, B_MN>;
   auto kfn = gemm_bf16_kernel<BN, A_MN, B_MN, CG>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -912,6 +916,58 @@ static int gemm_cg_choice() {
 // Pairs of thread blocks serve a fused collective when every rank's range of tile rows starts on an even tile row:
 // both blocks of a pair then work for the same owner.
 static bool pairs_fit_ranges(int num_m_blocks, int world) { return num_m_blocks % (2 * world) == 0; }
+// Tile of a launch: BN columns wide, 128 rows (cg = 1) or 256 rows by a pair of thread blocks (cg = 2).
+struct TileChoice {
+  int bn, cg;
+};
+// Microseconds of one 64-deep k block and of one tile's epilogue and hand-over, by operand layout (0: both K-major; 1: B
+// MN-major; 2: A MN-major), fitted to 192 shapes (77..8192 tokens x the projections of the vision and language models,
+// forward, input-gradient and weight-gradient form) with each of the five tiles; the fit is within 10 to 15 %.
+struct TileCost {
+  int bn, cg;
+  float k_us[3], tile_us[3];
+};
+constexpr TileCost TILE_COSTS[5] = {
+    {256, 2, {0.345f, 0.36f, 0.38f}, {2.6f, 2.4f, 1.8f}},
+    {192, 2, {0.26f, 0.32f, 0.36f}, {2.5f, 1.8f, 1.7f}},
+    {128, 2, {0.24f, 0.26f, 0.28f}, {1.2f, 1.0f, 1.3f}},
+    {256, 1, {0.40f, 0.40f, 0.44f}, {1.6f, 2.4f, 0.9f}},
+    {128, 1, {0.24f, 0.31f, 0.32f}, {0.7f, 0.8f, 0.6f}},
+};
+static float tile_cost(const TileCost& c, int layout, int M, int N, int K) {
+  const long units = (M + BM * c.cg - 1) / (BM * c.cg);
+  const long tiles = units * ((N + c.bn - 1) / c.bn);
+  const long slots = sm_count() / c.cg;
+  const long rounds = (tiles + slots - 1) / slots;
+  return 6.f + rounds * (c.k_us[layout] * ((K + BK - 1) / BK) + c.tile_us[layout]);
+}
+// What a launch costs is the number of rounds its tiles take times the time of a tile: a last round that is nearly empty, or
+// a width that does not divide N, costs as much as a full one (2916 x 1152 x 4304: 60 pairs of 256 columns, or 207 blocks of
+// 128 in two rounds, take 39 and 46 us; 72 pairs of 192 columns fill one round, 27 us).  The widest tile moves the fewest
+// bytes per FLOP and is kept unless another is predicted at least 7 % faster, half the spread of the fit: on the 192 shapes
+// 75 then change tile, two of them lose more than 3 %, and all together gain 5.8 %.
+// `max_ctas` > 0 (the launch shares the GPU with another kernel) keeps single blocks and the width by size alone.
+static TileChoice choose_tile(int M, int N, int K, int tile_n, int max_ctas, bool a_mn_major, bool b_mn_major) {
+  const long m_blocks = (M + BM - 1) / BM;
+  const bool pairs = gemm_cg_choice() == 2 && max_ctas <= 0;
+  TileChoice d;
+  d.bn = tile_n;
+  if (d.bn != 128 && d.bn != 256) d.bn = (N >= 256 && m_blocks * ((N + 255) / 256) >= sm_count()) ? 256 : 128;
+  d.cg = (d.bn == 256 && pairs && m_blocks >= 2) ? 2 : 1;
+  if (tile_n == 128 || tile_n == 256 || !pairs) return d;
+  const int layout = a_mn_major ? 2 : (b_mn_major ? 1 : 0);
+  float best = 0.f;
+  for (const TileCost& c : TILE_COSTS)
+    if (c.bn == d.bn && c.cg == d.cg) best = 0.93f * tile_cost(c, layout, M, N, K);
+  for (const TileCost& c : TILE_COSTS) {
+    const float t = tile_cost(c, layout, M, N, K);
+    if (t < best) {
+      best = t;
+      d = {c.bn, c.cg};
+    }
+  }
+  return d;
+}
 static void no_collective(GemmParams& p) {
   p.group_rows = 0;
   p.ar_scatter = 0; p.ar_row_offset = 0;
@@ -931,12 +987,8 @@ CSB_API int csb_gemm_bf16(const void* A, const void* B, void* C, const void* bia
   using namespace csb;
   if (M <= 0 || N <= 0 || K <= 0 || (lda & 7) || (ldb & 7)) return CSB_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return CSB_ERR_BAD_ARG;
-  int bn = tile_n;
-  if (bn != 128 && bn != 256) {
-    // 256-wide tiles halve the A re-reads; fall back to 128 when N is small or the tile count is low.
-    long t256 = (long)((M + BM - 1) / BM) * ((N + 255) / 256);
-    bn = (N >= 256 && t256 >= sm_count()) ? 256 : 128;
-  }
+  const TileChoice tc = choose_tile(M, N, K, tile_n, max_ctas, a_mn_major != 0, b_mn_major != 0);
+  const int bn = tc.bn;
   GemmParams p;
   p.C = C;
   p.bias = bias;
@@ -954,22 +1006,18 @@ CSB_API int csb_gemm_bf16(const void* A, const void* B, void* C, const void* bia
   for (int i = 0; i < 8; ++i) { p.ar_inbox[i] = nullptr; p.ar_final[i] = nullptr; p.ar_cnt_part[i] = nullptr; p.ar_cnt_final[i] = nullptr; }
   no_collective(p);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-#define CSB_DISPATCH(BNV)                                                                       \
-  if (!a_mn_major && !b_mn_major) return launch_gemm<BNV, false, false>(A, B, p, lda, ldb, max_ctas, s); \
-  if (!a_mn_major && b_mn_major) return launch_gemm<BNV, false, true>(A, B, p, lda, ldb, max_ctas, s);   \
-  if (a_mn_major && !b_mn_major) return launch_gemm<BNV, true, false>(A, B, p, lda, ldb, max_ctas, s);   \
-  return launch_gemm<BNV, true, true>(A, B, p, lda, ldb, max_ctas, s);
-  // Pairs of thread blocks on one 256 x 256 tile (cta_group::2) when the problem has at least two tile rows and the
-  // caller did not restrict the number of thread blocks (a restricted launch shares the GPU with another kernel).
-  const int cg = gemm_cg_choice();
-  if (bn == 256 && cg == 2 && p.num_m_blocks >= 2 && max_ctas <= 0) {
-    if (!a_mn_major && !b_mn_major) return launch_gemm<256, false, false, 2>(A, B, p, lda, ldb, 0, s);
-    if (!a_mn_major && b_mn_major) return launch_gemm<256, false, true, 2>(A, B, p, lda, ldb, 0, s);
-    if (a_mn_major && !b_mn_major) return launch_gemm<256, true, false, 2>(A, B, p, lda, ldb, 0, s);
-    return launch_gemm<256, true, true, 2>(A, B, p, lda, ldb, 0, s);
+#define CSB_DISPATCH(BNV, CGV)                                                                                   \
+  if (!a_mn_major && !b_mn_major) return launch_gemm<BNV, false, false, CGV>(A, B, p, lda, ldb, max_ctas, s);   \
+  if (!a_mn_major && b_mn_major) return launch_gemm<BNV, false, true, CGV>(A, B, p, lda, ldb, max_ctas, s);     \
+  if (a_mn_major && !b_mn_major) return launch_gemm<BNV, true, false, CGV>(A, B, p, lda, ldb, max_ctas, s);     \
+  return launch_gemm<BNV, true, true, CGV>(A, B, p, lda, ldb, max_ctas, s);
+  if (tc.cg == 2) {
+    if (bn == 256) { CSB_DISPATCH(256, 2) }
+    if (bn == 192) { CSB_DISPATCH(192, 2) }
+    CSB_DISPATCH(128, 2)
   }
-  if (bn == 256) { CSB_DISPATCH(256) }
-  CSB_DISPATCH(128)
+  if (bn == 256) { CSB_DISPATCH(256, 1) }
+  CSB_DISPATCH(128, 1)
 #undef CSB_DISPATCH
 }
 
