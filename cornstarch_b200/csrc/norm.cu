@@ -11,23 +11,26 @@
 
 namespace csb {
 
-constexpr int NORM_THREADS = 256;
-constexpr int NORM_MAX_VEC = 4;  // 256 threads * 8 elems * 4 = 8192 max hidden
+constexpr int NORM_MAX_H = 8192;  // one 16-byte vector per thread, 1024 threads
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ __forceinline__ float block_sum(float v, float* sh) {
+
+// Sum over the threads that share a row: a warp (ONE_WARP) or the whole block.  One barrier per sum: the warp sums of
+// consecutive calls go to alternating halves of `sh`, and whoever writes a half again has passed the barrier of the call in
+// between, which every reader of that half's old contents reached after reading.
+template <bool ONE_WARP>
+__device__ __forceinline__ float row_sum(float v, float* sh, uint32_t& n_calls) {
   v = warp_sum(v);
+  if constexpr (ONE_WARP) return v;
+  float* buf = sh + (n_calls++ & 1) * 32;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) buf[w] = v;
   __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  float t = (l < (blockDim.x >> 5)) ? sh[l] : 0.f;
-  t = warp_sum(t);
-  return t;
+  return warp_sum(l < (int)(blockDim.x >> 5) ? buf[l] : 0.f);
 }
 
 struct Vec8 {
@@ -54,87 +57,6 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const Vec8& v) {
   *reinterpret_cast<uint4*>(p) = u;
 }
 
-// IS_LN: LayerNorm (mean subtraction + bias) else RMSNorm.  w_offset: Gemma-style (1 + w).
-template <bool IS_LN>
-__global__ void __launch_bounds__(NORM_THREADS)
-norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
-                const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
-                __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out, float* __restrict__ mean_out,
-                float* __restrict__ rstd_out, int rows, int H, float eps, float w_offset) {
-  __shared__ float sh[32];
-  const int nvec = H / 8;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const size_t base = static_cast<size_t>(row) * H;
-    Vec8 v[NORM_MAX_VEC];
-    float s = 0.f, ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < NORM_MAX_VEC; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nvec) {
-        v[i] = load8(x + base + c * 8);
-        if (res) {
-          Vec8 r = load8(res + base + c * 8);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[i].f[j] += r.f[j];
-        }
-        if (h_out) {
-          // the residual stream is stored in bf16; normalise the rounded value so that the
-          // backward (which re-reads h) sees exactly what the forward normalised
-          store8(h_out + base + c * 8, v[i]);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[i].f[j] = __bfloat162float(__float2bfloat16(v[i].f[j]));
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          s += v[i].f[j];
-          ss += v[i].f[j] * v[i].f[j];
-        }
-      }
-    }
-    float mean = 0.f;
-    if (IS_LN) {
-      mean = block_sum(s, sh) / H;
-      // two-pass variance on the register-resident row
-      float d2 = 0.f;
-#pragma unroll
-      for (int i = 0; i < NORM_MAX_VEC; ++i) {
-        const int c = threadIdx.x + i * NORM_THREADS;
-        if (c < nvec) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float d = v[i].f[j] - mean;
-            d2 += d * d;
-          }
-        }
-      }
-      ss = d2;
-    }
-    const float var = block_sum(ss, sh) / H;
-    const float rstd = rsqrtf(var + eps);
-    if (threadIdx.x == 0) {
-      if (IS_LN && mean_out) mean_out[row] = mean;
-      rstd_out[row] = rstd;
-    }
-#pragma unroll
-    for (int i = 0; i < NORM_MAX_VEC; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nvec) {
-        Vec8 wv = load8(w + c * 8);
-        Vec8 o;
-        if (IS_LN && b) {
-          Vec8 bv = load8(b + c * 8);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o.f[j] = (v[i].f[j] - mean) * rstd * (wv.f[j] + w_offset) + bv.f[j];
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o.f[j] = (v[i].f[j] - mean) * rstd * (wv.f[j] + w_offset);
-        }
-        store8(y + base + c * 8, o);
-      }
-    }
-  }
-}
-
 __device__ __forceinline__ Vec8 unpack8(const uint4& u) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
   Vec8 v;
@@ -147,112 +69,188 @@ __device__ __forceinline__ Vec8 unpack8(const uint4& u) {
   return v;
 }
 
+// IS_LN: LayerNorm (mean subtraction + bias) else RMSNorm.  w_offset: Gemma-style (1 + w).
+// Every thread holds ONE 16-byte vector of the row (ONE_WARP: H <= 256, a warp per row and eight rows per block; else a
+// block per row, rounded up to whole warps).  HBM bounds this kernel; what kept it from that were the dependent phases of a
+// row (load, reduce, store), so the next row of the block is loaded before the current one is reduced and several small
+// blocks per SM are in different phases.
+template <bool IS_LN, bool ONE_WARP>
+__global__ void __launch_bounds__(1024)
+norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
+                const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
+                __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out, float* __restrict__ mean_out,
+                float* __restrict__ rstd_out, int rows, int H, float eps, float w_offset) {
+  __shared__ float sh[64];
+  uint32_t n_sums = 0;
+  const int c = ONE_WARP ? (threadIdx.x & 31) : threadIdx.x;  // this thread's vector of the row
+  const bool on = c < H / 8;
+  const int first = ONE_WARP ? blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x;
+  const int step = ONE_WARP ? gridDim.x * (blockDim.x >> 5) : gridDim.x;
+  Vec8 wv, bv;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) wv.f[j] = bv.f[j] = 0.f;
+  if (on) {
+    wv = load8(w + c * 8);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) wv.f[j] += w_offset;
+    if (IS_LN && b) bv = load8(b + c * 8);
+  }
+  uint4 n_x = make_uint4(0u, 0u, 0u, 0u), n_r = n_x;
+  auto fetch = [&](int row) {
+    const size_t at = static_cast<size_t>(row) * H + c * 8;
+    if (on) {
+      n_x = *reinterpret_cast<const uint4*>(x + at);
+      if (res) n_r = *reinterpret_cast<const uint4*>(res + at);
+    }
+  };
+  if (first < rows) fetch(first);
+  for (int row = first; row < rows; row += step) {
+    const size_t at = static_cast<size_t>(row) * H + c * 8;
+    Vec8 v = unpack8(n_x);
+    if (res) {
+      const Vec8 r = unpack8(n_r);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v.f[j] += r.f[j];
+    }
+    if (row + step < rows) fetch(row + step);
+    if (h_out) {
+      // the residual stream is stored in bf16; normalise the rounded value so that the
+      // backward (which re-reads h) sees exactly what the forward normalised
+      if (on) store8(h_out + at, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v.f[j] = __bfloat162float(__float2bfloat16(v.f[j]));
+    }
+    float mean = 0.f, ss = 0.f;
+    if (IS_LN) {
+      float s = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += v.f[j];
+      mean = row_sum<ONE_WARP>(s, sh, n_sums) / H;
+      // two-pass variance on the register-resident row
+      if (on) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float d = v.f[j] - mean;
+          ss += d * d;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += v.f[j] * v.f[j];
+    }
+    const float var = row_sum<ONE_WARP>(ss, sh, n_sums) / H;
+    const float rstd = rsqrtf(var + eps);
+    if (c == 0) {
+      if (IS_LN && mean_out) mean_out[row] = mean;
+      rstd_out[row] = rstd;
+    }
+    if (on) {
+      Vec8 o;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o.f[j] = (v.f[j] - mean) * rstd * wv.f[j] + (IS_LN ? bv.f[j] : 0.f);
+      store8(y + at, o);
+    }
+  }
+}
+
 // dx = rstd * (g - xhat * mean(g*xhat) [- mean(g)])  with g = dy * w;  dw += dy * xhat;  db += dy
-// NVEC = 16-byte vectors per thread (H <= NVEC * 2048).  The raw vectors of the CTA's next row are fetched before the
-// current row is reduced, so that loads stay in flight across the block-wide reduction.
-template <bool IS_LN, int NVEC>
-__global__ void __launch_bounds__(NORM_THREADS)
+// One 16-byte vector per thread, as in the forward kernel, with the next row's three inputs and its statistics in flight
+// while the current row is reduced.  (Two vectors per thread in blocks of 256 needed so many registers that two blocks
+// fitted an SM, paid two or four barriers per row, and read the row's statistics only when it needed them.)
+template <bool IS_LN, bool ONE_WARP>
+__global__ void __launch_bounds__(1024)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
                 const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean_in,
                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                 __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial, float* __restrict__ db_partial,
                 int rows, int H, float w_offset) {
-  __shared__ float sh[32];
-  const int nvec = H / 8;
-  float dw_acc[NVEC][8];
-  float db_acc[NVEC][8];
+  __shared__ float sh[64];
+  uint32_t n_sums = 0;
+  const int c = ONE_WARP ? (threadIdx.x & 31) : threadIdx.x;
+  const bool on = c < H / 8;
+  const int first = ONE_WARP ? blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x;
+  const int step = ONE_WARP ? gridDim.x * (blockDim.x >> 5) : gridDim.x;
+  float dw_acc[8], db_acc[8];
 #pragma unroll
-  for (int i = 0; i < NVEC; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      dw_acc[i][j] = 0.f;
-      db_acc[i][j] = 0.f;
-    }
-  Vec8 wv[NVEC];
-#pragma unroll
-  for (int i = 0; i < NVEC; ++i) {
-    const int c = threadIdx.x + i * NORM_THREADS;
-    if (c < nvec) {
-      wv[i] = load8(w + c * 8);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) wv[i].f[j] += w_offset;
-    }
-  }
-  uint4 n_dy[NVEC], n_h[NVEC], n_dr[NVEC];
+  for (int j = 0; j < 8; ++j) dw_acc[j] = db_acc[j] = 0.f;
+  uint4 w_raw = make_uint4(0u, 0u, 0u, 0u);
+  if (on) w_raw = *reinterpret_cast<const uint4*>(w + c * 8);
+  uint4 n_dy = make_uint4(0u, 0u, 0u, 0u), n_h = n_dy, n_dr = n_dy;
+  float n_mean = 0.f, n_rstd = 0.f;
   auto fetch = [&](int row) {
-    const size_t base = static_cast<size_t>(row) * H;
-#pragma unroll
-    for (int i = 0; i < NVEC; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nvec) {
-        n_dy[i] = __ldcs(reinterpret_cast<const uint4*>(dy + base + c * 8));
-        n_h[i] = __ldcs(reinterpret_cast<const uint4*>(h + base + c * 8));
-        if (dres) n_dr[i] = __ldcs(reinterpret_cast<const uint4*>(dres + base + c * 8));
-      }
+    const size_t at = static_cast<size_t>(row) * H + c * 8;
+    n_rstd = rstd_in[row];
+    if (IS_LN) n_mean = mean_in[row];
+    if (on) {
+      n_dy = __ldcs(reinterpret_cast<const uint4*>(dy + at));
+      n_h = __ldcs(reinterpret_cast<const uint4*>(h + at));
+      if (dres) n_dr = __ldcs(reinterpret_cast<const uint4*>(dres + at));
     }
   };
-  if (blockIdx.x < rows) fetch(blockIdx.x);
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const size_t base = static_cast<size_t>(row) * H;
-    uint4 c_dy[NVEC], c_h[NVEC], c_dr[NVEC];
-#pragma unroll
-    for (int i = 0; i < NVEC; ++i) {
-      c_dy[i] = n_dy[i];
-      c_h[i] = n_h[i];
-      c_dr[i] = n_dr[i];
-    }
-    if (row + (int)gridDim.x < rows) fetch(row + gridDim.x);
-    const float mean = IS_LN ? mean_in[row] : 0.f;
-    const float rstd = rstd_in[row];
-    Vec8 g[NVEC], xh[NVEC];
+  if (first < rows) fetch(first);
+  for (int row = first; row < rows; row += step) {
+    // the row is kept as it was loaded and unpacked again after the reduction: half the registers
+    const uint4 c_dy = n_dy, c_h = n_h, c_dr = n_dr;
+    const float mean = n_mean, rstd = n_rstd;
+    if (row + step < rows) fetch(row + step);
     float s1 = 0.f, s2 = 0.f;
+    {
+      const Vec8 d = unpack8(c_dy), hv = unpack8(c_h), wv = unpack8(w_raw);
 #pragma unroll
-    for (int i = 0; i < NVEC; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nvec) {
-        const Vec8 d = unpack8(c_dy[i]);
-        const Vec8 hv = unpack8(c_h[i]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          xh[i].f[j] = (hv.f[j] - mean) * rstd;
-          g[i].f[j] = d.f[j] * wv[i].f[j];
-          s1 += g[i].f[j] * xh[i].f[j];
-          s2 += g[i].f[j];
-          dw_acc[i][j] += d.f[j] * xh[i].f[j];
-          db_acc[i][j] += d.f[j];
-        }
+      for (int j = 0; j < 8; ++j) {
+        const float xh = (hv.f[j] - mean) * rstd;
+        const float g = d.f[j] * (wv.f[j] + w_offset);
+        s1 += g * xh;
+        if (IS_LN) s2 += g;
+        dw_acc[j] += d.f[j] * xh;
+        if (IS_LN) db_acc[j] += d.f[j];
       }
     }
-    const float m1 = block_sum(s1, sh) / H;
-    const float m2 = IS_LN ? block_sum(s2, sh) / H : 0.f;
+    if (!on) s1 = s2 = 0.f;
+    const float m1 = row_sum<ONE_WARP>(s1, sh, n_sums) / H;
+    const float m2 = IS_LN ? row_sum<ONE_WARP>(s2, sh, n_sums) / H : 0.f;
+    if (on) {
+      const Vec8 d = unpack8(c_dy), hv = unpack8(c_h), wv = unpack8(w_raw);
+      Vec8 o;
 #pragma unroll
-    for (int i = 0; i < NVEC; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nvec) {
-        Vec8 o;
+      for (int j = 0; j < 8; ++j) o.f[j] = rstd * (d.f[j] * (wv.f[j] + w_offset) - (hv.f[j] - mean) * rstd * m1 - m2);
+      if (dres) {
+        const Vec8 r = unpack8(c_dr);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o.f[j] = rstd * (g[i].f[j] - xh[i].f[j] * m1 - m2);
-        if (dres) {
-          const Vec8 r = unpack8(c_dr[i]);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o.f[j] += r.f[j];
-        }
-        store8(dx + base + c * 8, o);
+        for (int j = 0; j < 8; ++j) o.f[j] += r.f[j];
       }
+      store8(dx + static_cast<size_t>(row) * H + c * 8, o);
     }
   }
+  if constexpr (ONE_WARP) {
+    // the warps of a block add up their sums: one partial row per block
+    __shared__ float part[8][2][256];
+    const int wi = threadIdx.x >> 5;
+    if (on) {
 #pragma unroll
-  for (int i = 0; i < NVEC; ++i) {
-    const int c = threadIdx.x + i * NORM_THREADS;
-    if (c < nvec) {
-      float* pw = dw_partial + static_cast<size_t>(blockIdx.x) * H + c * 8;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) pw[j] = dw_acc[i][j];
-      if (IS_LN && db_partial) {
-        float* pb = db_partial + static_cast<size_t>(blockIdx.x) * H + c * 8;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) pb[j] = db_acc[i][j];
+      for (int j = 0; j < 8; ++j) {
+        part[wi][0][c * 8 + j] = dw_acc[j];
+        if (IS_LN) part[wi][1][c * 8 + j] = db_acc[j];
       }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < H; i += blockDim.x) {
+      float sw = 0.f, sb = 0.f;
+      for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
+        sw += part[k][0][i];
+        if (IS_LN) sb += part[k][1][i];
+      }
+      dw_partial[static_cast<size_t>(blockIdx.x) * H + i] = sw;
+      if (IS_LN && db_partial) db_partial[static_cast<size_t>(blockIdx.x) * H + i] = sb;
+    }
+  } else if (on) {
+    float* pw = dw_partial + static_cast<size_t>(blockIdx.x) * H + c * 8;
+    *reinterpret_cast<float4*>(pw) = make_float4(dw_acc[0], dw_acc[1], dw_acc[2], dw_acc[3]);
+    *reinterpret_cast<float4*>(pw + 4) = make_float4(dw_acc[4], dw_acc[5], dw_acc[6], dw_acc[7]);
+    if (IS_LN && db_partial) {
+      float* pb = db_partial + static_cast<size_t>(blockIdx.x) * H + c * 8;
+      *reinterpret_cast<float4*>(pb) = make_float4(db_acc[0], db_acc[1], db_acc[2], db_acc[3]);
+      *reinterpret_cast<float4*>(pb + 4) = make_float4(db_acc[4], db_acc[5], db_acc[6], db_acc[7]);
     }
   }
 }
@@ -266,8 +264,10 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
   float s = 0.f;
-  if (c < H)
+  if (c < H) {
+#pragma unroll 4
     for (int r = ty; r < nparts; r += 8) s += partial[static_cast<size_t>(r) * H + c];
+  }
   sh[ty][tx] = s;
   __syncthreads();
   if (ty == 0 && c < H) {
@@ -283,21 +283,34 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
   }
 }
 
-// Column sum of a bf16 matrix [rows][H] (bias gradients): partial per CTA then reduce_partials.
+// Column sum of a bf16 matrix [rows][H] (bias gradients): partial sums per row slice, then reduce_partials.
+// A block owns 256 columns (a warp reads 512 contiguous bytes of a row) and one slice of the rows, which its eight warps
+// share; columns x slices fill the GPU.  (One block for all columns walked its few rows once per 2048 columns with a single
+// load in flight per thread.)
+constexpr int COLSUM_COLS = 256;
 __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16* __restrict__ x,
                                                             float* __restrict__ partial, int rows, int H) {
-  // each thread owns 8 consecutive columns; CTAs stride over rows
-  const int nvec = H / 8;
-  for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-      Vec8 v = load8(x + static_cast<size_t>(r) * H + c * 8);
+  __shared__ float part[8][COLSUM_COLS];
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int col = blockIdx.x * COLSUM_COLS + lane * 8;
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (col < H) {
+#pragma unroll 4
+    for (int r = blockIdx.y * 8 + wi; r < rows; r += gridDim.y * 8) {
+      const Vec8 v = load8(x + static_cast<size_t>(r) * H + col);
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] += v.f[j];
     }
-    float* p = partial + static_cast<size_t>(blockIdx.x) * H + c * 8;
+  }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) p[j] = acc[j];
+  for (int j = 0; j < 8; ++j) part[wi][lane * 8 + j] = acc[j];
+  __syncthreads();
+  const int c = blockIdx.x * COLSUM_COLS + threadIdx.x;
+  if (c < H) {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += part[k][threadIdx.x];
+    partial[static_cast<size_t>(blockIdx.y) * H + c] = s;
   }
 }
 
@@ -305,9 +318,21 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
 
 using namespace csb;
 
+// Upper bound of the partial rows of a launch (what csb_norm_bwd_parts promises the caller).
 static int norm_grid(int rows) {
   int g = sm_count() * 4;
   return rows < g ? rows : g;
+}
+// Threads of a block and blocks of a launch for rows of H elements: up to 256 elements a warp per row and eight rows per
+// block, above that one block of H / 8 threads (whole warps) per row; blocks for two rows' worth of threads per SM slot.
+static void norm_shape(int rows, int H, int* threads, int* grid) {
+  const int nvec = H / 8;
+  const bool one_warp = nvec <= 32;
+  *threads = one_warp ? 256 : (nvec + 31) / 32 * 32;
+  const long units = one_warp ? (rows + 7) / 8 : rows;
+  long g = (long)sm_count() * (2048 / *threads < 4 ? 2048 / *threads : 4);
+  if (*threads > 512) g = sm_count() * 2;
+  *grid = (int)(units < g ? units : g);
 }
 
 // Number of fp32 rows the caller must provide in the dw/db partial buffers for a given row count.
@@ -316,7 +341,7 @@ CSB_API int csb_norm_bwd_parts(int rows) { return norm_grid(rows); }
 CSB_API int csb_norm_fwd(int is_layernorm, const void* x, const void* res, const void* w, const void* b, void* y,
                          void* h_out, float* mean, float* rstd, int rows, int H, float eps, float w_offset,
                          void* stream) {
-  if (H % 8 != 0 || H > NORM_THREADS * 8 * NORM_MAX_VEC || rows <= 0) return CSB_ERR_BAD_ARG;
+  if (H % 8 != 0 || H > NORM_MAX_H || rows <= 0) return CSB_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   auto X = reinterpret_cast<const __nv_bfloat16*>(x);
   auto R = reinterpret_cast<const __nv_bfloat16*>(res);
@@ -324,10 +349,15 @@ CSB_API int csb_norm_fwd(int is_layernorm, const void* x, const void* res, const
   auto B = reinterpret_cast<const __nv_bfloat16*>(b);
   auto Y = reinterpret_cast<__nv_bfloat16*>(y);
   auto Ho = reinterpret_cast<__nv_bfloat16*>(h_out);
-  if (is_layernorm)
-    norm_fwd_kernel<true><<<norm_grid(rows), NORM_THREADS, 0, s>>>(X, R, W, B, Y, Ho, mean, rstd, rows, H, eps, w_offset);
-  else
-    norm_fwd_kernel<false><<<norm_grid(rows), NORM_THREADS, 0, s>>>(X, R, W, B, Y, Ho, mean, rstd, rows, H, eps, w_offset);
+  int threads, grid;
+  norm_shape(rows, H, &threads, &grid);
+#define CSB_NORM_FWD(LN, OW) norm_fwd_kernel<LN, OW><<<grid, threads, 0, s>>>(X, R, W, B, Y, Ho, mean, rstd, rows, H, eps, w_offset)
+  if (is_layernorm) {
+    if (H <= 256) CSB_NORM_FWD(true, true); else CSB_NORM_FWD(true, false);
+  } else {
+    if (H <= 256) CSB_NORM_FWD(false, true); else CSB_NORM_FWD(false, false);
+  }
+#undef CSB_NORM_FWD
   return launch_result();
 }
 
@@ -336,21 +366,21 @@ CSB_API int csb_norm_bwd(int is_layernorm, const void* dy, const void* h, const 
                          const float* rstd, const void* dres, void* dx, float* dw_partial, float* db_partial,
                          void* dw_out, void* db_out, int grads_fp32, int accumulate, int rows, int H,
                          float w_offset, void* stream) {
-  if (H % 8 != 0 || H > NORM_THREADS * 8 * NORM_MAX_VEC || rows <= 0) return CSB_ERR_BAD_ARG;
+  if (H % 8 != 0 || H > NORM_MAX_H || rows <= 0) return CSB_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const int grid = norm_grid(rows);
+  int threads, grid;
+  norm_shape(rows, H, &threads, &grid);
   auto DY = reinterpret_cast<const __nv_bfloat16*>(dy);
   auto Hh = reinterpret_cast<const __nv_bfloat16*>(h);
   auto W = reinterpret_cast<const __nv_bfloat16*>(w);
   auto DR = reinterpret_cast<const __nv_bfloat16*>(dres);
   auto DX = reinterpret_cast<__nv_bfloat16*>(dx);
-#define CSB_NORM_BWD(LN, NV) \
-  norm_bwd_kernel<LN, NV><<<grid, NORM_THREADS, 0, s>>>(DY, Hh, W, mean, rstd, DR, DX, dw_partial, db_partial, rows, H, w_offset)
-  const int nv = H <= 2048 ? 1 : (H <= 4096 ? 2 : 4);
+#define CSB_NORM_BWD(LN, OW) \
+  norm_bwd_kernel<LN, OW><<<grid, threads, 0, s>>>(DY, Hh, W, mean, rstd, DR, DX, dw_partial, db_partial, rows, H, w_offset)
   if (is_layernorm) {
-    if (nv == 1) CSB_NORM_BWD(true, 1); else if (nv == 2) CSB_NORM_BWD(true, 2); else CSB_NORM_BWD(true, 4);
+    if (H <= 256) CSB_NORM_BWD(true, true); else CSB_NORM_BWD(true, false);
   } else {
-    if (nv == 1) CSB_NORM_BWD(false, 1); else if (nv == 2) CSB_NORM_BWD(false, 2); else CSB_NORM_BWD(false, 4);
+    if (H <= 256) CSB_NORM_BWD(false, true); else CSB_NORM_BWD(false, false);
   }
 #undef CSB_NORM_BWD
   int r = launch_result();
@@ -371,9 +401,13 @@ CSB_API int csb_colsum(const void* x, float* partial, void* out, int out_fp32, i
   if (H % 8 != 0 || rows <= 0) return CSB_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return CSB_ERR_BAD_ARG;  // 16-byte loads
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const int grid = csb_colsum_parts(rows);
-  colsum_partial_kernel<<<grid, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), partial, rows, H);
+  // row slices: enough blocks to fill the GPU four times, at least 8 rows (one per warp) in each, never more than promised
+  const int col_blocks = (H + COLSUM_COLS - 1) / COLSUM_COLS;
+  int slices = (sm_count() * 4 + col_blocks - 1) / col_blocks;
+  if (slices > (rows + 7) / 8) slices = (rows + 7) / 8;
+  if (slices > csb_colsum_parts(rows)) slices = csb_colsum_parts(rows);
+  colsum_partial_kernel<<<dim3(col_blocks, slices), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), partial, rows, H);
   if (int e = launch_result()) return e;
-  reduce_partials_kernel<<<(H + 31) / 32, 256, 0, s>>>(partial, out, grid, H, out_fp32, accumulate);
+  reduce_partials_kernel<<<(H + 31) / 32, 256, 0, s>>>(partial, out, slices, H, out_fp32, accumulate);
   return launch_result();
 }
