@@ -34,17 +34,20 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 // In place on the first `n_heads` heads of each token row of a [T][row_stride] buffer (the fused
 // q|k|v projection output): rotate-half convention, cos/sin tables fp32 [max_pos][D/2].
 // sign = +1 forward, -1 backward (the transpose of a rotation).
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __restrict__ cos_t,
+// A row of the block (threadIdx.y, 64 threads) takes one token at a time: no 64-bit index arithmetic per vector.
+// VEC: the tables are 16-byte aligned and read as float4.
+template <bool VEC>
+__global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const int* __restrict__ pos_ids, long T, int S,
                             int row_stride, int n_heads, int D, int rot_dim, float sign, int table_rows) {
   const int half = rot_dim / 2;
   const int vec_per_head = half / 8;
-  const long total = T * n_heads * vec_per_head;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+  const int per_row = n_heads * vec_per_head;  // a block row (threadIdx.y) takes one token row at a time
+  for (long t = blockIdx.x * (long)blockDim.y + threadIdx.y; t < T; t += (long)gridDim.x * blockDim.y) {
+#pragma unroll 2
+  for (int i = threadIdx.x; i < per_row; i += blockDim.x) {
     const int vc = i % vec_per_head;
-    const long th = i / vec_per_head;
-    const int hd = th % n_heads;
-    const long t = th / n_heads;
+    const int hd = i / vec_per_head;
     const int pos = pos_ids ? pos_ids[t] : static_cast<int>(t % S);
     if (!CSB_IN_BOUNDS(pos, table_rows, BND_ROPE_POS)) continue;
     __nv_bfloat16* p = buf + t * row_stride + hd * D + vc * 8;
@@ -55,22 +58,40 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __rest
     unpack8(u2, x2);
     const float* c = cos_t + static_cast<size_t>(pos) * half + vc * 8;
     const float* s = sin_t + static_cast<size_t>(pos) * half + vc * 8;
+    float cs[8], sn[8];
+    if constexpr (VEC) {
+      *reinterpret_cast<float4*>(cs) = __ldg(reinterpret_cast<const float4*>(c));
+      *reinterpret_cast<float4*>(cs + 4) = __ldg(reinterpret_cast<const float4*>(c) + 1);
+      *reinterpret_cast<float4*>(sn) = __ldg(reinterpret_cast<const float4*>(s));
+      *reinterpret_cast<float4*>(sn + 4) = __ldg(reinterpret_cast<const float4*>(s) + 1);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        cs[j] = c[j];
+        sn[j] = s[j];
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float cs = c[j], sn = sign * s[j];
-      o1[j] = x1[j] * cs - x2[j] * sn;
-      o2[j] = x2[j] * cs + x1[j] * sn;
+      o1[j] = x1[j] * cs[j] - x2[j] * (sign * sn[j]);
+      o2[j] = x2[j] * cs[j] + x1[j] * (sign * sn[j]);
     }
     *reinterpret_cast<uint4*>(p) = pack8(o1);
     *reinterpret_cast<uint4*>(p + half) = pack8(o2);
   }
+  }
 }
 
 // ------------------------------------------------------------------------------------ gated MLP activation
+// The tanh form of GELU is written with 0.5 (1 + tanh u) = 1 / (1 + exp(-2u)): one exponential instead of tanhf, and no
+// cancellation in 1 + tanh u for negative u.
+__device__ __forceinline__ float gelu_tanh_gate(float g) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  return 1.f / (1.f + __expf(-2.f * k0 * (g + k1 * g * g * g)));
+}
 __device__ __forceinline__ float act_fwd(float g, int act) {
   if (act == 0) return g / (1.f + __expf(-g));  // silu
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;  // gelu_tanh
-  return 0.5f * g * (1.f + tanhf(k0 * (g + k1 * g * g * g)));
+  return g * gelu_tanh_gate(g);
 }
 __device__ __forceinline__ float act_bwd(float g, int act) {
   if (act == 0) {
@@ -78,45 +99,86 @@ __device__ __forceinline__ float act_bwd(float g, int act) {
     return sg * (1.f + g * (1.f - sg));
   }
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float t = tanhf(k0 * (g + k1 * g * g * g));
-  return 0.5f * (1.f + t) + 0.5f * g * (1.f - t * t) * k0 * (1.f + 3.f * k1 * g * g);
+  const float sg = gelu_tanh_gate(g);
+  return sg + 2.f * g * sg * (1.f - sg) * k0 * (1.f + 3.f * k1 * g * g);
+}
+// silu forward and derivative from one exponential
+__device__ __forceinline__ void act_both(float g, int act, float& f, float& d) {
+  if (act == 0) {
+    const float sg = 1.f / (1.f + __expf(-g));
+    f = g * sg;
+    d = sg * (1.f + g * (1.f - sg));
+  } else {
+    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+    const float sg = gelu_tanh_gate(g);
+    f = g * sg;
+    d = sg + 2.f * g * sg * (1.f - sg) * k0 * (1.f + 3.f * k1 * g * g);
+  }
 }
 
+// The gated kernels: a thread owns one 8-column vector of the row (blockIdx.x) and walks the rows (blockIdx.y), two at a
+// time, so that no index is divided and the loads of two rows are in flight.
 // gu: [T][2I] (gate | up), y: [T][I].   y = act(gate) * up
-__global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, long T, int I,
-                               int act) {
-  const int vec = I / 8;
-  const long total = T * vec;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const long t = i / vec;
-    const int c = (i % vec) * 8;
-    float g[8], u[8], o[8];
-    unpack8(*reinterpret_cast<const uint4*>(gu + t * 2 * I + c), g);
-    unpack8(*reinterpret_cast<const uint4*>(gu + t * 2 * I + I + c), u);
+__global__ void __launch_bounds__(256) glu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, long T, int I,
+                                                      int act) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (c >= I) return;
+  for (long t = blockIdx.y; t < T; t += 2L * gridDim.y) {
+    const long t1 = t + gridDim.y;
+    uint4 rg[2], ru[2];
+    rg[0] = *reinterpret_cast<const uint4*>(gu + t * 2 * I + c);
+    ru[0] = *reinterpret_cast<const uint4*>(gu + t * 2 * I + I + c);
+    if (t1 < T) {
+      rg[1] = *reinterpret_cast<const uint4*>(gu + t1 * 2 * I + c);
+      ru[1] = *reinterpret_cast<const uint4*>(gu + t1 * 2 * I + I + c);
+    }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = act_fwd(g[j], act) * u[j];
-    *reinterpret_cast<uint4*>(y + t * I + c) = pack8(o);
+    for (int k = 0; k < 2; ++k) {
+      const long tk = k == 0 ? t : t1;
+      if (tk >= T) break;
+      float g[8], u[8], o[8];
+      unpack8(rg[k], g);
+      unpack8(ru[k], u);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = act_fwd(g[j], act) * u[j];
+      *reinterpret_cast<uint4*>(y + tk * I + c) = pack8(o);
+    }
   }
 }
 // dgu: [T][2I] <- (dy * up * act'(gate) | dy * act(gate))
-__global__ void glu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dy,
-                               __nv_bfloat16* __restrict__ dgu, long T, int I, int act) {
-  const int vec = I / 8;
-  const long total = T * vec;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const long t = i / vec;
-    const int c = (i % vec) * 8;
-    float g[8], u[8], d[8], og[8], ou[8];
-    unpack8(*reinterpret_cast<const uint4*>(gu + t * 2 * I + c), g);
-    unpack8(*reinterpret_cast<const uint4*>(gu + t * 2 * I + I + c), u);
-    unpack8(*reinterpret_cast<const uint4*>(dy + t * I + c), d);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      og[j] = d[j] * u[j] * act_bwd(g[j], act);
-      ou[j] = d[j] * act_fwd(g[j], act);
+__global__ void __launch_bounds__(256) glu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dy,
+                                                      __nv_bfloat16* __restrict__ dgu, long T, int I, int act) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (c >= I) return;
+  for (long t = blockIdx.y; t < T; t += 2L * gridDim.y) {
+    const long t1 = t + gridDim.y;
+    uint4 rg[2], ru[2], rd[2];
+    rg[0] = *reinterpret_cast<const uint4*>(gu + t * 2 * I + c);
+    ru[0] = *reinterpret_cast<const uint4*>(gu + t * 2 * I + I + c);
+    rd[0] = *reinterpret_cast<const uint4*>(dy + t * I + c);
+    if (t1 < T) {
+      rg[1] = *reinterpret_cast<const uint4*>(gu + t1 * 2 * I + c);
+      ru[1] = *reinterpret_cast<const uint4*>(gu + t1 * 2 * I + I + c);
+      rd[1] = *reinterpret_cast<const uint4*>(dy + t1 * I + c);
     }
-    *reinterpret_cast<uint4*>(dgu + t * 2 * I + c) = pack8(og);
-    *reinterpret_cast<uint4*>(dgu + t * 2 * I + I + c) = pack8(ou);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const long tk = k == 0 ? t : t1;
+      if (tk >= T) break;
+      float g[8], u[8], d[8], og[8], ou[8];
+      unpack8(rg[k], g);
+      unpack8(ru[k], u);
+      unpack8(rd[k], d);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float f, df;
+        act_both(g[j], act, f, df);
+        og[j] = d[j] * u[j] * df;
+        ou[j] = d[j] * f;
+      }
+      *reinterpret_cast<uint4*>(dgu + tk * 2 * I + c) = pack8(og);
+      *reinterpret_cast<uint4*>(dgu + tk * 2 * I + I + c) = pack8(ou);
+    }
   }
 }
 
@@ -256,6 +318,89 @@ adamw_kernel(__nv_bfloat16* __restrict__ param, void* __restrict__ master_v, flo
       if (zero_grad) {
         if constexpr (sizeof(GradT) == 4) __stcs(reinterpret_cast<float4*>(grad) + i, make_float4(0.f, 0.f, 0.f, 0.f));
         else __stcs(reinterpret_cast<uint2*>(grad) + i, make_uint2(0u, 0u));
+      }
+    }
+  }
+}
+
+// 32-byte accesses (sm_100): one instruction moves eight fp32 values of a thread, 1 KB of consecutive bytes of a warp.
+__device__ __forceinline__ void load_f32x8(const float* p, float (&f)[8]) {
+  asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]), "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7])
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void store_f32x8(float* p, const float (&f)[8]) {
+  asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.f32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]),
+               "f"(f[4]), "f"(f[5]), "f"(f[6]), "f"(f[7]), "l"(p)
+               : "memory");
+}
+
+// The update of adamw_kernel<GradT, true> with eight elements per thread: 16-byte accesses to the 16-bit arrays (parameter,
+// remainder, bf16 gradient), 32-byte accesses to the fp32 arrays.
+constexpr int ADAMW8_UNROLL = 1;
+template <typename GradT>
+__global__ void __launch_bounds__(256, 4)
+adamw_split8_kernel(__nv_bfloat16* __restrict__ param, uint4* __restrict__ resid, float* __restrict__ m,
+                    float* __restrict__ v, GradT* __restrict__ grad, long n, float lr, float b1, float b2,
+                    float eps, float wd, float bc1, float bc2, const float* __restrict__ grad_scale,
+                    const int* __restrict__ skip, int zero_grad) {
+  if (skip && *skip) return;
+  const float gs = grad_scale ? *grad_scale : 1.f;
+  const float inv_bc1 = 1.f / bc1, inv_bc2 = 1.f / bc2, decay = 1.f - lr * wd;
+  const long n8 = n / 8;
+  const long pass = (long)blockDim.x * ADAMW8_UNROLL;
+  for (long base = blockIdx.x * pass; base < n8; base += (long)gridDim.x * pass) {
+    uint4 pb[ADAMW8_UNROLL], rb[ADAMW8_UNROLL], gb[ADAMW8_UNROLL];
+    float mm[ADAMW8_UNROLL][8], vv[ADAMW8_UNROLL][8], gf[ADAMW8_UNROLL][8];
+#pragma unroll
+    for (int u = 0; u < ADAMW8_UNROLL; ++u) {
+      const long i = base + u * blockDim.x + threadIdx.x;
+      if (i < n8) {
+        pb[u] = __ldcs(reinterpret_cast<const uint4*>(param) + i);
+        rb[u] = __ldcs(resid + i);
+        if constexpr (sizeof(GradT) == 4) load_f32x8(reinterpret_cast<const float*>(grad) + i * 8, gf[u]);
+        else gb[u] = __ldcs(reinterpret_cast<const uint4*>(grad) + i);
+        load_f32x8(m + i * 8, mm[u]);
+        load_f32x8(v + i * 8, vv[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < ADAMW8_UNROLL; ++u) {
+      const long i = base + u * blockDim.x + threadIdx.x;
+      if (i >= n8) continue;
+      if constexpr (sizeof(GradT) == 2) unpack8(gb[u], gf[u]);
+      const uint32_t ph[4] = {pb[u].x, pb[u].y, pb[u].z, pb[u].w}, rh[4] = {rb[u].x, rb[u].y, rb[u].z, rb[u].w};
+      uint32_t po[4], ro[4];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t hi = (ph[j / 2] >> (16 * (j & 1))) & 0xffffu;
+        const int32_t lo = static_cast<int16_t>((rh[j / 2] >> (16 * (j & 1))) & 0xffffu);
+        float w = __uint_as_float((hi << 16) + static_cast<uint32_t>(lo));
+        const float gj = gf[u][j] * gs;
+        mm[u][j] = b1 * mm[u][j] + (1.f - b1) * gj;
+        vv[u][j] = b2 * vv[u][j] + (1.f - b2) * gj * gj;
+        const float denom = sqrtf(vv[u][j] * inv_bc2) + eps;
+        w = w * decay - lr * (mm[u][j] * inv_bc1) / denom;
+        const uint32_t bits = __float_as_uint(w);
+        const uint32_t hb = (bits + 0x8000u) >> 16;  // round half away from zero: the remainder is in [-32768, 32767]
+        const uint32_t lb = (bits - (hb << 16)) & 0xffffu;
+        if (j & 1) {
+          po[j / 2] |= hb << 16;
+          ro[j / 2] |= lb << 16;
+        } else {
+          po[j / 2] = hb;
+          ro[j / 2] = lb;
+        }
+      }
+      store_f32x8(m + i * 8, mm[u]);
+      store_f32x8(v + i * 8, vv[u]);
+      __stcs(resid + i, make_uint4(ro[0], ro[1], ro[2], ro[3]));
+      reinterpret_cast<uint4*>(param)[i] = make_uint4(po[0], po[1], po[2], po[3]);
+      if (zero_grad) {
+        const float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if constexpr (sizeof(GradT) == 4) store_f32x8(reinterpret_cast<float*>(grad) + i * 8, z);
+        else __stcs(reinterpret_cast<uint4*>(grad) + i, make_uint4(0u, 0u, 0u, 0u));
       }
     }
   }
@@ -517,26 +662,49 @@ static inline int ew_grid(long work, int threads) {
   return (int)(g < cap ? (g > 0 ? g : 1) : cap);
 }
 
+// Blocks of the gated kernels: columns x row slices, eight blocks of 256 threads per SM.
+static dim3 glu_grid(long T, int I, int* threads) {
+  const int vec = I / 8;
+  *threads = vec >= 256 ? 256 : (vec + 31) / 32 * 32;
+  const int bx = (vec + *threads - 1) / *threads;
+  long by = ((long)sm_count() * 8 * 256 / *threads + bx - 1) / bx;
+  if (by > T) by = T;
+  if (by > 65535) by = 65535;
+  return dim3((unsigned)bx, (unsigned)by);
+}
+
 // table_rows: rows of the cos / sin tables (what positions are checked against in the bounds-checked build).
 CSB_API int csb_rope(void* buf, const float* cos_t, const float* sin_t, const int* pos_ids, long T, int S,
                      int row_stride, int n_heads, int D, int rot_dim, float sign, int table_rows, void* stream) {
   if (rot_dim % 16 != 0 || rot_dim > D || (row_stride % 8) || (D % 8)) return CSB_ERR_BAD_ARG;
   if (pos_ids == nullptr && S > table_rows) return CSB_ERR_BAD_ARG;  // implicit positions 0..S-1 must fit the tables
-  const long work = T * n_heads * (rot_dim / 16);
-  rope_kernel<<<ew_grid(work, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<__nv_bfloat16*>(buf), cos_t, sin_t, pos_ids, T, S, row_stride, n_heads, D, rot_dim, sign, table_rows);
+  const bool vec = ((reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15) == 0;
+  const dim3 block(64, 4);
+  const int grid = ew_grid(T, 4);
+  if (vec)
+    rope_kernel<true><<<grid, block, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<__nv_bfloat16*>(buf), cos_t, sin_t, pos_ids, T, S, row_stride, n_heads, D, rot_dim, sign, table_rows);
+  else
+    rope_kernel<false><<<grid, block, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<__nv_bfloat16*>(buf), cos_t, sin_t, pos_ids, T, S, row_stride, n_heads, D, rot_dim, sign, table_rows);
   return launch_result();
 }
 
 CSB_API int csb_glu_fwd(const void* gu, void* y, long T, int I, int act, void* stream) {
   if (I % 8) return CSB_ERR_BAD_ARG;
-  glu_fwd_kernel<<<ew_grid(T * (I / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  if (T <= 0) return 0;
+  int threads;
+  const dim3 grid = glu_grid(T, I, &threads);
+  glu_fwd_kernel<<<grid, threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const __nv_bfloat16*>(gu), reinterpret_cast<__nv_bfloat16*>(y), T, I, act);
   return launch_result();
 }
 CSB_API int csb_glu_bwd(const void* gu, const void* dy, void* dgu, long T, int I, int act, void* stream) {
   if (I % 8) return CSB_ERR_BAD_ARG;
-  glu_bwd_kernel<<<ew_grid(T * (I / 8), 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  if (T <= 0) return 0;
+  int threads;
+  const dim3 grid = glu_grid(T, I, &threads);
+  glu_bwd_kernel<<<grid, threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const __nv_bfloat16*>(gu), reinterpret_cast<const __nv_bfloat16*>(dy),
       reinterpret_cast<__nv_bfloat16*>(dgu), T, I, act);
   return launch_result();
@@ -585,6 +753,19 @@ CSB_API int csb_adamw_split(void* param, short* resid, float* m, float* v, void*
                             const int* skip, int zero_grad, void* stream) {
   if (n % 4) return CSB_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  auto aligned = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
+  if (n % 8 == 0 && aligned(param, 16) && aligned(resid, 16) && aligned(m, 32) && aligned(v, 32) && aligned(grad, grad_fp32 ? 32 : 16)) {
+    const int grid8 = ew_grid(n / 8 / ADAMW8_UNROLL + 1, 256);
+    if (grad_fp32)
+      adamw_split8_kernel<float><<<grid8, 256, 0, s>>>(reinterpret_cast<__nv_bfloat16*>(param), reinterpret_cast<uint4*>(resid), m, v,
+                                                       reinterpret_cast<float*>(grad), n, lr, b1, b2, eps, wd, bc1, bc2,
+                                                       grad_scale, skip, zero_grad);
+    else
+      adamw_split8_kernel<__nv_bfloat16><<<grid8, 256, 0, s>>>(reinterpret_cast<__nv_bfloat16*>(param), reinterpret_cast<uint4*>(resid), m, v,
+                                                               reinterpret_cast<__nv_bfloat16*>(grad), n, lr, b1, b2, eps, wd,
+                                                               bc1, bc2, grad_scale, skip, zero_grad);
+    return launch_result();
+  }
   const int grid = ew_grid(n / 4 / ADAMW_UNROLL + 1, 256);
   if (grad_fp32)
     adamw_kernel<float, true><<<grid, 256, 0, s>>>(reinterpret_cast<__nv_bfloat16*>(param), resid, m, v,
