@@ -134,6 +134,12 @@ class AttnMask:
         return c
 
 
+    def by_index(self) -> bool:
+        """Whether the token indices alone decide the mask: the kernels then work the tile classes out themselves and no
+        class map is made (one launch less in front of a call's first use of a mask)."""
+        return self.mode == MASK_FULL or (self.mode == MASK_CAUSAL and self.q_pos is None and self.k_pos is None)
+
+
 def dense_mask(mask: AttnMask, B: int, Sq: int, Sk: int, device="cpu") -> torch.Tensor:
     """Boolean ``[B, Sq, Sk]`` (True = may attend): direct statement of the per-element predicate."""
     qp = mask.q_pos.to(device).long() if mask.q_pos is not None else torch.arange(Sq, device=device).expand(B, Sq)
@@ -240,7 +246,7 @@ def attention_forward(q, k, v, mask: AttnMask, scale: float | None = None):
         _check_layout(t, n)
     out = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device)
     lse = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device)
-    cls = mask.classes(B, Sq, Sk, q.device)
+    cls = None if mask.by_index() else mask.classes(B, Sq, Sk, q.device)
     st = nat.status_word(q.device)
     ex, keep = mask.extras(B, Hq, Sq, Sk, q.device)
     if ex is not None:
@@ -248,7 +254,7 @@ def attention_forward(q, k, v, mask: AttnMask, scale: float | None = None):
             nat.lib().csb_attn_fwd_dense(
                 q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), B, Sq, Sk, Hq, Hk, D,
                 q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1), v.stride(0), out.stride(1), out.stride(0),
-                scale, mask.mode, cls.data_ptr(), C.addressof(ex), st.data_ptr(), nat.stream(),
+                scale, mask.mode, nat.ptr(cls), C.addressof(ex), st.data_ptr(), nat.stream(),
             ),
             "csb_attn_fwd_dense",
         )
@@ -258,7 +264,7 @@ def attention_forward(q, k, v, mask: AttnMask, scale: float | None = None):
         nat.lib().csb_attn_fwd(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), B, Sq, Sk, Hq, Hk, D,
             q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1), v.stride(0), out.stride(1), out.stride(0),
-            scale, mask.mode, nat.ptr(qb), nat.ptr(kb), nat.ptr(qp), nat.ptr(kp), cls.data_ptr(), st.data_ptr(),
+            scale, mask.mode, nat.ptr(qb), nat.ptr(kb), nat.ptr(qp), nat.ptr(kp), nat.ptr(cls), st.data_ptr(),
             nat.stream(),
         ),
         "csb_attn_fwd",
@@ -278,7 +284,7 @@ def attention_backward(do, q, k, v, out, lse, mask: AttnMask, scale: float | Non
     dv = torch.empty((B, Sk, Hk, D), dtype=q.dtype, device=q.device) if dv is None else dv
     dq_acc = torch.zeros((B, Sq, Hq, D), dtype=torch.float32, device=q.device)
     delta = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device)
-    cls = mask.classes(B, Sq, Sk, q.device)
+    cls = None if mask.by_index() else mask.classes(B, Sq, Sk, q.device)
     st = nat.status_word(q.device)
     ex, keep = mask.extras(B, Hq, Sq, Sk, q.device)
     if ex is not None:
@@ -288,7 +294,7 @@ def attention_backward(do, q, k, v, out, lse, mask: AttnMask, scale: float | Non
                 dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, Sq, Sk, Hq, Hk, D,
                 q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1), v.stride(0), out.stride(1), out.stride(0),
                 do.stride(1), do.stride(0), dq.stride(1), dq.stride(0), dk.stride(1), dk.stride(0), dv.stride(1),
-                dv.stride(0), scale, mask.mode, cls.data_ptr(), C.addressof(ex), st.data_ptr(), nat.stream(),
+                dv.stride(0), scale, mask.mode, nat.ptr(cls), C.addressof(ex), st.data_ptr(), nat.stream(),
             ),
             "csb_attn_bwd_dense",
         )
@@ -300,7 +306,7 @@ def attention_backward(do, q, k, v, out, lse, mask: AttnMask, scale: float | Non
             dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, Sq, Sk, Hq, Hk, D,
             q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1), v.stride(0), out.stride(1), out.stride(0),
             do.stride(1), do.stride(0), dq.stride(1), dq.stride(0), dk.stride(1), dk.stride(0), dv.stride(1),
-            dv.stride(0), scale, mask.mode, nat.ptr(qb), nat.ptr(kb), nat.ptr(qp), nat.ptr(kp), cls.data_ptr(),
+            dv.stride(0), scale, mask.mode, nat.ptr(qb), nat.ptr(kb), nat.ptr(qp), nat.ptr(kp), nat.ptr(cls),
             st.data_ptr(), nat.stream(),
         ),
         "csb_attn_bwd",
