@@ -234,13 +234,10 @@ class Attention(nn.Module):
             qkv = torch.cat([q, k, v], dim=-1)
         if rope is not None:
             qkv = E.rope_(qkv, rope[0], rope[1], pos, Hq + Hk, D)
-        q = qkv[..., : Hq * D].view(B, S, Hq, D)
-        k = qkv[..., Hq * D : (Hq + Hk) * D].view(B, S, Hk, D)
-        v = qkv[..., (Hq + Hk) * D :].view(B, S, Hk, D)
         if self.attn_impl is not None:
-            o = self.attn_impl(q, k, v, mask, self.scale)
+            o = self.attn_impl(*A.split_qkv(qkv, Hq, Hk, D), mask, self.scale)
         else:
-            o = A.attention(q, k, v, mask, self.scale)
+            o = A.attention_qkv(qkv, Hq, Hk, D, mask, self.scale)
         o = o.reshape(B, S, Hq * D)
         if ulysses:
             o = comm.all_to_all_comm(o, self.pc.sp_group, 1, 2)

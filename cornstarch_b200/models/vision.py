@@ -78,13 +78,10 @@ def encoder_block(x, ln1, q, k, v, o, ln2, fc1, fc2, act: str, num_heads: int, m
     biases = [q.bias, k.bias, v.bias] if (q.bias is not None or k.bias is not None or v.bias is not None) else None
     qkv = multi_linear(hin, [q.weight, k.weight, v.weight], biases, tp=q.tp_spec(h))
     nh = q.weight.shape[0] // D
-    qh = qkv[..., : nh * D].view(B, S, nh, D)
-    kh = qkv[..., nh * D : 2 * nh * D].view(B, S, nh, D)
-    vh = qkv[..., 2 * nh * D :].view(B, S, nh, D)
     if attn_impl is not None:
-        a = attn_impl(qh, kh, vh, mask, scale)
+        a = attn_impl(*A.split_qkv(qkv, nh, nh, D), mask, scale)
     else:
-        a = A.attention(qh, kh, vh, mask, scale)
+        a = A.attention_qkv(qkv, nh, nh, D, mask, scale)
     a = o(a.reshape(B, S, nh * D))
     h2, x = ln2(a, x)  # x <- x + a ; h2 = LN(x)
     m = fc2(E.activation(fc1(h2), act))

@@ -345,6 +345,37 @@ class _AttnReplayFn(torch.autograd.Function):
         return dq, dk, dv, None, None, None, None
 
 
+def split_qkv(qkv: torch.Tensor, Hq: int, Hk: int, D: int):
+    """``q [B,S,Hq,D]``, ``k``, ``v [B,S,Hk,D]`` as views of a fused ``[B, S, (Hq + 2 Hk) D]`` projection output."""
+    B, S, _ = qkv.shape
+    q = qkv[..., : Hq * D].view(B, S, Hq, D)
+    k = qkv[..., Hq * D : (Hq + Hk) * D].view(B, S, Hk, D)
+    v = qkv[..., (Hq + Hk) * D :].view(B, S, Hk, D)
+    return q, k, v
+
+
+class _AttnQkvFn(torch.autograd.Function):
+    """Attention on a fused q|k|v buffer.  The backward kernel writes dQ, dK and dV straight into one gradient buffer of the
+    same layout; as three slices they would come back through autograd as three zero-filled buffers of the full width that
+    are then added up (about 1 GB of memory traffic per 8192 tokens of a 32/8-head, 128-wide layer).  ``kept``: output and
+    LSE of an earlier run of the same call (activation recomputation), the forward kernel is then skipped."""
+
+    @staticmethod
+    def forward(ctx, qkv, Hq, Hk, D, mask, scale, kept):
+        out, lse = kept if kept is not None else attention_forward(*split_qkv(qkv, Hq, Hk, D), mask, scale)
+        ctx.save_for_backward(qkv, out, lse)
+        ctx.dims, ctx.mask, ctx.scale = (Hq, Hk, D), mask, scale
+        return out if kept is None else out.view_as(out)
+
+    @staticmethod
+    def backward(ctx, do):
+        qkv, out, lse = ctx.saved_tensors
+        dqkv = torch.empty(qkv.shape, dtype=qkv.dtype, device=qkv.device)
+        dq, dk, dv = split_qkv(dqkv, *ctx.dims)
+        attention_backward(do, *split_qkv(qkv, *ctx.dims), out, lse, ctx.mask, ctx.scale, dq=dq, dk=dk, dv=dv)
+        return dqkv, None, None, None, None, None, None
+
+
 _TAPE = threading.local()
 
 
@@ -418,3 +449,14 @@ def attention(q, k, v, mask: AttnMask | None = None, scale: float | None = None)
         return _AttnFn.apply(q, k, v, mask, scale)
     o, _ = attention_reference(q, k, v, mask, scale)
     return o
+
+
+def attention_qkv(qkv, Hq: int, Hk: int, D: int, mask: AttnMask | None = None, scale: float | None = None) -> torch.Tensor:
+    """:func:`attention` of a fused ``[B, S, (Hq + 2 Hk) D]`` projection output (q heads, then k heads, then v heads)."""
+    native = qkv.is_cuda and qkv.dtype == torch.bfloat16 and not nat.LIBRARY_MODE
+    if not native or qkv.shape[-1] != (Hq + 2 * Hk) * D or not torch.is_grad_enabled() or not qkv.requires_grad:
+        return attention(*split_qkv(qkv, Hq, Hk, D), mask, scale)
+    mask = mask or AttnMask.causal()
+    tape = getattr(_TAPE, "cur", None)
+    kept = tape.items.pop(0) if tape is not None and tape.mode == "replay" and tape.items else None
+    return _AttnQkvFn.apply(qkv, Hq, Hk, D, mask, scale, kept)
