@@ -110,6 +110,7 @@ class _CountingLib:
                         launch_count += 1
                         return _t(*a)
             self._cache[name] = fn
+            setattr(self, name, fn)  # later calls find it without coming back here
         return fn
 
 
@@ -152,7 +153,9 @@ def ptr(t: torch.Tensor | None):
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (what ``torch.cuda.current_stream().cuda_stream`` is, without the
+    stream object and the device look-ups around it: 0.3 against 3 us, once per launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def check(code: int, what: str) -> None:

@@ -171,6 +171,18 @@ class _LinearFn(torch.autograd.Function):
                         else:
                             dws[i] = gemm(dy2[:, o : o + n], x2, a_mn_major=True, b_mn_major=True)
                     o += n
+        if (ctx.has_bias and n_w > 1 and dy2.is_contiguous() and all(b is not None for b in ctx.biases)
+                and all(ctx.needs_input_grad[4 + n_w :])):
+            # one column sum over all projections' outputs instead of a copy and a sum for each
+            mains = [getattr(b, "main_grad", None) for b in ctx.biases]
+            fused_main = fuse_adjacent_1d(mains)
+            if fused_main is not None:
+                colsum(dy2, out=fused_main, accumulate=True)
+                for b in ctx.biases:
+                    b.grad_added_to_main_grad = True
+                return (dx, None, None, None, *dws, *dbs)
+            if all(m is None for m in mains):
+                return (dx, None, None, None, *dws, *torch.split(colsum(dy2), [w.shape[0] for w in weights]))
         if ctx.has_bias:
             o = 0
             for i, (w, b) in enumerate(zip(weights, ctx.biases)):
