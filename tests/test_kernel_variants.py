@@ -1,0 +1,217 @@
+"""The variants that a size, type or alignment selects inside one entry point, at the sizes where the selection or the
+variant's own edges lie, against the oracles of the modules (or against the general variant, bit for bit)."""
+
+import pytest
+import torch
+
+from cornstarch_b200.ops import attention as A
+from cornstarch_b200.ops import elementwise as E
+from cornstarch_b200.ops.gemm import gemm, gemm_reference
+from cornstarch_b200.ops.linear import colsum, multi_linear
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+# Outputs are bf16 (half a unit in the last place: 2^-9 of the value) computed from operands that are rounded to bf16 once
+# more inside the attention kernels: a relative 2-norm error of 2^-8 = 3.9e-3 is what a correct kernel stays below.
+REL = 2.0**-8
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm().clamp(min=1e-30)).item()
+
+
+def _bits(B, S, pad):
+    text, image = (1 << 62) | 3, 2
+    bits = torch.full((B, S), text, dtype=torch.int64, device="cuda")
+    for b in range(B):
+        bits[b, 5 + b * 40 : 5 + b * 40 + S // 3] = image
+    bits[-1, S - pad :] = 0
+    return bits
+
+
+# 148 or more blocks of two query tiles select the paired kernel; 1, 2 and 3 tiles per head, ragged last tiles, widths on
+# both sides of 64, one and several query heads per key head
+@pytest.mark.parametrize("S", [128, 129, 256, 257, 390])
+@pytest.mark.parametrize("Hq,Hk,D", [(16, 16, 72), (32, 8, 64), (32, 4, 128), (16, 8, 16)])
+@pytest.mark.parametrize("mode", ["causal", "full", "bitfield", "prefix"])
+def test_paired_attention_forward(S, Hq, Hk, D, mode):
+    B = 10
+    g = torch.Generator(device="cuda").manual_seed(S + D)
+    q, k, v = (torch.randn(B, S, h, D, generator=g, device="cuda").to(BF16) for h in (Hq, Hk, Hk))
+    mask = {"causal": A.AttnMask.causal(), "full": A.AttnMask.full(), "bitfield": A.AttnMask.bitfield(_bits(B, S, 9)),
+            "prefix": A.AttnMask.bitfield(_bits(B, S, 9), prefix_causal=True)}[mode]
+    o, lse = A.attention_forward(q, k, v, mask)
+    ro, rlse = A.attention_reference(q, k, v, mask)
+    assert _rel(o, ro) <= REL
+    live = torch.isfinite(rlse)
+    assert torch.equal(torch.isfinite(lse), live)
+    assert (lse[live] - rlse[live]).abs().max().item() <= 1e-4  # fp32 sums of at most 390 terms around 1..10
+
+
+@pytest.mark.parametrize("S,Sk", [(57, 57), (128, 128), (257, 257), (129, 300), (300, 129)])
+@pytest.mark.parametrize("B", [1, 12])
+def test_index_masks_equal_the_class_map(S, Sk, B):
+    """Causal and full masks without positions need no class map; with explicit positions 0, 1, 2, ... the same mask goes
+    through the map.  Same tiles, same arithmetic: the same bits (dQ is summed by reduce-adds in no fixed order)."""
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, do = (torch.randn(B, S, 16, 64, generator=g, device="cuda").to(BF16) for _ in range(2))
+    k, v = (torch.randn(B, Sk, 16, 64, generator=g, device="cuda").to(BF16) for _ in range(2))
+    pos = dict(q_pos=torch.arange(S, device="cuda")[None].int(), k_pos=torch.arange(Sk, device="cuda")[None].int())
+    for plain, mapped in ((A.AttnMask.causal(), A.AttnMask(mode=A.MASK_CAUSAL, **pos)), (A.AttnMask.full(), A.AttnMask(mode=A.MASK_FULL, **pos))):
+        mapped_cls = A.classify_mask(mapped, B, S, Sk, "cuda")
+        assert torch.equal(mapped_cls.cpu(), A.classify_mask(A.AttnMask(mode=plain.mode), B, S, Sk, "cpu"))
+        o1, l1 = A.attention_forward(q, k, v, plain)
+        o2, l2 = A.attention_forward(q, k, v, mapped)
+        assert torch.equal(o1, o2) and torch.equal(l1, l2)
+        g1, g2 = (A.attention_backward(do, q, k, v, o1, l1, m) for m in (plain, mapped))
+        assert torch.equal(g1[1], g2[1]) and torch.equal(g1[2], g2[2]) and _rel(g1[0], g2[0]) <= REL
+
+
+@pytest.mark.parametrize("Hq,Hk,D", [(8, 2, 64), (4, 4, 72)])
+def test_fused_qkv_attention_matches_slices(Hq, Hk, D):
+    g = torch.Generator(device="cuda").manual_seed(D)
+    base = torch.randn(2, 200, (Hq + 2 * Hk) * D, generator=g, device="cuda").to(BF16)
+    do = torch.randn(2, 200, Hq, D, generator=g, device="cuda").to(BF16)
+    grads = []
+    for fused in (True, False):
+        x = base.clone().requires_grad_()
+        o = A.attention_qkv(x, Hq, Hk, D) if fused else A.attention(*A.split_qkv(x, Hq, Hk, D))
+        o.backward(do)
+        grads.append((o.detach(), x.grad))
+    assert torch.equal(grads[0][0], grads[1][0])
+    kv = slice(Hq * D, None)
+    assert torch.equal(grads[0][1][..., kv], grads[1][1][..., kv]) and _rel(grads[0][1], grads[1][1]) <= REL
+    with torch.no_grad():
+        assert torch.equal(A.attention_qkv(base, Hq, Hk, D), grads[0][0])
+
+
+# shapes whose cheapest tile is 192 or 128 columns of a pair, 256 columns of one block, or the width by size; remainders in
+# every dimension, rows that leave the second block of a pair without work, N that is no multiple of the width
+@pytest.mark.parametrize("M,N,K", [(2916, 1152, 4304), (1500, 1160, 1000), (77, 4096, 6144), (130, 200, 4104), (4304, 1152, 2916),
+                                   (4096, 1160, 264), (6144, 4096, 72), (300, 4304, 1160), (1, 392, 2056)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+def test_gemm_tiles(M, N, K, a_mn, b_mn):
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    Mp = (M + 7) // 8 * 8
+    a = torch.randn(*((K, Mp) if a_mn else (M, K)), generator=g, device="cuda").to(BF16)
+    a = a[:, :M] if a_mn else a
+    b = torch.randn(*((K, N) if b_mn else (N, K)), generator=g, device="cuda").to(BF16)
+    ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    assert _rel(gemm(a, b, a_mn, b_mn), ref) <= REL
+    acc = torch.randn(M, N, generator=g, device="cuda")
+    want = ref + acc.double()
+    gemm(a, b, a_mn, b_mn, out=acc, accumulate=True)
+    assert _rel(acc, want) <= 1e-5  # fp32 sums
+
+
+@pytest.mark.parametrize("H", [8, 248, 256, 264, 1152, 4104, 8192])
+@pytest.mark.parametrize("rows", [1, 7, 9, 1201])
+@pytest.mark.parametrize("ln", [False, True])
+def test_norm_row_splits(H, rows, ln):
+    """A warp per row up to 256 elements, a block of H / 8 threads above."""
+    g = torch.Generator(device="cuda").manual_seed(H + rows)
+    x, r, dy, dh = (torch.randn(rows, H, generator=g, device="cuda").to(BF16) for _ in range(4))
+    w, b = (torch.randn(H, generator=g, device="cuda").to(BF16) for _ in range(2))
+    ins = [t.requires_grad_() for t in ([x, r, w, b] if ln else [x, r, w])]
+    y, h = E.layer_norm(x, w, b, 1e-5, r) if ln else E.rms_norm(x, w, 1e-5, r)
+    got = torch.autograd.grad([y, h], ins, [dy, dh])
+    # the kernels normalise the bf16 sum that they store
+    hd = h.detach().double().requires_grad_()
+    wd, bd = w.detach().double().requires_grad_(), b.detach().double().requires_grad_()
+    yd = (torch.nn.functional.layer_norm(hd, (H,), wd, bd, 1e-5) if ln
+          else hd * torch.rsqrt(hd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd)
+    ref = torch.autograd.grad([yd], [hd, wd] + ([bd] if ln else []), [dy.double()])
+    assert _rel(y, yd) <= REL
+    # (a layer norm over 8 elements subtracts nearly equal terms: compare with the size of what is summed)
+    assert _rel(got[0], ref[0] + dh.double()) <= REL and torch.equal(got[0], got[1])
+    for a, c in zip(got[2:], ref[1:]):
+        assert _rel(a, c) <= REL
+
+
+@pytest.mark.parametrize("rows,H", [(1, 8), (8, 256), (9, 264), (1201, 4304), (297, 4096)])
+def test_colsum_slices(rows, H):
+    x = torch.randn(rows, H, device="cuda").to(BF16)
+    out = torch.randn(H, device="cuda")
+    want = out.double() + x.double().sum(0)
+    colsum(x, out=out, accumulate=True)
+    assert (out.double() - want).abs().max().item() <= 1e-4  # fp32 sums of up to 1201 values around 1
+
+
+def test_bias_gradients_of_fused_projections():
+    x = torch.randn(100, 64, device="cuda").to(BF16).requires_grad_()
+    ws = [torch.randn(n, 64, device="cuda").to(BF16).requires_grad_() for n in (64, 24, 40)]
+    bs = [torch.randn(n, device="cuda").to(BF16).requires_grad_() for n in (64, 24, 40)]
+    dy = torch.randn(100, 128, device="cuda").to(BF16)
+    multi_linear(x, ws, bs).backward(dy)
+    for b, part in zip(bs, torch.split(dy.double().sum(0), [64, 24, 40])):
+        assert _rel(b.grad, part) <= REL
+
+
+@pytest.mark.parametrize("grad_dtype", [BF16, torch.float32])
+def test_adamw_eight_wide_equals_general(grad_dtype):
+    """n a multiple of 8 and aligned pointers take 32-byte accesses; arrays that start 4 elements in take the general kernel.
+    The same update: the same bits."""
+    from cornstarch_b200.ops import _native as nat
+
+    n = 8 * 1237
+    g = torch.Generator(device="cuda").manual_seed(0)
+    src = dict(param=torch.randn(n, generator=g, device="cuda").to(BF16), resid=torch.randint(-32768, 32768, (n,), generator=g, device="cuda").to(torch.int16),
+               m=torch.randn(n, generator=g, device="cuda") * 1e-3, v=torch.rand(n, generator=g, device="cuda") * 1e-6,
+               grad=(torch.randn(n, generator=g, device="cuda") * 1e-3).to(grad_dtype))
+    scale, skip = torch.full((1,), 0.5, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    res = []
+    for off in (0, 4):
+        t = {}
+        for k, x in src.items():
+            buf = torch.zeros(n + 16, dtype=x.dtype, device="cuda")
+            t[k] = buf[off : off + n]
+            t[k].copy_(x)
+        nat.check(nat.lib().csb_adamw_split(*(t[k].data_ptr() for k in ("param", "resid", "m", "v", "grad")), int(grad_dtype == torch.float32), n,
+                                            1e-3, 0.9, 0.999, 1e-8, 0.01, 0.1, 0.01, scale.data_ptr(), skip.data_ptr(), 1, nat.stream()), "adamw")
+        res.append(t)
+    for k in src:
+        assert torch.equal(res[0][k], res[1][k]), k
+    assert not res[0]["grad"].any() and not torch.equal(res[0]["param"], src["param"])
+
+
+@pytest.mark.parametrize("T,I", [(1, 8), (3, 40), (5, 2056), (700, 264)])
+@pytest.mark.parametrize("act", ["silu", "gelu_pytorch_tanh"])
+def test_gated_activation_columns_and_rows(T, I, act):
+    gu = (3 * torch.randn(T, 2 * I, device="cuda")).to(BF16).requires_grad_()
+    dy = torch.randn(T, I, device="cuda").to(BF16)
+    y = E.glu(gu, act)
+    (got,) = torch.autograd.grad(y, gu, dy)
+    x = gu.detach().double().requires_grad_()
+    f = torch.nn.functional.silu(x[:, :I]) if act == "silu" else torch.nn.functional.gelu(x[:, :I], approximate="tanh")
+    ref = f * x[:, I:]
+    (want,) = torch.autograd.grad(ref, x, dy.double())
+    assert _rel(y, ref) <= REL and _rel(got, want) <= REL
+
+
+def test_tanh_gelu_error_over_the_range_of_bf16():
+    """The sigmoid form of the tanh GELU against 64 bits over every finite bf16 value up to 2^40: half a unit in the last
+    place of the result, plus fp32 rounding where the value is tiny."""
+    x = torch.arange(-32768, 32768, device="cuda").to(torch.int16).view(BF16)
+    x = x[torch.isfinite(x) & (x.abs() < 2.0**40)]
+    x = x[: x.numel() // 8 * 8].requires_grad_()
+    y = E.activation(x, "gelu_pytorch_tanh")
+    (got,) = torch.autograd.grad(y, x, torch.ones_like(y))
+    d = x.detach().double().requires_grad_()
+    ref = torch.nn.functional.gelu(d, approximate="tanh")
+    (want,) = torch.autograd.grad(ref, d, torch.ones_like(ref))
+    for a, r in ((y, ref), (got, want)):
+        err = (a.double() - r).abs()
+        fine = torch.isfinite(r) & torch.isfinite(a.double())
+        assert bool((err[fine] <= 2.0**-8 * r[fine].abs() + 1e-6).all())
+
+
+def test_rope_with_tables_off_the_16_byte_boundary():
+    T, H, D = 50, 3, 32
+    cos, sin = E.rope_tables(64, D, device="cuda")
+    off = [torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view_as(t) for t in (cos, sin)]
+    assert off[0].data_ptr() % 16 != 0
+    x = torch.randn(1, T, H * D, device="cuda").to(BF16)
+    a = E.rope_(x.clone(), cos, sin, None, H, D)
+    b = E.rope_(x.clone(), *off, None, H, D)
+    want = E._rope_ref(x.view(1, T, H, D), cos, sin, None, D).view_as(x)
+    assert torch.equal(a, b) and _rel(a, want) <= REL
