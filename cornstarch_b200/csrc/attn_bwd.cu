@@ -16,12 +16,12 @@
 // accumulator by TMA reduce-add (one 32x32 block per warp), then converted to bf16 by a final pass.
 //
 // Warp roles (768 threads by default): warp 0 = TMA producer (K/V once, Q/dO ring of 3 stages), warp 1 = MMA
-// issuer, warps 4..7 = dQ^T drain, warps 8..23 = 512 compute threads (or 8..15 = 256).  Thread (r, group) owns KV row r (TMEM lane r) and 16
+// issuer, warps 2 and 3 = query metadata, warps 4..7 = dQ^T drain, warps 8..23 = 512 compute threads (or 8..15 = 256).  Thread (r, group) owns KV row r (TMEM lane r) and 16
 // (32) of the 64 query columns of S^T / dP^T; a drain thread moves head-dim row r of dQ^T.  The pipeline keeps S^T one
 // iteration ahead: while the compute warps turn S^T(i), dP^T(i) into P^T, dS^T, the tensor core
 // already holds S^T(i+1); dP^T(i+1) is issued as soon as dP^T(i) has been read, before the
 // dV/dK/dQ^T MMAs of iteration i, so the next exponentials overlap those MMAs.  Per-tile query
-// metadata (LSE, delta, positions, bitfields) is prefetched into registers one iteration early.
+// metadata (LSE, delta, mask rules) is staged in shared memory by two warps of its own, a ring stage with Q / dO.
 //
 // Replaces cornstarch/kernel/bitfield_attention.py:526-929 (T8, T9: fp32 atomics for dQ, dK and dV)
 // and cornstarch/kernel/attention.py:348-852.
@@ -72,9 +72,9 @@ struct BwdSmem {
   static constexpr int DO_OFF = Q_OFF + QSTAGES * 2 * Q_CHUNK;
   static constexpr int DST_OFF = DO_OFF + QSTAGES * 2 * Q_CHUNK;  // dS^T [128 kv][64 q] bf16
   static constexpr int DQ_OFF = DST_OFF + KV_CHUNK;           // dQ staging: 8 warps x [32 q][32 d] fp32 (row-major, 4 KB each)
-  static constexpr int META_OFF = DQ_OFF + 8 * 4096;          // three buffers of: -lse2[64] f32, -delta*scale[64] f32, and the mask rules lim[64] i32, am[64] i64, qe[64] i64
+  static constexpr int META_OFF = DQ_OFF + 8 * 4096;          // one buffer per Q stage of: -lse2[64] f32, -delta*scale[64] f32, and the mask rules lim[64] i32, am[64] i64, qe[64] i64
   static constexpr int META_STAGE = 64 * 4 * 3 + 2 * 64 * 8;
-  static constexpr int LIST_OFF = META_OFF + 3 * META_STAGE;  // valid 64-row query tiles of this key block: int16 index, int8 class
+  static constexpr int LIST_OFF = META_OFF + QSTAGES * META_STAGE;  // valid 64-row query tiles of this key block: int16 index, int8 class
   static constexpr int MAX_TILES = 1024;                      // sequences up to 65536 tokens
   static constexpr int BAR_OFF = LIST_OFF + MAX_TILES * 4;
   static constexpr int NBAR = 1 + QSTAGES + QSTAGES + 1 + 1 + 1 + 1 + 1 + 1;
@@ -109,45 +109,84 @@ __device__ __forceinline__ bool bw_wait(uint64_t* bar, uint32_t phase, volatile 
   return false;
 }
 
-// delta[b][h][q] = sum_d O[b][q][h][d] * dO[b][q][h][d]
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO,
-                                  float* __restrict__ delta, int B, int Sq, int Hq, int D, long o_sb, long o_ss,
-                                  long do_sb, long do_ss) {
-  const long row = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;  // one warp per (b, q, h)
-  const int lane = threadIdx.x & 31;
-  const long total = (long)B * Sq * Hq;
-  if (row >= total) return;
-  const int h = row % Hq;
-  const long bq = row / Hq;
-  const int q = bq % Sq;
-  const int b = bq / Sq;
-  const __nv_bfloat16* o = O + b * o_sb + (long)q * o_ss + (long)h * D;
-  const __nv_bfloat16* d = dO + b * do_sb + (long)q * do_ss + (long)h * D;
-  float acc = 0.f;
-  for (int i = lane * 2; i < D; i += 64) {
-    float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(o + i));
-    float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(d + i));
-    acc += a.x * c.x + a.y * c.y;
+// delta[b][h][q] = sum_d O[b][q][h][d] * dO[b][q][h][d].  Sixteen lanes share a row (8 elements each, D <= 128) and take
+// DELTA_ROWS queries of one head, so that every thread has 2 x DELTA_ROWS 16-byte loads in flight and the results of a block
+// are consecutive.  VEC: rows of both tensors start on 16-byte boundaries.
+constexpr int DELTA_ROWS = 4;
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __restrict__ dO, float* __restrict__ delta, int Sq,
+                  int Hq, int D, long o_sb, long o_ss, long do_sb, long do_ss) {
+  const int lane16 = threadIdx.x & 15, row = threadIdx.x >> 4;
+  const int n_qb = (Sq + 16 * DELTA_ROWS - 1) / (16 * DELTA_ROWS);
+  const int hb = blockIdx.x / n_qb;
+  const int h = hb % Hq, b = hb / Hq;
+  const int q0 = (blockIdx.x - hb * n_qb) * (16 * DELTA_ROWS) + row;
+  const int c = lane16 * 8;
+  uint4 uo[DELTA_ROWS], ud[DELTA_ROWS];
+#pragma unroll
+  for (int i = 0; i < DELTA_ROWS; ++i) {
+    const int q = q0 + i * 16;
+    uo[i] = ud[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (q < Sq && c < D) {
+      const __nv_bfloat16* o = O + b * o_sb + (long)q * o_ss + (long)h * D + c;
+      const __nv_bfloat16* d = dO + b * do_sb + (long)q * do_ss + (long)h * D + c;
+      if constexpr (VEC) {
+        uo[i] = *reinterpret_cast<const uint4*>(o);
+        ud[i] = *reinterpret_cast<const uint4*>(d);
+      } else {
+        __align__(16) __nv_bfloat16 to[8], td[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          to[j] = o[j];
+          td[j] = d[j];
+        }
+        uo[i] = *reinterpret_cast<const uint4*>(to);
+        ud[i] = *reinterpret_cast<const uint4*>(td);
+      }
+    }
   }
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (lane == 0) delta[((long)b * Hq + h) * Sq + q] = acc;
+  for (int i = 0; i < DELTA_ROWS; ++i) {
+    const uint32_t wo[4] = {uo[i].x, uo[i].y, uo[i].z, uo[i].w}, wd[4] = {ud[i].x, ud[i].y, ud[i].z, ud[i].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc += __uint_as_float(wo[j] << 16) * __uint_as_float(wd[j] << 16);
+      acc += __uint_as_float(wo[j] & 0xffff0000u) * __uint_as_float(wd[j] & 0xffff0000u);
+    }
+#pragma unroll
+    for (int s = 8; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    const int q = q0 + i * 16;
+    if (lane16 == 0 && q < Sq) delta[((long)b * Hq + h) * Sq + q] = acc;
+  }
 }
 
-// dq (bf16, strided) = dq_acc (fp32, dense [B][Sq][Hq][D])
-__global__ void attn_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long n_rows,
-                                       int Sq, int HD, long dq_sb, long dq_ss) {
-  const int vec = HD / 4;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n_rows * vec; i += (long)gridDim.x * blockDim.x) {
-    const long row = i / vec;
-    const int c = (i % vec) * 4;
+// dq (bf16, strided) = dq_acc (fp32, dense [B][Sq][Hq][D]); a thread owns 8 columns (blockIdx.x) and walks the token rows.
+// VEC: rows of dq start on 16-byte boundaries (8-byte boundaries otherwise).
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+attn_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long n_rows, int Sq, int HD, long dq_sb, long dq_ss) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (c >= HD) return;
+#pragma unroll 2
+  for (long row = blockIdx.y; row < n_rows; row += gridDim.y) {
     const int q = row % Sq;
     const long b = row / Sq;
-    const float4 f = *reinterpret_cast<const float4*>(acc + row * HD + c);
-    uint2 u;
+    const float4 f = __ldcs(reinterpret_cast<const float4*>(acc + row * HD + c));
+    const float4 g = __ldcs(reinterpret_cast<const float4*>(acc + row * HD + c + 4));
+    uint4 u;
     u.x = pack_bf16x2(f.x, f.y);
     u.y = pack_bf16x2(f.z, f.w);
-    *reinterpret_cast<uint2*>(dq + b * dq_sb + (long)q * dq_ss + c) = u;
+    u.z = pack_bf16x2(g.x, g.y);
+    u.w = pack_bf16x2(g.z, g.w);
+    __nv_bfloat16* dst = dq + b * dq_sb + (long)q * dq_ss + c;
+    if constexpr (VEC) {
+      *reinterpret_cast<uint4*>(dst) = u;
+    } else {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(u.x, u.y);
+      *reinterpret_cast<uint2*>(dst + 4) = make_uint2(u.z, u.w);
+    }
   }
 }
 
@@ -195,7 +234,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int i = 0; i < QS; ++i) {
-      mbar_init(&q_full[i], 1);
+      mbar_init(&q_full[i], 1 + BW_BQ);  // the TMA thread and the 64 metadata threads
       mbar_init(&q_empty[i], 1);
     }
     mbar_init(sdp_full, 1);
@@ -368,6 +407,36 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
     }
     __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ query metadata (warps 2 and 3, one query row each)
+    // Statistics and mask rules of the stage's 64 query rows, one ring stage with its Q / dO tiles.  (When two of the compute
+    // warps loaded them on the side, every iteration waited for their global loads: 1400 of its 3700 cycles.)
+    const float LOG2E = 1.4426950408889634f;
+    const int r = (warp - 2) * 32 + lane;
+    for (int it = 0; it < n_iter; ++it) {
+      const int st = it % QS;
+      const int h = hk * group + it / n_valid;
+      const int q = tile_idx[it % n_valid] * BW_BQ + r;
+      const bool qv = q < p.Sq;
+      const long idx = ((long)b * p.Hq + h) * p.Sq + q;
+      const float lse = qv ? -(p.lse[idx] * LOG2E) : -INFINITY;  // both negated: their uses are one packed FMA each
+      const float delta = qv ? -(p.delta[idx] * p.scale) : 0.f;
+      const int qpos = qv ? (p.q_pos ? p.q_pos[(long)b * p.Sq + q] : q) : 0;
+      const int64_t qbits = (qv && p.q_bits) ? p.q_bits[(long)b * p.Sq + q] : 0;
+      const QueryRule rule = make_query_rule(p.mask_mode, qv && qpos >= 0, qbits, qpos);
+      if (!bw_wait(&q_empty[st], ((it / QS) & 1) ^ 1, abort_flag)) {
+        if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY);
+        *abort_flag = 1;
+        break;
+      }
+      float* m = reinterpret_cast<float*>(smem + L::META_OFF + st * L::META_STAGE);
+      m[r] = lse;
+      m[64 + r] = delta;
+      reinterpret_cast<int*>(m + 128)[r] = rule.lim;
+      reinterpret_cast<int64_t*>(m + 192)[r] = rule.am;
+      reinterpret_cast<int64_t*>(m + 320)[r] = rule.qe;
+      mbar_arrive(&q_full[st]);
+    }
   }
   } else if (warp >= 8) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CFG::COMPUTE_REGS));
@@ -383,53 +452,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const bool k_valid = krow < p.seg.rows[sg];
     const int64_t kb = mask_key_bits(p.mask_mode, k_valid, (k_valid && p.k_bits) ? p.k_bits[(long)b * p.Sk + kidx] : 0);
     const int kpos = k_valid ? (p.k_pos ? p.k_pos[(long)b * p.Sk + kidx] : kidx) : -1;
-    const float LOG2E = 1.4426950408889634f;
     const uint64_t scale_log2_2 = pack_f32x2(p.scale_log2, p.scale_log2), scale_2 = pack_f32x2(p.scale, p.scale);
     const bool by_index = p.mask_mode == MASK_FULL || (p.mask_mode == MASK_CAUSAL && p.q_pos == nullptr && p.k_pos == nullptr);
-    // the 64 threads with half == 0 and r < 64 stage the metadata of query row (tile * 64 + r)
-    const bool stager = (half == 0) && (r < 64);
-
-    float pf_lse = 0.f, pf_delta = 0.f;
-    int pf_qpos = 0;
-    bool pf_exists = false;
-    int64_t pf_qbits = 0;
-    auto prefetch_meta = [&](int it) {
-      if (!stager || it >= n_iter) return;
-      const int h = hk * group + it / n_valid;
-      const int q = tile_idx[it % n_valid] * BW_BQ + r;
-      const bool qv = q < p.Sq;
-      const long idx = ((long)b * p.Hq + h) * p.Sq + q;
-      pf_lse = qv ? -(p.lse[idx] * LOG2E) : -INFINITY;  // negated: the two uses below are one packed FMA each
-      pf_delta = qv ? -(p.delta[idx] * p.scale) : 0.f;
-      pf_qpos = qv ? (p.q_pos ? p.q_pos[(long)b * p.Sq + q] : q) : 0;
-      pf_exists = qv && pf_qpos >= 0;
-      pf_qbits = (qv && p.q_bits) ? p.q_bits[(long)b * p.Sq + q] : 0;
-    };
-
     bool ok = true;
-    // Query metadata of iteration it lives in buffer it % 3.  The stagers write the metadata of iteration it + 1 right
-    // after they hold S^T / dP^T of iteration it in registers and BEFORE they arrive on dp_read(it); the MMA warp issues
-    // dP^T(it + 1) only after dp_read(it) is complete, so sdp_full(it + 1) also tells every thread that the metadata is
-    // staged.  Three buffers: whoever stages it + 1 has seen sdp_full(it), i.e. every thread is past its loads of it - 1
-    // and therefore done with the metadata of it - 2, the previous tenant of that buffer.
-    auto stage_meta = [&](int it) {
-      if (!stager || it >= n_iter) return;
-      float* m = reinterpret_cast<float*>(smem + L::META_OFF + (it % 3) * L::META_STAGE);
-      m[r] = pf_lse;
-      m[64 + r] = pf_delta;
-      const QueryRule rule = make_query_rule(p.mask_mode, pf_exists, pf_qbits, pf_qpos);
-      reinterpret_cast<int*>(m + 128)[r] = rule.lim;
-      reinterpret_cast<int64_t*>(m + 192)[r] = rule.am;
-      reinterpret_cast<int64_t*>(m + 320)[r] = rule.qe;
-    };
-    prefetch_meta(0);
-    stage_meta(0);
-    prefetch_meta(1);
-    // the metadata of iteration 0 is ordered by a barrier of its own (named barrier 1 over the compute threads)
-    asm volatile("bar.sync 1, %0;" ::"n"(CFG::COMPUTE_THREADS) : "memory");
+    // The statistics and mask rules of iteration it (buffer it % QS) were staged before its Q / dO stage counted as full, so
+    // sdp_full(it) covers them too.
     for (int it = 0; it < n_iter && ok; ++it) {
       const int c = tile_cls[it % n_valid];
-      float* m_lse = reinterpret_cast<float*>(smem + L::META_OFF + (it % 3) * L::META_STAGE);
+      float* m_lse = reinterpret_cast<float*>(smem + L::META_OFF + (it % QS) * L::META_STAGE);
       float* m_delta = m_lse + 64;
       const int* m_lim = reinterpret_cast<const int*>(m_lse + 128);
       const int64_t* m_am = reinterpret_cast<const int64_t*>(m_lse + 192);
@@ -445,8 +475,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       tmem_ld_cols<COLS>(tmem_base + (it & 1) * 64 + col0 + lane_addr, sv);
       tmem_ld_cols<COLS>(tmem_dPT + col0 + lane_addr, dv);
       tmem_ld_wait();
-      stage_meta(it + 1);
-      prefetch_meta(it + 2);  // global loads for the tile after next fly while this one is processed
       tc_fence_before();
       mbar_arrive(dp_read);
       float pv[COLS], ds[COLS];
@@ -658,12 +686,13 @@ static int attn_bwd_seg_impl(const void* q, const CsbKvSegments* kv, const void*
   if ((q_ss % 8) || (do_ss % 8) || (dq_ss % 4)) return CSB_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   {
-    const long rows = (long)B * Sq * Hq;
-    const int threads = 256;
-    const long blocks = (rows * 32 + threads - 1) / threads;
-    attn_delta_kernel<<<(unsigned)blocks, threads, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(out),
-                                                           reinterpret_cast<const __nv_bfloat16*>(dout), delta, B, Sq, Hq,
-                                                           D, o_sb, o_ss, do_sb, do_ss);
+    const long grid = (long)((Sq + 16 * DELTA_ROWS - 1) / (16 * DELTA_ROWS)) * B * Hq;
+    if (grid > 0x7fffffffL) return CSB_ERR_TOO_LARGE;
+    const bool vec = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(dout)) & 15) == 0 && o_ss % 8 == 0 &&
+                     o_sb % 8 == 0 && do_ss % 8 == 0 && do_sb % 8 == 0;
+    auto kfn = vec ? attn_delta_kernel<true> : attn_delta_kernel<false>;
+    kfn<<<(unsigned)grid, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(dout), delta, Sq,
+                             Hq, D, o_sb, o_ss, do_sb, do_ss);
     if (int e = launch_result()) return e;
   }
   AttnBwdParams p;
@@ -736,9 +765,14 @@ static int attn_bwd_seg_impl(const void* q, const CsbKvSegments* kv, const void*
   if (e) return e;
   const long n_rows = (long)B * Sq;
   const int HD = Hq * D;
-  long work = n_rows * (HD / 4);
-  int blocks = (int)((work + 255) / 256 < (long)sm_count() * 16 ? (work + 255) / 256 : (long)sm_count() * 16);
-  attn_dq_convert_kernel<<<blocks, 256, 0, s>>>(dq_acc, reinterpret_cast<__nv_bfloat16*>(dq), n_rows, Sq, HD, dq_sb, dq_ss);
+  {
+    const int bx = (HD / 8 + 255) / 256;
+    long by = ((long)sm_count() * 8 + bx - 1) / bx;
+    if (by > n_rows) by = n_rows;
+    const bool vec = (reinterpret_cast<uintptr_t>(dq) & 15) == 0 && dq_ss % 8 == 0 && dq_sb % 8 == 0;
+    auto kfn = vec ? attn_dq_convert_kernel<true> : attn_dq_convert_kernel<false>;
+    kfn<<<dim3(bx, (unsigned)by), 256, 0, s>>>(dq_acc, reinterpret_cast<__nv_bfloat16*>(dq), n_rows, Sq, HD, dq_sb, dq_ss);
+  }
   return launch_result();
 }
 
