@@ -255,24 +255,31 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
   }
 }
 
-// out[c] (+)= sum_r partial[r][c]; out is fp32 (main-grad accumulation) or bf16.
-// One CTA = 32 columns x 8 row groups: every warp reads 128 contiguous bytes of a row, the 8 groups are summed in
-// shared memory (a column-per-thread loop over all rows left the partial buffer to 16 CTAs).
-__global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, void* __restrict__ out,
-                                                              int nparts, int H, int out_fp32, int accumulate) {
-  __shared__ float sh[8][33];
+// out[c] (+)= sum_r partial[r][c]; out is fp32 (main-grad accumulation) or bf16.  blockIdx.y = 1: the second pair of arrays.
+// One CTA = 32 columns x 32 row groups: every warp reads 128 contiguous bytes of a row, the groups are summed in shared
+// memory.  The loads of a thread are what takes the time (592 rows of partial sums: 74 in a row with 8 groups, 5.9 us).
+struct PartialSums {
+  const float* partial[2];
+  void* out[2];
+};
+constexpr int REDUCE_GROUPS = 32;
+__global__ void __launch_bounds__(32 * REDUCE_GROUPS) reduce_partials_kernel(const PartialSums p, int nparts, int H, int out_fp32,
+                                                                             int accumulate) {
+  __shared__ float sh[REDUCE_GROUPS][33];
+  const float* __restrict__ partial = p.partial[blockIdx.y];
+  void* __restrict__ out = p.out[blockIdx.y];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
   float s = 0.f;
   if (c < H) {
-#pragma unroll 4
-    for (int r = ty; r < nparts; r += 8) s += partial[static_cast<size_t>(r) * H + c];
+#pragma unroll 8
+    for (int r = ty; r < nparts; r += REDUCE_GROUPS) s += partial[static_cast<size_t>(r) * H + c];
   }
   sh[ty][tx] = s;
   __syncthreads();
   if (ty == 0 && c < H) {
 #pragma unroll
-    for (int k = 1; k < 8; ++k) s += sh[k][tx];
+    for (int k = 1; k < REDUCE_GROUPS; ++k) s += sh[k][tx];
     if (out_fp32) {
       float* o = reinterpret_cast<float*>(out);
       o[c] = accumulate ? o[c] + s : s;
@@ -385,9 +392,17 @@ CSB_API int csb_norm_bwd(int is_layernorm, const void* dy, const void* h, const 
 #undef CSB_NORM_BWD
   int r = launch_result();
   if (r) return r;
-  if (dw_out) reduce_partials_kernel<<<(H + 31) / 32, 256, 0, s>>>(dw_partial, dw_out, grid, H, grads_fp32, accumulate);
-  if (is_layernorm && db_out && db_partial)
-    reduce_partials_kernel<<<(H + 31) / 32, 256, 0, s>>>(db_partial, db_out, grid, H, grads_fp32, accumulate);
+  PartialSums ps = {};
+  int n = 0;
+  if (dw_out) {
+    ps.partial[n] = dw_partial;
+    ps.out[n++] = dw_out;
+  }
+  if (is_layernorm && db_out && db_partial) {
+    ps.partial[n] = db_partial;
+    ps.out[n++] = db_out;
+  }
+  if (n > 0) reduce_partials_kernel<<<dim3((H + 31) / 32, n), 32 * REDUCE_GROUPS, 0, s>>>(ps, grid, H, grads_fp32, accumulate);
   return launch_result();
 }
 
@@ -408,6 +423,7 @@ CSB_API int csb_colsum(const void* x, float* partial, void* out, int out_fp32, i
   if (slices > csb_colsum_parts(rows)) slices = csb_colsum_parts(rows);
   colsum_partial_kernel<<<dim3(col_blocks, slices), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), partial, rows, H);
   if (int e = launch_result()) return e;
-  reduce_partials_kernel<<<(H + 31) / 32, 256, 0, s>>>(partial, out, slices, H, out_fp32, accumulate);
+  PartialSums ps = {{partial, nullptr}, {out, nullptr}};
+  reduce_partials_kernel<<<(H + 31) / 32, 32 * REDUCE_GROUPS, 0, s>>>(ps, slices, H, out_fp32, accumulate);
   return launch_result();
 }
