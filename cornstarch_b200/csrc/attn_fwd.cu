@@ -314,9 +314,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tc_fence_after();
         // descriptors of the k-th 16-wide slice: the tile's descriptor plus the slice's byte offset / 16
         const uint64_t k_desc = make_desc_kmajor_sw128(smem_u32(smem + L::K_OFF + st * L::KV_BYTES));
-        for (int kk = 0; kk < ksteps_s; ++kk) {
+#pragma unroll
+        for (int kk = 0; kk < 4 * NCH; ++kk) {  // unrolled to the maximum, cut by a uniform test
           const uint64_t off = static_cast<uint64_t>(((kk >> 2) * CHUNK_BYTES + (kk & 3) * 32) >> 4);
-          umma_f16_w(tmem_S + st * 128, q_desc + off, k_desc + off, idesc_s, kk > 0 ? 1u : 0u);
+          if (kk < ksteps_s) umma_f16_w(tmem_S + st * 128, q_desc + off, k_desc + off, idesc_s, kk > 0 ? 1u : 0u);
         }
         umma_commit_w(&k_empty[st]);
         umma_commit_w(&s_full[st]);
@@ -676,7 +677,12 @@ static int attn_fwd_seg_impl(const void* q, const CsbKvSegments* kv, void* out, 
   int r;
   if ((r = make_qkv_tmap(&tq, q, D, Hq, Sq, B, q_stride_s, q_stride_b))) return r;
   for (int i = 0; i < CSB_MAX_SEG; ++i) {
-    const int g = i < kv->n_seg ? i : 0;  // unused slots repeat segment 0 (never dereferenced)
+    if (i >= kv->n_seg) {  // unused slots repeat segment 0 (never dereferenced)
+      kvm.k[i] = kvm.k[0];
+      kvm.v[i] = kvm.v[0];
+      continue;
+    }
+    const int g = i;
     if ((kv->k_stride_s[g] % 8) || (kv->v_stride_s[g] % 8)) return CSB_ERR_BAD_ARG;
     // with pulling blocks the tiles of a remote segment are read from its local copy
     const bool local_copy = p.seg.pull_ctas > 0 && g != kv->my_seg;

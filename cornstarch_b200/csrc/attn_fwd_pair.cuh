@@ -188,9 +188,10 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     auto issue_s = [&](int s, uint32_t it) {
       const uint64_t q_desc = make_desc_kmajor_sw128(smem_u32(smem + L::Q_OFF + s * L::TILE_BYTES));
       const uint64_t k_desc = make_desc_kmajor_sw128(smem_u32(smem + L::K_OFF + (it & 1) * L::TILE_BYTES));
-      for (int kk = 0; kk < ksteps_s; ++kk) {
+#pragma unroll
+      for (int kk = 0; kk < 4 * NCH; ++kk) {  // unrolled to the maximum, cut by a uniform test
         const uint64_t off = static_cast<uint64_t>(((kk >> 2) * CHUNK_BYTES + (kk & 3) * 32) >> 4);
-        umma_f16_w(tmem_S + s * 128, q_desc + off, k_desc + off, idesc_s, kk > 0 ? 1u : 0u);
+        if (kk < ksteps_s) umma_f16_w(tmem_S + s * 128, q_desc + off, k_desc + off, idesc_s, kk > 0 ? 1u : 0u);
       }
       umma_commit_w(&s_full[s]);
     };
