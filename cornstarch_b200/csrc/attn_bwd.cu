@@ -13,11 +13,11 @@
 //
 // dK/dV need no atomics and are bit-reproducible: every query head that shares the KV head is
 // handled by the same CTA.  dQ^T tiles are staged in shared memory as [q][d] rows and added into an fp32
-// accumulator by TMA reduce-add (one 32x32 block per warp), then converted to bf16 by a final pass.
+// accumulator by TMA reduce-add (one 32 x 64 block per warp), then converted to bf16 by a final pass.
 //
-// Warp roles (768 threads by default): warp 0 = TMA producer (K/V once, Q/dO ring of 3 stages), warp 1 = MMA
-// issuer, warps 2 and 3 = query metadata, warps 4..7 = dQ^T drain, warps 8..23 = 512 compute threads (or 8..15 = 256).  Thread (r, group) owns KV row r (TMEM lane r) and 16
-// (32) of the 64 query columns of S^T / dP^T; a drain thread moves head-dim row r of dQ^T.  The pipeline keeps S^T one
+// Warp roles (512 threads): warp 0 = TMA producer (K/V once, Q/dO ring of 3 stages), warp 1 = MMA issuer, warps 2 and 3 =
+// query metadata, warps 4..7 = dQ^T drain, warps 8..15 = 256 compute threads.  Thread (r, group) owns KV row r (TMEM lane r)
+// and 32 of the 64 query columns of S^T / dP^T; a drain thread moves head-dim row r of dQ^T.  The pipeline keeps S^T one
 // iteration ahead: while the compute warps turn S^T(i), dP^T(i) into P^T, dS^T, the tensor core
 // already holds S^T(i+1); dP^T(i+1) is issued as soon as dP^T(i) has been read, before the
 // dV/dK/dQ^T MMAs of iteration i, so the next exponentials overlap those MMAs.  Per-tile query
@@ -54,6 +54,10 @@ struct AttnBwdParams {
   __nv_bfloat16* dV[CSB_MAX_SEG];
   long dk_stride_b[CSB_MAX_SEG], dk_stride_s[CSB_MAX_SEG], dv_stride_b[CSB_MAX_SEG], dv_stride_s[CSB_MAX_SEG];
   int* status;
+  // Several blocks per key block (nsplit > 1, one local segment): block `split` takes an equal share of the iterations and
+  // writes its fp32 part of dK and dV to part[0 / 1][split][B][Sk][Hk][D]; attn_dkv_reduce_kernel adds the parts in order.
+  int nsplit;
+  float* part;
   int kj_slowest;  // block order: 1 = key block slowest (masks that leave key blocks unequal work), 0 = key block fastest
   // dense boolean mask (MASK_DENSE) and additive bias, as in the forward kernel
   const uint8_t* dmask;
@@ -64,6 +68,19 @@ struct AttnBwdParams {
   SegInfo seg;
 };
 
+// Position in a block's list of (query head, query tile) iterations, advanced without divisions (a division and a
+// remainder per iteration in every compute warp: 8192 tokens causal 1976 us with, 1903 us without).
+struct BwdCursor {
+  int h, t, n_valid;
+  __device__ __forceinline__ BwdCursor(int it, int n) : h(n > 0 ? it / n : 0), t(n > 0 ? it % n : 0), n_valid(n) {}
+  __device__ __forceinline__ void next() {
+    if (++t == n_valid) {
+      t = 0;
+      ++h;
+    }
+  }
+};
+
 struct BwdSmem {
   static constexpr int QSTAGES = 3;
   static constexpr int K_OFF = 0;
@@ -71,7 +88,7 @@ struct BwdSmem {
   static constexpr int Q_OFF = V_OFF + 2 * KV_CHUNK;          // QSTAGES x (2 chunks x 8 KB)
   static constexpr int DO_OFF = Q_OFF + QSTAGES * 2 * Q_CHUNK;
   static constexpr int DST_OFF = DO_OFF + QSTAGES * 2 * Q_CHUNK;  // dS^T [128 kv][64 q] bf16
-  static constexpr int DQ_OFF = DST_OFF + KV_CHUNK;           // dQ staging: 8 warps x [32 q][32 d] fp32 (row-major, 4 KB each)
+  static constexpr int DQ_OFF = DST_OFF + KV_CHUNK;           // dQ staging: 4 warps x [64 q][32 d] fp32 (row-major, 8 KB each)
   static constexpr int META_OFF = DQ_OFF + 8 * 4096;          // one buffer per Q stage of: -lse2[64] f32, -delta*scale[64] f32, and the mask rules lim[64] i32, am[64] i64, qe[64] i64
   static constexpr int META_STAGE = 64 * 4 * 3 + 2 * 64 * 8;
   static constexpr int LIST_OFF = META_OFF + QSTAGES * META_STAGE;  // valid 64-row query tiles of this key block: int16 index, int8 class
@@ -82,17 +99,15 @@ struct BwdSmem {
   static constexpr int DYN_BYTES = TOTAL + 1024;
 };
 
-// NCW compute warps (8 or 16): NCW / 4 warps share a TMEM lane quarter and split the 64 query columns between them.
-template <int NCW>
+// Eight compute warps: two share a TMEM lane quarter and split the 64 query columns between them.  Their loop is bound by
+// instruction issue, and what does not depend on the number of columns (waits, addresses, hand-overs) is paid per warp: sixteen
+// warps of 16 columns took 1903 us where eight of 32 take 1816 (8192 tokens causal, 32 / 8 heads of 128; full mask 3769 / 3510).
 struct BwdCfg {
-  static constexpr int COMPUTE_THREADS = NCW * 32;
+  static constexpr int COMPUTE_THREADS = 8 * 32;
   static constexpr int DRAIN_THREADS = 128;  // four warps that only move dQ^T out (one per TMEM lane quarter)
   static constexpr int THREADS = 128 + DRAIN_THREADS + COMPUTE_THREADS;
-  // Registers a thread after the split (warpgroups of 128 threads: TMA + MMA + two spare warps, drain, compute): with 16
-  // compute warps 80 + 48 + 4 x 88 = 6 x 80, with 8 compute warps 80 + 48 + 2 x 192 = 4 x 128 (what the launch allocates).
-  static constexpr int COMPUTE_REGS = NCW == 16 ? 88 : 192;
-  static constexpr int GROUPS = NCW / 4;       // column groups
-  static constexpr int COLS = BW_BQ / GROUPS;  // query columns of S^T / dP^T per thread: 32 or 16
+  static constexpr int GROUPS = 2;             // column groups
+  static constexpr int COLS = BW_BQ / GROUPS;  // query columns of S^T / dP^T per thread
 };
 
 __device__ __forceinline__ bool bw_wait(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
@@ -112,6 +127,8 @@ __device__ __forceinline__ bool bw_wait(uint64_t* bar, uint32_t phase, volatile 
 // delta[b][h][q] = sum_d O[b][q][h][d] * dO[b][q][h][d].  Sixteen lanes share a row (8 elements each, D <= 128) and take
 // DELTA_ROWS queries of one head, so that every thread has 2 x DELTA_ROWS 16-byte loads in flight and the results of a block
 // are consecutive.  VEC: rows of both tensors start on 16-byte boundaries.
+// (A warp per row with 4-byte loads took 13.7 us for the 13 MB of 4 x 729 tokens, 16 heads of 72; the whole backward call went
+// from 124 to 112 us with this pass, the conversion below and the statistics warps.)
 constexpr int DELTA_ROWS = 4;
 template <bool VEC>
 __global__ void __launch_bounds__(256)
@@ -190,13 +207,12 @@ attn_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict_
   }
 }
 
-template <int NCW>
-__global__ void __launch_bounds__(BwdCfg<NCW>::THREADS, 1)
+__global__ void __launch_bounds__(BwdCfg::THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ KvMaps kvm,
                 const __grid_constant__ CUtensorMap tm_do, const __grid_constant__ CUtensorMap tm_dq,
                 const AttnBwdParams p) {
   using L = BwdSmem;
-  using CFG = BwdCfg<NCW>;
+  using CFG = BwdCfg;
   constexpr int QS = L::QSTAGES;
   constexpr int COLS = CFG::COLS;
   extern __shared__ uint8_t smem_raw[];
@@ -209,7 +225,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint64_t* pds_full = sdp_full + 1;      //       P^T and dS^T tiles written to smem (256 arrivals)
   uint64_t* pds_empty = pds_full + 1;     //       ... and consumed by the MMAs
   uint64_t* dq_full = pds_empty + 1;      //       dQ^T ready in TMEM
-  uint64_t* dq_free = dq_full + 1;        //       dQ^T drained (256 arrivals)
+  uint64_t* dq_free = dq_full + 1;        //       dQ^T drained (128 arrivals)
   uint64_t* dp_read = dq_free + 1;      //       S^T and dP^T of an iteration are in registers (256 arrivals): dP^T may be overwritten
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -223,8 +239,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // the heavy blocks of every head start first and the light ones fill the tail.
   // (With a full mask every block is equally heavy; key block fastest then keeps the Q / dO tiles of few heads in L2.)
   const int n_hb = p.Hk * p.B;
-  const int hb = p.kj_slowest ? blockIdx.x % n_hb : blockIdx.x / p.nK;
-  const int kj = p.kj_slowest ? blockIdx.x / n_hb : blockIdx.x % p.nK;
+  const int split = blockIdx.x % p.nsplit;
+  const int blk = blockIdx.x / p.nsplit;
+  const int hb = p.kj_slowest ? blk % n_hb : blk / p.nK;
+  const int kj = p.kj_slowest ? blk / n_hb : blk % p.nK;
   const int hk = hb % p.Hk, b = hb / p.Hk;
   const int group = p.Hq / p.Hk;
   const int k0 = kj * BW_BKV;                              // index into k_bits / k_pos (padded gathered space)
@@ -285,15 +303,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
   const int n_valid = *n_valid_slot;
   const bool peer_ready = *peer_ok_slot != 0;
-  const int n_iter = peer_ready ? n_valid * group : 0;
+  // this block's share [it0, it0 + n_iter) of the (query head, query tile) list
+  const int n_all = peer_ready ? n_valid * group : 0;
+  const int it0 = (int)((long)n_all * split / p.nsplit);
+  const int n_iter = (int)((long)n_all * (split + 1) / p.nsplit) - it0;
   // TMEM columns: S^T[0] 0..63, S^T[1] 64..127, dP^T 128..191, dQ^T 192..255, dV 256..383, dK 384..511
   const uint32_t tmem_dPT = tmem_base + 128;
   const uint32_t tmem_dQT = tmem_base + 192;
   const uint32_t tmem_dV = tmem_base + 256;
   const uint32_t tmem_dK = tmem_base + 384;
 
-  if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -307,9 +326,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           tma_load_4d(smem + L::V_OFF + c * KV_CHUNK, &kvm.v[sg], kv_full, c * 64, hk, row0, b);
         }
       }
-      for (int it = 0; peer_ok && it < n_iter; ++it) {
-        const int h = hk * group + it / n_valid;
-        const int i = tile_idx[it % n_valid];
+      BwdCursor cur(it0, n_valid);
+      for (int it = 0; peer_ok && it < n_iter; ++it, cur.next()) {
+        const int h = hk * group + cur.h;
+        const int i = tile_idx[cur.t];
         const int st = it % QS;
         if (!bw_wait(&q_empty[st], ((it / QS) & 1) ^ 1, abort_flag)) {
           atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY);
@@ -337,6 +357,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const uint64_t k_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::K_OFF), KV_CHUNK);
       const uint64_t dst_km = make_desc_kmajor_sw128(smem_u32(smem + L::DST_OFF));
       const uint64_t dst_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::DST_OFF), KV_CHUNK);
+      // steps of the contractions over D: their loops are unrolled to the maximum and cut by a uniform test
       const int ksteps_d = p.dk16 / 16;
       bool ok = bw_wait(kv_full, 0, abort_flag);
       if (!ok) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; }
@@ -351,16 +372,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tc_fence_after();
         const uint64_t q_km = make_desc_kmajor_sw128(smem_u32(smem + L::Q_OFF + st * 2 * Q_CHUNK));
         const uint32_t t_st = tmem_base + (it & 1) * 64;
-        for (int kk = 0; kk < ksteps_d; ++kk)
-          umma_f16_w(t_st, k_km + kslice(kk, KV_CHUNK), q_km + kslice(kk, Q_CHUNK), idesc_s, kk > 0);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          if (kk < ksteps_d) umma_f16_w(t_st, k_km + kslice(kk, KV_CHUNK), q_km + kslice(kk, Q_CHUNK), idesc_s, kk > 0);
         return true;
       };
       // dP^T(it) = V dO^T; its commit also covers S^T(it), issued earlier
       auto issue_dpt = [&](int it) {
         const int st = it % QS;
         const uint64_t do_km = make_desc_kmajor_sw128(smem_u32(smem + L::DO_OFF + st * 2 * Q_CHUNK));
-        for (int kk = 0; kk < ksteps_d; ++kk)
-          umma_f16_w(tmem_dPT, v_km + kslice(kk, KV_CHUNK), do_km + kslice(kk, Q_CHUNK), idesc_s, kk > 0);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          if (kk < ksteps_d) umma_f16_w(tmem_dPT, v_km + kslice(kk, KV_CHUNK), do_km + kslice(kk, Q_CHUNK), idesc_s, kk > 0);
         umma_commit_w(sdp_full);
       };
 
@@ -407,16 +430,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
     }
     __syncwarp();
-  } else {
+  } else if (warp < 4) {
     // ------------------------------------------------------------------ query metadata (warps 2 and 3, one query row each)
     // Statistics and mask rules of the stage's 64 query rows, one ring stage with its Q / dO tiles.  (When two of the compute
     // warps loaded them on the side, every iteration waited for their global loads: 1400 of its 3700 cycles.)
     const float LOG2E = 1.4426950408889634f;
     const int r = (warp - 2) * 32 + lane;
-    for (int it = 0; it < n_iter; ++it) {
+    BwdCursor cur(it0, n_valid);
+    for (int it = 0; it < n_iter; ++it, cur.next()) {
       const int st = it % QS;
-      const int h = hk * group + it / n_valid;
-      const int q = tile_idx[it % n_valid] * BW_BQ + r;
+      const int h = hk * group + cur.h;
+      const int q = tile_idx[cur.t] * BW_BQ + r;
       const bool qv = q < p.Sq;
       const long idx = ((long)b * p.Hq + h) * p.Sq + q;
       const float lse = qv ? -(p.lse[idx] * LOG2E) : -INFINITY;  // both negated: their uses are one packed FMA each
@@ -437,10 +461,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       reinterpret_cast<int64_t*>(m + 320)[r] = rule.qe;
       mbar_arrive(&q_full[st]);
     }
-  }
   } else if (warp >= 8) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(CFG::COMPUTE_REGS));
-    // ------------------------------------------------------------------ compute threads (NCW warps)
+    // ------------------------------------------------------------------ compute threads (8 warps)
     const int cw = warp - 8;
     const int quarter = warp & 3;       // TMEM lane quarter this warp may touch
     const int half = cw >> 2;           // which group of COLS query columns (of 64) this warp handles
@@ -457,9 +479,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     bool ok = true;
     // The statistics and mask rules of iteration it (buffer it % QS) were staged before its Q / dO stage counted as full, so
     // sdp_full(it) covers them too.
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const int c = tile_cls[it % n_valid];
-      float* m_lse = reinterpret_cast<float*>(smem + L::META_OFF + (it % QS) * L::META_STAGE);
+    BwdCursor cur(it0, n_valid);
+    int stage = 0;  // it % QS
+    for (int it = 0; it < n_iter && ok; ++it, cur.next(), stage = stage + 1 == QS ? 0 : stage + 1) {
+      const int c = tile_cls[cur.t];
+      float* m_lse = reinterpret_cast<float*>(smem + L::META_OFF + stage * L::META_STAGE);
       float* m_delta = m_lse + 64;
       const int* m_lim = reinterpret_cast<const int*>(m_lse + 128);
       const int64_t* m_am = reinterpret_cast<const int64_t*>(m_lse + 192);
@@ -478,9 +502,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       tc_fence_before();
       mbar_arrive(dp_read);
       float pv[COLS], ds[COLS];
-      const int q_base = tile_idx[it % n_valid] * BW_BQ + col0;  // first query row of this thread's columns
+      const int q_base = tile_idx[cur.t] * BW_BQ + col0;  // first query row of this thread's columns
       if (p.bias != nullptr && k_valid) {
-        const int hh = hk * group + it / n_valid;
+        const int hh = hk * group + cur.h;
         const float* bcol = p.bias + (long)b * p.bias_sb + (long)hh * p.bias_sh + kidx;
 #pragma unroll
         for (int x = 0; x < COLS; ++x)
@@ -557,13 +581,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       tc_fence_before();
       mbar_arrive(pds_full);
     }
-    // ---- epilogue: dV and dK tiles (every MMA has retired once the last dS^T was consumed);
+    // ---- epilogue: dV and dK tiles (every MMA has retired once the last dS^T was consumed); the warps of a lane quarter split
+    //      the head-dim columns
     if (ok && n_iter > 0 && !bw_wait(pds_empty, (n_iter - 1) & 1, abort_flag)) {
       if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_MISC);
       *abort_flag = 1;
       ok = false;
     }
-    //      the warps of a lane quarter split the head-dim columns
     if (ok && peer_ready) {
       tc_fence_after();
 #pragma unroll
@@ -583,7 +607,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
             for (int x = 0; x < 32; ++x) v[x] = 0u;
           }
-          if (k_valid) {
+          if (k_valid && p.nsplit > 1) {
+            float* dst = p.part + ((((long)(which == 0 ? 1 : 0) * p.nsplit + split) * p.B + b) * p.Sk + kidx) * p.Hk * p.D + (long)hk * p.D;
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+              const int col = cc * 32 + g * 4;
+              if (col + 4 <= p.D)
+                *reinterpret_cast<float4*>(dst + col) = make_float4(__uint_as_float(v[g * 4]), __uint_as_float(v[g * 4 + 1]),
+                                                                    __uint_as_float(v[g * 4 + 2]), __uint_as_float(v[g * 4 + 3]));
+            }
+          } else if (k_valid) {
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
               const int col = cc * 32 + g * 8;
@@ -601,14 +634,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
     }
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
     // ------------------------------------------------------------------ dQ^T drain: TMEM -> smem [q][d] rows -> reduce-add
     // Warps of their own, so that the compute warps go straight from dS^T(it) to S^T(it + 1): with the drain in their loop
     // the next exponentials waited for the tensor-memory loads and staging stores of an iteration that was long over.
     const int quarter = warp & 3;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     float* stage = reinterpret_cast<float*>(smem + L::DQ_OFF + quarter * (BW_BQ * 128));
-    for (int it = 0; it < n_iter; ++it) {
+    BwdCursor cur(it0, n_valid);
+    for (int it = 0; it < n_iter; ++it, cur.next()) {
       if (!bw_wait(dq_full, it & 1, abort_flag)) {
         if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
@@ -633,7 +666,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0 && quarter * 32 < p.D) {
-        tma_reduce_add_4d(&tm_dq, stage, quarter * 32, hk * group + it / n_valid, tile_idx[it % n_valid] * BW_BQ, b);  // box: 32 d x 64 q
+        tma_reduce_add_4d(&tm_dq, stage, quarter * 32, hk * group + cur.h, tile_idx[cur.t] * BW_BQ, b);  // box: 32 d x 64 q
         tma_store_commit();
       }
     }
@@ -646,6 +679,30 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// dK (blockIdx.z = 0) / dV (1) = sum over the splits, in order, of their fp32 parts [split][rows][HD], rounded to bf16 once.
+// A thread owns 8 columns; the parts are dense, the results strided.
+__global__ void __launch_bounds__(128)
+attn_dkv_reduce_kernel(const float* __restrict__ part, int nsplit, long n_rows, int Sk, int HD, __nv_bfloat16* __restrict__ dk,
+                       __nv_bfloat16* __restrict__ dv, long dk_sb, long dk_ss, long dv_sb, long dv_ss) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (c >= HD) return;
+  const float* src = part + (long)blockIdx.z * nsplit * n_rows * HD;
+  for (long row = blockIdx.y; row < n_rows; row += gridDim.y) {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int sp = 0; sp < nsplit; ++sp) {
+      const float* q = src + ((long)sp * n_rows + row) * HD + c;
+      const float4 f = *reinterpret_cast<const float4*>(q), g = *reinterpret_cast<const float4*>(q + 4);
+      acc[0] += f.x; acc[1] += f.y; acc[2] += f.z; acc[3] += f.w;
+      acc[4] += g.x; acc[5] += g.y; acc[6] += g.z; acc[7] += g.w;
+    }
+    const long b = row / Sk, k = row - b * Sk;
+    __nv_bfloat16* dst = (blockIdx.z == 0 ? dk + b * dk_sb + k * dk_ss : dv + b * dv_sb + k * dv_ss) + c;
+    *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
+                                                pack_bf16x2(acc[6], acc[7]));
   }
 }
 
@@ -677,7 +734,9 @@ static int attn_bwd_seg_impl(const void* q, const CsbKvSegments* kv, const void*
                              float* delta, float* dq_acc, void* dq, int B, int Sq, int Sk, int Hq, int Hk, int D, long q_ss,
                              long q_sb, long o_ss, long o_sb, long do_ss, long do_sb, long dq_ss, long dq_sb, float scale,
                              int mask_mode, const long* q_bits, const long* k_bits, const int* q_pos, const int* k_pos,
-                             const signed char* cls, int* status, void* stream, const CsbAttnExtras* ex) {
+                             const signed char* cls, int* status, void* stream, const CsbAttnExtras* ex, float* part = nullptr,
+                             int nsplit = 1) {
+  if (nsplit < 1 || (nsplit > 1 && (part == nullptr || kv == nullptr || kv->n_seg != 1 || kv->ready_flags != nullptr))) return CSB_ERR_BAD_ARG;
   if (D % 8 || D > 128 || D < 16 || Hq % Hk) return CSB_ERR_BAD_ARG;
   if (cls == nullptr && !(mask_mode == MASK_FULL || (mask_mode == MASK_CAUSAL && q_pos == nullptr && k_pos == nullptr))) return CSB_ERR_BAD_ARG;
   if (mask_mode == MASK_DENSE && (ex == nullptr || ex->dmask == nullptr)) return CSB_ERR_BAD_ARG;
@@ -716,6 +775,8 @@ static int attn_bwd_seg_impl(const void* q, const CsbKvSegments* kv, const void*
   p.bias_sb = ex ? ex->bias_sb : 0; p.bias_sh = ex ? ex->bias_sh : 0; p.bias_sq = ex ? ex->bias_sq : 0;
   p.inv_scale = scale != 0.f ? 1.f / scale : 0.f;
   p.kj_slowest = mask_mode != MASK_FULL;
+  p.nsplit = nsplit;
+  p.part = part;
   fill_seg_info(&p.seg, kv, BW_BKV);
   if (p.seg.tile_start[kv->n_seg] != p.nK) return CSB_ERR_BAD_ARG;
   CUtensorMap tq, tdo;
@@ -724,21 +785,20 @@ static int attn_bwd_seg_impl(const void* q, const CsbKvSegments* kv, const void*
   if ((r = make_tmap_4d(&tq, q, D, Hq, Sq, B, q_ss, q_sb, BW_BQ))) return r;
   if ((r = make_tmap_4d(&tdo, dout, D, Hq, Sq, B, do_ss, do_sb, BW_BQ))) return r;
   for (int i = 0; i < CSB_MAX_SEG; ++i) {
-    const int g = i < kv->n_seg ? i : 0;
+    const int g = i < kv->n_seg ? i : 0;  // unused slots repeat segment 0 (never dereferenced)
     if ((kv->k_stride_s[g] % 8) || (kv->v_stride_s[g] % 8) || (kv->dk_stride_s[g] % 8) || (kv->dv_stride_s[g] % 8)) return CSB_ERR_BAD_ARG;
-    if ((r = make_tmap_4d(&kvm.k[i], kv->k[g], D, Hk, kv->rows[g], B, kv->k_stride_s[g], kv->k_stride_b[g], BW_BKV))) return r;
-    if ((r = make_tmap_4d(&kvm.v[i], kv->v[g], D, Hk, kv->rows[g], B, kv->v_stride_s[g], kv->v_stride_b[g], BW_BKV))) return r;
+    if (i < kv->n_seg) {
+      if ((r = make_tmap_4d(&kvm.k[i], kv->k[g], D, Hk, kv->rows[g], B, kv->k_stride_s[g], kv->k_stride_b[g], BW_BKV))) return r;
+      if ((r = make_tmap_4d(&kvm.v[i], kv->v[g], D, Hk, kv->rows[g], B, kv->v_stride_s[g], kv->v_stride_b[g], BW_BKV))) return r;
+    } else {
+      kvm.k[i] = kvm.k[0];
+      kvm.v[i] = kvm.v[0];
+    }
     p.dK[i] = reinterpret_cast<__nv_bfloat16*>(kv->dk[g]);
     p.dV[i] = reinterpret_cast<__nv_bfloat16*>(kv->dv[g]);
     p.dk_stride_s[i] = kv->dk_stride_s[g]; p.dk_stride_b[i] = kv->dk_stride_b[g];
     p.dv_stride_s[i] = kv->dv_stride_s[g]; p.dv_stride_b[i] = kv->dv_stride_b[g];
   }
-  // 16 compute warps (four per scheduler: they hide the tensor-memory load and dependency latencies of each other;
-  // measured 3 % faster than 8 at S = 8192 once the MMA warp issued as a converged warp), or 8 when the environment asks
-  static const bool wide = []() {
-    const char* e = getenv("CORNSTARCH_B200_ATTN_BWD_WARPS");
-    return !(e && atoi(e) == 8);
-  }();
   CUtensorMap tdq;
   {
     // dq_acc is dense fp32 [B][Sq][Hq][D]; a block is 32 head-dim elements (128 B) x 64 query rows
@@ -749,20 +809,24 @@ static int attn_bwd_seg_impl(const void* q, const CsbKvSegments* kv, const void*
   }
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(attn_bwd_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::DYN_BYTES) != cudaSuccess ||
-        cudaFuncSetAttribute(attn_bwd_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::DYN_BYTES) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::DYN_BYTES) != cudaSuccess)
       return launch_result();
     attr = true;
   }
-  const long n_blocks = (long)p.nK * Hk * B;
+  const long n_blocks = (long)p.nK * Hk * B * nsplit;
   if (n_blocks > 0x7fffffffL) return CSB_ERR_TOO_LARGE;
   dim3 grid((unsigned)n_blocks);
-  if (wide)
-    attn_bwd_kernel<16><<<grid, BwdCfg<16>::THREADS, BwdSmem::DYN_BYTES, s>>>(tq, kvm, tdo, tdq, p);
-  else
-    attn_bwd_kernel<8><<<grid, BwdCfg<8>::THREADS, BwdSmem::DYN_BYTES, s>>>(tq, kvm, tdo, tdq, p);
+  attn_bwd_kernel<<<grid, BwdCfg::THREADS, BwdSmem::DYN_BYTES, s>>>(tq, kvm, tdo, tdq, p);
   int e = launch_result();
   if (e) return e;
+  if (nsplit > 1) {
+    const long k_rows = (long)B * Sk;
+    const int hd = Hk * D, bx = (hd / 8 + 127) / 128;
+    const dim3 rgrid(bx, (unsigned)(k_rows < 2048 ? k_rows : 2048), 2);
+    attn_dkv_reduce_kernel<<<rgrid, 128, 0, s>>>(part, nsplit, k_rows, Sk, hd, p.dK[0], p.dV[0], p.dk_stride_b[0], p.dk_stride_s[0],
+                                                 p.dv_stride_b[0], p.dv_stride_s[0]);
+    if ((e = launch_result())) return e;
+  }
   const long n_rows = (long)B * Sq;
   const int HD = Hq * D;
   {
@@ -805,13 +869,49 @@ CSB_API int csb_attn_bwd_dense(const void* q, const void* k, const void* v, cons
                            dq_ss, dq_sb, scale, mask_mode, nullptr, nullptr, nullptr, nullptr, cls, status, stream, ex);
 }
 
-// One local K/V tensor ([B][Sk][Hk][D] views) with dK / dV of the same shape.
+// Blocks per 128-row key block that csb_attn_bwd should be given for these sizes.  Without a split a key block of one KV head is
+// one thread block that walks all query heads of its group: 64 blocks for 1024 tokens and 8 KV heads on 148 SMs, and under a
+// causal mask the longest block alone decides.  Each further block costs its set-up and epilogue again (about 8 us) and the
+// parts are written and read once more.  The count with the smallest predicted time is taken: about 1.9 us per 128 x 64 tile,
+// whole rounds of equal blocks under a full mask, the longest block or the average load of the SMs otherwise.
+// Measured, one against several blocks (split by "two blocks per SM", which this rule replaces where it lost): 1024 tokens
+// causal, 32 / 8 heads: 146 against 87 us; 2048: 296 / 203; 1500 tokens, 8 / 1 heads: 406 / 53; but 729 tokens, 16 / 16
+// heads, full: 37 / 47, 2 x 900 tokens, 8 / 8 heads: 44 / 60.
+CSB_API int csb_attn_bwd_splits(int mask_mode, int B, int Sq, int Sk, int Hq, int Hk) {
+  if (B < 1 || Sq < 1 || Sk < 1 || Hk < 1 || Hq < Hk) return 1;
+  const float setup_us = 8.f, tile_us = 1.9f;
+  const int sms = sm_count();
+  const long blocks = (long)((Sk + BW_BKV - 1) / BW_BKV) * Hk * B;
+  const long iters = (long)((Sq + BW_BQ - 1) / BW_BQ) * (Hq / Hk);  // of the longest block
+  int best = 1;
+  float best_us = 0.f;
+  for (int n = 1; n <= 16 && (n == 1 || n <= iters / 2); ++n) {
+    const float longest = setup_us + tile_us * iters / n;
+    float us;
+    if (mask_mode == MASK_FULL) {
+      us = longest * ((blocks * n + sms - 1) / sms);
+    } else {
+      const float average = (blocks * n * setup_us + blocks * (0.5f * iters) * tile_us) / sms;
+      us = longest > average ? longest : average;
+    }
+    if (n > 1) us += 4.f + 0.052f * n * blocks;  // the parts: 128 rows x 128 columns, fp32, dK and dV, written and read
+    if (n == 1 || us < best_us) {
+      best_us = us;
+      best = n;
+    }
+  }
+  return best;
+}
+
+// One local K/V tensor ([B][Sk][Hk][D] views) with dK / dV of the same shape.  nsplit > 1: `part` holds 2 * nsplit * B * Sk * Hk
+// * D floats of scratch.
 CSB_API int csb_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout,
                          const float* lse, float* delta, float* dq_acc, void* dq, void* dk, void* dv, int B, int Sq,
                          int Sk, int Hq, int Hk, int D, long q_ss, long q_sb, long k_ss, long k_sb, long v_ss, long v_sb,
                          long o_ss, long o_sb, long do_ss, long do_sb, long dq_ss, long dq_sb, long dk_ss, long dk_sb,
                          long dv_ss, long dv_sb, float scale, int mask_mode, const long* q_bits, const long* k_bits,
-                         const int* q_pos, const int* k_pos, const signed char* cls, int* status, void* stream) {
+                         const int* q_pos, const int* k_pos, const signed char* cls, int* status, void* stream, float* part,
+                         int nsplit) {
   CsbKvSegments kv = {};
   kv.n_seg = 1;
   kv.my_seg = 0;
@@ -821,8 +921,8 @@ CSB_API int csb_attn_bwd(const void* q, const void* k, const void* v, const void
   kv.dk[0] = dk; kv.dv[0] = dv;
   kv.dk_stride_s[0] = dk_ss; kv.dk_stride_b[0] = dk_sb; kv.dv_stride_s[0] = dv_ss; kv.dv_stride_b[0] = dv_sb;
   kv.ready_flags = nullptr;
-  return csb_attn_bwd_seg(q, &kv, out, dout, lse, delta, dq_acc, dq, B, Sq, Sk, Hq, Hk, D, q_ss, q_sb, o_ss, o_sb, do_ss,
-                          do_sb, dq_ss, dq_sb, scale, mask_mode, q_bits, k_bits, q_pos, k_pos, cls, status, stream);
+  return attn_bwd_seg_impl(q, &kv, out, dout, lse, delta, dq_acc, dq, B, Sq, Sk, Hq, Hk, D, q_ss, q_sb, o_ss, o_sb, do_ss, do_sb,
+                           dq_ss, dq_sb, scale, mask_mode, q_bits, k_bits, q_pos, k_pos, cls, status, stream, nullptr, part, nsplit);
 }
 
 // --------------------------------------------------------------------------------------------- context-parallel glue

@@ -81,7 +81,7 @@ def lib():
 class _CountingLib:
     """Forwards attribute access to the CDLL and counts calls of kernel-launching entry points."""
 
-    _NO_LAUNCH = {"csb_norm_bwd_parts", "csb_colsum_parts"}
+    _NO_LAUNCH = {"csb_norm_bwd_parts", "csb_colsum_parts", "csb_attn_bwd_splits"}
 
     def __init__(self, raw):
         self._raw = raw

@@ -40,8 +40,9 @@ nat.declare(
 )
 nat.declare(
     "csb_attn_bwd",
-    [vp] * 11 + [i32] * 6 + [i64] * 16 + [f32, i32, vp, vp, vp, vp, vp, vp, vp],
+    [vp] * 11 + [i32] * 6 + [i64] * 16 + [f32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32],
 )
+nat.declare("csb_attn_bwd_splits", [i32] * 6)
 nat.declare("csb_mask_classify_dense", [vp, i64, i64, i32, i32, i32, vp, vp, vp])
 nat.declare("csb_attn_fwd_dense", [vp] * 5 + [i32] * 6 + [i64] * 8 + [f32, i32, vp, vp, vp, vp])
 nat.declare("csb_attn_bwd_dense", [vp] * 11 + [i32] * 6 + [i64] * 16 + [f32, i32, vp, vp, vp, vp])
@@ -300,6 +301,9 @@ def attention_backward(do, q, k, v, out, lse, mask: AttnMask, scale: float | Non
         )
         return dq, dk, dv
     qb, kb, qp, kp = _mask_ptrs(mask, B)
+    # small grids: several blocks share a key block and leave fp32 parts of dK and dV that are added in a fixed order
+    splits = nat.lib().csb_attn_bwd_splits(mask.mode, B, Sq, Sk, Hq, Hk)
+    part = torch.empty(2 * splits * B * Sk * Hk * D, dtype=torch.float32, device=q.device) if splits > 1 else None
     nat.check(
         nat.lib().csb_attn_bwd(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(),
@@ -307,7 +311,7 @@ def attention_backward(do, q, k, v, out, lse, mask: AttnMask, scale: float | Non
             q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1), v.stride(0), out.stride(1), out.stride(0),
             do.stride(1), do.stride(0), dq.stride(1), dq.stride(0), dk.stride(1), dk.stride(0), dv.stride(1),
             dv.stride(0), scale, mask.mode, nat.ptr(qb), nat.ptr(kb), nat.ptr(qp), nat.ptr(kp), nat.ptr(cls),
-            st.data_ptr(), nat.stream(),
+            st.data_ptr(), nat.stream(), nat.ptr(part), splits,
         ),
         "csb_attn_bwd",
     )

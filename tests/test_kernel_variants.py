@@ -215,3 +215,28 @@ def test_rope_with_tables_off_the_16_byte_boundary():
     b = E.rope_(x.clone(), *off, None, H, D)
     want = E._rope_ref(x.view(1, T, H, D), cos, sin, None, D).view_as(x)
     assert torch.equal(a, b) and _rel(a, want) <= REL
+
+
+# sizes whose key blocks are shared by several thread blocks: causal with one, two and eight query heads per key head, uneven
+# shares of the iterations, key blocks without a query (Sk > Sq under a causal mask), widths that are no multiple of 32
+@pytest.mark.parametrize("B,S,Sk,Hq,Hk,D", [(1, 1024, 1024, 8, 1, 128), (1, 333, 333, 32, 8, 72), (2, 513, 513, 8, 4, 64),
+                                            (1, 200, 700, 16, 2, 128), (1, 640, 640, 8, 1, 24)])
+@pytest.mark.parametrize("mode", ["causal", "full", "bitfield"])
+def test_split_attention_backward(B, S, Sk, Hq, Hk, D, mode):
+    if mode == "bitfield" and S != Sk:
+        pytest.skip("one bitfield per sequence")
+    g = torch.Generator(device="cuda").manual_seed(S + D)
+    q, do = (torch.randn(B, S, Hq, D, generator=g, device="cuda").to(BF16) for _ in range(2))
+    k, v = (torch.randn(B, Sk, Hk, D, generator=g, device="cuda").to(BF16) for _ in range(2))
+    mask = {"causal": A.AttnMask.causal(), "full": A.AttnMask.full(), "bitfield": None if S != Sk else A.AttnMask.bitfield(_bits(B, S, 9))}[mode]
+    o, lse = A.attention_forward(q, k, v, mask)
+    got = A.attention_backward(do, q, k, v, o, lse, mask)
+    again = A.attention_backward(do, q, k, v, o, lse, mask)
+    assert torch.equal(got[1], again[1]) and torch.equal(got[2], again[2])  # the parts are added in a fixed order
+    x = [t.double().requires_grad_() for t in (q, k, v)]
+    s = torch.einsum("bqhd,bkhd->bhqk", x[0], x[1].repeat_interleave(Hq // Hk, 2)) / D**0.5
+    ok = A.dense_mask(mask, B, S, Sk, "cuda")[:, None]
+    p = torch.nan_to_num(torch.softmax(s.masked_fill(~ok, float("-inf")), -1))
+    ref = torch.autograd.grad(torch.einsum("bhqk,bkhd->bqhd", p, x[2].repeat_interleave(Hq // Hk, 2)), x, do.double())
+    for a, r in zip(got, ref):
+        assert _rel(a, r) <= 1.5 * REL  # P and dS are rounded to bf16 as well as the result
