@@ -1,0 +1,62 @@
+"""The branch-free mask rule and the class of a tile by its indices (``csrc/mask.cuh``) against the predicate that defines the
+masks, compiled for the host."""
+
+import ctypes
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "cornstarch_b200" / "csrc"
+SOURCE = r"""
+#include "mask.cuh"
+using namespace csb;
+// number of (query, key) pairs for which the rule and the predicate differ
+extern "C" int rule_differences(int mode) {
+  const long bits[] = {0, 1, 2, 3, 4, 5, 6, 7, (1L << 61), (1L << 61) | 1, (1L << 62), (1L << 62) | 1, (1L << 62) | 3, (1L << 62) | 2,
+                       (1L << 33) | 1, (1L << 33), -1L, (1L << 63) | 2};
+  int bad = 0;
+  for (long qb : bits)
+    for (long kb : bits)
+      for (int qp = 0; qp < 4; ++qp)
+        for (int kp = -1; kp < 5; ++kp)
+          for (int q_exists = 0; q_exists < 2; ++q_exists) {
+            const bool k_exists = kp >= 0;
+            const bool want = q_exists && k_exists && mask_allowed(mode, qb, kb, qp, kp);
+            const QueryRule r = make_query_rule(mode, q_exists != 0, qb, qp);
+            bad += rule_allows(r, mask_key_bits(mode, k_exists, kb), kp) != want;
+          }
+  return bad;
+}
+extern "C" int tile_class(int mode, int qi, int kj, int Sq, int Sk) { return index_tile_class(mode, qi, kj, Sq, Sk); }
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("no host compiler")
+    d = tmp_path_factory.mktemp("mask")
+    (d / "m.cpp").write_text(SOURCE)
+    flags = ["-D__host__=", "-D__device__=", "-D__forceinline__=inline", "-std=c++17", "-shared", "-fPIC", f"-I{CSRC}"]
+    subprocess.run([cxx, *flags, "-x", "c++", str(d / "m.cpp"), "-o", str(d / "m.so")], check=True)
+    return ctypes.CDLL(str(d / "m.so"))
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_rule_equals_predicate(lib, mode):
+    assert lib.rule_differences(mode) == 0
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("Sq,Sk", [(1, 1), (127, 128), (128, 127), (129, 257), (300, 129), (640, 640)])
+def test_index_class_equals_count(lib, mode, Sq, Sk):
+    for qi in range((Sq + 127) // 128):
+        rows = range(qi * 128, min(Sq, qi * 128 + 128))
+        for kj in range((Sk + 127) // 128):
+            keys = range(kj * 128, min(Sk, kj * 128 + 128))
+            n = sum(1 for q in rows for k in keys if mode == 0 or k <= q)
+            want = 0 if n == 0 else (2 if n == len(rows) * 128 else 1)
+            assert lib.tile_class(mode, qi, kj, Sq, Sk) == want, (qi, kj)
