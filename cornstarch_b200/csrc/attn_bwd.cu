@@ -69,7 +69,7 @@ struct AttnBwdParams {
 };
 
 // Position in a block's list of (query head, query tile) iterations, advanced without divisions (a division and a
-// remainder per iteration in every compute warp: 8192 tokens causal 1976 us with, 1903 us without).
+// remainder per iteration on the compute warps' chain: 8192 tokens causal 1976 us with, 1903 us without).
 struct BwdCursor {
   int h, t, n_valid;
   __device__ __forceinline__ BwdCursor(int it, int n) : h(n > 0 ? it / n : 0), t(n > 0 ? it % n : 0), n_valid(n) {}
@@ -99,9 +99,9 @@ struct BwdSmem {
   static constexpr int DYN_BYTES = TOTAL + 1024;
 };
 
-// Eight compute warps: two share a TMEM lane quarter and split the 64 query columns between them.  Their loop is bound by
-// instruction issue, and what does not depend on the number of columns (waits, addresses, hand-overs) is paid per warp: sixteen
-// warps of 16 columns took 1903 us where eight of 32 take 1816 (8192 tokens causal, 32 / 8 heads of 128; full mask 3769 / 3510).
+// Eight compute warps: two share a TMEM lane quarter and split the 64 query columns between them.  Their loop is a chain
+// of hand-overs with the MMA warp (issue slots are 28 % used), and what does not depend on the number of columns (waits,
+// addresses, arrivals of every thread) is on it once per warp of a scheduler: sixteen warps of 16 columns took 1903 us where eight of 32 take 1816 (8192 tokens causal, 32 / 8 heads of 128; full mask 3769 / 3510).
 struct BwdCfg {
   static constexpr int COMPUTE_THREADS = 8 * 32;
   static constexpr int DRAIN_THREADS = 128;  // four warps that only move dQ^T out (one per TMEM lane quarter)
