@@ -1023,6 +1023,21 @@ CSB_API int csb_gemm_bf16(const void* A, const void* B, void* C, const void* bia
 #undef CSB_DISPATCH
 }
 
+CSB_API int csb_colsum(const void* x, float* partial, void* out, int out_fp32, int accumulate, int rows, int H, void* stream);
+
+// Gradients of y = x w^T + b in one call (host time: the three launches are small next to a call from Python each):
+//   dx[T,K] = dy w (null: not wanted)     dw[N,K] (+)= dy^T x     db[N] (+)= column sums of dy (null: no bias)
+// `scratch` as csb_colsum takes it; dy has row pitch N when db is given.
+CSB_API int csb_linear_bwd(const void* dy, const void* x, const void* w, void* dx, void* dw, void* db, float* scratch, int T, int N,
+                           int K, int lddy, int ldx, int ldw, int lddw, int dw_fp32, int dw_acc, int db_fp32, int db_acc, int* status,
+                           void* stream) {
+  if (db != nullptr && lddy != N) return CSB_ERR_BAD_ARG;
+  int r = 0;
+  if (dx != nullptr) r = csb_gemm_bf16(dy, w, dx, nullptr, T, K, N, lddy, ldw, K, 0, 1, 0, 0, 0, 0, 0, status, stream);
+  if (!r) r = csb_gemm_bf16(dy, x, dw, nullptr, N, K, T, lddy, ldx, lddw, 1, 1, dw_fp32, dw_acc, 0, 0, 0, status, stream);
+  if (!r && db != nullptr) r = csb_colsum(dy, scratch, db, db_fp32, db_acc, T, N, stream);
+  return r;
+}
 
 // Grouped GEMM: `groups` problems of the same shape in ONE launch.  A is [groups * group_rows][K] (K-major) and C is
 // [groups * group_rows][N]; rows [g * group_rows, (g + 1) * group_rows) use B_ptrs[g] (a HOST array of `groups` device

@@ -87,6 +87,70 @@ def fuse_adjacent_1d(tensors: Sequence[torch.Tensor | None]) -> torch.Tensor | N
     return torch.as_strided(t0, (n,), (1,), t0.storage_offset())
 
 
+def _fused_grads(tensors, fuse):
+    """``(one, True)``: the ``main_grad`` buffers of ``tensors`` as one; ``(None, True)``: none of them has any; ``(None, False)``:
+    neither."""
+    mains = [getattr(t, "main_grad", None) for t in tensors]
+    if all(m is None for m in mains):
+        return None, True
+    if any(m is None for m in mains):
+        return None, False
+    one = fuse(mains) if len(mains) > 1 else mains[0]
+    return one, one is not None
+
+
+def _native_backward(ctx, dy2, x2, weights, fused_w):
+    """The gradients of a linear layer whose weights (and biases) are all wanted, in one native call: dX, dW and the column
+    sum for the bias are issued without coming back to Python between them, which bounds layers of a few thousand tokens (forward
+    and backward of 2916 tokens, 1152 -> 4304 with a bias, back to back: 182 -> 157 us).  Several projections without buffers of
+    their own get views of one gradient.  ``None``: this layer is not of that form."""
+    n_w, biases = ctx.n_w, ctx.biases
+    T, (N, K) = dy2.shape[0], fused_w.shape
+    if ctx.tp is not None or T == 0 or not all(ctx.needs_input_grad[4 : 4 + n_w]) or fused_w.stride(1) != 1:
+        return None
+    if N % 8 or K % 8 or fused_w.stride(0) % 8 or fused_w.data_ptr() % 16 or not dy2.dtype == x2.dtype == fused_w.dtype == torch.bfloat16:
+        return None
+    dW, ok = _fused_grads(weights, fuse_adjacent)
+    if not ok or (dW is not None and (dW.dim() != 2 or dW.stride(1) != 1 or dW.shape != fused_w.shape)):
+        return None
+    db, scratch = None, None
+    if ctx.has_bias:
+        if any(b is None for b in biases) or not all(ctx.needs_input_grad[4 + n_w :]) or not dy2.is_contiguous():
+            return None
+        db, ok = _fused_grads(biases, fuse_adjacent_1d)
+        if not ok or (db is not None and (not db.is_contiguous() or db.numel() != N)):
+            return None
+    dev, lib = dy2.device, nat.lib()
+    acc_w, acc_b = int(dW is not None), int(db is not None)
+    if dW is None:
+        dW = torch.empty((N, K), dtype=dy2.dtype, device=dev)
+    if ctx.has_bias:
+        scratch = torch.empty(lib.csb_colsum_parts(T) * N, dtype=torch.float32, device=dev)
+        if db is None:
+            db = torch.empty(N, dtype=dy2.dtype, device=dev)
+    dx = torch.empty((T, K), dtype=dy2.dtype, device=dev) if ctx.needs_input_grad[0] else None
+    nat.check(
+        lib.csb_linear_bwd(dy2.data_ptr(), x2.data_ptr(), fused_w.data_ptr(), nat.ptr(dx), dW.data_ptr(), nat.ptr(db), nat.ptr(scratch),
+                           T, N, K, dy2.stride(0), x2.stride(0), fused_w.stride(0), dW.stride(0), int(dW.dtype == torch.float32),
+                           acc_w, int(db is not None and db.dtype == torch.float32), acc_b, nat.status_word(dev).data_ptr(), nat.stream()),
+        "csb_linear_bwd",
+    )
+    sizes = [w.shape[0] for w in weights]
+    dws, dbs = [None] * n_w, [None] * n_w
+    if acc_w:
+        for w in weights:
+            w.grad_added_to_main_grad = True
+    else:
+        dws = [dW] if n_w == 1 else torch.split(dW, sizes)
+    if ctx.has_bias:
+        if acc_b:
+            for b in biases:
+                b.grad_added_to_main_grad = True
+        else:
+            dbs = [db] if n_w == 1 else torch.split(db, sizes)
+    return (dx.view(ctx.x_shape) if dx is not None else None, None, None, None, *dws, *dbs)
+
+
 class _LinearFn(torch.autograd.Function):
     """y = x W^T + b with native backward; several (weight, bias) pairs share one input."""
 
@@ -128,6 +192,10 @@ class _LinearFn(torch.autograd.Function):
         n_w = ctx.n_w
         dy2 = _as_2d(dy)
         fused_w = fuse_adjacent(weights) if n_w > 1 else weights[0]
+        if fused_w is not None:
+            grads = _native_backward(ctx, dy2, x2, weights, fused_w)
+            if grads is not None:
+                return grads
         dx = None
         if ctx.needs_input_grad[0]:
             if fused_w is not None and ctx.tp is not None and ctx.tp[0] == "col":
