@@ -285,7 +285,7 @@ def attention_backward(do, q, k, v, out, lse, mask: AttnMask, scale: float | Non
     dq = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device) if dq is None else dq
     dk = torch.empty((B, Sk, Hk, D), dtype=q.dtype, device=q.device) if dk is None else dk
     dv = torch.empty((B, Sk, Hk, D), dtype=q.dtype, device=q.device) if dv is None else dv
-    dq_acc = torch.zeros((B, Sq, Hq, D), dtype=torch.float32, device=q.device)
+    dq_acc = torch.empty((B, Sq, Hq, D), dtype=torch.float32, device=q.device)
     delta = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device)
     cls = None if mask.by_index() else mask.classes(B, Sq, Sk, q.device)
     st = nat.status_word(q.device)

@@ -220,7 +220,7 @@ class FusedContextParallelAttention:
             do = do.contiguous()
         q = q if (q.stride(3) == 1 and q.stride(2) == D and q.stride(1) % 8 == 0) else q.contiguous()
         dq = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device)
-        dq_acc = torch.zeros((B, Sq, Hq, D), dtype=torch.float32, device=q.device)
+        dq_acc = torch.empty((B, Sq, Hq, D), dtype=torch.float32, device=q.device)
         delta = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device)
         cls = mask.classes(B, Sq, Sk, q.device)
         qb, kb, qp, kp = A._mask_ptrs(mask, B)
@@ -361,7 +361,7 @@ def attention_segments_local(q, ks, vs, mask: A.AttnMask, scale=None, my_seg: in
     dvs = [torch.empty_like(v) for v in vs]
     seg = local_segments(ks, vs, my_seg, dks, dvs)
     dq = torch.empty_like(q)
-    dq_acc = torch.zeros((B, Sq, Hq, D), dtype=torch.float32, device=q.device)
+    dq_acc = torch.empty((B, Sq, Hq, D), dtype=torch.float32, device=q.device)
     delta = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device)
     nat.check(nat.lib().csb_attn_bwd_seg(
         q.data_ptr(), C.addressof(seg), out.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),
