@@ -908,6 +908,8 @@ static int launch_gemm(const void* A, const void* B, const GemmParams& p, int ld
 
 }  // namespace csb
 
+#include "gemm_splitk.cuh"
+
 namespace csb {
 static int gemm_cg_choice() {
   static const int cg_env = []() { const char* e = getenv("CORNSTARCH_B200_GEMM_CG"); return e ? atoi(e) : 0; }();
@@ -970,6 +972,33 @@ static TileChoice choose_tile(int M, int N, int K, int tile_n, int max_ctas, boo
   }
   return d;
 }
+// Blocks that share the contraction of a tile (gemm_splitk_kernel), or 1.  A split costs two cluster barriers and the exchange of the
+// parts, SPLIT_US, and its tiles must all find room at one time (74 pairs of blocks, fewer of the larger clusters); it is taken where
+// it is predicted at least 7 % faster than the tile that choose_tile took (the spread of the fit).  Both sides measured, weights from
+// memory, 8 us of which are the launch and the events around it:
+//   77 tokens: 4096 -> 6144 26.6 / 22.6 us (2 blocks), 4096 -> 4096 24.6 / 18.4 (4), 14336 -> 4096 65.5 / 36.9 (4), 4304 -> 1152
+//   24.6 / 14.3 (8), dX of 4096 -> 28672 106.5 / 55.3 (4); 200 tokens: 14336 -> 4096 65.5 / 51.2 (2), 4304 -> 1152 24.6 / 16.4 (6);
+//   729 tokens: 4304 -> 1152 26.6 / 22.5 (2).  Kept whole: contractions of 1152 (14.3 / 12.3 at best) and, below sixteen k blocks,
+//   weight gradients.  Of 66 calls of 1 to 729 tokens with up to 74 tiles none got slower by more than the timer's 2 us.
+constexpr float SPLIT_US = 6.f, SPLIT_K_US = 0.26f;
+static int choose_split(int M, int N, int K, TileChoice tc, bool a_mn_major, bool b_mn_major) {
+  const long tiles = (long)((M + BM - 1) / BM) * ((N + SK_BN - 1) / SK_BN);
+  const int kb = (K + BK - 1) / BK;
+  if (kb < 16 || tiles * 2 > sm_count()) return 1;
+  const int layout = a_mn_major ? 2 : (b_mn_major ? 1 : 0);
+  float best = 0.f;
+  for (const TileCost& c : TILE_COSTS)
+    if (c.bn == tc.bn && c.cg == tc.cg) best = 0.93f * tile_cost(c, layout, M, N, K);
+  int split = 1;
+  for (int n : {2, 3, 4, 6, 8}) {
+    const float t = 6.f + SPLIT_US + SPLIT_K_US * ((kb + n - 1) / n);
+    if (t < best && tiles <= splitk_clusters(n)) {
+      best = t;
+      split = n;
+    }
+  }
+  return split;
+}
 static void no_collective(GemmParams& p) {
   p.group_rows = 0;
   p.ar_scatter = 0; p.ar_row_offset = 0;
@@ -990,7 +1019,8 @@ CSB_API int csb_gemm_bf16(const void* A, const void* B, void* C, const void* bia
   if (M <= 0 || N <= 0 || K <= 0 || (lda & 7) || (ldb & 7)) return CSB_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return CSB_ERR_BAD_ARG;
   const TileChoice tc = choose_tile(M, N, K, tile_n, max_ctas, a_mn_major != 0, b_mn_major != 0);
-  const int bn = tc.bn;
+  const int split = tile_n != 128 && tile_n != 256 && max_ctas <= 0 ? choose_split(M, N, K, tc, a_mn_major != 0, b_mn_major != 0) : 1;
+  const int bn = split > 1 ? SK_BN : tc.bn;
   GemmParams p;
   p.C = C;
   p.bias = bias;
@@ -1008,6 +1038,12 @@ CSB_API int csb_gemm_bf16(const void* A, const void* B, void* C, const void* bia
   for (int i = 0; i < 8; ++i) { p.ar_inbox[i] = nullptr; p.ar_final[i] = nullptr; p.ar_cnt_part[i] = nullptr; p.ar_cnt_final[i] = nullptr; }
   no_collective(p);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (split > 1) {
+    if (!a_mn_major && !b_mn_major) return launch_splitk<false, false>(A, B, p, lda, ldb, split, s);
+    if (!a_mn_major && b_mn_major) return launch_splitk<false, true>(A, B, p, lda, ldb, split, s);
+    if (a_mn_major && !b_mn_major) return launch_splitk<true, false>(A, B, p, lda, ldb, split, s);
+    return launch_splitk<true, true>(A, B, p, lda, ldb, split, s);
+  }
 #define CSB_DISPATCH(BNV, CGV)                                                                                   \
   if (!a_mn_major && !b_mn_major) return launch_gemm<BNV, false, false, CGV>(A, B, p, lda, ldb, max_ctas, s);   \
   if (!a_mn_major && b_mn_major) return launch_gemm<BNV, false, true, CGV>(A, B, p, lda, ldb, max_ctas, s);     \
