@@ -129,7 +129,8 @@ __device__ __forceinline__ bool bw_wait(uint64_t* bar, uint32_t phase, volatile 
 // DELTA_ROWS queries of one head, so that every thread has 2 x DELTA_ROWS 16-byte loads in flight and the results of a block
 // are consecutive.  VEC: rows of both tensors start on 16-byte boundaries.
 // The same threads write the zeros that the dQ accumulator starts from: one launch and one fill less in front of each call, which
-// small calls are bound by (issued and run one by one, 32 / 8 heads of 128 causal: 333 tokens 56 -> 42 us, 1024 tokens 96 -> 87).
+// small calls are bound by (issued and run one by one: 333 tokens causal, 32 / 8 heads of 128, 54 -> 46 us; 4 x 729 tokens, 16 heads
+// of 72, 110 -> 105; long sequences unchanged).
 // (A warp per row with 4-byte loads took 13.7 us for the 13 MB of 4 x 729 tokens, 16 heads of 72; the whole backward call went
 // from 124 to 112 us with this pass, the conversion below and the statistics warps.)
 constexpr int DELTA_ROWS = 4;
