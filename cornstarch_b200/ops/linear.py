@@ -25,6 +25,9 @@ from . import _native as nat
 from .gemm import gemm
 
 
+_GRAD_TYPES = (torch.bfloat16, torch.float32)  # what the GEMM and the column sum write (the native calls know only "fp32 or not")
+
+
 def _use_native(x: torch.Tensor) -> bool:
     return x.is_cuda and x.dtype == torch.bfloat16 and not nat.LIBRARY_MODE
 
@@ -39,7 +42,7 @@ def _as_2d(x: torch.Tensor) -> torch.Tensor:
 def colsum(x2: torch.Tensor, out: torch.Tensor | None = None, accumulate: bool = False) -> torch.Tensor:
     """Column sums of a bf16 ``[rows, H]`` matrix (bias gradients) on the native kernel."""
     rows, H = x2.shape
-    if not _use_native(x2) or H % 8 or not x2.is_contiguous():
+    if not _use_native(x2) or H % 8 or not x2.is_contiguous() or (out is not None and out.dtype not in _GRAD_TYPES):
         s = x2.float().sum(0)
         if out is None:
             return s.to(x2.dtype)
@@ -89,11 +92,11 @@ def fuse_adjacent_1d(tensors: Sequence[torch.Tensor | None]) -> torch.Tensor | N
 
 def _fused_grads(tensors, fuse):
     """``(one, True)``: the ``main_grad`` buffers of ``tensors`` as one; ``(None, True)``: none of them has any; ``(None, False)``:
-    neither."""
+    neither, or a buffer of a type that the kernels do not write."""
     mains = [getattr(t, "main_grad", None) for t in tensors]
     if all(m is None for m in mains):
         return None, True
-    if any(m is None for m in mains):
+    if any(m is None or m.dtype not in _GRAD_TYPES for m in mains):
         return None, False
     one = fuse(mains) if len(mains) > 1 else mains[0]
     return one, one is not None

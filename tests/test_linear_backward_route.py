@@ -1,0 +1,70 @@
+"""Which linear backward passes go through the one native call, and that every other form gets its gradients on the general
+path.  Runs on the CPU: ``gemm`` is its fp32 statement there, and the native library is one that records the calls."""
+
+import pytest
+import torch
+
+from cornstarch_b200.ops import _native as nat
+from cornstarch_b200.ops import linear as L
+
+BF16 = torch.bfloat16
+
+
+class _Recorder:
+    def __init__(self):
+        self.calls = 0
+
+    def csb_colsum_parts(self, rows):
+        return rows
+
+    def csb_linear_bwd(self, *args):
+        self.calls += 1
+        return 0
+
+
+@pytest.fixture
+def lib(monkeypatch):
+    rec = _Recorder()
+    monkeypatch.setattr(nat, "lib", lambda: rec)
+    monkeypatch.setattr(nat, "status_word", lambda device=None: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(nat, "stream", lambda: 0)
+    return rec
+
+
+def _randn(*shape):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(sum(shape))).to(BF16)
+
+
+def _layer(x, w, b, dy, main_w=None, main_b=None):
+    """Gradients of x, w and b as a program sees them: in ``main_grad`` where there is one."""
+    x, w = x.detach().requires_grad_(), w.detach().requires_grad_()
+    b = b.detach().requires_grad_() if b is not None else None
+    for t, m in ((w, main_w), (b, main_b)):
+        if t is not None and m is not None:
+            t.main_grad = m
+    L._LinearFn.apply(x, 1, None, None, w, b).backward(dy)
+    return [x.grad, *(t.main_grad if hasattr(t, "main_grad") else t.grad for t in (w, b) if t is not None)]
+
+
+def _check(got, x, w, b, dy, base=0.0):
+    want = [dy.double() @ w.double(), dy.double().t() @ x.double() + base] + ([dy.double().sum(0) + base] if b is not None else [])
+    for a, r in zip(got, want):
+        # one rounding to bf16 (2^-9 of the value), two where the result is added to a buffer
+        assert (a.double() - r).norm() <= 2.0**-8 * r.norm()
+
+
+def test_plain_layers_take_the_native_call(lib):
+    _layer(_randn(9, 40), _randn(24, 40), _randn(24), _randn(9, 24))
+    _layer(_randn(9, 40), _randn(24, 40), None, _randn(9, 24), torch.zeros(24, 40))
+    assert lib.calls == 2
+
+
+@pytest.mark.parametrize("w_dtype,b_dtype", [(torch.float16, None), (torch.float64, None), (torch.float16, torch.float16),
+                                             (BF16, torch.float16), (torch.float32, torch.float64)])
+def test_buffers_of_other_types_are_not_the_kernels(lib, w_dtype, b_dtype):
+    """The kernels write bf16 and fp32.  A buffer of another type goes the general way (where the GEMM refuses it on the GPU) and
+    is never taken for bf16."""
+    x, w, dy, b = _randn(9, 40), _randn(24, 40), _randn(9, 24), _randn(24) if b_dtype is not None else None
+    got = _layer(x, w, b, dy, torch.ones(24, 40, dtype=w_dtype), None if b is None else torch.ones(24, dtype=b_dtype))
+    assert lib.calls == 0
+    _check(got, x, w, b, dy, base=1.0)
