@@ -111,7 +111,10 @@ def _native_backward(ctx, dy2, x2, weights, fused_w):
     T, (N, K) = dy2.shape[0], fused_w.shape
     if ctx.tp is not None or T == 0 or not all(ctx.needs_input_grad[4 : 4 + n_w]) or fused_w.stride(1) != 1:
         return None
-    if N % 8 or K % 8 or fused_w.stride(0) % 8 or fused_w.data_ptr() % 16 or not dy2.dtype == x2.dtype == fused_w.dtype == torch.bfloat16:
+    # (_as_2d leaves an operand that is contiguous off the 16-byte grid where it is: gemm repacks it)
+    if N % 8 or K % 8 or any(t.stride(0) % 8 or t.data_ptr() % 16 for t in (dy2, x2, fused_w)):
+        return None
+    if not dy2.dtype == x2.dtype == fused_w.dtype == torch.bfloat16:
         return None
     dW, ok = _fused_grads(weights, fuse_adjacent)
     if not ok or (dW is not None and (dW.dim() != 2 or dW.stride(1) != 1 or dW.shape != fused_w.shape)):

@@ -68,3 +68,44 @@ def test_buffers_of_other_types_are_not_the_kernels(lib, w_dtype, b_dtype):
     got = _layer(x, w, b, dy, torch.ones(24, 40, dtype=w_dtype), None if b is None else torch.ones(24, dtype=b_dtype))
     assert lib.calls == 0
     _check(got, x, w, b, dy, base=1.0)
+
+
+def _misaligned(t):
+    """``t`` as a contiguous view four elements into a flat buffer: 8 bytes off the 16-byte grid."""
+    flat = torch.zeros(t.numel() + 8, dtype=t.dtype)
+    flat[4 : 4 + t.numel()] = t.flatten()
+    return flat[4 : 4 + t.numel()].view(t.shape)
+
+
+def _row_of_wider(t):
+    """The one row ``t`` from columns 4.. of a wider row: contiguous, and off the grid."""
+    wide = torch.zeros(3, t.shape[1] + 12, dtype=t.dtype)
+    wide[0, 4 : 4 + t.shape[1]] = t[0]
+    return wide[:1, 4 : 4 + t.shape[1]]
+
+
+@pytest.mark.parametrize("which", ["x", "dy", "both"])
+@pytest.mark.parametrize("form,T", [(_misaligned, 9), (_misaligned, 1), (_row_of_wider, 1)])
+@pytest.mark.parametrize("main", [False, True])
+def test_operands_off_the_grid_take_the_general_path(lib, which, form, T, main):
+    """The TMA loads of the native call need 16-byte aligned rows; the general path repacks such an operand."""
+    x, w, dy = _randn(T, 40), _randn(24, 40), _randn(T, 24)
+    xs, dys = (form(x) if which != "dy" else x), (form(dy) if which != "x" else dy)
+    for t, u in ((xs, x), (dys, dy)):
+        assert t.is_contiguous() and torch.equal(t, u)
+
+    class GivesDy(torch.autograd.Function):  # the gradient that reaches the layer is this tensor, not a copy
+        @staticmethod
+        def forward(ctx, y):
+            return y.float().sum()
+
+        @staticmethod
+        def backward(ctx, g):
+            return dys
+
+    xr, wr = xs.detach().requires_grad_(), w.detach().requires_grad_()
+    if main:
+        wr.main_grad = torch.zeros(24, 40)
+    GivesDy.apply(L._LinearFn.apply(xr, 1, None, None, wr, None)).backward()
+    assert lib.calls == 0
+    _check([xr.grad, wr.main_grad if main else wr.grad], x, w, None, dy)
