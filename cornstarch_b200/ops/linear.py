@@ -102,11 +102,17 @@ def _fused_grads(tensors, fuse):
     return one, one is not None
 
 
+def _parts(grad, sizes):
+    """The gradients of several parameters out of one buffer, each with a version counter of its own."""
+    return [t.data for t in torch.split(grad, sizes)]
+
+
 def _native_backward(ctx, dy2, x2, weights, fused_w):
     """The gradients of a linear layer whose weights (and biases) are all wanted, in one native call: dX, dW and the column
     sum for the bias are issued without coming back to Python between them, which bounds layers of a few thousand tokens (forward
     and backward of 2916 tokens, 1152 -> 4304 with a bias, back to back: 182 -> 157 us).  Several projections without buffers of
-    their own get views of one gradient.  ``None``: this layer is not of that form."""
+    their own get parts of one gradient, whose memory is given back with the last of them.  ``None``: this layer is not of that
+    form."""
     n_w, biases = ctx.n_w, ctx.biases
     T, (N, K) = dy2.shape[0], fused_w.shape
     if ctx.tp is not None or T == 0 or not all(ctx.needs_input_grad[4 : 4 + n_w]) or fused_w.stride(1) != 1:
@@ -147,13 +153,13 @@ def _native_backward(ctx, dy2, x2, weights, fused_w):
         for w in weights:
             w.grad_added_to_main_grad = True
     else:
-        dws = [dW] if n_w == 1 else torch.split(dW, sizes)
+        dws = [dW] if n_w == 1 else _parts(dW, sizes)
     if ctx.has_bias:
         if acc_b:
             for b in biases:
                 b.grad_added_to_main_grad = True
         else:
-            dbs = [db] if n_w == 1 else torch.split(db, sizes)
+            dbs = [db] if n_w == 1 else _parts(db, sizes)
     return (dx.view(ctx.x_shape) if dx is not None else None, None, None, None, *dws, *dbs)
 
 
@@ -256,7 +262,7 @@ class _LinearFn(torch.autograd.Function):
                     b.grad_added_to_main_grad = True
                 return (dx, None, None, None, *dws, *dbs)
             if all(m is None for m in mains):
-                return (dx, None, None, None, *dws, *torch.split(colsum(dy2), [w.shape[0] for w in weights]))
+                return (dx, None, None, None, *dws, *_parts(colsum(dy2), [w.shape[0] for w in weights]))
         if ctx.has_bias:
             o = 0
             for i, (w, b) in enumerate(zip(weights, ctx.biases)):

@@ -109,3 +109,24 @@ def test_operands_off_the_grid_take_the_general_path(lib, which, form, T, main):
     GivesDy.apply(L._LinearFn.apply(xr, 1, None, None, wr, None)).backward()
     assert lib.calls == 0
     _check([xr.grad, wr.main_grad if main else wr.grad], x, w, None, dy)
+
+
+def test_gradients_of_several_projections_change_one_by_one(lib):
+    """They may lie in one buffer, but a change of one in place is no change of the others: an autograd graph that holds one of
+    them stays valid."""
+    w, b = _randn(48, 40), _randn(48)
+    ws = [t.detach().requires_grad_() for t in torch.split(w, [24, 8, 16])]
+    bs = [t.detach().requires_grad_() for t in torch.split(b, [24, 8, 16])]
+    x = _randn(9, 40).requires_grad_()
+    L._LinearFn.apply(x, 3, None, None, *ws, *bs).backward(_randn(9, 48))
+    assert lib.calls == 1
+    for ts in (ws, bs):
+        with torch.no_grad():
+            ts[0].grad.fill_(2.0)
+            ts[2].grad.fill_(3.0)
+        z = torch.ones_like(ts[0], requires_grad=True)
+        loss = (z * ts[0].grad).sum()
+        torch.optim.SGD(ts[1:], lr=0.1).zero_grad(set_to_none=False)
+        ts[2].grad.mul_(0.5)
+        loss.backward()
+        assert (z.grad == 2).all() and (ts[0].grad == 2).all() and not ts[1].grad.any() and not ts[2].grad.any()
