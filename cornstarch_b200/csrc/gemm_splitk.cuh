@@ -252,22 +252,26 @@ struct SplitKLaunch {
 };
 template <bool A_MN, bool B_MN>
 static cudaError_t splitk_prepare() {
-  static const cudaError_t e =
+  static bool done = false;
+  if (done) return cudaSuccess;
+  const cudaError_t e =
       cudaFuncSetAttribute(gemm_splitk_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitKSmem::DYN_BYTES);
+  done = e == cudaSuccess;
   return e;
 }
-// Clusters of `split` blocks that the GPU holds at one time: an SM belongs to one GPC, and what a GPC has left over is lost.
+// Clusters of `split` blocks that the GPU holds at one time when nothing else runs: an SM belongs to one GPC, and what a GPC has left
+// over is lost.
 static int splitk_clusters(int split) {
-  static int n[SK_MAX_SPLIT + 1] = {};  // (a race writes the same number twice)
+  static int n[SK_MAX_SPLIT + 1] = {};  // (a race writes the same number twice; a query that failed is not kept)
   if (n[split] == 0) {
     int c = 0;
     SplitKLaunch l(1, split, nullptr);
     if (splitk_prepare<false, false>() != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&c, (const void*)gemm_splitk_kernel<false, false>, &l.cfg) != cudaSuccess) {
       cudaGetLastError();
-      c = 0;
+      return 0;
     }
-    n[split] = c > 0 ? c : -1;
+    n[split] = c;
   }
   return n[split];
 }
