@@ -981,7 +981,9 @@ static TileChoice choose_tile(int M, int N, int K, int tile_n, int max_ctas, boo
 //   729 tokens: 4304 -> 1152 26.6 / 22.5 (2).  Kept whole: contractions of 1152 (14.3 / 12.3 at best) and, below sixteen k blocks,
 //   weight gradients.  Of 66 calls of 1 to 729 tokens with up to 74 tiles none got slower by more than the timer's 2 us.
 constexpr float SPLIT_US = 6.f, SPLIT_K_US = 0.26f;
-static int choose_split(int M, int N, int K, TileChoice tc, bool a_mn_major, bool b_mn_major) {
+// (`tile_n`, `max_ctas` and CORNSTARCH_B200_GEMM_CG=1 ask for blocks that work alone.)
+static int choose_split(int M, int N, int K, int tile_n, int max_ctas, TileChoice tc, bool a_mn_major, bool b_mn_major) {
+  if (tile_n == 128 || tile_n == 256 || max_ctas > 0 || gemm_cg_choice() == 1) return 1;
   const long tiles = (long)((M + BM - 1) / BM) * ((N + SK_BN - 1) / SK_BN);
   const int kb = (K + BK - 1) / BK;
   if (kb < 16 || tiles * 2 > sm_count()) return 1;
@@ -1008,6 +1010,18 @@ static void no_collective(GemmParams& p) {
 }
 }  // namespace csb
 
+// What csb_gemm_bf16 takes for a call: columns of a tile, blocks that work on one tile side by side (1 or 2), blocks
+// that share its contraction.
+CSB_API int csb_gemm_choice(int M, int N, int K, int a_mn_major, int b_mn_major, int tile_n, int max_ctas, int* bn, int* cg, int* split) {
+  using namespace csb;
+  if (M <= 0 || N <= 0 || K <= 0) return CSB_ERR_BAD_ARG;
+  const TileChoice tc = choose_tile(M, N, K, tile_n, max_ctas, a_mn_major != 0, b_mn_major != 0);
+  *split = choose_split(M, N, K, tile_n, max_ctas, tc, a_mn_major != 0, b_mn_major != 0);
+  *bn = *split > 1 ? SK_BN : tc.bn;
+  *cg = *split > 1 ? 1 : tc.cg;
+  return 0;
+}
+
 // C[M,N] (+)= act(op(A) * op(B)^T + bias).  a_mn_major=0: A is [M][K] with row stride lda;
 // a_mn_major=1: A is [K][M] with row stride lda.  Same for B with N in place of M.
 // Leading dimensions are in elements and must be multiples of 8 (16-byte TMA strides).
@@ -1019,7 +1033,7 @@ CSB_API int csb_gemm_bf16(const void* A, const void* B, void* C, const void* bia
   if (M <= 0 || N <= 0 || K <= 0 || (lda & 7) || (ldb & 7)) return CSB_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return CSB_ERR_BAD_ARG;
   const TileChoice tc = choose_tile(M, N, K, tile_n, max_ctas, a_mn_major != 0, b_mn_major != 0);
-  const int split = tile_n != 128 && tile_n != 256 && max_ctas <= 0 ? choose_split(M, N, K, tc, a_mn_major != 0, b_mn_major != 0) : 1;
+  const int split = choose_split(M, N, K, tile_n, max_ctas, tc, a_mn_major != 0, b_mn_major != 0);
   const int bn = split > 1 ? SK_BN : tc.bn;
   GemmParams p;
   p.C = C;
