@@ -973,20 +973,27 @@ static TileChoice choose_tile(int M, int N, int K, int tile_n, int max_ctas, boo
   return d;
 }
 // Blocks that share the contraction of a tile (gemm_splitk_kernel), or 1.  A split costs two cluster barriers and the exchange of the
-// parts, SPLIT_US, and its tiles must all find room at one time (74 pairs of blocks, fewer of the larger clusters); it is taken where
-// it is predicted at least 7 % faster than the tile that choose_tile took (the spread of the fit).  Both sides measured, weights from
-// memory, 8 us of which are the launch and the events around it:
-//   77 tokens: 4096 -> 6144 26.6 / 22.6 us (2 blocks), 4096 -> 4096 24.6 / 18.4 (4), 14336 -> 4096 65.5 / 36.9 (4), 4304 -> 1152
-//   24.6 / 14.3 (8), dX of 4096 -> 28672 106.5 / 55.3 (4); 200 tokens: 14336 -> 4096 65.5 / 51.2 (2), 4304 -> 1152 24.6 / 16.4 (6);
-//   729 tokens: 4304 -> 1152 26.6 / 22.5 (2).  Kept whole: contractions of 1152 (14.3 / 12.3 at best) and, below sixteen k blocks,
-//   weight gradients.  Of 66 calls of 1 to 729 tokens with up to 74 tiles none got slower by more than the timer's 2 us.
-constexpr float SPLIT_US = 6.f, SPLIT_K_US = 0.26f;
+// parts, SPLIT_US, and its tiles must all find room at one time; it is taken where it is predicted at least 7 % faster than the tile
+// that choose_tile took (the spread of the fit).  Both sides measured, weights from memory, replayed back to back:
+//   77 tokens: 4096 -> 6144 20.1 / 16.2 us (2 blocks), 4096 -> 4096 19.4 / 12.2 (4), 14336 -> 4096 52.4 / 24.9 (4), 4304 -> 1152
+//   20.5 / 9.3 (8); 200 tokens: 14336 -> 4096 53.2 / 35.4 (2), 4304 -> 1152 21.6 / 10.5 (6); 729 tokens: 4304 -> 1152 22.1 / 16.9 (2);
+//   weight gradients added to fp32: 768 x 768 of 2048 tokens 15.1 / 13.5 (3), of 8192 39.1 / 23.1; 1024 x 1024 of 8192 39.9 / 31.5 (2).
+// 159 forward and input-gradient calls (1 to 8192 tokens) that are split take 0.47 of the time in the geometric mean, the worst 0.84;
+// 201 weight gradients (of 1536 to 16384 tokens; fresh, added to bf16 and to fp32) 0.64, the worst 0.98.  One SPLIT_K_US does for
+// all operand orders: the loads bound it.  The parts are shorter fp32 sums: 0.1 to 0.5 of the whole tile's error against 64 bits.
+// Kept whole: contractions of 1152 and, below sixteen k blocks, weight gradients.
+// Room: SPLIT_CLUSTERS is what runs at one time beside 16 blocks of another kernel (the overlapped gradient reduction; an idle GPU
+// holds 74 / 45 / 33 / 22 / 15).  One cluster more and a second round starts: 128 rows x 4096, 66 tiles in pairs 21.1 us beside it,
+// 67 tiles 33.5, whole 23.1; 40 tiles in threes 16.0, 42 tiles 26.6, whole 21.1.  Beside more blocks than that, 24 or 32 of
+// them, 64 tiles in pairs meet that second round (33.3); fours and more are then no slower than whole tiles.
 // (`tile_n`, `max_ctas` and CORNSTARCH_B200_GEMM_CG=1 ask for blocks that work alone.)
+constexpr float SPLIT_US = 6.f, SPLIT_K_US = 0.26f;
+constexpr int SPLIT_CLUSTERS[SK_MAX_SPLIT + 1] = {0, 0, 66, 40, 33, 0, 18, 0, 15};
 static int choose_split(int M, int N, int K, int tile_n, int max_ctas, TileChoice tc, bool a_mn_major, bool b_mn_major) {
   if (tile_n == 128 || tile_n == 256 || max_ctas > 0 || gemm_cg_choice() == 1) return 1;
   const long tiles = (long)((M + BM - 1) / BM) * ((N + SK_BN - 1) / SK_BN);
   const int kb = (K + BK - 1) / BK;
-  if (kb < 16 || tiles * 2 > sm_count()) return 1;
+  if (kb < 16 || tiles > SPLIT_CLUSTERS[2]) return 1;
   const int layout = a_mn_major ? 2 : (b_mn_major ? 1 : 0);
   float best = 0.f;
   for (const TileCost& c : TILE_COSTS)
@@ -994,7 +1001,7 @@ static int choose_split(int M, int N, int K, int tile_n, int max_ctas, TileChoic
   int split = 1;
   for (int n : {2, 3, 4, 6, 8}) {
     const float t = 6.f + SPLIT_US + SPLIT_K_US * ((kb + n - 1) / n);
-    if (t < best && tiles <= splitk_clusters(n)) {
+    if (t < best && tiles <= SPLIT_CLUSTERS[n] && tiles <= splitk_clusters(n)) {
       best = t;
       split = n;
     }
