@@ -984,8 +984,8 @@ static TileChoice choose_tile(int M, int N, int K, int tile_n, int max_ctas, boo
 // Kept whole: contractions of 1152 and, below sixteen k blocks, weight gradients.
 // Room: SPLIT_CLUSTERS is what runs at one time beside 16 blocks of another kernel (the overlapped gradient reduction; an idle GPU
 // holds 74 / 45 / 33 / 22 / 15).  One cluster more and a second round starts: 128 rows x 4096, 66 tiles in pairs 21.1 us beside it,
-// 67 tiles 33.5, whole 23.1; 40 tiles in threes 16.0, 42 tiles 26.6, whole 21.1.  Beside more blocks than that, 24 or 32 of
-// them, 64 tiles in pairs meet that second round (33.3); fours and more are then no slower than whole tiles.
+// 67 tiles 33.5, whole 23.1; 40 tiles in threes 16.0, 42 tiles 26.6, whole 21.1.  Beside more blocks than that the largest
+// splits meet it too: beside 24, 64 tiles in pairs take 33.3 us and 30 in fours 22.7 (whole 23.0 and 20.3).
 // (`tile_n`, `max_ctas` and CORNSTARCH_B200_GEMM_CG=1 ask for blocks that work alone.)
 constexpr float SPLIT_US = 6.f, SPLIT_K_US = 0.26f;
 constexpr int SPLIT_CLUSTERS[SK_MAX_SPLIT + 1] = {0, 0, 66, 40, 33, 0, 18, 0, 15};

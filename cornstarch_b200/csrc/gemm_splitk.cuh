@@ -9,7 +9,8 @@
 // memory, no second launch, no atomics: results repeat themselves bit for bit.
 //
 // What bounds it is the latency of the loads, then the memory: six stages of 32 KB and one block per SM (77 tokens, 14336 -> 4096 in
-// four parts: 43.0 us with three stages and two blocks per SM, 36.9 with six; whole 65.5; the weights alone take 18 at 6.5 TB/s).
+// four parts: 43.0 us with three stages and two blocks per SM, 36.9 with six; whole 65.5; 8 us of each are the launch and the events
+// around it; the weights alone take 18 at 6.5 TB/s).
 // Set-up, cluster barriers and the exchange of the parts are about 6 us: measured on both sides at choose_split.
 #pragma once
 

@@ -110,7 +110,7 @@ def _parts(grad, sizes):
 def _native_backward(ctx, dy2, x2, weights, fused_w):
     """The gradients of a linear layer whose weights (and biases) are all wanted, in one native call: dX, dW and the column
     sum for the bias are issued without coming back to Python between them, which bounds layers of a few thousand tokens (forward
-    and backward of 2916 tokens, 1152 -> 4304 with a bias, back to back: 182 -> 157 us).  Several projections without buffers of
+    and backward of 2916 tokens, 1152 -> 4304 with a bias, back to back: 167 -> 151 us).  Several projections without buffers of
     their own get parts of one gradient, whose memory is given back with the last of them.  ``None``: this layer is not of that
     form."""
     n_w, biases = ctx.n_w, ctx.biases
