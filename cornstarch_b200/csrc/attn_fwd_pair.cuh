@@ -8,14 +8,22 @@
 //
 // so that one group computes exponentials while the tensor core works for the other, and the two softmax warps of a
 // scheduler are in different phases of a tile.  (With one tile per block both warps of a scheduler load, take maxima and
-// store at the same time; the special-function unit and the tensor core then idle in turns.)  One thread per row takes the
-// maximum with three-input instructions and scales and sums in packed pairs; nothing is exchanged between threads.
-// Measured (B200, 32 / 8 heads of 128): 8192 tokens causal 788 -> 495 us (1110 TFLOP/s), full 1329 -> 928 us (1185 TFLOP/s).
+// store at the same time; the special-function unit and the tensor core then idle in turns.  An MMA warp per stream has the
+// same effect: the streams fall into step, 939 us for the case below that takes 833.)  One thread per row takes the maximum
+// with three-input instructions and scales and sums in packed pairs; nothing is exchanged between threads.
 //
-// Hand-overs per stream and tile: s_full (MMA -> softmax) and p_full (softmax -> MMA), strictly alternating, so no parity
-// wait can be two phases behind.  S(next) of a stream is issued after P V of its current tile, whose operand P lives in
-// the columns that S(next) overwrites; s_full of the next tile therefore also says that P V has retired, which is what
-// the lazy rescale of O needs.
+// What bounds it: the chain of a stream, P V and the next S (1024 cycles of the tensor pipe, of which the other stream takes
+// as many) and the softmax in between, about 3050 cycles per key tile and pair where the pipe needs 2048; on long runs the
+// power cap (990 W at 1.63 GHz).  Before, it was the MMA warp's own instructions: 90 cycles to issue an MMA that takes 64, 550 to
+// 1000 per tile for tile classes and waits.  Hence runs of MMAs (umma_f16_run_w), classes as bits in registers and one wait per
+// tile for K and V; P goes over in two halves so that P V starts beside the second half's exponentials.
+// Measured (B200, 32 / 8 heads of 128, before -> now): 8192 tokens causal 507 -> 455 us (1209 TFLOP/s), full 920 -> 830 us (1325
+// TFLOP/s); 1024 causal 23.4 -> 21.1 us; 4 x 729 tokens, 16 heads of 72: 35.7 -> 34.7 us.
+//
+// Hand-overs per stream and tile: s_full (MMA -> softmax) and p_full, one per half of the keys (softmax -> MMA), strictly
+// alternating, so no parity wait can be two phases behind.  S(next) of a stream is issued after P V of its current tile, whose
+// operand P lives in the columns that S(next) overwrites; s_full of the next tile therefore also says that P V has retired,
+// which is what the lazy rescale of O needs.
 #pragma once
 
 namespace csb {
@@ -35,7 +43,7 @@ struct PairSmem {
   static constexpr int CLS_OFF = META_OFF + 8 * META_WARP;  // tile classes of both streams
   static constexpr int MAX_NK = AttnSmem<NCH>::MAX_NK;
   static constexpr int BAR_OFF = CLS_OFF + 2 * MAX_NK;
-  static constexpr int NBAR = 16;
+  static constexpr int NBAR = 13;
   static constexpr int TOTAL = BAR_OFF + NBAR * 8 + 16;
   static constexpr int DYN_BYTES = TOTAL + 1024;
 };
@@ -83,14 +91,12 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-  uint64_t* q_full = bars;        // [2] per stream
-  uint64_t* k_full = bars + 2;    // [2] per stage
-  uint64_t* k_empty = bars + 4;   // [2]
-  uint64_t* v_full = bars + 6;    // [2]
-  uint64_t* v_empty = bars + 8;   // [2]
-  uint64_t* s_full = bars + 10;   // [2] per stream
-  uint64_t* p_full = bars + 12;   // [2] per stream, 128 arrivals
-  uint64_t* o_full = bars + 14;   // [2] per stream: its last P V has retired
+  uint64_t* q_full = bars;        // both query tiles and the first K tile
+  uint64_t* vk_full = bars + 1;   // [2] V of ring position i and K of position i + 1
+  uint64_t* vk_empty = bars + 3;  // [2]
+  uint64_t* s_full = bars + 5;    // [2] per stream
+  uint64_t* o_full = bars + 7;    // [2] per stream: its last P V has retired
+  uint64_t* p_full = bars + 9;    // [2][2] per stream and half of the keys, 128 arrivals
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int8_t* cls_s = reinterpret_cast<int8_t*>(smem + L::CLS_OFF);
@@ -110,11 +116,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       cls_s[s * L::MAX_NK + j] = s < n_streams ? tile_class(p, b, qp0 + s, j) : int8_t(0);
   }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 12; ++i) mbar_init(&bars[i], 1);
-    mbar_init(&p_full[0], 128);
-    mbar_init(&p_full[1], 128);
-    mbar_init(&o_full[0], 1);
-    mbar_init(&o_full[1], 1);
+    for (int i = 0; i < 9; ++i) mbar_init(&bars[i], 1);
+    for (int i = 0; i < 4; ++i) mbar_init(&p_full[i], 128);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -144,29 +147,29 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
-      const int t0 = next_tile(0);
+      auto load = [&](int off, const CUtensorMap* tm, uint64_t* bar, int head, int tile) {
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) tma_load_4d(smem + off + c * CHUNK_BYTES, tm, bar, c * 64, head, tile * 128, b);
+      };
+      int t = next_tile(0);
       // Without a key tile (queries that are all padding) nobody waits for the query tiles, so they are not loaded: the block
       // would exit with the copies in flight, into shared memory and barriers that the SM's next block already uses.
-      for (int s = 0; t0 < p.nK && s < n_streams; ++s) {
-        mbar_expect_tx(&q_full[s], L::TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < NCH; ++c)
-          tma_load_4d(smem + L::Q_OFF + s * L::TILE_BYTES + c * CHUNK_BYTES, &tm_q, &q_full[s], c * 64, h, (qp0 + s) * AT_BM, b);
+      if (t < p.nK) {
+        mbar_expect_tx(q_full, (n_streams + 1) * L::TILE_BYTES);
+        load(L::Q_OFF, &tm_q, q_full, h, qp0);
+        load(L::K_OFF, &tm_k, q_full, hk, t);
+        if (n_streams == 2) load(L::Q_OFF + L::TILE_BYTES, &tm_q, q_full, h, qp0 + 1);
       }
-      uint32_t it = 0;
-      for (int t = t0; t < p.nK; t = next_tile(t + 1), ++it) {
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        if (!at_wait(&k_empty[st], ph ^ 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
-        mbar_expect_tx(&k_full[st], L::TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < NCH; ++c)
-          tma_load_4d(smem + L::K_OFF + st * L::TILE_BYTES + c * CHUNK_BYTES, &tm_k, &k_full[st], c * 64, hk, t * AT_BN, b);
-        if (!at_wait(&v_empty[st], ph ^ 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
-        mbar_expect_tx(&v_full[st], L::TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < NCH; ++c)
-          tma_load_4d(smem + L::V_OFF + st * L::TILE_BYTES + c * CHUNK_BYTES, &tm_v, &v_full[st], c * 64, hk, t * AT_BN, b);
+      for (uint32_t it = 0; t < p.nK; ++it) {
+        const int st = it & 1, tn = next_tile(t + 1);
+        // Free are the V stage (P V of position it - 2 is done; the first two are free at the start) and the K stage that position
+        // it + 1 takes (S of position it - 1 is done; the first one at the start).  S is issued a position ahead of P V, so one
+        // commit after position it - 2 says both; for it = 1 there is one after the first S.
+        if (!at_wait(&vk_empty[st], ((it >> 1) ^ it ^ 1) & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
+        mbar_expect_tx(&vk_full[st], (tn < p.nK ? 2 : 1) * L::TILE_BYTES);
+        load(L::V_OFF + st * L::TILE_BYTES, &tm_v, &vk_full[st], hk, t);
+        if (tn < p.nK) load(L::K_OFF + (st ^ 1) * L::TILE_BYTES, &tm_k, &vk_full[st], hk, tn);
+        t = tn;
       }
     }
     __syncwarp();
@@ -175,67 +178,85 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t idesc_s = make_idesc_bf16(AT_BM, AT_BN, 0, 0);
     const uint32_t idesc_o = make_idesc_bf16(AT_BM, p.dk16, 0, 1);
     const int ksteps_s = p.dk16 / 16;
-    int last[2] = {-1, -1};  // last key tile of each stream
-    for (int t = 0; t < p.nK; ++t) {
-      if (cls0[t] != 0) last[0] = t;
-      if (cls1[t] != 0) last[1] = t;
-    }
+    const uint64_t q_desc = make_desc_kmajor_sw128(smem_u32(smem + L::Q_OFF));
+    const uint64_t k_desc = make_desc_kmajor_sw128(smem_u32(smem + L::K_OFF));
+    const uint64_t v_desc = make_desc_mnmajor_sw128(smem_u32(smem + L::V_OFF), CHUNK_BYTES);
+    constexpr uint64_t TILE_STEP = L::TILE_BYTES >> 4;  // from one tile to the next, in a descriptor's address field
     bool ok = true;
     auto fail = [&](int code) {
       atomicCAS(p.status, 0, code);
       *abort_flag = 1;
       ok = false;
     };
-    // S_s = Q_s K^T with the K tile of ring position it
+    // S of stream s = Q_s K^T with the K tile of ring position it
     auto issue_s = [&](int s, uint32_t it) {
-      const uint64_t q_desc = make_desc_kmajor_sw128(smem_u32(smem + L::Q_OFF + s * L::TILE_BYTES));
-      const uint64_t k_desc = make_desc_kmajor_sw128(smem_u32(smem + L::K_OFF + (it & 1) * L::TILE_BYTES));
-#pragma unroll
-      for (int kk = 0; kk < 4 * NCH; ++kk) {  // unrolled to the maximum, cut by a uniform test
-        const uint64_t off = static_cast<uint64_t>(((kk >> 2) * CHUNK_BYTES + (kk & 3) * 32) >> 4);
-        if (kk < ksteps_s) umma_f16_w(tmem_S + s * 128, q_desc + off, k_desc + off, idesc_s, kk > 0 ? 1u : 0u);
-      }
+      umma_f16_run_w(tmem_S + s * 128, q_desc + s * TILE_STEP, k_desc + (it & 1) * TILE_STEP, CHUNK_BYTES, CHUNK_BYTES, idesc_s, ksteps_s, 0u);
       umma_commit_w(&s_full[s]);
     };
+    // Key tiles as bits of 32, per stream: no shared-memory reads on the way from one MMA to the next.
+    int base = -32;
+    uint32_t bits[2] = {0, 0};
+    auto next = [&](uint32_t& who) -> int {  // the next tile that a stream needs (nK at the end); who: bit s = stream s needs it
+      while ((bits[0] | bits[1]) == 0) {
+        base += 32;
+        if (base >= p.nK) {
+          who = 0;
+          return p.nK;
+        }
+        const bool in = base + lane < p.nK;
+        bits[0] = __ballot_sync(0xffffffffu, in && cls0[base + lane] != 0);
+        bits[1] = __ballot_sync(0xffffffffu, in && cls1[base + lane] != 0);
+      }
+      const uint32_t low = (bits[0] | bits[1]) & (0u - (bits[0] | bits[1]));
+      who = ((bits[0] & low) ? 1u : 0u) | ((bits[1] & low) ? 2u : 0u);
+      bits[0] &= ~low;
+      bits[1] &= ~low;
+      return base + __ffs(low) - 1;
+    };
+    int last[2] = {-1, -1};  // last key tile of each stream
+    for (int b0 = 0; b0 < p.nK; b0 += 32) {
+      const bool in = b0 + lane < p.nK;
+      const uint32_t m0 = __ballot_sync(0xffffffffu, in && cls0[b0 + lane] != 0), m1 = __ballot_sync(0xffffffffu, in && cls1[b0 + lane] != 0);
+      if (m0 != 0) last[0] = b0 + 31 - __clz(m0);
+      if (m1 != 0) last[1] = b0 + 31 - __clz(m1);
+    }
     uint32_t done[2] = {0, 0};  // tiles of each stream whose P V was issued
-    int t = next_tile(0);
+    uint32_t who, who_next;
+    int t = next(who);
     if (t < p.nK) {
-      for (int s = 0; s < n_streams && ok; ++s)
-        if (!at_wait(&q_full[s], 0, abort_flag)) fail(ST_TIMEOUT_FULL);
-      if (ok && !at_wait(&k_full[0], 0, abort_flag)) fail(ST_TIMEOUT_FULL);
+      if (!at_wait(q_full, 0, abort_flag)) fail(ST_TIMEOUT_FULL);
       if (ok) {
         tc_fence_after();
-        if (cls0[t] != 0) issue_s(0, 0);
-        if (cls1[t] != 0) issue_s(1, 0);
-        umma_commit_w(&k_empty[0]);
+        if (who & 1u) issue_s(0, 0);
+        if (who & 2u) issue_s(1, 0);
+        umma_commit_w(&vk_empty[1]);
       }
     }
     for (uint32_t it = 0; ok && t < p.nK; ++it) {
-      const int tn = next_tile(t + 1);
+      const int tn = next(who_next);
       const int st = it & 1;
-      if (!at_wait(&v_full[st], (it >> 1) & 1, abort_flag)) { fail(ST_TIMEOUT_FULL); break; }
-      if (tn < p.nK && !at_wait(&k_full[st ^ 1], ((it + 1) >> 1) & 1, abort_flag)) { fail(ST_TIMEOUT_FULL); break; }
+      if (!at_wait(&vk_full[st], (it >> 1) & 1, abort_flag)) { fail(ST_TIMEOUT_FULL); break; }
       tc_fence_after();
-      const uint64_t v_desc = make_desc_mnmajor_sw128(smem_u32(smem + L::V_OFF + st * L::TILE_BYTES), CHUNK_BYTES);
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const int8_t* cl = s == 0 ? cls0 : cls1;
-        if (cl[t] != 0) {
-          if (!at_wait(&p_full[s], done[s] & 1, abort_flag)) { fail(ST_TIMEOUT_MISC); break; }
-          tc_fence_after();
+        if (who & (1u << s)) {
 #pragma unroll
-          for (int kk = 0; kk < AT_BN / 16; ++kk)
-            umma_f16_ts_w(tmem_O + s * 128, tmem_S + s * 128 + kk * 8, v_desc + static_cast<uint64_t>((kk * 2048) >> 4), idesc_o,
-                          (done[s] > 0 || kk > 0) ? 1u : 0u);
+          for (int u = 0; u < 2; ++u) {
+            if (!at_wait(&p_full[s * 2 + u], done[s] & 1, abort_flag)) { fail(ST_TIMEOUT_MISC); break; }
+            tc_fence_after();
+            umma_f16_ts_run4_w(tmem_O + s * 128, tmem_S + s * 128 + u * 32,
+                               v_desc + st * TILE_STEP + static_cast<uint64_t>((u * 4 * 2048) >> 4), idesc_o, done[s] > 0 || u > 0 ? 1u : 0u);
+          }
+          if (!ok) break;
           ++done[s];
           if (t == last[s]) umma_commit_w(&o_full[s]);
         }
-        if (tn < p.nK && cl[tn] != 0) issue_s(s, it + 1);
+        if (who_next & (1u << s)) issue_s(s, it + 1);
       }
       if (!ok) break;
-      umma_commit_w(&v_empty[st]);
-      if (tn < p.nK) umma_commit_w(&k_empty[st ^ 1]);
+      umma_commit_w(&vk_empty[st]);
       t = tn;
+      who = who_next;
     }
     __syncwarp();
   }
@@ -286,52 +307,68 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[g][i] = ((w[g] >> i) & 1u) ? v[g][i] : 0xff800000u;  // -inf
       }
-      float mx[4];
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        mx[g] = max3(__uint_as_float(v[g][0]), __uint_as_float(v[g][1]), __uint_as_float(v[g][2]));
-#pragma unroll
-        for (int i = 3; i + 1 < 32; i += 2) mx[g] = max3(mx[g], __uint_as_float(v[g][i]), __uint_as_float(v[g][i + 1]));
-        mx[g] = fmaxf(mx[g], __uint_as_float(v[g][31]));
-      }
-      const float m_new = fmaxf(max3(mx[0], mx[1], mx[2]), fmaxf(mx[3], m_used));
-      const bool need = (m_new - m_used) * p.scale_log2 > 8.f;  // also true when m_used is -inf and m_new is finite
-      if (it > 0 && __any_sync(0xffffffffu, need)) {
-        // rare (lazy rescale); s_full of this tile says that the previous P V of this stream has retired
-        float alpha = 1.f;
-        if (need) alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * p.scale_log2);
-#pragma unroll 1
-        for (int cc = 0; cc < 4 * NCH; ++cc) {
-          uint32_t o[16];
-          tmem_ld_32x16(t_O + cc * 16, o);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st_32x16(t_O + cc * 16, o);
-        }
-        l_sum *= alpha;
-      }
-      if (need) m_used = m_new;
-      const float m_eff = (m_used == -INFINITY) ? 0.f : m_used * p.scale_log2;
-      const uint64_t negm2 = pack_f32x2(-m_eff, -m_eff);
       uint64_t ls[2] = {0ull, 0ull};
+      // exponentials of 64 keys with the maximum that is in use: P over the first 64 columns of S (all of S is in registers)
+      auto half_tile = [&](int u) {
+        const float m_eff = (m_used == -INFINITY) ? 0.f : m_used * p.scale_log2;
+        const uint64_t negm2 = pack_f32x2(-m_eff, -m_eff);
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        uint32_t pk[16];
+        for (int g = 2 * u; g < 2 * u + 2; ++g) {
+          uint32_t pk[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const uint64_t x2 = pack_u32x2(v[g][2 * i], v[g][2 * i + 1]);
-          float y0, y1;
-          unpack_f32x2(fma_f32x2(x2, scale2, negm2), y0, y1);
-          const float e0 = fast_exp2(y0), e1 = fast_exp2(y1);
-          ls[i & 1] = add_f32x2(ls[i & 1], pack_f32x2(e0, e1));
-          pk[i] = pack_bf16x2(e0, e1);
+          for (int i = 0; i < 16; ++i) {
+            const uint64_t y2 = fma_f32x2(pack_u32x2(v[g][2 * i], v[g][2 * i + 1]), scale2, negm2);
+            float y0, y1;
+            unpack_f32x2(y2, y0, y1);
+            const float e0 = fast_exp2(y0), e1 = fast_exp2(y1);
+            ls[i & 1] = add_f32x2(ls[i & 1], pack_f32x2(e0, e1));
+            pk[i] = pack_bf16x2(e0, e1);
+          }
+          tmem_st_32x16(t_S + g * 16, pk);
         }
-        tmem_st_32x16(t_S + g * 16, pk);  // P over the first 64 columns of this stream's S (all of S is in registers)
+      };
+      // The first half's exponentials are taken with the maximum that is in use, beside the search for the tile's, and once more
+      // where that has grown by more than 2^8 (a row's first tile, rarely later): the tensor core does not wait for the maximum.
+#pragma unroll 1
+      for (bool again = false;; again = true) {
+        ls[0] = ls[1] = 0ull;
+        float mx[4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          mx[g] = max3(__uint_as_float(v[g][0]), __uint_as_float(v[g][1]), __uint_as_float(v[g][2]));
+#pragma unroll
+          for (int i = 3; i + 1 < 32; i += 2) mx[g] = max3(mx[g], __uint_as_float(v[g][i]), __uint_as_float(v[g][i + 1]));
+          mx[g] = fmaxf(mx[g], __uint_as_float(v[g][31]));
+        }
+        half_tile(0);
+        if (again) break;
+        const float m_new = fmaxf(max3(mx[0], mx[1], mx[2]), fmaxf(mx[3], m_used));
+        const bool need = (m_new - m_used) * p.scale_log2 > 8.f;  // also true when m_used is -inf and m_new is finite
+        if (!__any_sync(0xffffffffu, need)) break;
+        if (it > 0) {
+          // lazy rescale; s_full of this tile says that the previous P V of this stream has retired
+          float alpha = 1.f;
+          if (need) alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * p.scale_log2);
+#pragma unroll 1
+          for (int cc = 0; cc < 4 * NCH; ++cc) {
+            uint32_t o[16];
+            tmem_ld_32x16(t_O + cc * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x16(t_O + cc * 16, o);
+          }
+          l_sum *= alpha;
+        }
+        if (need) m_used = m_new;
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&p_full[s_id]);
+      mbar_arrive(&p_full[s_id * 2]);
+      half_tile(1);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&p_full[s_id * 2 + 1]);
       {
         float a0, a1;
         unpack_f32x2(add_f32x2(ls[0], ls[1]), a0, a1);

@@ -296,6 +296,50 @@ __device__ __forceinline__ void umma_f16_ts_w(uint32_t d_tmem, uint32_t a_tmem, 
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Runs of MMAs of one tile pair as one block of instructions: one elect.sync for all of them and 32-bit steps of the descriptors'
+// address fields, where a call per MMA pays an election and 64-bit additions each time.  Short MMAs (128 x 64 or 128 x 128 x 16 take
+// the pipe 48 or 64 cycles) are issued no faster than that otherwise: eight 128 x 64 x 16 next to busy warps 750 cycles one by
+// one, 450 as a run.
+// D (+)= A B^T over K-major 128-byte-swizzled operands: `n` steps of 16 (at most 8); a 64-wide chunk of A / B is 4 steps.
+__device__ __forceinline__ void umma_f16_run_w(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t a_chunk_bytes,
+                                               uint32_t b_chunk_bytes, uint32_t idesc, int n, uint32_t accumulate) {
+  const uint32_t a0 = static_cast<uint32_t>(a_desc), ah = static_cast<uint32_t>(a_desc >> 32);
+  const uint32_t b0 = static_cast<uint32_t>(b_desc), bh = static_cast<uint32_t>(b_desc >> 32);
+  const uint32_t a1 = a0 + (a_chunk_bytes >> 4), b1 = b0 + (b_chunk_bytes >> 4);
+#define CSB_UMMA_STEP(k, a, b, off)                                                                   \
+  "setp.gt.and.s32 q, %9, " #k ", e;\n\tadd.u32 x, " a ", " #off ";\n\tadd.u32 y, " b ", " #off ";\n\t" \
+  "mov.b64 da, {x, %2};\n\tmov.b64 db, {y, %4};\n\t"                                                \
+  "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %7, 1;\n\t"
+  asm volatile(
+      "{\n\t.reg .pred p, q, e;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %8, 0;\n\t"
+      "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %7, p;\n\t"
+      CSB_UMMA_STEP(1, "%1", "%3", 2) CSB_UMMA_STEP(2, "%1", "%3", 4) CSB_UMMA_STEP(3, "%1", "%3", 6)
+      CSB_UMMA_STEP(4, "%5", "%6", 0) CSB_UMMA_STEP(5, "%5", "%6", 2) CSB_UMMA_STEP(6, "%5", "%6", 4) CSB_UMMA_STEP(7, "%5", "%6", 6)
+      "}" ::"r"(d_tmem), "r"(a0), "r"(ah), "r"(b0), "r"(bh), "r"(a1), "r"(b1), "r"(idesc), "r"(accumulate), "r"(n)
+      : "memory");
+#undef CSB_UMMA_STEP
+}
+// D (+)= A B with A = 64 columns (of bf16 pairs: 8 tensor-memory columns a step of 16) and B MN-major in shared memory (16 rows of
+// 128 bytes a step): four steps.
+__device__ __forceinline__ void umma_f16_ts_run4_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  const uint32_t b0 = static_cast<uint32_t>(b_desc), bh = static_cast<uint32_t>(b_desc >> 32);
+#define CSB_UMMA_STEP(ao, bo)                                                                    \
+  "add.u32 x, %1, " #ao ";\n\tadd.u32 y, %2, " #bo ";\n\tmov.b64 db, {y, %3};\n\t"              \
+  "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [x], db, %4, 1;\n\t"
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t.reg .b32 x, y;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t"
+      CSB_UMMA_STEP(8, 128) CSB_UMMA_STEP(16, 256) CSB_UMMA_STEP(24, 384)
+      "}" ::"r"(d_tmem), "r"(a_tmem), "r"(b0), "r"(bh), "r"(idesc), "r"(accumulate)
+      : "memory");
+#undef CSB_UMMA_STEP
+}
 __device__ __forceinline__ void umma_f16_2cta_w(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                 uint32_t accumulate) {
   asm volatile(
