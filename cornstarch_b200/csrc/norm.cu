@@ -33,6 +33,33 @@ __device__ __forceinline__ float row_sum(float v, float* sh, uint32_t& n_calls) 
   return warp_sum(l < (int)(blockDim.x >> 5) ? buf[l] : 0.f);
 }
 
+// Two such sums with the barrier of one; `sh` holds 128 floats.
+template <bool ONE_WARP>
+__device__ __forceinline__ void row_sum2(float& a, float& b, float* sh, uint32_t& n_calls) {
+  a = warp_sum(a);
+  b = warp_sum(b);
+  if constexpr (ONE_WARP) return;
+  float* buf = sh + (n_calls++ & 1) * 64;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, n = blockDim.x >> 5;
+  if (l == 0) *reinterpret_cast<float2*>(buf + 2 * w) = make_float2(a, b);
+  __syncthreads();
+  const float2 v = l < n ? *reinterpret_cast<const float2*>(buf + 2 * l) : make_float2(0.f, 0.f);
+  a = warp_sum(v.x);
+  b = warp_sum(v.y);
+}
+
+// Eight bf16 values as four packed pairs of fp32: half the issue slots of an element-wise loop.
+struct Pair4 {
+  uint64_t p[4];
+};
+__device__ __forceinline__ Pair4 unpack_pairs(const uint4& u) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  Pair4 r;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) r.p[i] = pack_u32x2(w[i] << 16, w[i] & 0xffff0000u);
+  return r;
+}
+
 struct Vec8 {
   float f[8];
 };
@@ -206,85 +233,124 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 }
 
 // dx = rstd * (g - xhat * mean(g*xhat) [- mean(g)])  with g = dy * w;  dw += dy * xhat;  db += dy
-// One 16-byte vector per thread, with the next row's three inputs and its statistics in flight
-// while the current row is reduced.  (Two vectors per thread in blocks of 256 needed so many registers that two blocks
-// fitted an SM, paid two or four barriers per row, and read the row's statistics only when it needed them.)
-// With the sums below and the residual's gradient, in a CUDA graph: 8192 x 4096 RMSNorm 68 -> 52 us, LayerNorm 134 -> 74 us;
-// 262144 x 128: 377 -> 70 us.
-template <bool IS_LN, bool ONE_WARP>
-__global__ void __launch_bounds__(1024)
+// NV 16-byte vectors per thread, with the next row's inputs and statistics in flight while the current row is reduced.
+// The arithmetic of a row, not HBM, took the time (three unpackings and a conversion of the weight per element and pass, 19
+// instructions; LayerNorm's two sums behind two barriers): products and sums go in packed pairs of fp32 now, dy * w and xhat stay in
+// registers between the passes (6 instructions), and one barrier serves both sums.  NV and MIN_BLOCKS: see norm_bwd_shape.
+// With the sums below and the residual's gradient, inputs from HBM, before -> now: 8192 x 4096 RMSNorm 56.5 -> 53.1 us (5.0 TB/s),
+// LayerNorm 77 -> 60.4; 16384 x 1152 LayerNorm 48.6 -> 38.2; 16384 x 5120 RMSNorm 162 -> 118; 1531 x 4096 17.6 -> 14.9; 262144 x
+// 128 LayerNorm 108 -> 83.  (Rows in shared memory by bulk copies, up to eight ahead: 0.81 at 8192 elements, but 1.02 to 1.14 up
+// to 4096, and 1.2 to 1.6 for the forward kernel.)
+template <bool IS_LN, bool ONE_WARP, int NV, int MAX_THREADS, int MIN_BLOCKS>
+__global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
                 const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean_in,
                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                 __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial, float* __restrict__ db_partial,
                 int rows, int H, float w_offset) {
-  __shared__ float sh[64];
+  __shared__ float sh[128];
   uint32_t n_sums = 0;
-  const int c = ONE_WARP ? (threadIdx.x & 31) : threadIdx.x;
-  const bool on = c < H / 8;
+  const int lanes = ONE_WARP ? 32 : blockDim.x;
+  const int c = ONE_WARP ? (threadIdx.x & 31) : threadIdx.x;  // this thread's vectors of the row: c, c + lanes, ...
+  const int nvec = H / 8;
   const int first = ONE_WARP ? blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x;
   const int step = ONE_WARP ? gridDim.x * (blockDim.x >> 5) : gridDim.x;
-  float dw_acc[8], db_acc[8];
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  Pair4 dw_acc[NV], db_acc[IS_LN ? NV : 1], w2[NV];
+  uint4 n_dy[NV], n_h[NV], n_dr[NV], w_raw[NV];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) dw_acc[j] = db_acc[j] = 0.f;
-  uint4 w_raw = make_uint4(0u, 0u, 0u, 0u);
-  if (on) w_raw = *reinterpret_cast<const uint4*>(w + c * 8);
-  uint4 n_dy = make_uint4(0u, 0u, 0u, 0u), n_h = n_dy, n_dr = n_dy;
+  for (int i = 0; i < NV; ++i) {
+    n_dy[i] = n_h[i] = n_dr[i] = zero;
+    w_raw[i] = c + i * lanes < nvec ? *reinterpret_cast<const uint4*>(w + (c + i * lanes) * 8) : zero;
+  }
   float n_mean = 0.f, n_rstd = 0.f;
   auto fetch = [&](int row) {
-    const size_t at = static_cast<size_t>(row) * H + c * 8;
     n_rstd = rstd_in[row];
     if (IS_LN) n_mean = mean_in[row];
-    if (on) {
-      n_dy = __ldcs(reinterpret_cast<const uint4*>(dy + at));
-      n_h = __ldcs(reinterpret_cast<const uint4*>(h + at));
-      if (dres) n_dr = __ldcs(reinterpret_cast<const uint4*>(dres + at));
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const size_t at = static_cast<size_t>(row) * H + (c + i * lanes) * 8;
+      if (c + i * lanes < nvec) {
+        n_dy[i] = __ldcs(reinterpret_cast<const uint4*>(dy + at));
+        n_h[i] = __ldcs(reinterpret_cast<const uint4*>(h + at));
+        if (dres) n_dr[i] = __ldcs(reinterpret_cast<const uint4*>(dres + at));
+      }
     }
   };
   if (first < rows) fetch(first);
-  for (int row = first; row < rows; row += step) {
-    // the row is kept as it was loaded and unpacked again after the reduction: half the registers
-    const uint4 c_dy = n_dy, c_h = n_h, c_dr = n_dr;
-    const float mean = n_mean, rstd = n_rstd;
-    if (row + step < rows) fetch(row + step);
-    float s1 = 0.f, s2 = 0.f;
-    {
-      const Vec8 d = unpack8(c_dy), hv = unpack8(c_h), wv = unpack8(w_raw);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float xh = (hv.f[j] - mean) * rstd;
-        const float g = d.f[j] * (wv.f[j] + w_offset);
-        s1 += g * xh;
-        if (IS_LN) s2 += g;
-        dw_acc[j] += d.f[j] * xh;
-        if (IS_LN) db_acc[j] += d.f[j];
+  for (int i = 0; i < NV; ++i) {  // (not before the first row is on its way: few rows are bound by these latencies)
+    w2[i] = unpack_pairs(w_raw[i]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      w2[i].p[j] = add_f32x2(w2[i].p[j], pack_f32x2(w_offset, w_offset));
+      dw_acc[i].p[j] = 0ull;
+      if (IS_LN) db_acc[i].p[j] = 0ull;
+    }
+  }
+  for (int row = first; row < rows; row += step) {
+    const float rstd = n_rstd;
+    const uint64_t rstd2 = pack_f32x2(rstd, rstd), neg_mean2 = pack_f32x2(-n_mean, -n_mean);
+    uint4 c_dr[NV];
+    Pair4 g[NV], xh[NV];
+    uint64_t s1 = 0ull, s2 = 0ull;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {  // vectors beyond the row are zeros: dy = 0, nothing is added
+      const Pair4 d = unpack_pairs(n_dy[i]), hv = unpack_pairs(n_h[i]);
+      c_dr[i] = n_dr[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        xh[i].p[j] = mul_f32x2(IS_LN ? add_f32x2(hv.p[j], neg_mean2) : hv.p[j], rstd2);
+        g[i].p[j] = mul_f32x2(d.p[j], w2[i].p[j]);
+        s1 = fma_f32x2(g[i].p[j], xh[i].p[j], s1);
+        dw_acc[i].p[j] = fma_f32x2(d.p[j], xh[i].p[j], dw_acc[i].p[j]);
+        if (IS_LN) {
+          s2 = add_f32x2(s2, g[i].p[j]);
+          db_acc[i].p[j] = add_f32x2(db_acc[i].p[j], d.p[j]);
+        }
       }
     }
-    if (!on) s1 = s2 = 0.f;
-    const float m1 = row_sum<ONE_WARP>(s1, sh, n_sums) / H;
-    const float m2 = IS_LN ? row_sum<ONE_WARP>(s2, sh, n_sums) / H : 0.f;
-    if (on) {
-      const Vec8 d = unpack8(c_dy), hv = unpack8(c_h), wv = unpack8(w_raw);
-      Vec8 o;
+    if (row + step < rows) fetch(row + step);
+    float s1a, s1b, m1, m2 = 0.f;
+    unpack_f32x2(s1, s1a, s1b);
+    m1 = s1a + s1b;
+    if (IS_LN) {
+      float s2a, s2b;
+      unpack_f32x2(s2, s2a, s2b);
+      m2 = s2a + s2b;
+      row_sum2<ONE_WARP>(m1, m2, sh, n_sums);
+      m2 /= H;
+    } else {
+      m1 = row_sum<ONE_WARP>(m1, sh, n_sums);
+    }
+    m1 /= H;
+    const uint64_t neg_m1 = pack_f32x2(-m1, -m1), neg_m2 = pack_f32x2(-m2, -m2);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o.f[j] = rstd * (d.f[j] * (wv.f[j] + w_offset) - (hv.f[j] - mean) * rstd * m1 - m2);
-      if (dres) {
-        const Vec8 r = unpack8(c_dr);
+    for (int i = 0; i < NV; ++i) {
+      if (c + i * lanes < nvec) {
+        const Pair4 r = unpack_pairs(c_dr[i]);  // zeros without a second gradient
+        uint32_t o[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o.f[j] += r.f[j];
+        for (int j = 0; j < 4; ++j) {
+          uint64_t t = fma_f32x2(xh[i].p[j], neg_m1, g[i].p[j]);
+          if (IS_LN) t = add_f32x2(t, neg_m2);
+          float lo, hi;
+          unpack_f32x2(fma_f32x2(t, rstd2, r.p[j]), lo, hi);
+          o[j] = pack_bf16x2(lo, hi);
+        }
+        *reinterpret_cast<uint4*>(dx + static_cast<size_t>(row) * H + (c + i * lanes) * 8) = make_uint4(o[0], o[1], o[2], o[3]);
       }
-      store8(dx + static_cast<size_t>(row) * H + c * 8, o);
     }
   }
   if constexpr (ONE_WARP) {
     // the warps of a block add up their sums: one partial row per block
     __shared__ float part[8][2][256];
     const int wi = threadIdx.x >> 5;
-    if (on) {
+    if (c < nvec) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        part[wi][0][c * 8 + j] = dw_acc[j];
-        if (IS_LN) part[wi][1][c * 8 + j] = db_acc[j];
+      for (int j = 0; j < 4; ++j) {
+        *reinterpret_cast<uint64_t*>(&part[wi][0][c * 8 + 2 * j]) = dw_acc[0].p[j];
+        if (IS_LN) *reinterpret_cast<uint64_t*>(&part[wi][1][c * 8 + 2 * j]) = db_acc[0].p[j];
       }
     }
     __syncthreads();
@@ -297,14 +363,22 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
       dw_partial[static_cast<size_t>(blockIdx.x) * H + i] = sw;
       if (IS_LN && db_partial) db_partial[static_cast<size_t>(blockIdx.x) * H + i] = sb;
     }
-  } else if (on) {
-    float* pw = dw_partial + static_cast<size_t>(blockIdx.x) * H + c * 8;
-    *reinterpret_cast<float4*>(pw) = make_float4(dw_acc[0], dw_acc[1], dw_acc[2], dw_acc[3]);
-    *reinterpret_cast<float4*>(pw + 4) = make_float4(dw_acc[4], dw_acc[5], dw_acc[6], dw_acc[7]);
-    if (IS_LN && db_partial) {
-      float* pb = db_partial + static_cast<size_t>(blockIdx.x) * H + c * 8;
-      *reinterpret_cast<float4*>(pb) = make_float4(db_acc[0], db_acc[1], db_acc[2], db_acc[3]);
-      *reinterpret_cast<float4*>(pb + 4) = make_float4(db_acc[4], db_acc[5], db_acc[6], db_acc[7]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      if (c + i * lanes < nvec) {
+        const size_t at = static_cast<size_t>(blockIdx.x) * H + (c + i * lanes) * 8;
+        ulonglong2* pw = reinterpret_cast<ulonglong2*>(dw_partial + at);
+        pw[0] = make_ulonglong2(dw_acc[i].p[0], dw_acc[i].p[1]);
+        pw[1] = make_ulonglong2(dw_acc[i].p[2], dw_acc[i].p[3]);
+        if constexpr (IS_LN) {
+          if (db_partial) {
+            ulonglong2* pb = reinterpret_cast<ulonglong2*>(db_partial + at);
+            pb[0] = make_ulonglong2(db_acc[i].p[0], db_acc[i].p[1]);
+            pb[1] = make_ulonglong2(db_acc[i].p[2], db_acc[i].p[3]);
+          }
+        }
+      }
     }
   }
 }
@@ -386,16 +460,28 @@ static int norm_grid(int rows) {
   int g = sm_count() * 4;
   return rows < g ? rows : g;
 }
-// Threads of a block and blocks of a backward launch for rows of H elements: up to 256 elements a warp per row and eight rows
-// per block, above that one block of H / 8 threads (whole warps) per row; at most four blocks per SM, two above 512 threads.
-static void norm_shape(int rows, int H, int* threads, int* grid) {
+// Threads, vectors per thread and blocks of a backward launch for rows of H elements: up to 256 elements a warp per row and eight
+// rows per block, above that one block per row.
+// - Two vectors per thread above 2048 elements, two blocks of up to 320 threads per SM: with one vector, blocks of 512 threads at 64
+//   registers take 1.03 to 1.2 times as long (1000 x 4096 RMSNorm with residual 14.8 / 12.7 us, 8192 rows 55.1 / 53.1, LayerNorm
+//   65.0 / 60.4), at 640 to 1024 threads only one fits (16384 x 5120: 157 / 118).  Three blocks at 80 registers spill (8192 x 4096:
+//   61 us).  One vector with no more rows than SMs, where a row's latency counts (77 x 4096 LayerNorm: 7.5 / 8.0 us).
+// - Four blocks up to 1280 elements at up to 102 registers, three of those with a warp per row: at 64 LayerNorm spills (4096 x 768:
+//   15.3 / 13.3 us; 262144 x 128: 84 / 83 but 700 x 256 RMSNorm 4.9 / 5.0).
+struct NormBwdShape {
+  int threads, nv, blocks, grid;  // blocks per SM
+};
+static NormBwdShape norm_bwd_shape(int rows, int H) {
+  NormBwdShape r;
   const int nvec = H / 8;
-  const bool one_warp = nvec <= 32;
-  *threads = one_warp ? 256 : (nvec + 31) / 32 * 32;
-  const long units = one_warp ? (rows + 7) / 8 : rows;
-  long g = (long)sm_count() * (2048 / *threads < 4 ? 2048 / *threads : 4);
-  if (*threads > 512) g = sm_count() * 2;
-  *grid = (int)(units < g ? units : g);
+  r.nv = nvec > 512 || (nvec > 256 && rows > sm_count()) ? 2 : 1;
+  r.threads = nvec <= 32 ? 256 : ((nvec + r.nv - 1) / r.nv + 31) / 32 * 32;
+  const long units = nvec <= 32 ? (rows + 7) / 8 : rows;
+  r.blocks = r.threads > 320 && r.nv == 2 ? 1 : (r.nv == 2 || r.threads > 256 ? 2 : 4);
+  if (nvec <= 32) r.blocks = 3;
+  const long g = (long)sm_count() * r.blocks;
+  r.grid = (int)(units < g ? units : g);
+  return r;
 }
 
 // Number of fp32 rows the caller must provide in the dw/db partial buffers for a given row count.
@@ -457,20 +543,24 @@ CSB_API int csb_norm_bwd(int is_layernorm, const void* dy, const void* h, const 
                          float w_offset, void* stream) {
   if (H % 8 != 0 || H > NORM_MAX_H || rows <= 0) return CSB_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  int threads, grid;
-  norm_shape(rows, H, &threads, &grid);
+  const NormBwdShape shape = norm_bwd_shape(rows, H);
+  const int grid = shape.grid;
   auto DY = reinterpret_cast<const __nv_bfloat16*>(dy);
   auto Hh = reinterpret_cast<const __nv_bfloat16*>(h);
   auto W = reinterpret_cast<const __nv_bfloat16*>(w);
   auto DR = reinterpret_cast<const __nv_bfloat16*>(dres);
   auto DX = reinterpret_cast<__nv_bfloat16*>(dx);
-#define CSB_NORM_BWD(LN, OW) \
-  norm_bwd_kernel<LN, OW><<<grid, threads, 0, s>>>(DY, Hh, W, mean, rstd, DR, DX, dw_partial, db_partial, rows, H, w_offset)
-  if (is_layernorm) {
-    if (H <= 256) CSB_NORM_BWD(true, true); else CSB_NORM_BWD(true, false);
-  } else {
-    if (H <= 256) CSB_NORM_BWD(false, true); else CSB_NORM_BWD(false, false);
-  }
+#define CSB_NORM_BWD(LN, OW, NV, MT, MB)                                                                                     \
+  norm_bwd_kernel<LN, OW, NV, MT, MB><<<grid, shape.threads, 0, s>>>(DY, Hh, W, mean, rstd, DR, DX, dw_partial, db_partial, rows, H, w_offset)
+#define CSB_NORM_BWD_LN(OW, NV, MT, MB) \
+  if (is_layernorm) CSB_NORM_BWD(true, OW, NV, MT, MB); else CSB_NORM_BWD(false, OW, NV, MT, MB)
+  if (H <= 256) { CSB_NORM_BWD_LN(true, 1, 256, 3); }
+  else if (shape.nv == 1 && shape.threads <= 160) { CSB_NORM_BWD_LN(false, 1, 160, 4); }
+  else if (shape.nv == 1) { CSB_NORM_BWD_LN(false, 1, 512, 2); }
+  else if (shape.threads <= 256) { CSB_NORM_BWD_LN(false, 2, 256, 2); }
+  else if (shape.threads <= 320) { CSB_NORM_BWD_LN(false, 2, 320, 2); }
+  else { CSB_NORM_BWD_LN(false, 2, 512, 1); }
+#undef CSB_NORM_BWD_LN
 #undef CSB_NORM_BWD
   int r = launch_result();
   if (r) return r;
