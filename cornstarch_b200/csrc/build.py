@@ -3,8 +3,9 @@
 Every ``*.cu`` file in this directory is compiled with nvcc for ``sm_100a`` only and linked into
 ``cornstarch_b200/lib/libcornstarch_b200.so``.  The library exposes a plain C ABI (see the
 ``CSB_API`` functions) that :mod:`cornstarch_b200.ops._native` loads with ``ctypes``; no torch
-headers are involved, so a full rebuild takes well under a minute and works on a machine without a
-GPU (nvcc cross-compiles).
+headers are involved there.  ``host_ops.cpp`` (the host side of the hot calls, torch's C++ interface) becomes the Python module
+``cornstarch_b200/lib/_host_ops.so``.  A full rebuild takes about a minute and works on a machine without a GPU (nvcc
+cross-compiles).
 
 Run ``python -m cornstarch_b200.csrc.build`` (add ``--force`` to rebuild everything, ``-v`` for the
 ptxas resource report, ``--bounds-check`` for the debug library with index checks).
@@ -13,10 +14,12 @@ ptxas resource report, ``--bounds-check`` for the debug library with index check
 from __future__ import annotations
 
 import concurrent.futures as cf
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent
@@ -108,7 +111,30 @@ def build(force: bool = False, verbose: bool = False, bounds_check: bool = False
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    build_host_ops(force)
     return lib_path
+
+
+HOST_OPS_PATH = LIB_DIR / "_host_ops.so"
+
+
+def build_host_ops(force: bool = False) -> Path:
+    """The Python module of ``host_ops.cpp`` (torch's C++ interface around the library's entry points; no device code)."""
+    src = CSRC / "host_ops.cpp"
+    torch_dir = Path(importlib.util.find_spec("torch").submodule_search_locations[0])
+    newest = max(src.stat().st_mtime, (torch_dir / "version.py").stat().st_mtime)
+    if not force and HOST_OPS_PATH.exists() and HOST_OPS_PATH.stat().st_mtime >= newest:
+        return HOST_OPS_PATH
+    cuda = Path(_nvcc()).resolve().parent.parent
+    inc = [torch_dir / "include", torch_dir / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
+    tmp = HOST_OPS_PATH.with_suffix(".tmp.so")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *[f"-I{i}" for i in inc], str(src), "-o",
+           str(tmp), f"-L{torch_dir / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{torch_dir / 'lib'}"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed for {src.name}:\n{res.stdout}\n{res.stderr}")
+    os.replace(tmp, HOST_OPS_PATH)
+    return HOST_OPS_PATH
 
 
 if __name__ == "__main__":

@@ -98,8 +98,8 @@ class _CountingLib:
             else:
                 if KERNEL_TIMES:
                     def fn(*a, _t=target, _n=name):
-                        global launch_count
-                        launch_count += 1
+                        global _launches
+                        _launches += 1
                         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                         e0.record()
                         r = _t(*a)
@@ -108,15 +108,23 @@ class _CountingLib:
                         return r
                 else:
                     def fn(*a, _t=target):
-                        global launch_count
-                        launch_count += 1
+                        global _launches
+                        _launches += 1
                         return _t(*a)
             self._cache[name] = fn
             setattr(self, name, fn)  # later calls find it without coming back here
         return fn
 
 
-launch_count = 0
+_launches = 0  # through ctypes; nat.launch_count adds what host_ops launched
+
+
+def __getattr__(name):
+    if name == "launch_count":
+        return _launches + (_HOST.launches() if _HOST else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
 # CORNSTARCH_B200_KERNEL_TIMES=1: bracket every native call with a CUDA event pair on the launching stream and sum the
 # device time per entry point (kernel_times()); a few microseconds of host time per call, for in-situ breakdowns.
 KERNEL_TIMES = os.environ.get("CORNSTARCH_B200_KERNEL_TIMES", "0") == "1"
@@ -130,6 +138,35 @@ def kernel_times(reset: bool = True) -> dict:
     if reset:
         _TIMES.clear()
     return out
+
+
+_HOST = None  # the module; False where calls go through ctypes one by one
+_HOST_ENTRIES = ("csb_gemm_bf16", "csb_linear_bwd", "csb_colsum_parts", "csb_norm_fwd", "csb_norm_bwd", "csb_norm_bwd_parts", "csb_act_fwd",
+                 "csb_act_bwd", "csb_glu_fwd", "csb_glu_bwd", "csb_attn_fwd", "csb_attn_bwd", "csb_attn_bwd_splits")
+
+
+def host_ops():
+    """``csrc/host_ops.cpp``: checks, output allocation and launch of one operator on CUDA tensors in one native call (each answers
+    ``None`` for a form that it does not take).  ``None`` while every call is timed on its own (KERNEL_TIMES).  Like the library it
+    is mandatory on a machine with a GPU."""
+    global _HOST
+    if _HOST is None:
+        if KERNEL_TIMES:
+            _HOST = False
+        else:
+            import importlib.util
+
+            path = _LIB_PATH.parent / "_host_ops.so"
+            if not path.exists():
+                raise RuntimeError(f"{path} not found: run `python -m cornstarch_b200.csrc.build`")
+            spec = importlib.util.spec_from_file_location("_host_ops", path)
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+            raw = lib()._raw
+            mod.bind({n: C.cast(getattr(raw, n), vp).value for n in _HOST_ENTRIES},
+                     lambda index: status_word(torch.device("cuda", index)).data_ptr())
+            _HOST = mod
+    return _HOST or None
 
 
 def declare(name: str, argtypes: list) -> None:

@@ -240,11 +240,23 @@ def _mask_ptrs(mask: AttnMask, B: int | None = None):
     return _rows(mask.q_bits, B), _rows(mask.k_bits, B), _rows(mask.q_pos, B, True), _rows(mask.k_pos, B, True)
 
 
+def _mask_args(mask: AttnMask, B: int, Sq: int, Sk: int, device):
+    """Bits, positions and class map of a mask without dense parts, as the native calls take them."""
+    if mask.by_index() and mask.q_bits is None and mask.k_bits is None:
+        return None, None, None, None, None
+    return (*_mask_ptrs(mask, B), None if mask.by_index() else mask.classes(B, Sq, Sk, device))
+
+
 def attention_forward(q, k, v, mask: AttnMask, scale: float | None = None):
     """Native forward; returns ``(out [B,Sq,Hq,D] bf16, lse [B,Hq,Sq] fp32)``."""
     B, Sq, Hq, D = q.shape
     Sk, Hk = k.shape[1], k.shape[2]
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
+    host = nat.host_ops() if mask.dense is None and mask.bias is None and q.is_cuda else None
+    if host is not None:
+        got = host.attn_fwd(q, k, v, scale, mask.mode, *_mask_args(mask, B, Sq, Sk, q.device))
+        if got is not None:
+            return got
     for t, n in ((q, "q"), (k, "k"), (v, "v")):
         _check_layout(t, n)
     out = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device)
@@ -280,6 +292,12 @@ def attention_backward(do, q, k, v, out, lse, mask: AttnMask, scale: float | Non
     B, Sq, Hq, D = q.shape
     Sk, Hk = k.shape[1], k.shape[2]
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
+    host = nat.host_ops() if mask.dense is None and mask.bias is None and q.is_cuda else None
+    if host is not None:
+        dq_acc = torch.empty((B, Sq, Hq, D), dtype=torch.float32, device=q.device)
+        got = host.attn_bwd(do, q, k, v, out, lse, dq_acc, scale, mask.mode, *_mask_args(mask, B, Sq, Sk, q.device), dq, dk, dv)
+        if got is not None:
+            return got
     if do.stride(3) != 1 or do.stride(2) != D or do.stride(1) % 8:
         do = do.contiguous()
     dq = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device) if dq is None else dq

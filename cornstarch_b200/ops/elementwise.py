@@ -50,6 +50,14 @@ def _norm_ref(x, w, b, eps, is_ln, w_offset):
 class _NormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, res, w, b, eps, is_ln, w_offset):
+        host = nat.host_ops()
+        got = host.norm_fwd(x, res, w, b, eps, is_ln, w_offset) if host is not None else None
+        if got is not None:
+            y, h, hs, mean, rstd = got
+            ctx.save_for_backward(hs, w, mean, rstd)
+            ctx.is_ln, ctx.w_offset, ctx.shape, ctx.has_res, ctx.has_b = is_ln, w_offset, x.shape, res is not None, b is not None
+            ctx.w_ref, ctx.b_ref = w, b
+            return y, h
         H = x.shape[-1]
         x2 = x.reshape(-1, H)
         x2 = x2 if x2.is_contiguous() else x2.contiguous()
@@ -78,6 +86,14 @@ class _NormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, dh):
         hs, w, mean, rstd = ctx.saved_tensors
+        w_main = getattr(ctx.w_ref, "main_grad", None)
+        b_main = getattr(ctx.b_ref, "main_grad", None) if ctx.has_b else None
+        use_main = w_main is not None and (not ctx.has_b or b_main is not None)
+        host = nat.host_ops()
+        got = host.norm_bwd(dy, dh, hs, w, mean, rstd, ctx.is_ln, ctx.has_b, ctx.w_offset, w_main if use_main else None,
+                            b_main if use_main else None) if host is not None else None
+        if got is not None:
+            return _NormFn._results(ctx, *got, use_main)
         rows, H = hs.shape
         dy2 = dy.reshape(-1, H)
         dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
@@ -89,9 +105,6 @@ class _NormFn(torch.autograd.Function):
         parts = nat.lib().csb_norm_bwd_parts(rows)
         dw_part = torch.empty(parts * H, dtype=torch.float32, device=hs.device)
         db_part = torch.empty(parts * H, dtype=torch.float32, device=hs.device) if (ctx.is_ln and ctx.has_b) else None
-        w_main = getattr(ctx.w_ref, "main_grad", None)
-        b_main = getattr(ctx.b_ref, "main_grad", None) if ctx.has_b else None
-        use_main = w_main is not None and (not ctx.has_b or b_main is not None)
         if use_main:
             dw_out, db_out, acc = w_main, b_main, 1
         else:
@@ -105,6 +118,10 @@ class _NormFn(torch.autograd.Function):
                                    ctx.w_offset, nat.stream()),
             "csb_norm_bwd",
         )
+        return _NormFn._results(ctx, dx, dw_out, db_out, use_main)
+
+    @staticmethod
+    def _results(ctx, dx, dw_out, db_out, use_main):
         dx = dx.view(ctx.shape)
         if use_main:
             ctx.w_ref.grad_added_to_main_grad = True
@@ -237,6 +254,11 @@ def _act_ref(x, name):
 class _GluFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gu, act):
+        if (host := nat.host_ops()) is not None:
+            y, g2 = host.glu_fwd(gu, act)
+            ctx.save_for_backward(g2)
+            ctx.act, ctx.shape = act, gu.shape
+            return y
         I = gu.shape[-1] // 2
         g2 = gu.reshape(-1, 2 * I)
         g2 = g2 if g2.is_contiguous() else g2.contiguous()
@@ -249,6 +271,8 @@ class _GluFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         (g2,) = ctx.saved_tensors
+        if (host := nat.host_ops()) is not None:
+            return host.glu_bwd(g2, dy, ctx.act).view(ctx.shape), None
         I = g2.shape[1] // 2
         d2 = dy.reshape(-1, I)
         d2 = d2 if d2.is_contiguous() else d2.contiguous()
@@ -269,6 +293,11 @@ def glu(gate_up: torch.Tensor, act: str = "silu") -> torch.Tensor:
 class _ActFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, kind):
+        if (host := nat.host_ops()) is not None:
+            y, xc = host.act_fwd(x, kind)
+            ctx.save_for_backward(xc)
+            ctx.kind = kind
+            return y
         xc = x if x.is_contiguous() else x.contiguous()
         y = torch.empty_like(xc)
         nat.check(nat.lib().csb_act_fwd(xc.data_ptr(), y.data_ptr(), xc.numel(), kind, nat.stream()), "csb_act_fwd")
@@ -279,6 +308,8 @@ class _ActFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         (xc,) = ctx.saved_tensors
+        if (host := nat.host_ops()) is not None:
+            return host.act_bwd(xc, dy, ctx.kind), None
         d = dy if dy.is_contiguous() else dy.contiguous()
         dx = torch.empty_like(xc)
         nat.check(nat.lib().csb_act_bwd(xc.data_ptr(), d.data_ptr(), dx.data_ptr(), xc.numel(), ctx.kind, nat.stream()),

@@ -82,6 +82,11 @@ def gemm(
         return gemm_reference(a, b, a_mn_major, b_mn_major, bias, act, out, accumulate, out_dtype)
     if nat.LIBRARY_MODE:
         return gemm_library(a, b, a_mn_major, b_mn_major, bias, act, out, accumulate, out_dtype)
+    host = nat.host_ops()
+    if host is not None and out_dtype is None:
+        r = host.gemm(a, b, a_mn_major, b_mn_major, bias, ACT[act], out, accumulate, tile_n, max_ctas)
+        if r is not None:
+            return r
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "native GEMM is bf16 x bf16 -> fp32 accumulate"
     assert a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
     if a_mn_major:

@@ -33,6 +33,8 @@ def _use_native(x: torch.Tensor) -> bool:
 
 
 def _as_2d(x: torch.Tensor) -> torch.Tensor:
+    if x.is_cuda and (host := nat.host_ops()) is not None:
+        return host.as_2d(x)
     x2 = x.reshape(-1, x.shape[-1])
     if x2.stride(1) != 1 or (x2.stride(0) % 8) or (x2.data_ptr() % 16):
         x2 = x2.contiguous()
@@ -64,6 +66,8 @@ def colsum(x2: torch.Tensor, out: torch.Tensor | None = None, accumulate: bool =
 def fuse_adjacent(tensors: Sequence[torch.Tensor]) -> torch.Tensor | None:
     """If 2-D row-major tensors with equal width sit back to back in one storage, return the stacked view."""
     t0 = tensors[0]
+    if t0.is_cuda and (host := nat.host_ops()) is not None:
+        return host.fuse_adjacent(tensors)
     if any(t.dim() != 2 or not t.is_contiguous() or t.shape[1] != t0.shape[1] or t.dtype != t0.dtype for t in tensors):
         return None
     end = t0.data_ptr() + t0.numel() * t0.element_size()
@@ -132,8 +136,12 @@ def _native_backward(ctx, dy2, x2, weights, fused_w):
         db, ok = _fused_grads(biases, fuse_adjacent_1d)
         if not ok or (db is not None and (not db.is_contiguous() or db.numel() != N)):
             return None
-    dev, lib = dy2.device, nat.lib()
     acc_w, acc_b = int(dW is not None), int(db is not None)
+    host = nat.host_ops() if dy2.is_cuda else None
+    got = host.linear_bwd(dy2, x2, fused_w, ctx.needs_input_grad[0], dW, ctx.has_bias, db) if host is not None else None
+    if got is not None:
+        return _native_results(ctx, *got, weights, acc_w, acc_b)
+    dev, lib = dy2.device, nat.lib()
     if dW is None:
         dW = torch.empty((N, K), dtype=dy2.dtype, device=dev)
     if ctx.has_bias:
@@ -147,6 +155,12 @@ def _native_backward(ctx, dy2, x2, weights, fused_w):
                            acc_w, int(db is not None and db.dtype == torch.float32), acc_b, nat.status_word(dev).data_ptr(), nat.stream()),
         "csb_linear_bwd",
     )
+    return _native_results(ctx, dx, dW, db, weights, acc_w, acc_b)
+
+
+def _native_results(ctx, dx, dW, db, weights, acc_w, acc_b):
+    """What autograd is told: gradients that were added to buffers of their own count as such."""
+    n_w, biases = ctx.n_w, ctx.biases
     sizes = [w.shape[0] for w in weights]
     dws, dbs = [None] * n_w, [None] * n_w
     if acc_w:
@@ -170,8 +184,15 @@ class _LinearFn(torch.autograd.Function):
     def forward(ctx, x, n_w, act, tp, *params):
         weights = params[:n_w]
         biases = params[n_w:]
-        x2 = _as_2d(x)
         ctx.tp = tp
+        host = nat.host_ops() if tp is None and act is None and x.is_cuda else None
+        got = host.linear_fwd(x, weights, biases) if host is not None else None
+        if got is not None:
+            out, x2 = got
+            ctx.save_for_backward(x2, *weights)
+            ctx.n_w, ctx.has_bias, ctx.x_shape, ctx.biases = n_w, biases[0] is not None, x.shape, biases
+            return out
+        x2 = _as_2d(x)
         fused_w = fuse_adjacent(weights) if n_w > 1 else weights[0]
         has_bias = biases[0] is not None
         fused_b = (fuse_adjacent_1d(biases) if n_w > 1 else biases[0]) if has_bias else None

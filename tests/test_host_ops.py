@@ -1,0 +1,167 @@
+"""The native host path (``csrc/host_ops.cpp``) against the Python statement of the same operators: the same kernels with the same
+arguments, so the same bits, and every form that it does not take still goes where it went."""
+
+import pytest
+import torch
+
+from cornstarch_b200.ops import _native as nat
+from cornstarch_b200.ops import attention as A
+from cornstarch_b200.ops import elementwise as E
+from cornstarch_b200.ops import linear as L
+from cornstarch_b200.ops.gemm import gemm
+
+BF16 = torch.bfloat16
+
+
+def _both(monkeypatch, fn):
+    """Results of ``fn`` on the native host path and call by call, and how many launches each made."""
+    out = []
+    host = nat.host_ops()
+    assert host is not None
+    for h in (host, False):
+        monkeypatch.setattr(nat, "_HOST", h)
+        before = nat._launches + host.launches()
+        out.append((fn(), nat._launches + host.launches() - before))
+    monkeypatch.setattr(nat, "_HOST", host)
+    (a, na), (b, nb) = out
+    assert na == nb
+    return a, b
+
+
+def _same(a, b):
+    assert len(a) == len(b)
+    for x, y in zip(a, b):
+        assert (x is None) == (y is None)
+        if x is not None:
+            assert x.shape == y.shape and x.dtype == y.dtype and x.stride() == y.stride() and torch.equal(x, y)
+
+
+def _randn(*shape, seed=0):
+    return torch.randn(*shape, generator=torch.Generator(device="cuda").manual_seed(sum(shape) + seed), device="cuda").to(BF16)
+
+
+def _leaves(ts):
+    return [t if t is None else t.detach().requires_grad_() for t in ts]
+
+
+X_FORMS = {"plain": lambda: _randn(3, 13, 40), "one row": lambda: _randn(40), "slice": lambda: _randn(3, 13, 80)[..., 24:64],
+           "transposed": lambda: _randn(13, 3, 40).transpose(0, 1), "odd pitch": lambda: _randn(9, 44)[:, :40],
+           "off the grid": lambda: _randn(9 * 40 + 1)[1:].view(9, 40), "no rows": lambda: _randn(0, 40)}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", list(X_FORMS))
+@pytest.mark.parametrize("widths,adjacent", [((24,), True), ((24, 8, 16), True), ((24, 8, 16), False), ((12, 20), True)])
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("main", [None, BF16, torch.float32])
+def test_linear(form, widths, adjacent, bias, main, monkeypatch):
+    if form == "no rows" and bias:
+        pytest.skip("a column sum over no rows is refused on either path")
+    n = sum(widths)
+
+    def run():
+        x = X_FORMS[form]()
+        ws = torch.split(_randn(n, 40, seed=1), widths)
+        bs = torch.split(_randn(n, seed=2), widths) if bias else [None] * len(widths)
+        if not adjacent:
+            ws, bs = [w.clone() for w in ws], [b if b is None else b.clone() for b in bs]
+        x, ws, bs = _leaves([x])[0], _leaves(ws), _leaves(bs)
+        for t in [*ws, *bs]:
+            if t is not None and main is not None:
+                t.main_grad = torch.ones_like(t, dtype=main)
+        y = L.multi_linear(x, ws, bs)
+        y.backward(_randn(*y.shape, seed=3))
+        return [y.detach(), x.grad] + [t.main_grad if main is not None else t.grad for t in [*ws, *bs] if t is not None]
+
+    _same(*_both(monkeypatch, run))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("out", [None, "bf16", "fp32", "strided"])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
+def test_gemm(out, a_mn, b_mn, monkeypatch):
+    def run():
+        res = []
+        for M, N, K in ((33, 24, 40), (8, 16, 24), (5, 7, 9), (0, 8, 8), (8, 8, 0)):
+            a, b = _randn(*((K, M) if a_mn else (M, K))), _randn(*((K, N) if b_mn else (N, K)), seed=1)
+            o = {None: None, "bf16": torch.ones(M, N, device="cuda", dtype=BF16), "fp32": torch.ones(M, N, device="cuda"),
+                 "strided": torch.ones(M, N + 8, device="cuda")[:, :N]}[out]
+            res.append(gemm(a, b, a_mn, b_mn, out=o, accumulate=out is not None))
+        return res
+
+    _same(*_both(monkeypatch, run))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["plain", "one row", "slice", "transposed"])
+@pytest.mark.parametrize("kind", ["rms", "ln", "ln without bias"])
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("main", [None, BF16, torch.float32])
+def test_norms(form, kind, residual, main, monkeypatch):
+    def run():
+        x = X_FORMS[form]()
+        r = _randn(*x.shape, seed=1) if residual else None
+        w, b = _randn(40, seed=2), _randn(40, seed=3) if kind == "ln" else None
+        x, r, w, b = _leaves([x, r, w, b])
+        for t in (w, b):
+            if t is not None and main is not None:
+                t.main_grad = torch.ones_like(t, dtype=main)
+        y = E.rms_norm(x, w, 1e-5, r, 1.0) if kind == "rms" else E.layer_norm(x, w, b, 1e-5, r)
+        outs = list(y) if residual else [y]
+        torch.autograd.backward(outs, [_randn(*x.shape, seed=4 + i) for i in range(len(outs))])
+        return [o.detach() for o in outs] + [x.grad, r.grad if residual else None] + [
+            t.main_grad if main is not None else t.grad for t in (w, b) if t is not None]
+
+    _same(*_both(monkeypatch, run))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["plain", "slice", "transposed"])
+def test_activations(form, monkeypatch):
+    def run():
+        res = []
+        for f in (lambda t: E.activation(t, "gelu_pytorch_tanh"), lambda t: E.glu(t[..., :32], "silu")):
+            x = _leaves([X_FORMS[form]()])[0]
+            y = f(x)
+            y.backward(_randn(*y.shape, seed=1))
+            res += [y.detach(), x.grad]
+        return res
+
+    _same(*_both(monkeypatch, run))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["causal", "full", "bitfield", "shared bits", "positions", "dense"])
+@pytest.mark.parametrize("S", [60, 300])
+def test_attention(mode, S, monkeypatch):
+    bits = torch.full((2, S), (1 << 62) | 1, dtype=torch.int64, device="cuda")
+    bits[1, S - 7 :] = 0
+    pos = torch.arange(S, device="cuda")[None]
+
+    def run():
+        mask = {"causal": A.AttnMask.causal, "full": A.AttnMask.full, "bitfield": lambda: A.AttnMask.bitfield(bits),
+                "shared bits": lambda: A.AttnMask.bitfield(bits[1:]), "positions": lambda: A.AttnMask(mode=A.MASK_CAUSAL, q_pos=pos, k_pos=pos),
+                "dense": lambda: A.AttnMask.from_dense(torch.ones(2, S, S, dtype=torch.bool, device="cuda").tril())}[mode]()
+        qkv = _leaves([_randn(2, S, 8 * 64)])[0]
+        q, k, v = A.split_qkv(qkv, 4, 2, 64)
+        o = A.attention(q, k, v, mask)
+        o.backward(_randn(2, S, 64, 4, seed=1).transpose(2, 3))  # a gradient whose heads are not dense
+        return [o.detach(), qkv.grad]
+
+    (o, g), (ro, rg) = _both(monkeypatch, run)
+    assert torch.equal(o, ro) and torch.equal(g[..., 256:], rg[..., 256:])
+    # dQ is summed by reduce-adds in no fixed order: fp32 sums of the same terms, rounded to bf16 once
+    assert (g.double() - rg.double()).norm() <= 2.0**-9 * rg.double().norm()
+
+
+@pytest.mark.gpu
+def test_refused_layouts_are_refused(monkeypatch):
+    q = _randn(1, 20, 64, 4).transpose(2, 3)  # heads not dense
+    for host in (nat.host_ops(), False):
+        monkeypatch.setattr(nat, "_HOST", host)
+        with pytest.raises(AssertionError, match="dense heads"):
+            A.attention_forward(q, q, q, A.AttnMask.full())
+        with pytest.raises(AssertionError, match="contraction mismatch"):
+            gemm(_randn(8, 16), _randn(8, 24))
+        with pytest.raises(RuntimeError, match="csb_norm_fwd"):
+            E.rms_norm(_randn(0, 16), _randn(16))
