@@ -16,13 +16,20 @@
 // (csb_attn_bwd_splits, attn_dkv_reduce_kernel).  dQ^T tiles are staged in shared memory as [q][d] rows and added into an fp32
 // accumulator by TMA reduce-add (one 32 x 64 block per warp), then converted to bf16 by a final pass.
 //
-// Warp roles (512 threads): warp 0 = TMA producer (K/V once, Q/dO ring of 3 stages), warp 1 = MMA issuer, warps 2 and 3 =
-// query metadata, warps 4..7 = dQ^T drain, warps 8..15 = 256 compute threads.  Thread (r, group) owns KV row r (TMEM lane r)
-// and 32 of the 64 query columns of S^T / dP^T; a drain thread moves head-dim row r of dQ^T.  The pipeline keeps S^T one
-// iteration ahead: while the compute warps turn S^T(i), dP^T(i) into P^T, dS^T, the tensor core
-// already holds S^T(i+1); dP^T(i+1) is issued as soon as dP^T(i) has been read, before the
-// dV/dK/dQ^T MMAs of iteration i, so the next exponentials overlap those MMAs.  Per-tile query
-// metadata (LSE, delta, mask rules) is staged in shared memory by two warps of its own, a ring stage with Q / dO.
+// Warp roles (512 threads): warp 0 = MMA issuer of S^T and dP^T, warp 1 = of dV, dK and dQ^T, warps 2 and 3 = query metadata (and
+// TMA: K/V once, Q/dO ring of 3 stages), warps 4..7 = dQ^T drain, warps 8..15 = 256 compute threads.  Thread (r, group) owns KV
+// row r (TMEM lane r) and 32 of the 64 query columns of S^T / dP^T; a drain thread moves head-dim row r of dQ^T.  The pipeline keeps
+// S^T one iteration ahead: while the compute warps turn S^T(i), dP^T(i) into P^T, dS^T, the tensor core already holds S^T(i+1);
+// dP^T(i+1) is issued as soon as dP^T(i) has been read, so the next exponentials overlap the dV/dK/dQ^T MMAs of iteration i.
+// Per-tile query metadata (LSE, delta, mask rules) is staged in shared memory, a ring stage with Q / dO.
+//
+// What bounds it: shared memory.  The MMAs of an iteration read 192 KB of operands and everything else moves about 130 KB (Q / dO in,
+// dS^T, dQ through its staging, statistics): 2500 of the measured 2450 cycles at 128 B / cycle; the tensor pipe is busy 1676.  Long
+// runs are at the power cap.  Before, the one MMA warp was: 32 MMAs per iteration at 90 cycles of issue each, 3300 cycles; runs of
+// MMAs (umma_f16_run_w) and a second MMA warp, which has work for the pipe while the first waits, took that away.  (dQ^T straight from
+// registers by red.global, which spares its two passes through shared memory, takes 65 cycles per warp instruction: 2.0 x the time.)
+// Measured with the delta and conversion passes (32 / 8 heads of 128, before -> now): 8192 tokens causal 1679 -> 1411 us (975
+// TFLOP/s), full 3190 -> 2632 (1044 TFLOP/s), 4096 causal 476 -> 386, 1024 69 -> 62; 4 x 729 tokens, 16 heads of 72, 88 -> 78.
 //
 // Replaces cornstarch/kernel/bitfield_attention.py:526-929 (T8, T9: fp32 atomics for dQ, dK and dV)
 // and cornstarch/kernel/attention.py:348-852.
@@ -95,14 +102,14 @@ struct BwdSmem {
   static constexpr int LIST_OFF = META_OFF + QSTAGES * META_STAGE;  // valid 64-row query tiles of this key block: int16 index, int8 class
   static constexpr int MAX_TILES = 1024;                      // sequences up to 65536 tokens
   static constexpr int BAR_OFF = LIST_OFF + MAX_TILES * 4;
-  static constexpr int NBAR = 1 + QSTAGES + QSTAGES + 1 + 1 + 1 + 1 + 1 + 1;
+  static constexpr int NBAR = 1 + QSTAGES + QSTAGES + 5;
   static constexpr int TOTAL = BAR_OFF + NBAR * 8 + 32;
   static constexpr int DYN_BYTES = TOTAL + 1024;
 };
 
-// Eight compute warps: two share a TMEM lane quarter and split the 64 query columns between them.  Their loop is a chain
-// of hand-overs with the MMA warp (issue slots are 28 % used), and what does not depend on the number of columns (waits,
-// addresses, arrivals of every thread) is on it once per warp of a scheduler: sixteen warps of 16 columns took 1903 us where eight of 32 take 1816 (8192 tokens causal, 32 / 8 heads of 128; full mask 3769 / 3510).
+// Eight compute warps: two share a TMEM lane quarter and split the 64 query columns between them.  What does not depend on the
+// number of columns (waits, addresses, arrivals of every thread) is on their chain once per warp of a scheduler: sixteen warps of 16
+// columns took 1903 us where eight of 32 took 1816 (8192 tokens causal, with the MMA warp as the limit).
 struct BwdCfg {
   static constexpr int COMPUTE_THREADS = 8 * 32;
   static constexpr int DRAIN_THREADS = 128;  // four warps that only move dQ^T out (one per TMEM lane quarter)
@@ -112,6 +119,7 @@ struct BwdCfg {
 };
 
 __device__ __forceinline__ bool bw_wait(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
+  if (mbar_try_wait(bar, phase)) return true;  // in front of the loop and its set-up
   uint64_t t0 = 0;
   for (uint32_t i = 0; i < CSB_SPIN_LIMIT; ++i) {
     if (mbar_try_wait(bar, phase)) return true;
@@ -229,11 +237,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint64_t* kv_full = bars;
   uint64_t* q_full = bars + 1;            // [QS]  Q + dO stage landed
-  uint64_t* q_empty = q_full + QS;        // [QS]  stage consumed by the dV/dK MMAs
+  uint64_t* q_empty = q_full + QS;        // [QS]  stage consumed by the dV/dK MMAs (and P^T by dV)
   uint64_t* sdp_full = q_empty + QS;      //       S^T and dP^T of an iteration ready in TMEM
-  uint64_t* pds_full = sdp_full + 1;      //       P^T and dS^T tiles written to smem (256 arrivals)
-  uint64_t* pds_empty = pds_full + 1;     //       ... and consumed by the MMAs
-  uint64_t* dq_full = pds_empty + 1;      //       dQ^T ready in TMEM
+  uint64_t* pds_full = sdp_full + 1;      //       P^T and dS^T tiles written (256 arrivals)
+  uint64_t* dq_full = pds_full + 1;       //       dQ^T ready in TMEM, P^T and dS^T consumed: the iteration's last MMAs have retired
   uint64_t* dq_free = dq_full + 1;        //       dQ^T drained (128 arrivals)
   uint64_t* dp_read = dq_free + 1;      //       S^T and dP^T of an iteration are in registers (256 arrivals): dP^T may be overwritten
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBAR);
@@ -266,7 +273,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     mbar_init(sdp_full, 1);
     mbar_init(pds_full, CFG::COMPUTE_THREADS);
-    mbar_init(pds_empty, 1);
     mbar_init(dq_full, 1);
     mbar_init(dq_free, CFG::DRAIN_THREADS);
     mbar_init(dp_read, CFG::COMPUTE_THREADS);
@@ -322,153 +328,142 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tmem_dV = tmem_base + 256;
   const uint32_t tmem_dK = tmem_base + 384;
 
+  // The MMAs come from two warps, so that the pipe has work of one while the other waits for a hand-over: warp 0 issues S^T and dP^T,
+  // warp 1 dV, dK and dQ^T.  Whole warps walk this code in step (every lane waits on the barriers; one elected lane issues each run of
+  // MMAs and its commit).
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // ------------------------------------------------------------------ S^T and dP^T
+    const uint32_t idesc_s = make_idesc_bf16(128, BW_BQ, 0, 0);
+    const uint64_t k_km = make_desc_kmajor_sw128(smem_u32(smem + L::K_OFF));
+    const uint64_t v_km = make_desc_kmajor_sw128(smem_u32(smem + L::V_OFF));
+    const uint64_t q_km = make_desc_kmajor_sw128(smem_u32(smem + L::Q_OFF));
+    const uint64_t do_km = make_desc_kmajor_sw128(smem_u32(smem + L::DO_OFF));
+    constexpr uint64_t STAGE = (2 * Q_CHUNK) >> 4;
+    const int ksteps_d = p.dk16 / 16;
+    bool ok = n_iter == 0 || bw_wait(kv_full, 0, abort_flag);
+    if (!ok) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; }
+    int s_stage = 0, d_stage = 0;  // ring stages of the next S^T and dP^T
+    uint32_t s_phase = 0;
+    auto issue_st = [&](int it) -> bool {  // into ST[it & 1]; waits for the Q / dO stage of that iteration
+      if (!bw_wait(&q_full[s_stage], s_phase, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; return false; }
+      tc_fence_after();
+      umma_f16_run_w(tmem_base + (it & 1) * 64, k_km, q_km + s_stage * STAGE, KV_CHUNK, Q_CHUNK, idesc_s, ksteps_d, 0u);
+      if (++s_stage == QS) { s_stage = 0; s_phase ^= 1u; }
+      return true;
+    };
+    auto issue_dpt = [&]() {  // its commit also covers S^T of the iteration, issued earlier
+      umma_f16_run_w(tmem_dPT, v_km, do_km + d_stage * STAGE, KV_CHUNK, Q_CHUNK, idesc_s, ksteps_d, 0u);
+      umma_commit_w(sdp_full);
+      if (++d_stage == QS) d_stage = 0;
+    };
+    if (ok && n_iter > 0) {
+      ok = issue_st(0);
+      if (ok) issue_dpt();
+      if (ok && n_iter > 1) ok = issue_st(1);
+    }
+    int e_stage = 0;  // iteration it's stage and phase
+    uint32_t e_phase = 0;
+    for (int it = 0; ok && it + 1 < n_iter; ++it) {
+      // dP^T(it + 1) as soon as the compute warps hold dP^T(it) in registers, long before they are done with the iteration
+      if (!bw_wait(dp_read, it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; break; }
+      tc_fence_after();
+      issue_dpt();
+      if (it + 2 < n_iter) {
+        // S^T(it + 2) goes over P^T(it): dV(it) has to have retired, which is what releases the stage of iteration it
+        if (!bw_wait(&q_empty[e_stage], e_phase, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
+        if (++e_stage == QS) { e_stage = 0; e_phase ^= 1u; }
+        ok = issue_st(it + 2);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ dV, dK and dQ^T
+    const uint32_t idesc_dkv = make_idesc_bf16(128, p.dk16, 0, 1);
+    const uint32_t idesc_dq = make_idesc_bf16(128, BW_BQ, 1, 1);
+    const uint64_t k_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::K_OFF), KV_CHUNK);
+    const uint64_t q_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::Q_OFF), Q_CHUNK);
+    const uint64_t do_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::DO_OFF), Q_CHUNK);
+    const uint64_t dst_km = make_desc_kmajor_sw128(smem_u32(smem + L::DST_OFF));
+    const uint64_t dst_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::DST_OFF), KV_CHUNK);
+    constexpr uint64_t STAGE = (2 * Q_CHUNK) >> 4;
+    int st = 0;
+    uint32_t st_phase = 0;
+    bool ok = n_iter == 0 || bw_wait(kv_full, 0, abort_flag);
+    if (!ok) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; }
+    for (int it = 0; ok && it < n_iter; ++it) {
+      // (the stage is full long before; the wait orders this warp's MMAs behind the copies)
+      if (!bw_wait(&q_full[st], st_phase, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; break; }
+      if (!bw_wait(pds_full, it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; break; }
+      tc_fence_after();
+      // dV += P^T dO ; dK += dS^T Q   (contraction over the 64 query rows)
+      const uint32_t acc = it > 0 ? 1u : 0u;
+      umma_f16_ts_run4_w<COLS>(tmem_dV, tmem_base + (it & 1) * 64, do_mn + st * STAGE, idesc_dkv, acc);
+      umma_f16_run4_w<2, 128>(tmem_dK, dst_km, q_mn + st * STAGE, idesc_dkv, acc);  // 16 columns of dS^T, 16 rows of Q a step
+      umma_commit_w(&q_empty[st]);
+      if (it > 0) {
+        if (!bw_wait(dq_free, (it - 1) & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_EMPTY); *abort_flag = 1; break; }
+        tc_fence_after();
+      }
+      // dQ^T = K^T dS^T  (contraction over the 128 key rows)
+      umma_f16_run8_w<128, 128>(tmem_dQT, k_mn, dst_mn, idesc_dq, 0u);  // 16 rows of K and of dS^T a step
+      umma_commit_w(dq_full);
+      if (++st == QS) { st = 0; st_phase ^= 1u; }
+    }
+    __syncwarp();
+  } else if (warp < 4) {
+    // ------------------------------------------------------------------ TMA producer and query metadata (warps 2 and 3)
+    // Statistics and mask rules of the stage's 64 query rows, one row a thread and one ring stage with its Q / dO tiles, which lane 0
+    // of warp 2 loads.  (When two of the compute warps loaded them on the side, every iteration waited for their global loads: 1400 of
+    // its 3700 cycles.)
+    const float LOG2E = 1.4426950408889634f;
+    const int r = (warp - 2) * 32 + lane;
+    const bool producer = warp == 2 && lane == 0;
+    if (producer) {
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_do);
-      const bool peer_ok = peer_ready;
-      if (peer_ok && n_iter > 0) {  // a block without iterations only writes zeros
+      if (n_iter > 0) {  // (a block without iterations only writes zeros)
         mbar_expect_tx(kv_full, 4 * KV_CHUNK);
         for (int c = 0; c < 2; ++c) {
           tma_load_4d(smem + L::K_OFF + c * KV_CHUNK, &kvm.k[sg], kv_full, c * 64, hk, row0, b);
           tma_load_4d(smem + L::V_OFF + c * KV_CHUNK, &kvm.v[sg], kv_full, c * 64, hk, row0, b);
         }
       }
-      BwdCursor cur(it0, n_valid);
-      for (int it = 0; peer_ok && it < n_iter; ++it, cur.next()) {
-        const int h = hk * group + cur.h;
-        const int i = tile_idx[cur.t];
-        const int st = it % QS;
-        if (!bw_wait(&q_empty[st], ((it / QS) & 1) ^ 1, abort_flag)) {
-          atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY);
-          *abort_flag = 1;
-          break;
-        }
-        mbar_expect_tx(&q_full[st], 4 * Q_CHUNK);
-        for (int c = 0; c < 2; ++c) {
-          tma_load_4d(smem + L::Q_OFF + (st * 2 + c) * Q_CHUNK, &tm_q, &q_full[st], c * 64, h, i * BW_BQ, b);
-          tma_load_4d(smem + L::DO_OFF + (st * 2 + c) * Q_CHUNK, &tm_do, &q_full[st], c * 64, h, i * BW_BQ, b);
-        }
-      }
     }
-    __syncwarp();
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    // The whole warp walks this code in step (every lane waits on the barriers; one elected lane issues each MMA and
-    // commit): see umma_f16_w.  A 16-wide slice of a tile is the tile's descriptor plus the slice's byte offset / 16.
-    {
-      const uint32_t idesc_s = make_idesc_bf16(128, BW_BQ, 0, 0);
-      const uint32_t idesc_dkv = make_idesc_bf16(128, p.dk16, 0, 1);
-      const uint32_t idesc_dq = make_idesc_bf16(128, BW_BQ, 1, 1);
-      const uint64_t k_km = make_desc_kmajor_sw128(smem_u32(smem + L::K_OFF));
-      const uint64_t v_km = make_desc_kmajor_sw128(smem_u32(smem + L::V_OFF));
-      const uint64_t k_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::K_OFF), KV_CHUNK);
-      const uint64_t dst_km = make_desc_kmajor_sw128(smem_u32(smem + L::DST_OFF));
-      const uint64_t dst_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::DST_OFF), KV_CHUNK);
-      // steps of the contractions over D: their loops are unrolled to the maximum and cut by a uniform test
-      const int ksteps_d = p.dk16 / 16;
-      bool ok = n_iter == 0 || bw_wait(kv_full, 0, abort_flag);
-      if (!ok) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; }
-      auto kslice = [](int kk, int chunk_bytes) -> uint64_t {
-        return static_cast<uint64_t>(((kk >> 2) * chunk_bytes + (kk & 3) * 32) >> 4);
-      };
-
-      // S^T(it) = K Q^T into ST[it & 1]; waits for the Q/dO stage of that iteration
-      auto issue_st = [&](int it) -> bool {
-        const int st = it % QS;
-        if (!bw_wait(&q_full[st], (it / QS) & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; return false; }
-        tc_fence_after();
-        const uint64_t q_km = make_desc_kmajor_sw128(smem_u32(smem + L::Q_OFF + st * 2 * Q_CHUNK));
-        const uint32_t t_st = tmem_base + (it & 1) * 64;
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          if (kk < ksteps_d) umma_f16_w(t_st, k_km + kslice(kk, KV_CHUNK), q_km + kslice(kk, Q_CHUNK), idesc_s, kk > 0);
-        return true;
-      };
-      // dP^T(it) = V dO^T; its commit also covers S^T(it), issued earlier
-      auto issue_dpt = [&](int it) {
-        const int st = it % QS;
-        const uint64_t do_km = make_desc_kmajor_sw128(smem_u32(smem + L::DO_OFF + st * 2 * Q_CHUNK));
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          if (kk < ksteps_d) umma_f16_w(tmem_dPT, v_km + kslice(kk, KV_CHUNK), do_km + kslice(kk, Q_CHUNK), idesc_s, kk > 0);
-        umma_commit_w(sdp_full);
-      };
-
-      if (ok && n_iter > 0) {
-        ok = issue_st(0);
-        if (ok) issue_dpt(0);
-        if (ok && n_iter > 1) ok = issue_st(1);
-      }
-      for (int it = 0; ok && it < n_iter; ++it) {
-        const int st = it % QS;
-        // dP^T(it+1) is issued as soon as the compute warps hold dP^T(it) in registers, long before they are done with
-        // the iteration: S^T(it+1) and dP^T(it+1) are then ready when they come back for the next one
-        if (it + 1 < n_iter) {
-          if (!bw_wait(dp_read, it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; break; }
-          tc_fence_after();
-          issue_dpt(it + 1);
-        }
-        if (!bw_wait(pds_full, it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; break; }
-        tc_fence_after();
-        const uint64_t q_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::Q_OFF + st * 2 * Q_CHUNK), Q_CHUNK);
-        const uint64_t do_mn = make_desc_mnmajor_sw128(smem_u32(smem + L::DO_OFF + st * 2 * Q_CHUNK), Q_CHUNK);
-        // dV += P^T dO ; dK += dS^T Q   (contraction over the 64 query rows)
-#pragma unroll
-        for (int kk = 0; kk < BW_BQ / 16; ++kk)
-          umma_f16_ts_w(tmem_dV, tmem_base + (it & 1) * 64 + (kk / (COLS / 16)) * COLS + (kk % (COLS / 16)) * 8,
-                        do_mn + static_cast<uint64_t>((kk * 2048) >> 4), idesc_dkv, (it > 0 || kk > 0) ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < BW_BQ / 16; ++kk)
-          umma_f16_w(tmem_dK, dst_km + static_cast<uint64_t>((kk * 32) >> 4), q_mn + static_cast<uint64_t>((kk * 2048) >> 4),
-                     idesc_dkv, (it > 0 || kk > 0) ? 1u : 0u);
-        umma_commit_w(&q_empty[st]);
-        if (it > 0) {
-          if (!bw_wait(dq_free, (it - 1) & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_EMPTY); *abort_flag = 1; break; }
-          tc_fence_after();
-        }
-        // dQ^T = K^T dS^T  (contraction over the 128 key rows)
-#pragma unroll
-        for (int kk = 0; kk < BW_BKV / 16; ++kk)
-          umma_f16_w(tmem_dQT, k_mn + static_cast<uint64_t>((kk * 2048) >> 4), dst_mn + static_cast<uint64_t>((kk * 2048) >> 4),
-                     idesc_dq, kk > 0 ? 1u : 0u);
-        umma_commit_w(pds_empty);
-        umma_commit_w(dq_full);
-        if (it + 2 < n_iter) ok = issue_st(it + 2);  // ST[it & 1] was read before pds_full(it)
-      }
-    }
-    __syncwarp();
-  } else if (warp < 4) {
-    // ------------------------------------------------------------------ query metadata (warps 2 and 3, one query row each)
-    // Statistics and mask rules of the stage's 64 query rows, one ring stage with its Q / dO tiles.  (When two of the compute
-    // warps loaded them on the side, every iteration waited for their global loads: 1400 of its 3700 cycles.)
-    const float LOG2E = 1.4426950408889634f;
-    const int r = (warp - 2) * 32 + lane;
     BwdCursor cur(it0, n_valid);
+    int st = 0;
+    uint32_t st_phase = 1;
     for (int it = 0; it < n_iter; ++it, cur.next()) {
-      const int st = it % QS;
       const int h = hk * group + cur.h;
-      const int q = tile_idx[cur.t] * BW_BQ + r;
+      const int qt = tile_idx[cur.t];
+      const int q = qt * BW_BQ + r;
       const bool qv = q < p.Sq;
       const long idx = ((long)b * p.Hq + h) * p.Sq + q;
-      const float lse = qv ? -(p.lse[idx] * LOG2E) : -INFINITY;  // both negated: their uses are one packed FMA each
-      const float delta = qv ? -(p.delta[idx] * p.scale) : 0.f;
+      const float lse = qv ? p.lse[idx] : INFINITY;
+      const float delta = qv ? p.delta[idx] : 0.f;
       const int qpos = qv ? (p.q_pos ? p.q_pos[(long)b * p.Sq + q] : q) : 0;
       const int64_t qbits = (qv && p.q_bits) ? p.q_bits[(long)b * p.Sq + q] : 0;
-      const QueryRule rule = make_query_rule(p.mask_mode, qv && qpos >= 0, qbits, qpos);
-      if (!bw_wait(&q_empty[st], ((it / QS) & 1) ^ 1, abort_flag)) {
+      if (!bw_wait(&q_empty[st], st_phase, abort_flag)) {
         if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY);
         *abort_flag = 1;
         break;
       }
+      if (producer) {
+        mbar_expect_tx(&q_full[st], 4 * Q_CHUNK);
+        for (int c = 0; c < 2; ++c) {
+          tma_load_4d(smem + L::Q_OFF + (st * 2 + c) * Q_CHUNK, &tm_q, &q_full[st], c * 64, h, qt * BW_BQ, b);
+          tma_load_4d(smem + L::DO_OFF + (st * 2 + c) * Q_CHUNK, &tm_do, &q_full[st], c * 64, h, qt * BW_BQ, b);
+        }
+      }
+      __syncwarp();
+      const QueryRule rule = make_query_rule(p.mask_mode, qv && qpos >= 0, qbits, qpos);
       float* m = reinterpret_cast<float*>(smem + L::META_OFF + st * L::META_STAGE);
-      m[r] = lse;
-      m[64 + r] = delta;
+      m[r] = -(lse * LOG2E);  // both negated: their uses are one packed FMA each
+      m[64 + r] = -(delta * p.scale);
       reinterpret_cast<int*>(m + 128)[r] = rule.lim;
       reinterpret_cast<int64_t*>(m + 192)[r] = rule.am;
       reinterpret_cast<int64_t*>(m + 320)[r] = rule.qe;
       mbar_arrive(&q_full[st]);
+      if (++st == QS) { st = 0; st_phase ^= 1u; }
     }
   } else if (warp >= 8) {
     // ------------------------------------------------------------------ compute threads (8 warps)
@@ -490,14 +485,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // sdp_full(it) covers them too.
     BwdCursor cur(it0, n_valid);
     int stage = 0;  // it % QS
-    for (int it = 0; it < n_iter && ok; ++it, cur.next(), stage = stage + 1 == QS ? 0 : stage + 1) {
-      const int c = tile_cls[cur.t];
+    int c_next = n_iter > 0 ? tile_cls[cur.t] : 0, qt_next = n_iter > 0 ? tile_idx[cur.t] : 0;
+    for (int it = 0; it < n_iter && ok; ++it, stage = stage + 1 == QS ? 0 : stage + 1) {
+      const int c = c_next, qt = qt_next;
+      const int head = cur.h;
+      cur.next();  // (of the tile after the last one nothing is used)
+      c_next = tile_cls[cur.t];
+      qt_next = tile_idx[cur.t];
       float* m_lse = reinterpret_cast<float*>(smem + L::META_OFF + stage * L::META_STAGE);
       float* m_delta = m_lse + 64;
       const int* m_lim = reinterpret_cast<const int*>(m_lse + 128);
       const int64_t* m_am = reinterpret_cast<const int64_t*>(m_lse + 192);
       const int64_t* m_qe = reinterpret_cast<const int64_t*>(m_lse + 320);
-      const int q_base = tile_idx[cur.t] * BW_BQ + col0;  // first query row of this thread's columns
+      const int q_base = qt * BW_BQ + col0;  // first query row of this thread's columns
       // Mask bytes and biases of this thread's pairs, all loaded before the wait for the scores: rows that do not exist are
       // clamped, not branched around, so that the loads of the COLS columns are in flight together.
       uint32_t mask_word = 0xffffffffu;
@@ -515,7 +515,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
         if (p.bias != nullptr) {
-          const float* v = p.bias + (long)b * p.bias_sb + (long)(hk * group + cur.h) * p.bias_sh + q_first * p.bias_sq + k_at;
+          const float* v = p.bias + (long)b * p.bias_sb + (long)(hk * group + head) * p.bias_sh + q_first * p.bias_sq + k_at;
 #pragma unroll
           for (int x = 0; x < COLS; ++x) {
             bias_v[x] = __ldg(v);
@@ -579,6 +579,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
       }
+      // P^T -> packed bf16 pairs in tensor memory, over this thread's own S^T columns (the first half of them)
+      {
+        uint32_t pk[COLS / 2];
+#pragma unroll
+        for (int x = 0; x < COLS / 2; ++x) pk[x] = pack_bf16x2(pv[2 * x], pv[2 * x + 1]);
+        tmem_st_32x16(tmem_base + (it & 1) * 64 + col0 + lane_addr, pk);
+      }
 #pragma unroll
       for (int x4 = 0; x4 < COLS / 4; ++x4) {
         const float4 d4 = *reinterpret_cast<const float4*>(m_delta + col0 + x4 * 4);
@@ -588,21 +595,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         unpack_f32x2(mul_f32x2(pack_f32x2(pv[x4 * 4 + 2], pv[x4 * 4 + 3]), t1), ds[x4 * 4 + 2], ds[x4 * 4 + 3]);
       }
       if (it > 0) {
-        if (!bw_wait(pds_empty, (it - 1) & 1, abort_flag)) {
+        if (!bw_wait(dq_full, (it - 1) & 1, abort_flag)) {
           if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_MISC);
           *abort_flag = 1;
           ok = false;
           break;
         }
       }
-      // P^T -> packed bf16 pairs in tensor memory, over this thread's own S^T columns (the first half of them);
       // dS^T -> bf16 smem tile: row r, this warp's 16-byte pieces (8 query columns each)
-      {
-        uint32_t pk[COLS / 2];
-#pragma unroll
-        for (int x = 0; x < COLS / 2; ++x) pk[x] = pack_bf16x2(pv[2 * x], pv[2 * x + 1]);
-        tmem_st_32x16(tmem_base + (it & 1) * 64 + col0 + lane_addr, pk);
-      }
 #pragma unroll
       for (int pc = 0; pc < COLS / 8; ++pc) {
         uint4 w;
@@ -619,7 +619,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     // ---- epilogue: dV and dK tiles (every MMA has retired once the last dS^T was consumed); the warps of a lane quarter split
     //      the head-dim columns
-    if (ok && n_iter > 0 && !bw_wait(pds_empty, (n_iter - 1) & 1, abort_flag)) {
+    if (ok && n_iter > 0 && !bw_wait(dq_full, (n_iter - 1) & 1, abort_flag)) {
       if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_MISC);
       *abort_flag = 1;
       ok = false;
@@ -910,21 +910,21 @@ CSB_API int csb_attn_bwd_dense(const void* q, const void* k, const void* v, cons
 // one thread block that walks all query heads of its group: 64 blocks for 1024 tokens and 8 KV heads on 148 SMs, and under a
 // causal mask the longest block alone decides.  Each further block costs its set-up and epilogue again and the parts are written
 // and read once more.  The count with the smallest predicted time is taken: whole rounds of equal blocks under a full mask, the
-// longest block or the average load of the SMs otherwise.  The constants are rounded up from grids of a single round: 32 / 8
-// heads of 128, causal, 333 tokens (24 iterations) 55 us, 512 (32) 69 us, 1024 (64) 126 us, and 1500 tokens with 8 / 1 heads
-// (192) 351 us, delta and conversion passes included, are 1.75 us an iteration.
-// One block is kept unless another count is predicted at least 7 % faster (the prediction is no better than that: 4096 tokens
-// causal, 3 % predicted for two blocks, took 490 against 478 us), and the parts may take CSB_ATTN_BWD_PART_BYTES at most: long
-// sequences fill the GPU without a split, and must not need gigabytes for the last per cents.
-// Measured, one block against the count taken: 256 tokens causal, 32 / 8 heads: 41 / 26 us (6 blocks); 1024: 126 / 70 (4); 2048:
-// 246 / 154 (2); 1500 tokens, 8 / 1 heads: 351 / 50 (16); full mask, 3072 tokens: 688 / 520 (3), 8192: 3593 / 3176 (2, 128 MiB).
-// Kept whole: 729 tokens, 16 / 16 heads, full: 33 us, 45 with three blocks; 2 x 900 tokens, 8 / 8 heads: 40, 60 with two.  The
-// furthest from the best count found: 512 tokens causal, 44 us with the 6 blocks taken, 37 with 4; 6144 tokens, full: 2007 us
-// whole, 1898 with three blocks of 151 MB of parts.
+// longest block or the average load of the SMs otherwise.  An iteration takes 1.25 to 1.35 us on grids of a single round; the
+// constant is larger because more blocks also mean more blocks per SM and more parts.
+// One block is kept unless another count is predicted at least 7 % faster (the prediction is no better than that), and the parts
+// may take CSB_ATTN_BWD_PART_BYTES at most: long sequences fill the GPU without a split, and must not need gigabytes for the last
+// per cents.
+// Measured, delta and conversion passes included, one block against the count taken (32 / 8 heads, causal): 256 tokens 34.5 / 24.3 us
+// (6 blocks); 333: 45.2 / 28.5 (6); 1024: 99.9 / 61.8 (4); 2048: 191 / 131 (2); 1500 tokens, 8 / 1 heads: 251 / 46.4 (16); full
+// mask, 3072 tokens: 529 / 424 (3), 8192: 2828 / 2630 (2, 128 MiB).  Kept whole: 729 tokens, 16 / 16 heads, full: 33.5 us, 45 with
+// three blocks; 2 x 900 tokens, 8 / 8 heads: 37, 56 with two; 4096 tokens causal: 390, 410 with two.  The furthest from the best
+// count found: 512 tokens causal, 41.1 us with the 6 blocks taken, 33.5 with 4; 1024: 61.8, 58.1 with 3; 6144 tokens, full: 1611 us
+// whole, 1552 with three blocks of 151 MB of parts.
 constexpr long CSB_ATTN_BWD_PART_BYTES = 128L << 20;
 CSB_API int csb_attn_bwd_splits(int mask_mode, int B, int Sq, int Sk, int Hq, int Hk) {
   if (B < 1 || Sq < 1 || Sk < 1 || Hk < 1 || Hq < Hk) return 1;
-  const float setup_us = 8.f, tile_us = 1.9f;
+  const float setup_us = 8.f, tile_us = 1.6f;
   const int sms = sm_count();
   const long blocks = (long)((Sk + BW_BKV - 1) / BW_BKV) * Hk * B;
   const long iters = (long)((Sq + BW_BQ - 1) / BW_BQ) * (Hq / Hk);  // of the longest block

@@ -322,8 +322,40 @@ __device__ __forceinline__ void umma_f16_run_w(uint32_t d_tmem, uint64_t a_desc,
       : "memory");
 #undef CSB_UMMA_STEP
 }
-// D (+)= A B with A = 64 columns (of bf16 pairs: 8 tensor-memory columns a step of 16) and B MN-major in shared memory (16 rows of
-// 128 bytes a step): four steps.
+// The same with steps of A_STEP and B_STEP (in units of the descriptors' address fields, 16 bytes), four or eight of them.
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_f16_run4_w(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+#define CSB_UMMA_STEP                                                                                                  \
+  "add.u32 x, x, %7;\n\tadd.u32 y, y, %8;\n\tmov.b64 da, {x, %2};\n\tmov.b64 db, {y, %4};\n\t"                      \
+  "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, 1;\n\t"
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b32 x, %1;\n\tmov.b32 y, %3;\n\tmov.b64 da, {x, %2};\n\tmov.b64 db, {y, %4};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t"
+      CSB_UMMA_STEP CSB_UMMA_STEP CSB_UMMA_STEP
+      "}" ::"r"(d_tmem), "r"(static_cast<uint32_t>(a_desc)), "r"(static_cast<uint32_t>(a_desc >> 32)), "r"(static_cast<uint32_t>(b_desc)),
+      "r"(static_cast<uint32_t>(b_desc >> 32)), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
+      : "memory");
+}
+template <int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_f16_run8_w(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b32 x, %1;\n\tmov.b32 y, %3;\n\tmov.b64 da, {x, %2};\n\tmov.b64 db, {y, %4};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t"
+      CSB_UMMA_STEP CSB_UMMA_STEP CSB_UMMA_STEP CSB_UMMA_STEP CSB_UMMA_STEP CSB_UMMA_STEP CSB_UMMA_STEP
+      "}" ::"r"(d_tmem), "r"(static_cast<uint32_t>(a_desc)), "r"(static_cast<uint32_t>(a_desc >> 32)), "r"(static_cast<uint32_t>(b_desc)),
+      "r"(static_cast<uint32_t>(b_desc >> 32)), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
+      : "memory");
+#undef CSB_UMMA_STEP
+}
+// D (+)= A B with A = 64 columns of bf16 pairs in tensor memory (16 of them are 8 tensor-memory columns; step 2 starts at column HALF)
+// and B MN-major in shared memory (16 rows of 128 bytes a step): four steps.
+template <int HALF = 16>
 __device__ __forceinline__ void umma_f16_ts_run4_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   const uint32_t b0 = static_cast<uint32_t>(b_desc), bh = static_cast<uint32_t>(b_desc >> 32);
 #define CSB_UMMA_STEP(ao, bo)                                                                    \
@@ -335,8 +367,8 @@ __device__ __forceinline__ void umma_f16_ts_run4_w(uint32_t d_tmem, uint32_t a_t
       "setp.ne.b32 p, %5, 0;\n\t"
       "mov.b64 db, {%2, %3};\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t"
-      CSB_UMMA_STEP(8, 128) CSB_UMMA_STEP(16, 256) CSB_UMMA_STEP(24, 384)
-      "}" ::"r"(d_tmem), "r"(a_tmem), "r"(b0), "r"(bh), "r"(idesc), "r"(accumulate)
+      CSB_UMMA_STEP(8, 128) CSB_UMMA_STEP(%6, 256) CSB_UMMA_STEP(%7, 384)
+      "}" ::"r"(d_tmem), "r"(a_tmem), "r"(b0), "r"(bh), "r"(idesc), "r"(accumulate), "n"(HALF), "n"(HALF + 8)
       : "memory");
 #undef CSB_UMMA_STEP
 }
