@@ -311,13 +311,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const uint32_t ph = (it >> 1) & 1;
         if (!at_wait(&k_full[st], ph, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; return false; }
         tc_fence_after();
-        // descriptors of the k-th 16-wide slice: the tile's descriptor plus the slice's byte offset / 16
         const uint64_t k_desc = make_desc_kmajor_sw128(smem_u32(smem + L::K_OFF + st * L::KV_BYTES));
-#pragma unroll
-        for (int kk = 0; kk < 4 * NCH; ++kk) {  // unrolled to the maximum, cut by a uniform test
-          const uint64_t off = static_cast<uint64_t>(((kk >> 2) * CHUNK_BYTES + (kk & 3) * 32) >> 4);
-          if (kk < ksteps_s) umma_f16_w(tmem_S + st * 128, q_desc + off, k_desc + off, idesc_s, kk > 0 ? 1u : 0u);
-        }
+        umma_f16_run_w(tmem_S + st * 128, q_desc, k_desc, CHUNK_BYTES, CHUNK_BYTES, idesc_s, ksteps_s, 0u);
         umma_commit_w(&k_empty[st]);
         umma_commit_w(&s_full[st]);
         return true;
@@ -338,10 +333,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int hh = 0; hh < 2; ++hh) {
           if (!at_wait(&p_full[hh], it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; ok = false; break; }
           tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < AT_BN / 32; ++kk)
-            umma_f16_ts_w(tmem_O + hh * 128, tmem_S + st * 128 + hh * 64 + kk * 8,
-                          v_desc + static_cast<uint64_t>(((hh * 4 + kk) * 2048) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
+          umma_f16_ts_run4_w(tmem_O + hh * 128, tmem_S + st * 128 + hh * 64, v_desc + static_cast<uint64_t>((hh * 4 * 2048) >> 4), idesc_o,
+                             it > 0 ? 1u : 0u);
         }
         if (!ok) break;
         umma_commit_w(&v_empty[st]);

@@ -117,26 +117,25 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
   } else if (warp == 1) {
     // the whole warp walks this code in step (see umma_f16_w)
     constexpr uint32_t idesc = make_idesc_bf16(BM, SK_BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    constexpr int A_STEP = (A_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4, B_STEP = (B_MN ? UMMA_K * 128 : UMMA_K * 2) >> 4;
+    const uint32_t sa0 = smem_u32(smem), sb0 = sa0 + L::A_BYTES;
+    const uint64_t adesc = A_MN ? make_desc_mnmajor_sw128(sa0, 64 * BK * 2) : make_desc_kmajor_sw128(sa0);
+    const uint64_t bdesc = B_MN ? make_desc_mnmajor_sw128(sb0, 64 * BK * 2) : make_desc_kmajor_sw128(sb0);
+    int s = 0;
+    uint32_t ph = 0;
     bool ok = true;
-    for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
-      const int s = it % L::STAGES;
-      if (!wait_or_abort(&full_bar[s], (it / L::STAGES) & 1, abort_flag)) {
+    for (int kb = kb0; kb < kb1; ++kb) {
+      if (!wait_or_abort(&full_bar[s], ph, abort_flag)) {
         atomicExch(p.status, ST_TIMEOUT_FULL);
         *abort_flag = 1;
         ok = false;
         break;
       }
       tc_fence_after();
-      const uint32_t sa = smem_u32(smem + s * L::STAGE_BYTES), sb = sa + L::A_BYTES;
-      const uint64_t adesc = A_MN ? make_desc_mnmajor_sw128(sa, 64 * BK * 2) : make_desc_kmajor_sw128(sa);
-      const uint64_t bdesc = B_MN ? make_desc_mnmajor_sw128(sb, 64 * BK * 2) : make_desc_kmajor_sw128(sb);
-#pragma unroll
-      for (int k = 0; k < BK / UMMA_K; ++k) {
-        const uint64_t a_adv = A_MN ? (uint64_t)((k * UMMA_K * 128) >> 4) : (uint64_t)((k * UMMA_K * 2) >> 4);
-        const uint64_t b_adv = B_MN ? (uint64_t)((k * UMMA_K * 128) >> 4) : (uint64_t)((k * UMMA_K * 2) >> 4);
-        umma_f16_w(tmem_base, adesc + a_adv, bdesc + b_adv, idesc, (it > 0 || k > 0) ? 1u : 0u);
-      }
+      const uint64_t stage = static_cast<uint64_t>((s * L::STAGE_BYTES) >> 4);
+      umma_f16_run4_w<A_STEP, B_STEP>(tmem_base, adesc + stage, bdesc + stage, idesc, kb > kb0 ? 1u : 0u);
       umma_commit_w(&empty_bar[s]);
+      if (++s == L::STAGES) { s = 0; ph ^= 1u; }
     }
     if (ok) umma_commit_w(tmem_full);
     __syncwarp();

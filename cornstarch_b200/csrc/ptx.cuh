@@ -372,6 +372,28 @@ __device__ __forceinline__ void umma_f16_ts_run4_w(uint32_t d_tmem, uint32_t a_t
       : "memory");
 #undef CSB_UMMA_STEP
 }
+// umma_f16_run4_w for a CTA pair (CG = 2) or one block.
+template <int CG, int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_f16_run4_cg_w(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (CG == 1) {
+    umma_f16_run4_w<A_STEP, B_STEP>(d_tmem, a_desc, b_desc, idesc, accumulate);
+  } else {
+#define CSB_UMMA_STEP                                                                                                  \
+  "add.u32 x, x, %7;\n\tadd.u32 y, y, %8;\n\tmov.b64 da, {x, %2};\n\tmov.b64 db, {y, %4};\n\t"                      \
+  "@e tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, 1;\n\t"
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "mov.b32 x, %1;\n\tmov.b32 y, %3;\n\tmov.b64 da, {x, %2};\n\tmov.b64 db, {y, %4};\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t"
+        CSB_UMMA_STEP CSB_UMMA_STEP CSB_UMMA_STEP
+        "}" ::"r"(d_tmem), "r"(static_cast<uint32_t>(a_desc)), "r"(static_cast<uint32_t>(a_desc >> 32)), "r"(static_cast<uint32_t>(b_desc)),
+        "r"(static_cast<uint32_t>(b_desc >> 32)), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
+        : "memory");
+#undef CSB_UMMA_STEP
+  }
+}
 __device__ __forceinline__ void umma_f16_2cta_w(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                 uint32_t accumulate) {
   asm volatile(
