@@ -20,6 +20,7 @@ from .. import nn as cnn
 from ..ops import attention as A
 from ..ops import elementwise as E
 from ..ops.linear import multi_linear
+from ..ops.patch import patch_embed
 from .base import ModelOutput, PretrainedConfig, PreTrainedModel, is_released, register_model
 
 
@@ -151,8 +152,7 @@ class SiglipVisionEmbeddings(nn.Module):
         self.position_embedding = nn.Embedding(self.num_patches, config.hidden_size)
 
     def forward(self, pixel_values):
-        x = self.patch_embedding(pixel_values.to(self.patch_embedding.weight.dtype))
-        x = x.flatten(2).transpose(1, 2)
+        x = patch_embed(self.patch_embedding, pixel_values.to(self.patch_embedding.weight.dtype))
         return x + self.position_embedding.weight[: x.shape[1]].unsqueeze(0)
 
 
@@ -251,7 +251,7 @@ class CLIPVisionEmbeddings(nn.Module):
         self.position_embedding = nn.Embedding(self.num_positions, H)
 
     def forward(self, pixel_values):
-        x = self.patch_embedding(pixel_values.to(self.patch_embedding.weight.dtype)).flatten(2).transpose(1, 2)
+        x = patch_embed(self.patch_embedding, pixel_values.to(self.patch_embedding.weight.dtype))
         cls = self.class_embedding.expand(x.shape[0], 1, -1).to(x.dtype)
         x = torch.cat([cls, x], dim=1)
         return x + self.position_embedding.weight[: x.shape[1]].unsqueeze(0)
@@ -353,7 +353,7 @@ class ViTEmbeddings(nn.Module):
 
     def forward(self, pixel_values):
         w = self.patch_embeddings.projection.weight
-        x = self.patch_embeddings.projection(pixel_values.to(w.dtype)).flatten(2).transpose(1, 2)
+        x = patch_embed(self.patch_embeddings.projection, pixel_values.to(w.dtype))
         x = torch.cat([self.cls_token.expand(x.shape[0], -1, -1).to(x.dtype), x], dim=1)
         return x + self.position_embeddings[:, : x.shape[1]].to(x.dtype)
 

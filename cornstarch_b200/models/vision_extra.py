@@ -19,6 +19,7 @@ from .. import nn as cnn
 from ..ops import attention as A
 from ..ops import elementwise as E
 from ..ops.linear import multi_linear
+from ..ops.patch import patch_embed
 from .base import ModelOutput, PretrainedConfig, is_released, register_model
 from .vision import VisionConfig, _Encoder, _VisionBase
 
@@ -130,7 +131,7 @@ class Dinov2Embeddings(nn.Module):
 
     def forward(self, pixel_values):
         w = self.patch_embeddings.projection.weight
-        x = self.patch_embeddings.projection(pixel_values.to(w.dtype)).flatten(2).transpose(1, 2)
+        x = patch_embed(self.patch_embeddings.projection, pixel_values.to(w.dtype))
         x = torch.cat([self.cls_token.expand(x.shape[0], -1, -1).to(x.dtype), x], dim=1)
         return x + self.position_embeddings[:, : x.shape[1]].to(x.dtype)
 
@@ -229,7 +230,7 @@ class EvaCLIPVisionEmbeddings(nn.Module):
         self.position_embedding = nn.Embedding((config.image_size // config.patch_size) ** 2 + 1, H)
 
     def forward(self, pixel_values):
-        x = self.patch_embedding(pixel_values.to(self.patch_embedding.weight.dtype)).flatten(2).transpose(1, 2)
+        x = patch_embed(self.patch_embedding, pixel_values.to(self.patch_embedding.weight.dtype))
         x = torch.cat([self.class_embedding.expand(x.shape[0], 1, -1).to(x.dtype), x], dim=1)
         return x + self.position_embedding.weight[: x.shape[1]].unsqueeze(0)
 
@@ -329,7 +330,7 @@ class InternVisionEmbeddings(nn.Module):
         self.position_embedding = nn.Parameter(torch.randn(1, n + 1, H) * 0.02)
 
     def forward(self, pixel_values):
-        x = self.patch_embedding(pixel_values.to(self.patch_embedding.weight.dtype)).flatten(2).transpose(1, 2)
+        x = patch_embed(self.patch_embedding, pixel_values.to(self.patch_embedding.weight.dtype))
         x = torch.cat([self.class_embedding.expand(x.shape[0], -1, -1).to(x.dtype), x], dim=1)
         return x + self.position_embedding[:, : x.shape[1]].to(x.dtype)
 
@@ -453,9 +454,9 @@ class PixtralVisionModel(_VisionBase):
         from ..utils.recompute import checkpoint_layer
 
         if hidden_states is None:
-            x = self.patch_conv(pixel_values.to(self.patch_conv.weight.dtype))
-            B, H, gh, gw = x.shape
-            x = self.ln_pre(x.flatten(2).transpose(1, 2))
+            B, (ph, pw) = pixel_values.shape[0], self.patch_conv.kernel_size
+            gh, gw = pixel_values.shape[2] // ph, pixel_values.shape[3] // pw
+            x = self.ln_pre(patch_embed(self.patch_conv, pixel_values.to(self.patch_conv.weight.dtype)))
             side = self.patch_positional_embedding.side
             hh, ww = torch.meshgrid(torch.arange(gh, device=x.device), torch.arange(gw, device=x.device), indexing="ij")
             position_ids = (hh * side + ww).reshape(1, -1).expand(B, -1).int().contiguous()
