@@ -32,6 +32,7 @@ constexpr int UMMA_K = 16;
 
 enum Act : int { ACT_NONE = 0, ACT_GELU_TANH = 1, ACT_GELU_ERF = 2, ACT_SILU = 3 };
 
+constexpr int MAX_COL_GROUPS = 4;
 struct GemmParams {
   void* C;
   const void* bias;  // bf16 [N] or null
@@ -75,7 +76,19 @@ struct GemmParams {
   // multiplied with that group's own B (the local experts of a MoE layer in ONE launch).  group_rows is a multiple of
   // the tile height, so a tile never straddles two groups; the B tensor maps travel in EpiMaps (see group_b_map).
   int group_rows;
+  // ---- column groups (col_groups > 1): columns [col_first[g], col_first[g + 1]) * BN of C are A times the B of group g, a matrix of
+  // its own (projections of one input whose weights are not adjacent), plus its bias; widths are multiples of BN, so a tile never
+  // straddles two groups; the maps travel in EpiMaps.
+  int col_groups;
+  int col_first[MAX_COL_GROUPS + 1];
+  const void* col_bias[MAX_COL_GROUPS];
 };
+__device__ __forceinline__ int col_group(const GemmParams& p, int n_blk) {
+  int g = 0;
+#pragma unroll
+  for (int i = 1; i < MAX_COL_GROUPS; ++i) g += i < p.col_groups && n_blk >= p.col_first[i] ? 1 : 0;
+  return g;
+}
 
 constexpr int AR_MAX_ROWS = 512;
 
@@ -280,7 +293,7 @@ template <int BN, int EPI_OFF_BYTES_SLAB = 128 * 128>
 __device__ __forceinline__ void epilogue_tile_tma(const GemmParams& p, const EpiMaps& maps, uint8_t* epi_smem,
                                                   uint32_t t_row, int m_blk, int n_blk, int quarter, int lane, int warp,
                                                   uint32_t& slab_ctr, uint64_t* tmem_empty_bar, bool ar, int owner,
-                                                  bool mine, bool remote_leader = false) {
+                                                  bool mine, bool remote_leader, const void* bias) {
   const int r = quarter * 32 + lane;
   const int row = m_blk * BM + r;
   const bool e0 = (warp == 2 && lane == 0);
@@ -307,9 +320,9 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmParams& p, const Epi
       tc_fence_before();
       arrive_tmem_empty(tmem_empty_bar, remote_leader);  // the accumulator buffer can be overwritten by the next tile's MMAs
     }
-    if (p.bias) {
-      const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0;
-      if (col0 + 64 <= p.N && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
+    if (bias) {
+      const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(bias) + col0;
+      if (col0 + 64 <= p.N && (reinterpret_cast<uintptr_t>(b) & 15) == 0) {
         // Eight 16-byte loads, the same address in all lanes.  (One 2-byte load per column and thread took longer than the MMAs of a
         // short contraction: 2916 x 1152 -> 4304 45.8 us, 26.4 without a bias; 4096 x 1152 -> 4304 54.5 -> 32.2.)
         // (64 columns also for fp32 results, whose slabs have 32: the others are not used.)
@@ -504,10 +517,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         int m_blk, n_blk;
         tile_coords_rot<(CG == 2 ? 8 : 16)>(tile, num_m_units, p.num_n_blocks, rot, m_blk, n_blk);
         m_blk = m_blk * CG + cta_rank;
-        const int n_row0 = n_blk * BN + cta_rank * BNH;
+        int n_row0 = n_blk * BN + cta_rank * BNH;
         const CUtensorMap* map_a = &tma_a;
         int a_row0 = m_blk * BM;
         const CUtensorMap* map_b = p.group_rows > 0 ? group_b_map(epi_maps, a_row0 / p.group_rows) : &tma_b;
+        if (p.col_groups > 1) {
+          const int g = col_group(p, n_blk);
+          map_b = group_b_map(epi_maps, g);
+          n_row0 -= p.col_first[g] * BN;
+        }
         if (n_pull > 0) {
           const int o = ar_owner(m_blk, p.num_m_blocks, p.ag_world);
           if (o == p.ag_rank) {
@@ -632,8 +650,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             arrived = spin_until_ge(p.ar_cnt_part[p.ar_rank] + lane * AR_MAX_ROWS + m_blk, p.ar_base + p.num_n_blocks);
           if (!__all_sync(0xffffffffu, arrived) && lane == 0) atomicExch(p.status, ST_TIMEOUT_PEER_FLAG);
         }
+        const void* bias = p.bias;
+        if (p.col_groups > 1) {
+          const int g = col_group(p, n_blk);
+          bias = p.col_bias[g] ? reinterpret_cast<const __nv_bfloat16*>(p.col_bias[g]) - p.col_first[g] * BN : nullptr;
+        }
         epilogue_tile_tma<BN, L::EPI_SLAB_BYTES>(p, epi_maps, smem + L::EPI_OFFSET, t_row, m_blk, n_blk, quarter, lane, warp, slab_ctr,
-                                                 &tmem_empty[acc], ar, owner, mine, !leader);
+                                                 &tmem_empty[acc], ar, owner, mine, !leader, bias);
         continue;
       }
       if (mine) {
@@ -876,6 +899,15 @@ static int launch_gemm(const void* A, const void* B, const GemmParams& p, int ld
       if (r) return r;
     }
   }
+  if (q.col_groups > 1) {
+    if (A_MN || B_MN || q.ar_world > 1 || q.ag_world > 1 || q.group_rows > 0 || groups != q.col_groups || group_b == nullptr || !q.tma_epi)
+      return CSB_ERR_BAD_ARG;
+    for (int g = 0; g < groups; ++g) {
+      if (reinterpret_cast<uintptr_t>(group_b[g]) & 15) return CSB_ERR_BAD_ARG;
+      const int n = (q.col_first[g + 1] - q.col_first[g]) * BN;
+      if ((r = make_tmap_2d_bf16(const_cast<CUtensorMap*>(group_b_map(em, g)), group_b[g], n, q.K, ldb, BK, BN / CG))) return r;
+    }
+  }
   if (q.ag_world > 1) {
     if (A_MN) return CSB_ERR_BAD_ARG;
     const int own0 = ar_range_start(q.ag_rank, q.num_m_blocks, q.ag_world) * BM;
@@ -1023,6 +1055,7 @@ static int choose_split(int M, int N, int K, int tile_n, int max_ctas, TileChoic
 }
 static void no_collective(GemmParams& p) {
   p.group_rows = 0;
+  p.col_groups = 0;
   p.ar_scatter = 0; p.ar_row_offset = 0;
   p.ag_world = 1; p.ag_rank = 0; p.ag_pull_ctas = 0;
   for (int i = 0; i < 8; ++i) p.ag_src[i] = nullptr;
@@ -1107,6 +1140,75 @@ CSB_API int csb_linear_bwd(const void* dy, const void* x, const void* w, void* d
   if (!r) r = csb_gemm_bf16(dy, x, dw, nullptr, N, K, T, lddy, ldx, lddw, 1, 1, dw_fp32, dw_acc, 0, 0, 0, status, stream);
   if (!r && db != nullptr) r = csb_colsum(dy, scratch, db, db_fp32, db_acc, T, N, stream);
   return r;
+}
+
+// Projections of one input whose weights are matrices of their own, in ONE launch: C[:, o_g : o_g + N_g] = A * B_g^T + bias_g with
+// o_g the widths before.  A and all B are K-major (pitches lda, ldb); bias: one pointer per group (0 = none), or null.  Taken where a
+// tile width divides all N_g and the whole would not share its contractions (choose_split); CSB_ERR_NO_FIT otherwise, and the
+// caller makes one call per weight.  Each of those ends in a round of its own, mostly empty for narrow ones: 1531 x 4096 -> 4096, 1024
+// and 1024 40.4 + 20.3 + 20.3 us, together 53; 729 x 1152 -> 3 x 1152 with biases 3 x 9.5, together 12.
+CSB_API int csb_gemm_cols_bf16(const void* A, const void* const* B, const void* const* bias, const int* widths, int groups, void* C, int M, int K,
+                               int lda, int ldb, int ldc, int* status, void* stream) {
+  using namespace csb;
+  if (groups < 2 || groups > MAX_COL_GROUPS || M <= 0 || K <= 0 || (lda & 7) || (ldb & 7) || B == nullptr || widths == nullptr) return CSB_ERR_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(C)) & 15) return CSB_ERR_BAD_ARG;
+  long total = 0;
+  for (int g = 0; g < groups; ++g) {
+    if (widths[g] <= 0) return CSB_ERR_BAD_ARG;
+    total += widths[g];
+  }
+  if (total > 0x7fffffffL || ldc < total || (ldc & 7)) return CSB_ERR_BAD_ARG;
+  const int N = (int)total;
+  auto divides = [&](int bn) {
+    for (int g = 0; g < groups; ++g)
+      if (widths[g] % bn) return false;
+    return true;
+  };
+  TileChoice tc = choose_tile(M, N, K, 0, 0, false, false);
+  if (choose_split(M, N, K, 0, 0, tc, false, false) > 1) return CSB_ERR_NO_FIT;
+  if (!divides(tc.bn)) {  // the cheapest one that does
+    float best = 0.f;
+    tc.bn = 0;
+    for (const TileCost& c : TILE_COSTS) {
+      if (!divides(c.bn) || (c.cg == 2 && (gemm_cg_choice() != 2 || M <= BM))) continue;
+      const float t = tile_cost(c, 0, M, N, K);
+      if (tc.bn == 0 || t < best) {
+        best = t;
+        tc = {c.bn, c.cg};
+      }
+    }
+    if (tc.bn == 0) return CSB_ERR_NO_FIT;
+  }
+  GemmParams p;
+  p.C = C;
+  p.bias = nullptr;
+  p.M = M; p.N = N; p.K = K;
+  p.ldc = ldc;
+  p.out_fp32 = 0;
+  p.accumulate = 0;
+  p.act = 0;
+  p.num_m_blocks = (M + BM - 1) / BM;
+  p.num_n_blocks = N / tc.bn;
+  p.num_k_blocks = (K + BK - 1) / BK;
+  p.status = status;
+  p.tma_epi = 0;
+  p.ar_world = 1; p.ar_rank = 0; p.ar_base = 0; p.ar_slot_elems = 0;
+  for (int i = 0; i < 8; ++i) { p.ar_inbox[i] = nullptr; p.ar_final[i] = nullptr; p.ar_cnt_part[i] = nullptr; p.ar_cnt_final[i] = nullptr; }
+  no_collective(p);
+  p.col_groups = groups;
+  p.col_first[0] = 0;
+  for (int g = 0; g < groups; ++g) {
+    p.col_first[g + 1] = p.col_first[g] + widths[g] / tc.bn;
+    p.col_bias[g] = bias ? bias[g] : nullptr;
+  }
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (tc.cg == 2) {
+    if (tc.bn == 256) return launch_gemm<256, false, false, 2>(A, B[0], p, lda, ldb, 0, s, B, groups);
+    if (tc.bn == 192) return launch_gemm<192, false, false, 2>(A, B[0], p, lda, ldb, 0, s, B, groups);
+    return launch_gemm<128, false, false, 2>(A, B[0], p, lda, ldb, 0, s, B, groups);
+  }
+  if (tc.bn == 256) return launch_gemm<256, false, false>(A, B[0], p, lda, ldb, 0, s, B, groups);
+  return launch_gemm<128, false, false>(A, B[0], p, lda, ldb, 0, s, B, groups);
 }
 
 // Grouped GEMM: `groups` problems of the same shape in ONE launch.  A is [groups * group_rows][K] (K-major) and C is

@@ -15,6 +15,7 @@ enum : int {
   CSB_ERR_NO_DRIVER_SYMBOL = -2,
   CSB_ERR_TENSORMAP = -3,
   CSB_ERR_TOO_LARGE = -4,
+  CSB_ERR_NO_FIT = -5,  // a form that the entry point does not take: the caller has another way
 };
 
 namespace csb {

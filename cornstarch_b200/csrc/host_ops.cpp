@@ -127,6 +127,30 @@ py::object gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const Op
 }
 
 // ------------------------------------------------------------------------------------------------------- linear layers
+using ColsFn = int (*)(const void*, const void* const*, const void* const*, const int*, int, void*, int, int, int, int, int, int*, void*);
+Entry<ColsFn> e_gemm_cols("csb_gemm_cols_bf16");
+constexpr int MAX_COL_GROUPS = 4, ERR_NO_FIT = -5;
+
+// Weights that are not adjacent as one launch; false where the library has no tile for them.
+bool cols_gemm(const Tensor& x2, const std::vector<Tensor>& ws, const std::vector<Tensor>& biases, void* out, int64_t T, int64_t N, int64_t K) {
+  if (ws.size() > MAX_COL_GROUPS || (reinterpret_cast<uintptr_t>(out) & 15) || N % 8) return false;
+  const void* b[MAX_COL_GROUPS];
+  const void* bias[MAX_COL_GROUPS];
+  int widths[MAX_COL_GROUPS];
+  for (size_t i = 0; i < ws.size(); ++i) {
+    if (ws[i].stride(0) != ws[0].stride(0)) return false;
+    b[i] = ws[i].data_ptr();
+    bias[i] = biases.empty() ? nullptr : biases[i].data_ptr();
+    widths[i] = (int)ws[i].size(0);
+  }
+  const int r = e_gemm_cols.get()(x2.data_ptr(), b, biases.empty() ? nullptr : bias, widths, (int)ws.size(), out, (int)T, (int)K, (int)x2.stride(0),
+                                  (int)ws[0].stride(0), (int)N, status_word(x2), stream());
+  if (r == ERR_NO_FIT) return false;
+  ++g_launches;
+  check(r, "csb_gemm_cols_bf16");
+  return true;
+}
+
 // (out, x as 2-D): the concatenated projections of x; one GEMM where the weights (and biases) are adjacent, else one each.
 py::object linear_fwd(const Tensor& x, const std::vector<Tensor>& ws, const std::vector<OptTensor>& bs) {
   if (!x.is_cuda() || !bf16(x) || x.dim() < 1 || x.numel() == 0) return py::none();
@@ -161,7 +185,7 @@ py::object linear_fwd(const Tensor& x, const std::vector<Tensor>& ws, const std:
   }
   if (w && (!has_bias || b)) {
     launch_gemm(x2, *w, out.data_ptr(), ptr(b), T, N, K, N, false, false, false, false, 0, 0, 0);
-  } else {
+  } else if (!cols_gemm(x2, ws, biases, out.data_ptr(), T, N, K)) {
     char* o = static_cast<char*>(out.data_ptr());
     for (size_t i = 0; i < ws.size(); ++i) {
       launch_gemm(x2, ws[i], o, has_bias ? biases[i].data_ptr() : nullptr, T, ws[i].size(0), K, N, false, false, false, false, 0, 0, 0);

@@ -141,7 +141,7 @@ def kernel_times(reset: bool = True) -> dict:
 
 
 _HOST = None  # the module; False where calls go through ctypes one by one
-_HOST_ENTRIES = ("csb_gemm_bf16", "csb_linear_bwd", "csb_colsum_parts", "csb_norm_fwd", "csb_norm_bwd", "csb_norm_bwd_parts", "csb_act_fwd",
+_HOST_ENTRIES = ("csb_gemm_bf16", "csb_gemm_cols_bf16", "csb_linear_bwd", "csb_colsum_parts", "csb_norm_fwd", "csb_norm_bwd", "csb_norm_bwd_parts", "csb_act_fwd",
                  "csb_act_bwd", "csb_glu_fwd", "csb_glu_bwd", "csb_attn_fwd", "csb_attn_bwd", "csb_attn_bwd_splits")
 
 

@@ -165,3 +165,22 @@ def test_refused_layouts_are_refused(monkeypatch):
             gemm(_randn(8, 16), _randn(8, 24))
         with pytest.raises(RuntimeError, match="csb_norm_fwd"):
             E.rms_norm(_randn(0, 16), _randn(16))
+
+
+# weights that are not adjacent, one launch: widths that 256, 192 and 128 columns divide, one tile row and several, and none that
+# fits (then one call per weight, as with a single row that shares its contraction)
+@pytest.mark.gpu
+@pytest.mark.parametrize("widths,one", [((512, 256, 256), True), ((192, 384), True), ((128, 640, 128, 256), True), ((1152, 1152, 1152), True),
+                                        ((136, 256), False), ((64, 64), False), ((128,) * 5, False)])
+@pytest.mark.parametrize("T", [1, 130, 700, 3000])
+@pytest.mark.parametrize("bias", [False, True])
+def test_projections_of_separate_weights(widths, one, T, bias):
+    x, ws = _randn(T, 264), [_randn(n, 264, seed=i) for i, n in enumerate(widths)]
+    bs = [_randn(n + 1, seed=9 + i)[1:] if i == 1 else _randn(n, seed=9 + i) for i, n in enumerate(widths)] if bias else [None] * len(ws)
+    before = nat.launch_count
+    with torch.no_grad():
+        y = L.multi_linear(x, ws, bs)
+    one = one and (T > 128 or widths != (192, 384))  # 192 columns are a tile of a pair of blocks
+    assert nat.launch_count - before == (1 if one else len(widths))
+    ref = torch.cat([x.double() @ w.double().t() + (b.double() if b is not None else 0) for w, b in zip(ws, bs)], -1)
+    assert (y.double() - ref).norm() <= 2.0**-8 * ref.norm() and (y.double() - ref).abs().max() <= 2.0**-7 * ref.abs().max()
