@@ -82,6 +82,7 @@ struct GemmParams {
   int col_groups;
   int col_first[MAX_COL_GROUPS + 1];
   const void* col_bias[MAX_COL_GROUPS];
+  float2* ce_part;  // CE form: [num_n_blocks][M] maximum and sum of exponentials of a row of a tile
 };
 __device__ __forceinline__ int col_group(const GemmParams& p, int n_blk) {
   int g = 0;
@@ -289,7 +290,9 @@ __device__ __forceinline__ void arrive_tmem_empty(uint64_t* bar, bool remote_lea
   else mbar_arrive(bar);
 }
 
-template <int BN, int EPI_OFF_BYTES_SLAB = 128 * 128>
+// CE: besides storing them (bf16), take each row's maximum over the tile's columns and the sum of exp(x - maximum) of the ROUNDED values
+// and leave them in ce_part[column tile][row]: the statistics of a cross-entropy loss without a pass over the logits (csb_lm_stats).
+template <int BN, int EPI_OFF_BYTES_SLAB = 128 * 128, bool CE = false>
 __device__ __forceinline__ void epilogue_tile_tma(const GemmParams& p, const EpiMaps& maps, uint8_t* epi_smem,
                                                   uint32_t t_row, int m_blk, int n_blk, int quarter, int lane, int warp,
                                                   uint32_t& slab_ctr, uint64_t* tmem_empty_bar, bool ar, int owner,
@@ -299,6 +302,7 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmParams& p, const Epi
   const bool e0 = (warp == 2 && lane == 0);
   const int cps = p.out_fp32 ? 32 : 64;  // columns per 128-byte slab row
   const int n_slabs = BN / cps;
+  float ce_max = -INFINITY, ce_sum = 0.f;
   for (int s = 0; s < n_slabs; ++s, ++slab_ctr) {
     const int col0 = n_blk * BN + s * cps;
     const bool last = (s == n_slabs - 1) || (col0 + cps >= p.N);
@@ -373,6 +377,34 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmParams& p, const Epi
         }
       }
     }
+    if constexpr (CE) {
+      const int n_words = (min(64, p.N - col0)) >> 1;  // pairs of columns that exist (N is even)
+      uint32_t w[32];
+      float mx[2];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        w[j] = pack_bf16x2(f[2 * j], f[2 * j + 1]);
+        if (j >= n_words) w[j] = 0xff80ff80u;  // -inf: takes part in nothing
+        const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xffff0000u);
+        if (j < 2) mx[j] = fmaxf(lo, hi);
+        else mx[j & 1] = max3(mx[j & 1], lo, hi);
+      }
+      const float LOG2E = 1.4426950408889634f;
+      const float m_new = fmaxf(ce_max, fmaxf(mx[0], mx[1]));
+      const uint64_t neg_m = pack_f32x2(-m_new, -m_new), log2e = pack_f32x2(LOG2E, LOG2E);
+      uint64_t sum[2] = {0ull, 0ull};
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        float y0, y1;
+        unpack_f32x2(mul_f32x2(add_f32x2(pack_u32x2(w[j] << 16, w[j] & 0xffff0000u), neg_m), log2e), y0, y1);
+        sum[j & 1] = add_f32x2(sum[j & 1], pack_f32x2(fast_exp2(y0), fast_exp2(y1)));
+      }
+      float s0, s1;
+      unpack_f32x2(add_f32x2(sum[0], sum[1]), s0, s1);
+      ce_sum = ce_sum * fast_exp2((ce_max - m_new) * LOG2E) + (s0 + s1);
+      ce_max = m_new;
+      if (last && row < p.M) p.ce_part[static_cast<size_t>(n_blk) * p.M + row] = make_float2(ce_max, ce_sum);
+    }
     uint8_t* buf = epi_smem + (slab_ctr & 1) * EPI_OFF_BYTES_SLAB;
     if (e0) tma_store_wait_read<1>();  // the store that last used this slab has finished reading it
     asm volatile("bar.sync 2, 128;" ::: "memory");
@@ -435,7 +467,7 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmParams& p, const Epi
   }
 }
 
-template <int BN, bool A_MN, bool B_MN, int CG>
+template <int BN, bool A_MN, bool B_MN, int CG, bool CE>
 __global__ void __launch_bounds__(192, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const __grid_constant__ EpiMaps epi_maps, const GemmParams p) {
@@ -655,7 +687,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           const int g = col_group(p, n_blk);
           bias = p.col_bias[g] ? reinterpret_cast<const __nv_bfloat16*>(p.col_bias[g]) - p.col_first[g] * BN : nullptr;
         }
-        epilogue_tile_tma<BN, L::EPI_SLAB_BYTES>(p, epi_maps, smem + L::EPI_OFFSET, t_row, m_blk, n_blk, quarter, lane, warp, slab_ctr,
+        epilogue_tile_tma<BN, L::EPI_SLAB_BYTES, CE>(p, epi_maps, smem + L::EPI_OFFSET, t_row, m_blk, n_blk, quarter, lane, warp, slab_ctr,
                                                  &tmem_empty[acc], ar, owner, mine, !leader, bias);
         continue;
       }
@@ -847,7 +879,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
 }
 
-template <int BN, bool A_MN, bool B_MN, int CG = 1>
+template <int BN, bool A_MN, bool B_MN, int CG = 1, bool CE = false>
 static int launch_gemm(const void* A, const void* B, const GemmParams& p, int lda, int ldb, int max_ctas,
                        cudaStream_t stream, const void* const* group_b = nullptr, int groups = 0) {
   CUtensorMap ta, tb;
@@ -863,7 +895,7 @@ static int launch_gemm(const void* A, const void* B, const GemmParams& p, int ld
     r = make_tmap_2d_bf16(&tb, B, p.N, p.K, ldb, BK, BN / CG);
   if (r) return r;
   using L = SmemLayout<BN, CG, B_MN>;
-  auto kfn = gemm_bf16_kernel<BN, A_MN, B_MN, CG>;
+  auto kfn = gemm_bf16_kernel<BN, A_MN, B_MN, CG, CE>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN_BYTES);
@@ -1056,6 +1088,7 @@ static int choose_split(int M, int N, int K, int tile_n, int max_ctas, TileChoic
 static void no_collective(GemmParams& p) {
   p.group_rows = 0;
   p.col_groups = 0;
+  p.ce_part = nullptr;
   p.ar_scatter = 0; p.ar_row_offset = 0;
   p.ag_world = 1; p.ag_rank = 0; p.ag_pull_ctas = 0;
   for (int i = 0; i < 8; ++i) p.ag_src[i] = nullptr;
@@ -1209,6 +1242,95 @@ CSB_API int csb_gemm_cols_bf16(const void* A, const void* const* B, const void* 
   }
   if (tc.bn == 256) return launch_gemm<256, false, false>(A, B[0], p, lda, ldb, 0, s, B, groups);
   return launch_gemm<128, false, false>(A, B[0], p, lda, ldb, 0, s, B, groups);
+}
+
+namespace csb {
+// Row statistics from those of the column tiles, in a fixed order: 32 rows and sixteen shares of the tiles per block.
+constexpr int CE_SHARES = 16;
+__device__ __forceinline__ void ce_add(float& m, float& s, float om, float os) {
+  const float nm = fmaxf(m, om);
+  s = nm == -INFINITY ? s + os : s * __expf(m - nm) + os * __expf(om - nm);
+  m = nm;
+}
+__global__ void __launch_bounds__(32 * CE_SHARES) ce_merge_kernel(const float2* __restrict__ part, int n_blocks, int M, const __nv_bfloat16* __restrict__ logits,
+                                                                 long ld, const long* __restrict__ labels, int V, int vocab_start,
+                                                                 float* __restrict__ row_max, float* __restrict__ row_sum, float* __restrict__ tgt) {
+  __shared__ float2 sh[CE_SHARES][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, row = blockIdx.x * 32 + tx;
+  float m = -INFINITY, s = 0.f;
+  if (row < M) {
+#pragma unroll 8
+    for (int b = ty; b < n_blocks; b += CE_SHARES) {
+      const float2 q = part[static_cast<size_t>(b) * M + row];
+      ce_add(m, s, q.x, q.y);
+    }
+  }
+  sh[ty][tx] = make_float2(m, s);
+  __syncthreads();
+  if (ty == 0 && row < M) {
+    for (int k = 1; k < CE_SHARES; ++k) ce_add(m, s, sh[k][tx].x, sh[k][tx].y);
+    row_max[row] = m;
+    row_sum[row] = s;
+    const long lab = labels[row] - vocab_start;
+    tgt[row] = lab >= 0 && lab < V ? __bfloat162float(logits[row * ld + lab]) : 0.f;
+  }
+}
+}  // namespace csb
+
+CSB_API int csb_ce_stats(const void* logits, long ld, const long* labels, int V, int vocab_start, float* row_max, float* row_sum, float* tgt_logit,
+                         long rows, void* stream);
+
+// Logits of a language-model head and the row statistics of their cross-entropy: C[M, N] = A[M, K] B[N, K]^T in bf16, row_max, row_sum and
+// tgt as csb_ce_stats gives them.  `part`: csb_lm_stats_parts(N) * M pairs of floats.  The statistics come out of the epilogue, where
+// the exponentials of a tile (256 a row) hide behind the next tile's MMAs, instead of from a pass that reads the logits again; few
+// rows whose contraction is shared, an output off the 16-byte grid, and logits of less than CE_FUSED_MIN elements take that pass:
+// a block with one tile hides nothing (64 x 1000 of 1024: 11.2 us with the pass, 12.6 without; 500 x 1000 of 2048: 17.8 / 18.1).
+// Logits and statistics, with the pass / without: 4096 x 128256 of 4096 3104 / 2842 us, of 1024 1051 / 914; 4096 x 32000 of 4096
+// 778 / 716; 1000 x 128256 of 2048 436 / 379; 4096 x 1000 of 1024 31.6 / 19.7; 64 x 128256 of 4096 195 / 192.
+constexpr long CE_FUSED_MIN = 1L << 21;
+CSB_API int csb_lm_stats_parts(int N) { return (N + 127) / 128; }
+CSB_API int csb_lm_stats(const void* A, const void* B, void* C, float* part, const long* labels, int vocab_start, float* row_max, float* row_sum,
+                         float* tgt, int M, int N, int K, int lda, int ldb, int ldc, int* status, void* stream) {
+  using namespace csb;
+  if (M <= 0 || N <= 0 || K <= 0 || (lda & 7) || (ldb & 7) || (N & 7) || (ldc & 7)) return CSB_ERR_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) return CSB_ERR_BAD_ARG;
+  const TileChoice tc = choose_tile(M, N, K, 0, 0, false, false);
+  const bool fused = part != nullptr && (long)M * N >= CE_FUSED_MIN && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && choose_split(M, N, K, 0, 0, tc, false, false) == 1;
+  if (!fused) {
+    if (int e = csb_gemm_bf16(A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0, 0, 0, 0, 0, 0, 0, status, stream)) return e;
+    return csb_ce_stats(C, ldc, labels, N, vocab_start, row_max, row_sum, tgt, M, stream);
+  }
+  GemmParams p;
+  p.C = C;
+  p.bias = nullptr;
+  p.M = M; p.N = N; p.K = K;
+  p.ldc = ldc;
+  p.out_fp32 = 0;
+  p.accumulate = 0;
+  p.act = 0;
+  p.num_m_blocks = (M + BM - 1) / BM;
+  p.num_n_blocks = (N + tc.bn - 1) / tc.bn;
+  p.num_k_blocks = (K + BK - 1) / BK;
+  p.status = status;
+  p.tma_epi = 0;
+  p.ar_world = 1; p.ar_rank = 0; p.ar_base = 0; p.ar_slot_elems = 0;
+  for (int i = 0; i < 8; ++i) { p.ar_inbox[i] = nullptr; p.ar_final[i] = nullptr; p.ar_cnt_part[i] = nullptr; p.ar_cnt_final[i] = nullptr; }
+  no_collective(p);
+  p.ce_part = reinterpret_cast<float2*>(part);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  int e;
+  if (tc.cg == 2) {
+    if (tc.bn == 256) e = launch_gemm<256, false, false, 2, true>(A, B, p, lda, ldb, 0, s);
+    else if (tc.bn == 192) e = launch_gemm<192, false, false, 2, true>(A, B, p, lda, ldb, 0, s);
+    else e = launch_gemm<128, false, false, 2, true>(A, B, p, lda, ldb, 0, s);
+  } else {
+    if (tc.bn == 256) e = launch_gemm<256, false, false, 1, true>(A, B, p, lda, ldb, 0, s);
+    else e = launch_gemm<128, false, false, 1, true>(A, B, p, lda, ldb, 0, s);
+  }
+  if (e) return e;
+  ce_merge_kernel<<<(M + 31) / 32, 32 * CE_SHARES, 0, s>>>(p.ce_part, p.num_n_blocks, M, reinterpret_cast<const __nv_bfloat16*>(C), ldc, labels, N,
+                                                          vocab_start, row_max, row_sum, tgt);
+  return launch_result();
 }
 
 // Grouped GEMM: `groups` problems of the same shape in ONE launch.  A is [groups * group_rows][K] (K-major) and C is

@@ -43,6 +43,8 @@ _PROTOS = {
     "csb_sumsq": [vp, i32, i64, vp, vp, i32, vp],
     "csb_clip_scale": [vp, f32, f32, vp, vp, vp, vp, vp],
     "csb_mma_issue_probe": [i32, i32, i32, i32, vp, vp],
+    "csb_lm_stats_parts": [i32],
+    "csb_lm_stats": [vp] * 5 + [i32] + [vp] * 3 + [i32] * 6 + [vp, vp],
     "csb_ce_stats": [vp, i64, vp, i32, i32, vp, vp, vp, i64, vp],
     "csb_ce_grad": [vp, i64, vp, i32, i32, vp, vp, vp, vp, vp, i64, i64, vp],
     "csb_gather_merge": [vp, vp, vp, vp, i64, i32, i64, i64, vp],
@@ -83,7 +85,7 @@ def lib():
 class _CountingLib:
     """Forwards attribute access to the CDLL and counts calls of kernel-launching entry points."""
 
-    _NO_LAUNCH = {"csb_norm_bwd_parts", "csb_colsum_parts", "csb_attn_bwd_splits", "csb_gemm_choice"}
+    _NO_LAUNCH = {"csb_norm_bwd_parts", "csb_colsum_parts", "csb_attn_bwd_splits", "csb_gemm_choice", "csb_lm_stats_parts"}
 
     def __init__(self, raw):
         self._raw = raw

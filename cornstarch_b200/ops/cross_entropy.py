@@ -47,6 +47,25 @@ def _stats(logits, labels, vocab_start):
     return mx, sm, tg
 
 
+def _logits_and_stats(h, weight, lg, labels, vocab_start):
+    """``lg = h weight^T`` and its row statistics; one native call takes them out of the GEMM's epilogue."""
+    T, K = h.shape
+    V = weight.shape[0]
+    grid = all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (h, weight, lg))
+    if T == 0 or K == 0 or not grid or not h.dtype == weight.dtype == lg.dtype == torch.bfloat16:
+        gemm(h, weight, out=lg)
+        return _stats(lg, labels, vocab_start)
+    mx, sm, tg = torch.empty((3, T), dtype=torch.float32, device=h.device).unbind(0)
+    part = torch.empty(2 * nat.lib().csb_lm_stats_parts(V) * T, dtype=torch.float32, device=h.device)
+    nat.check(
+        nat.lib().csb_lm_stats(h.data_ptr(), weight.data_ptr(), lg.data_ptr(), part.data_ptr(), labels.data_ptr(), vocab_start, mx.data_ptr(),
+                               sm.data_ptr(), tg.data_ptr(), T, V, K, h.stride(0), weight.stride(0), lg.stride(0),
+                               nat.status_word(h.device).data_ptr(), nat.stream()),
+        "csb_lm_stats",
+    )
+    return mx, sm, tg
+
+
 def _combine_tp(mx, sm, tg, group):
     if group is None or dist.get_world_size(group) == 1:
         return mx, sm, tg
@@ -74,8 +93,7 @@ class _LinearCEFn(torch.autograd.Function):
         for s in range(0, T, chunk):
             e = min(T, s + chunk)
             lg = buf[s:e] if keep else buf[: e - s]
-            gemm(hidden[s:e], weight, out=lg)
-            mx, sm, tg = _stats(lg, labels[s:e], vocab_start)
+            mx, sm, tg = _logits_and_stats(hidden[s:e], weight, lg, labels[s:e], vocab_start)
             mx, sm, tg = _combine_tp(mx, sm, tg, group)
             row_max[s:e], row_sum[s:e], row_tgt[s:e] = mx, sm, tg
         valid = labels != ignore_index
