@@ -23,9 +23,11 @@
 // dP^T(i+1) is issued as soon as dP^T(i) has been read, so the next exponentials overlap the dV/dK/dQ^T MMAs of iteration i.
 // Per-tile query metadata (LSE, delta, mask rules) is staged in shared memory, a ring stage with Q / dO.
 //
-// What bounds it: shared memory.  The MMAs of an iteration read 192 KB of operands and everything else moves about 130 KB (Q / dO in,
-// dS^T, dQ through its staging, statistics): 2500 of the measured 2450 cycles at 128 B / cycle; the tensor pipe is busy 1676.  Long
-// runs are at the power cap.  Before, the one MMA warp was: 32 MMAs per iteration at 90 cycles of issue each, 3300 cycles; runs of
+// What bounds it: no single unit.  Of the measured 2450 cycles of an iteration the tensor pipe is busy 1676 and the chain of
+// the compute warps takes about 2000 without its waits; the MMAs read 192 KB of operands from shared memory and everything else (Q / dO in,
+// dS^T, dQ through its staging, statistics) moves about 130 KB, 2500 cycles if reads and writes share a port of 128 B (counters, 4096
+// tokens causal: bank reads 35 %, writes 12 %, tensor pipe 53 %, issue slots 34 % of peak).  Long runs are at the power
+// cap.  Before, the one MMA warp was: 32 MMAs per iteration at 90 cycles of issue each, 3300 cycles; runs of
 // MMAs (umma_f16_run_w) and a second MMA warp, which has work for the pipe while the first waits, took that away.  (dQ^T straight from
 // registers by red.global, which spares its two passes through shared memory, takes 65 cycles per warp instruction: 2.0 x the time.)
 // Measured with the delta and conversion passes (32 / 8 heads of 128, before -> now): 8192 tokens causal 1679 -> 1411 us (975

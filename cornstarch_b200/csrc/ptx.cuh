@@ -286,16 +286,6 @@ __device__ __forceinline__ void umma_f16_w(uint32_t d_tmem, uint64_t a_desc, uin
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void umma_f16_ts_w(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // Runs of MMAs of one tile pair as one block of instructions: one elect.sync for all of them and 32-bit steps of the descriptors'
 // address fields, where a call per MMA pays an election and 64-bit additions each time.  Short MMAs (128 x 64 or 128 x 128 x 16 take
 // the pipe 48 or 64 cycles) are issued no faster than that otherwise: eight 128 x 64 x 16 next to busy warps 750 cycles one by
@@ -393,16 +383,6 @@ __device__ __forceinline__ void umma_f16_run4_cg_w(uint32_t d_tmem, uint64_t a_d
         : "memory");
 #undef CSB_UMMA_STEP
   }
-}
-__device__ __forceinline__ void umma_f16_2cta_w(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 __device__ __forceinline__ void umma_commit_w(uint64_t* bar) {
   asm volatile(
