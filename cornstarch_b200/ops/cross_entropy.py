@@ -52,8 +52,8 @@ def _logits_and_stats(h, weight, lg, labels, vocab_start):
     T, K = h.shape
     V = weight.shape[0]
     grid = all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (h, weight, lg))
-    if T == 0 or K == 0 or not grid or not h.dtype == weight.dtype == lg.dtype == torch.bfloat16:
-        gemm(h, weight, out=lg)
+    if T == 0 or K == 0 or not grid or weight.shape[1] != K or not h.dtype == weight.dtype == lg.dtype == torch.bfloat16:
+        gemm(h, weight, out=lg)  # (which refuses what does not fit)
         return _stats(lg, labels, vocab_start)
     mx, sm, tg = torch.empty((3, T), dtype=torch.float32, device=h.device).unbind(0)
     part = torch.empty(2 * nat.lib().csb_lm_stats_parts(V) * T, dtype=torch.float32, device=h.device)
