@@ -394,7 +394,8 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmParams& p, const Epi
       }
       const float LOG2E = 1.4426950408889634f;
       const float m_new = fmaxf(ce_max, fmaxf(mx[0], mx[1]));
-      const uint64_t neg_m = pack_f32x2(-m_new, -m_new), log2e = pack_f32x2(LOG2E, LOG2E);
+      const float m_ref = m_new == -INFINITY ? 0.f : m_new;  // a slab of -inf adds zeros, not exp(-inf + inf)
+      const uint64_t neg_m = pack_f32x2(-m_ref, -m_ref), log2e = pack_f32x2(LOG2E, LOG2E);
       uint64_t sum[2] = {0ull, 0ull};
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
@@ -404,7 +405,7 @@ __device__ __forceinline__ void epilogue_tile_tma(const GemmParams& p, const Epi
       }
       float s0, s1;
       unpack_f32x2(add_f32x2(sum[0], sum[1]), s0, s1);
-      ce_sum = ce_sum * fast_exp2((ce_max - m_new) * LOG2E) + (s0 + s1);
+      ce_sum = ce_sum * fast_exp2((ce_max - m_ref) * LOG2E) + (s0 + s1);
       ce_max = m_new;
       if (last && row < p.M) p.ce_part[static_cast<size_t>(n_blk) * p.M + row] = make_float2(ce_max, ce_sum);
     }
