@@ -7,6 +7,8 @@
 // cornstarch/models/multimodal_language_model/modeling_multimodal_language_model.py:930-936,
 // cross-entropy) and torch.optim.Adam(fused=True)
 // (examples/distributed/run_vlm_hybrid.py:167-169).
+#include <cfloat>
+
 #include "host.h"
 #include "ptx.cuh"
 
@@ -457,7 +459,8 @@ __global__ void __launch_bounds__(512) ce_stats_kernel(const __nv_bfloat16* __re
   __shared__ float sh_m[16], sh_s[16];
   for (long row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* x = logits + row * ld;
-    float mx = -INFINITY, sm = 0.f;
+    // (below every bf16 value but -inf: columns of -inf add zeros, not exp(-inf + inf))
+    float mx = -FLT_MAX, sm = 0.f;
     const int nvec = V / 8;
     for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
       float f[8];
@@ -480,6 +483,7 @@ __global__ void __launch_bounds__(512) ce_stats_kernel(const __nv_bfloat16* __re
       }
       sm += __expf(f - mx);
     }
+    if (mx == -FLT_MAX) mx = -INFINITY;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float om = __shfl_xor_sync(0xffffffffu, mx, o);
