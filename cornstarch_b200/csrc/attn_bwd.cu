@@ -120,16 +120,18 @@ struct BwdCfg {
   static constexpr int COLS = BW_BQ / GROUPS;  // query columns of S^T / dP^T per thread
 };
 
+// For whole warps, with one verdict for all lanes: what follows is warp-wide (tensor-memory loads, elect.sync, __syncwarp), and a
+// lane that gave up alone would leave the others waiting there for good.  (A phase that is over for one lane stays over for all:
+// the next one needs this warp's own arrivals or MMAs.)
 __device__ __forceinline__ bool bw_wait(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, phase)) return true;  // in front of the loop and its set-up
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, phase))) return true;  // in front of the loop and its set-up
   uint64_t t0 = 0;
   for (uint32_t i = 0; i < CSB_SPIN_LIMIT; ++i) {
-    if (mbar_try_wait(bar, phase)) return true;
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, phase))) return true;
     if ((i & 511u) == 511u) {
-      if (*abort_flag) return false;
       const uint64_t now = global_timer_ns();
       if (t0 == 0) t0 = now;
-      else if (now - t0 > wait_limit_ns()) return false;
+      if (__any_sync(0xffffffffu, *abort_flag != 0 || now - t0 > wait_limit_ns())) return false;
     }
   }
   return false;
