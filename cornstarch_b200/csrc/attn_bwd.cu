@@ -120,23 +120,6 @@ struct BwdCfg {
   static constexpr int COLS = BW_BQ / GROUPS;  // query columns of S^T / dP^T per thread
 };
 
-// For whole warps, with one verdict for all lanes: what follows is warp-wide (tensor-memory loads, elect.sync, __syncwarp), and a
-// lane that gave up alone would leave the others waiting there for good.  (A phase that is over for one lane stays over for all:
-// the next one needs this warp's own arrivals or MMAs.)
-__device__ __forceinline__ bool bw_wait(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, phase))) return true;  // in front of the loop and its set-up
-  uint64_t t0 = 0;
-  for (uint32_t i = 0; i < CSB_SPIN_LIMIT; ++i) {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, phase))) return true;
-    if ((i & 511u) == 511u) {
-      const uint64_t now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      if (__any_sync(0xffffffffu, *abort_flag != 0 || now - t0 > wait_limit_ns())) return false;
-    }
-  }
-  return false;
-}
-
 // delta[b][h][q] = sum_d O[b][q][h][d] * dO[b][q][h][d].  Sixteen lanes share a row (8 elements each, D <= 128) and take
 // DELTA_ROWS queries of one head, so that every thread has 2 x DELTA_ROWS 16-byte loads in flight and the results of a block
 // are consecutive.  VEC: rows of both tensors start on 16-byte boundaries.
@@ -344,12 +327,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint64_t do_km = make_desc_kmajor_sw128(smem_u32(smem + L::DO_OFF));
     constexpr uint64_t STAGE = (2 * Q_CHUNK) >> 4;
     const int ksteps_d = p.dk16 / 16;
-    bool ok = n_iter == 0 || bw_wait(kv_full, 0, abort_flag);
+    bool ok = n_iter == 0 || mbar_wait_abort_w(kv_full, 0, abort_flag);
     if (!ok) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; }
     int s_stage = 0, d_stage = 0;  // ring stages of the next S^T and dP^T
     uint32_t s_phase = 0;
     auto issue_st = [&](int it) -> bool {  // into ST[it & 1]; waits for the Q / dO stage of that iteration
-      if (!bw_wait(&q_full[s_stage], s_phase, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; return false; }
+      if (!mbar_wait_abort_w(&q_full[s_stage], s_phase, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; return false; }
       tc_fence_after();
       umma_f16_run_w(tmem_base + (it & 1) * 64, k_km, q_km + s_stage * STAGE, KV_CHUNK, Q_CHUNK, idesc_s, ksteps_d, 0u);
       if (++s_stage == QS) { s_stage = 0; s_phase ^= 1u; }
@@ -369,12 +352,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     uint32_t e_phase = 0;
     for (int it = 0; ok && it + 1 < n_iter; ++it) {
       // dP^T(it + 1) as soon as the compute warps hold dP^T(it) in registers, long before they are done with the iteration
-      if (!bw_wait(dp_read, it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; break; }
+      if (!mbar_wait_abort_w(dp_read, it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; break; }
       tc_fence_after();
       issue_dpt();
       if (it + 2 < n_iter) {
         // S^T(it + 2) goes over P^T(it): dV(it) has to have retired, which is what releases the stage of iteration it
-        if (!bw_wait(&q_empty[e_stage], e_phase, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
+        if (!mbar_wait_abort_w(&q_empty[e_stage], e_phase, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
         if (++e_stage == QS) { e_stage = 0; e_phase ^= 1u; }
         ok = issue_st(it + 2);
       }
@@ -392,12 +375,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     constexpr uint64_t STAGE = (2 * Q_CHUNK) >> 4;
     int st = 0;
     uint32_t st_phase = 0;
-    bool ok = n_iter == 0 || bw_wait(kv_full, 0, abort_flag);
+    bool ok = n_iter == 0 || mbar_wait_abort_w(kv_full, 0, abort_flag);
     if (!ok) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; }
     for (int it = 0; ok && it < n_iter; ++it) {
       // (the stage is full long before; the wait orders this warp's MMAs behind the copies)
-      if (!bw_wait(&q_full[st], st_phase, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; break; }
-      if (!bw_wait(pds_full, it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; break; }
+      if (!mbar_wait_abort_w(&q_full[st], st_phase, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; break; }
+      if (!mbar_wait_abort_w(pds_full, it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; break; }
       tc_fence_after();
       // dV += P^T dO ; dK += dS^T Q   (contraction over the 64 query rows)
       const uint32_t acc = it > 0 ? 1u : 0u;
@@ -405,7 +388,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       umma_f16_run4_w<2, 128>(tmem_dK, dst_km, q_mn + st * STAGE, idesc_dkv, acc);  // 16 columns of dS^T, 16 rows of Q a step
       umma_commit_w(&q_empty[st]);
       if (it > 0) {
-        if (!bw_wait(dq_free, (it - 1) & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_EMPTY); *abort_flag = 1; break; }
+        if (!mbar_wait_abort_w(dq_free, (it - 1) & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_EMPTY); *abort_flag = 1; break; }
         tc_fence_after();
       }
       // dQ^T = K^T dS^T  (contraction over the 128 key rows)
@@ -446,7 +429,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const float delta = qv ? p.delta[idx] : 0.f;
       const int qpos = qv ? (p.q_pos ? p.q_pos[(long)b * p.Sq + q] : q) : 0;
       const int64_t qbits = (qv && p.q_bits) ? p.q_bits[(long)b * p.Sq + q] : 0;
-      if (!bw_wait(&q_empty[st], st_phase, abort_flag)) {
+      if (!mbar_wait_abort_w(&q_empty[st], st_phase, abort_flag)) {
         if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY);
         *abort_flag = 1;
         break;
@@ -532,7 +515,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int x = 0; x < COLS; ++x) mask_word |= (mb[x] != 0u ? 1u : 0u) << x;
         }
       }
-      if (!bw_wait(sdp_full, it & 1, abort_flag)) {
+      if (!mbar_wait_abort_w(sdp_full, it & 1, abort_flag)) {
         if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
         ok = false;
@@ -599,7 +582,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         unpack_f32x2(mul_f32x2(pack_f32x2(pv[x4 * 4 + 2], pv[x4 * 4 + 3]), t1), ds[x4 * 4 + 2], ds[x4 * 4 + 3]);
       }
       if (it > 0) {
-        if (!bw_wait(dq_full, (it - 1) & 1, abort_flag)) {
+        if (!mbar_wait_abort_w(dq_full, (it - 1) & 1, abort_flag)) {
           if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_MISC);
           *abort_flag = 1;
           ok = false;
@@ -623,7 +606,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     // ---- epilogue: dV and dK tiles (every MMA has retired once the last dS^T was consumed); the warps of a lane quarter split
     //      the head-dim columns
-    if (ok && n_iter > 0 && !bw_wait(dq_full, (n_iter - 1) & 1, abort_flag)) {
+    if (ok && n_iter > 0 && !mbar_wait_abort_w(dq_full, (n_iter - 1) & 1, abort_flag)) {
       if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_MISC);
       *abort_flag = 1;
       ok = false;
@@ -682,7 +665,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     float* stage = reinterpret_cast<float*>(smem + L::DQ_OFF + quarter * (BW_BQ * 128));
     BwdCursor cur(it0, n_valid);
     for (int it = 0; it < n_iter; ++it, cur.next()) {
-      if (!bw_wait(dq_full, it & 1, abort_flag)) {
+      if (!mbar_wait_abort_w(dq_full, it & 1, abort_flag)) {
         if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
         break;

@@ -157,21 +157,6 @@ struct AttnSmem {
   static constexpr int DYN_BYTES = TOTAL + 1024;
 };
 
-__device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, phase)) return true;  // in front of the loop and its set-up: 41 cycles for a wait that is over, 75 inside
-  uint64_t t0 = 0;
-  for (uint32_t i = 0; i < CSB_SPIN_LIMIT; ++i) {
-    if (mbar_try_wait(bar, phase)) return true;
-    if ((i & 511u) == 511u) {
-      if (*abort_flag) return false;
-      const uint64_t now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > wait_limit_ns()) return false;
-    }
-  }
-  return false;
-}
-
 template <int NCH>
 __global__ void __launch_bounds__(320, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ KvMaps kvm, const AttnFwdParams p) {
@@ -276,12 +261,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         const int st = it & 1;
         const uint32_t ph = (it >> 1) & 1;
-        if (!at_wait(&k_empty[st], ph ^ 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
+        if (!mbar_wait_abort(&k_empty[st], ph ^ 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
         mbar_expect_tx(&k_full[st], L::KV_BYTES);
 #pragma unroll
         for (int c = 0; c < NCH; ++c)
           tma_load_4d(smem + L::K_OFF + st * L::KV_BYTES + c * CHUNK_BYTES, &kvm.k[sg], &k_full[st], c * 64, hk, row0, b);
-        if (!at_wait(&v_empty[st], ph ^ 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
+        if (!mbar_wait_abort(&v_empty[st], ph ^ 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
         mbar_expect_tx(&v_full[st], L::KV_BYTES);
 #pragma unroll
         for (int c = 0; c < NCH; ++c)
@@ -299,7 +284,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const uint32_t idesc_o = make_idesc_bf16(AT_BM, p.dk16, 0, 1);
       const uint64_t q_desc = make_desc_kmajor_sw128(smem_u32(smem + L::Q_OFF));
       const int ksteps_s = p.dk16 / 16;
-      bool ok = at_wait(q_full, 0, abort_flag);
+      bool ok = mbar_wait_abort_w(q_full, 0, abort_flag);
       if (!ok) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; }
       // number of non-empty key blocks
       int n = 0;
@@ -311,7 +296,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       auto issue_s = [&](uint32_t it) -> bool {
         const int st = it & 1;
         const uint32_t ph = (it >> 1) & 1;
-        if (!at_wait(&k_full[st], ph, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; return false; }
+        if (!mbar_wait_abort_w(&k_full[st], ph, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; return false; }
         tc_fence_after();
         const uint64_t k_desc = make_desc_kmajor_sw128(smem_u32(smem + L::K_OFF + st * L::KV_BYTES));
         umma_f16_run_w(tmem_S + st * 128, q_desc, k_desc, CHUNK_BYTES, CHUNK_BYTES, idesc_s, ksteps_s, 0u);
@@ -327,13 +312,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         const int st = it & 1;
         const uint32_t ph = (it >> 1) & 1;
-        if (!at_wait(&v_full[st], ph, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; break; }
+        if (!mbar_wait_abort_w(&v_full[st], ph, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_FULL); *abort_flag = 1; break; }
         const uint64_t v_desc = make_desc_mnmajor_sw128(smem_u32(smem + L::V_OFF + st * L::KV_BYTES), CHUNK_BYTES);
         // O[h] += P_h V_h for the two column halves of the tile, each as soon as its threads have written P_h (packed
         // bf16 pairs in the first 32 columns of that half of the S buffer: 16 keys of a row = 8 columns per step)
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
-          if (!at_wait(&p_full[hh], it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; ok = false; break; }
+          if (!mbar_wait_abort_w(&p_full[hh], it & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_MISC); *abort_flag = 1; ok = false; break; }
           tc_fence_after();
           umma_f16_ts_run4_w(tmem_O + hh * 128, tmem_S + st * 128 + hh * 64, v_desc + static_cast<uint64_t>((hh * 4 * 2048) >> 4), idesc_o,
                              it > 0 ? 1u : 0u);
@@ -376,7 +361,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int c = cls_row[j];
       if (c == 0) continue;
       const int buf = it & 1;
-      if (!at_wait(&s_full[buf], (it >> 1) & 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); break; }
+      if (!mbar_wait_abort_w(&s_full[buf], (it >> 1) & 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); break; }
       tc_fence_after();
       float s[64];
       {
@@ -394,7 +379,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             kp_s[buf * 128 + r] = kp;
           }
           mbar_arrive(kb_full);
-          if (!at_wait(kb_full, n_partial & 1, abort_flag)) {
+          if (!mbar_wait_abort_w(kb_full, n_partial & 1, abort_flag)) {
             tmem_ld_wait();
             fail(ST_TIMEOUT_MISC);
             break;
@@ -445,7 +430,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const bool need = (m_new - m_used) * p.scale_log2 > 8.f;  // also true when m_used is -inf and m_new is finite
       if (it > 0 && __any_sync(0xffffffffu, need)) {
         // rare (lazy rescale): O[half] is only touched once the previous P V has retired
-        if (!at_wait(pv_done, (it - 1) & 1, abort_flag)) { fail(ST_TIMEOUT_MISC); break; }
+        if (!mbar_wait_abort_w(pv_done, (it - 1) & 1, abort_flag)) { fail(ST_TIMEOUT_MISC); break; }
         tc_fence_after();
         float alpha = 1.f;
         if (need) alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * p.scale_log2);
@@ -487,7 +472,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // run ahead of the MMA warp (S(it+1) is issued before it waits for p_full(it)): while it waits for a slow V tile,
       // p_full could complete two phases, which its parity wait cannot tell from none; a fast thread could also arrive
       // twice within one phase.  The exponentials above are already done, so the wait is normally free.
-      if (it > 0 && !at_wait(pv_done, (it - 1) & 1, abort_flag)) { fail(ST_TIMEOUT_MISC); break; }
+      if (it > 0 && !mbar_wait_abort_w(pv_done, (it - 1) & 1, abort_flag)) { fail(ST_TIMEOUT_MISC); break; }
       tc_fence_before();
       mbar_arrive(&p_full[half]);
       ++it;
@@ -495,14 +480,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // ---- epilogue
     if (ok && it > 0) {
       // (pv_done cannot be used here: two phases may still be pending, which a parity wait cannot tell from none)
-      if (!at_wait(o_done, 0, abort_flag)) fail(ST_TIMEOUT_MISC);
+      if (!mbar_wait_abort_w(o_done, 0, abort_flag)) fail(ST_TIMEOUT_MISC);
     }
     if (ok) {
       // merge the two halves' partial softmax results (running maximum, row sum, accumulator) of this row
       xm_s[half * 128 + r] = m_used;
       xm_s[(2 + half) * 128 + r] = l_sum;
       mbar_arrive(&pair_bar[quarter]);
-      if (!at_wait(&pair_bar[quarter], 0, abort_flag)) fail(ST_TIMEOUT_MISC);
+      if (!mbar_wait_abort_w(&pair_bar[quarter], 0, abort_flag)) fail(ST_TIMEOUT_MISC);
     }
     if (ok) {
       tc_fence_after();

@@ -165,7 +165,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // Free are the V stage (P V of position it - 2 is done; the first two are free at the start) and the K stage that position
         // it + 1 takes (S of position it - 1 is done; the first one at the start).  S is issued a position ahead of P V, so one
         // commit after position it - 2 says both; for it = 1 there is one after the first S.
-        if (!at_wait(&vk_empty[st], ((it >> 1) ^ it ^ 1) & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
+        if (!mbar_wait_abort(&vk_empty[st], ((it >> 1) ^ it ^ 1) & 1, abort_flag)) { atomicCAS(p.status, 0, ST_TIMEOUT_EMPTY); *abort_flag = 1; break; }
         mbar_expect_tx(&vk_full[st], (tn < p.nK ? 2 : 1) * L::TILE_BYTES);
         load(L::V_OFF + st * L::TILE_BYTES, &tm_v, &vk_full[st], hk, t);
         if (tn < p.nK) load(L::K_OFF + (st ^ 1) * L::TILE_BYTES, &tm_k, &vk_full[st], hk, tn);
@@ -224,7 +224,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     uint32_t who, who_next;
     int t = next(who);
     if (t < p.nK) {
-      if (!at_wait(q_full, 0, abort_flag)) fail(ST_TIMEOUT_FULL);
+      if (!mbar_wait_abort_w(q_full, 0, abort_flag)) fail(ST_TIMEOUT_FULL);
       if (ok) {
         tc_fence_after();
         if (who & 1u) issue_s(0, 0);
@@ -235,14 +235,14 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     for (uint32_t it = 0; ok && t < p.nK; ++it) {
       const int tn = next(who_next);
       const int st = it & 1;
-      if (!at_wait(&vk_full[st], (it >> 1) & 1, abort_flag)) { fail(ST_TIMEOUT_FULL); break; }
+      if (!mbar_wait_abort_w(&vk_full[st], (it >> 1) & 1, abort_flag)) { fail(ST_TIMEOUT_FULL); break; }
       tc_fence_after();
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
         if (who & (1u << s)) {
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
-            if (!at_wait(&p_full[s * 2 + u], done[s] & 1, abort_flag)) { fail(ST_TIMEOUT_MISC); break; }
+            if (!mbar_wait_abort_w(&p_full[s * 2 + u], done[s] & 1, abort_flag)) { fail(ST_TIMEOUT_MISC); break; }
             tc_fence_after();
             umma_f16_ts_run4_w(tmem_O + s * 128, tmem_S + s * 128 + u * 32,
                                v_desc + st * TILE_STEP + static_cast<uint64_t>((u * 4 * 2048) >> 4), idesc_o, done[s] > 0 || u > 0 ? 1u : 0u);
@@ -290,7 +290,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       if (c == 0) continue;
       uint32_t w[4] = {0u, 0u, 0u, 0u};
       if (c == 1) tile_mask_words(p, b, j, q, row_valid, rule, lane, kb_w, kp_w, w);  // while S is being computed
-      if (!at_wait(&s_full[s_id], it & 1, abort_flag)) {
+      if (!mbar_wait_abort_w(&s_full[s_id], it & 1, abort_flag)) {
         if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
         ok = false;
@@ -377,7 +377,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       ++it;
     }
     // ---- epilogue
-    if (ok && it > 0 && !at_wait(&o_full[s_id], 0, abort_flag)) {
+    if (ok && it > 0 && !mbar_wait_abort_w(&o_full[s_id], 0, abort_flag)) {
       if (lane == 0) atomicCAS(p.status, 0, ST_TIMEOUT_MISC);
       *abort_flag = 1;
       ok = false;

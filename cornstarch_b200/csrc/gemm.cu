@@ -124,21 +124,6 @@ struct SmemLayout {
   static constexpr int DYN_BYTES = TOTAL + 1024;  // slack for 1024-byte alignment
 };
 
-__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, phase)) return true;  // in front of the loop and its set-up: 41 cycles for a wait that is over, 75 inside
-  uint64_t t0 = 0;
-  for (uint32_t i = 0; i < CSB_SPIN_LIMIT; ++i) {
-    if (mbar_try_wait(bar, phase)) return true;
-    if ((i & 511u) == 511u) {
-      if (*abort_flag) return false;
-      const uint64_t now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > wait_limit_ns()) return false;
-    }
-  }
-  return false;
-}
-
 // Tiles are walked in groups of GROUP_M tile rows (all columns of a group before the next group), so that the thread
 // blocks running at one time share few rows of A and few columns of B (L2 reuse).  16 rows of 128 measured 2.7 % faster
 // than 8 at 8192 x 8192 x 4096 with one thread block per tile; pairs (rows of 256) keep 8.
@@ -584,7 +569,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         for (int kb = 0; kb < p.num_k_blocks; ++kb, ++it) {
           const int s = it % L::STAGES;
           const uint32_t ph = (it / L::STAGES) & 1;
-          if (!wait_or_abort(&empty_bar[s], ph ^ 1, abort_flag)) {
+          if (!mbar_wait_abort(&empty_bar[s], ph ^ 1, abort_flag)) {
             atomicExch(p.status, ST_TIMEOUT_EMPTY);
             *abort_flag = 1;
             ok = false;
@@ -630,7 +615,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       for (int tile = work_first; tile < num_tiles && ok; tile += work_step, ++local_tile) {
         const uint32_t acc = local_tile & 1;
         const uint32_t acc_ph = (local_tile >> 1) & 1;
-        if (!wait_or_abort(&tmem_empty[acc], acc_ph ^ 1, abort_flag)) {
+        if (!mbar_wait_abort_w(&tmem_empty[acc], acc_ph ^ 1, abort_flag)) {
           atomicExch(p.status, ST_TIMEOUT_TMEM_EMPTY);
           *abort_flag = 1;
           break;
@@ -638,7 +623,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-          if (!wait_or_abort(&full_bar[s], ph, abort_flag)) {
+          if (!mbar_wait_abort_w(&full_bar[s], ph, abort_flag)) {
             atomicExch(p.status, ST_TIMEOUT_FULL);
             *abort_flag = 1;
             ok = false;
@@ -666,7 +651,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       m_blk = m_blk * CG + cta_rank;
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
-      if (!wait_or_abort(&tmem_full[acc], acc_ph, abort_flag)) {
+      if (!mbar_wait_abort_w(&tmem_full[acc], acc_ph, abort_flag)) {
         if (lane == 0) atomicExch(p.status, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
         ok = false;

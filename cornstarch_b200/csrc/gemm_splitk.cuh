@@ -90,7 +90,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     if (lane == 0) {
       for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
         const int s = it % L::STAGES;
-        if (!wait_or_abort(&empty_bar[s], ((it / L::STAGES) & 1) ^ 1, abort_flag)) {
+        if (!mbar_wait_abort(&empty_bar[s], ((it / L::STAGES) & 1) ^ 1, abort_flag)) {
           atomicExch(p.status, ST_TIMEOUT_EMPTY);
           *abort_flag = 1;
           break;
@@ -125,7 +125,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     uint32_t ph = 0;
     bool ok = true;
     for (int kb = kb0; kb < kb1; ++kb) {
-      if (!wait_or_abort(&full_bar[s], ph, abort_flag)) {
+      if (!mbar_wait_abort_w(&full_bar[s], ph, abort_flag)) {
         atomicExch(p.status, ST_TIMEOUT_FULL);
         *abort_flag = 1;
         ok = false;
@@ -141,7 +141,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     __syncwarp();
   } else if (warp >= 4) {
     const int quarter = warp & 3, r = quarter * 32 + lane;
-    if (wait_or_abort(tmem_full, 0, abort_flag)) {  // every MMA has retired: the stages are free
+    if (mbar_wait_abort_w(tmem_full, 0, abort_flag)) {  // every MMA has retired: the stages are free
       tc_fence_after();
 #pragma unroll
       for (int g = 0; g < SK_BN / 32; ++g) {

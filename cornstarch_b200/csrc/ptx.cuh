@@ -159,6 +159,38 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase) {
   return false;
 }
 
+// The same for a thread of a block whose threads tell one another through `abort_flag` (shared memory) that one of them gave up.
+__device__ __forceinline__ bool mbar_wait_abort(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
+  if (mbar_try_wait(bar, phase)) return true;  // in front of the loop and its set-up: 41 cycles for a wait that is over, 75 inside
+  uint64_t t0 = 0;
+  for (uint32_t i = 0; i < CSB_SPIN_LIMIT; ++i) {
+    if (mbar_try_wait(bar, phase)) return true;
+    if ((i & 511u) == 511u) {
+      if (*abort_flag) return false;
+      const uint64_t now = global_timer_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > wait_limit_ns()) return false;
+    }
+  }
+  return false;
+}
+// For whole warps, with one verdict for all lanes: what follows is warp-wide (elect.sync, tensor-memory loads, __syncwarp), and a
+// lane that gave up alone would leave the others waiting there for good.  (A phase that is over for one lane stays over for all:
+// the next one needs this warp's own arrivals or MMAs.)
+__device__ __forceinline__ bool mbar_wait_abort_w(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, phase))) return true;
+  uint64_t t0 = 0;
+  for (uint32_t i = 0; i < CSB_SPIN_LIMIT; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, phase))) return true;
+    if ((i & 511u) == 511u) {
+      const uint64_t now = global_timer_ns();
+      if (t0 == 0) t0 = now;
+      if (__any_sync(0xffffffffu, *abort_flag != 0 || now - t0 > wait_limit_ns())) return false;
+    }
+  }
+  return false;
+}
+
 // ----------------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
