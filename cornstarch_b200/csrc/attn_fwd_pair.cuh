@@ -345,6 +345,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const float m_new = fmaxf(max3(mx[0], mx[1], mx[2]), fmaxf(mx[3], m_used));
         const bool need = (m_new - m_used) * p.scale_log2 > 8.f;  // also true when m_used is -inf and m_new is finite
         if (!__any_sync(0xffffffffu, need)) break;
+        tmem_st_wait();  // stores to one address are in no order without it: P of the new maximum goes over the first one
         if (it > 0) {
           // lazy rescale; s_full of this tile says that the previous P V of this stream has retired
           float alpha = 1.f;
