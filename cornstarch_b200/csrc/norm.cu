@@ -11,7 +11,7 @@
 
 namespace csb {
 
-constexpr int NORM_MAX_H = 8192;  // the backward's 1024 threads hold one 16-byte vector each
+constexpr int NORM_MAX_H = 8192;  // the backward's largest block: 512 threads with two 16-byte vectors each (norm_bwd_shape)
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -33,7 +33,7 @@ __device__ __forceinline__ float row_sum(float v, float* sh, uint32_t& n_calls) 
   return warp_sum(l < (int)(blockDim.x >> 5) ? buf[l] : 0.f);
 }
 
-// Two such sums with the barrier of one; `sh` holds 128 floats.
+// Two such sums with the barrier of one; `sh` holds 128 floats on an 8-byte boundary.
 template <bool ONE_WARP>
 __device__ __forceinline__ void row_sum2(float& a, float& b, float* sh, uint32_t& n_calls) {
   a = warp_sum(a);
@@ -248,7 +248,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                 const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
                 __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial, float* __restrict__ db_partial,
                 int rows, int H, float w_offset) {
-  __shared__ float sh[128];
+  __shared__ __align__(16) float sh[128];
   uint32_t n_sums = 0;
   const int lanes = ONE_WARP ? 32 : blockDim.x;
   const int c = ONE_WARP ? (threadIdx.x & 31) : threadIdx.x;  // this thread's vectors of the row: c, c + lanes, ...
@@ -344,7 +344,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
   }
   if constexpr (ONE_WARP) {
     // the warps of a block add up their sums: one partial row per block
-    __shared__ float part[8][2][256];
+    __shared__ __align__(16) float part[8][2][256];  // written in pairs
     const int wi = threadIdx.x >> 5;
     if (c < nvec) {
 #pragma unroll
@@ -550,6 +550,8 @@ CSB_API int csb_norm_bwd(int is_layernorm, const void* dy, const void* h, const 
   auto W = reinterpret_cast<const __nv_bfloat16*>(w);
   auto DR = reinterpret_cast<const __nv_bfloat16*>(dres);
   auto DX = reinterpret_cast<__nv_bfloat16*>(dx);
+  constexpr int LARGEST_NV = 2, LARGEST_THREADS = 512;
+  static_assert(LARGEST_NV * LARGEST_THREADS * 8 == NORM_MAX_H, "every admitted row has its threads");
 #define CSB_NORM_BWD(LN, OW, NV, MT, MB)                                                                                     \
   norm_bwd_kernel<LN, OW, NV, MT, MB><<<grid, shape.threads, 0, s>>>(DY, Hh, W, mean, rstd, DR, DX, dw_partial, db_partial, rows, H, w_offset)
 #define CSB_NORM_BWD_LN(OW, NV, MT, MB) \
@@ -559,7 +561,7 @@ CSB_API int csb_norm_bwd(int is_layernorm, const void* dy, const void* h, const 
   else if (shape.nv == 1) { CSB_NORM_BWD_LN(false, 1, 512, 2); }
   else if (shape.threads <= 256) { CSB_NORM_BWD_LN(false, 2, 256, 2); }
   else if (shape.threads <= 320) { CSB_NORM_BWD_LN(false, 2, 320, 2); }
-  else { CSB_NORM_BWD_LN(false, 2, 512, 1); }
+  else { CSB_NORM_BWD_LN(false, LARGEST_NV, LARGEST_THREADS, 1); }
 #undef CSB_NORM_BWD_LN
 #undef CSB_NORM_BWD
   int r = launch_result();
