@@ -4,8 +4,13 @@
 // What it replaces is Python around the same entry points of libcornstarch_b200.so: three to ten tensor methods and allocations
 // and one ctypes call of up to 45 arguments per operator, 20 to 45 us of host time where the kernels of a layer of a few thousand
 // tokens take 3 to 40 us.  The autograd functions stay in Python (hooks, saved tensors, transforms and buffers see the same
-// tensors as before); they hand their tensors over here.  Every function answers None for a form that it does not take: the
-// Python statement of the operator decides what happens then (another route, a copy, an error).
+// tensors as before); they hand their tensors over here.  A function answers None for a form that it does not take (activations
+// take all that Python sends them): the Python statement of the operator decides what happens then (another route, a copy, an
+// error).
+//
+// What allocates or launches runs without the GIL (60 ns a call), as calls through ctypes do: a launch waits while the stream's queue is full, an allocation
+// may wait for the device, and the threads that watch over a hanging step are Python threads.  What is Python (arguments, results, the
+// one look-up of a status word) is done before, after, or with the GIL taken back for it.
 //
 // The kernels' entry points are looked up once in the library that ctypes has loaded (bind), so there is one library per process
 // whichever file it came from.
@@ -17,34 +22,41 @@
 #include <optional>
 #include <stdexcept>
 #include <string>
+#include <tuple>
 #include <unordered_map>
 #include <vector>
 
 namespace py = pybind11;
 using at::Tensor;
 using OptTensor = std::optional<Tensor>;
+using Tensor2 = std::tuple<Tensor, Tensor>;  // (undefined tensors become None)
+using Tensor3 = std::tuple<Tensor, Tensor, Tensor>;
+using Tensor5 = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor>;
 
 namespace {
 
-std::unordered_map<std::string, void*> g_entry;
 std::atomic<long> g_launches{0};
 py::object* g_status_word = nullptr;  // Python: device index -> address of its status word
 constexpr int MAX_DEVICES = 64;
 std::atomic<int*> g_status[MAX_DEVICES];
 
 // One exported function of the library; counted like a call through ctypes.
-template <typename F>
-struct Entry {
+struct EntryPoint {
   const char* name;
-  F fn = nullptr;
-  explicit Entry(const char* n) : name(n) {}
+  std::atomic<void*> address{nullptr};  // set by bind, read without the GIL
+  explicit EntryPoint(const char* n) : name(n) { all().push_back(this); }
+  static std::vector<EntryPoint*>& all() {
+    static std::vector<EntryPoint*> list;
+    return list;
+  }
+};
+template <typename F>
+struct Entry : EntryPoint {
+  using EntryPoint::EntryPoint;
   F get() {
-    if (fn == nullptr) {
-      auto it = g_entry.find(name);
-      if (it == g_entry.end()) throw std::runtime_error(std::string("host_ops: no entry point ") + name);
-      fn = reinterpret_cast<F>(it->second);
-    }
-    return fn;
+    void* p = address.load();
+    if (p == nullptr) throw std::runtime_error(std::string("host_ops: no entry point ") + name);
+    return reinterpret_cast<F>(p);
   }
 };
 void check(int code, const char* what) {
@@ -59,6 +71,7 @@ int* status_word(const Tensor& t) {
   if (i < 0 || i >= MAX_DEVICES) throw std::runtime_error("host_ops: device index");
   int* p = g_status[i].load();
   if (p == nullptr) {
+    py::gil_scoped_acquire gil;
     p = reinterpret_cast<int*>((*g_status_word)(i).cast<uintptr_t>());
     g_status[i].store(p);
   }
@@ -108,22 +121,22 @@ void launch_gemm(const Tensor& a, const Tensor& b, void* out, const void* bias, 
                      fp32, acc, act, tile_n, max_ctas, status_word(a), stream()),
         "csb_gemm_bf16");
 }
-py::object gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const OptTensor& bias, int act, const OptTensor& out_, bool acc, int tile_n,
+OptTensor gemm(const Tensor& a, const Tensor& b, bool a_mn, bool b_mn, const OptTensor& bias, int act, const OptTensor& out_, bool acc, int tile_n,
                 int max_ctas) {
-  if (!gemm_operand(a) || !gemm_operand(b)) return py::none();
+  if (!gemm_operand(a) || !gemm_operand(b)) return std::nullopt;
   const int64_t M = a.size(a_mn ? 1 : 0), K = a.size(a_mn ? 0 : 1), N = b.size(b_mn ? 1 : 0);
-  if (b.size(b_mn ? 0 : 1) != K || M == 0 || N == 0 || K == 0) return py::none();
-  if (bias && (!bf16(*bias) || !bias->is_contiguous() || bias->numel() != N)) return py::none();
+  if (b.size(b_mn ? 0 : 1) != K || M == 0 || N == 0 || K == 0) return std::nullopt;
+  if (bias && (!bf16(*bias) || !bias->is_contiguous() || bias->numel() != N)) return std::nullopt;
   Tensor out;
   if (out_) {
     out = *out_;
-    if (out.dim() != 2 || out.size(0) != M || out.size(1) != N || out.stride(1) != 1 || !grad_type(out) || !fits_int(out.stride(0))) return py::none();
+    if (out.dim() != 2 || out.size(0) != M || out.size(1) != N || out.stride(1) != 1 || !grad_type(out) || !fits_int(out.stride(0))) return std::nullopt;
   } else {
     out = at::empty({M, N}, a.options());
     acc = false;
   }
   launch_gemm(a, b, out.data_ptr(), ptr(bias), M, N, K, out.stride(0), a_mn, b_mn, is_fp32(out), acc, act, tile_n, max_ctas);
-  return py::cast(out);
+  return out;
 }
 
 // ------------------------------------------------------------------------------------------------------- linear layers
@@ -152,25 +165,25 @@ bool cols_gemm(const Tensor& x2, const std::vector<Tensor>& ws, const std::vecto
 }
 
 // (out, x as 2-D): the concatenated projections of x; one GEMM where the weights (and biases) are adjacent, else one each.
-py::object linear_fwd(const Tensor& x, const std::vector<Tensor>& ws, const std::vector<OptTensor>& bs) {
-  if (!x.is_cuda() || !bf16(x) || x.dim() < 1 || x.numel() == 0) return py::none();
+std::optional<Tensor2> linear_fwd(const Tensor& x, const std::vector<Tensor>& ws, const std::vector<OptTensor>& bs) {
+  if (!x.is_cuda() || !bf16(x) || x.dim() < 1 || x.numel() == 0) return std::nullopt;
   const int64_t K = x.size(-1);
   int64_t N = 0;
   for (const Tensor& w : ws) {
-    if (!gemm_operand(w) || w.size(1) != K || w.size(0) == 0) return py::none();
+    if (!gemm_operand(w) || w.size(1) != K || w.size(0) == 0) return std::nullopt;
     N += w.size(0);
   }
   const bool has_bias = bs[0].has_value();
   std::vector<Tensor> biases;
   for (size_t i = 0; i < ws.size(); ++i) {
-    if (bs[i].has_value() != has_bias) return py::none();
+    if (bs[i].has_value() != has_bias) return std::nullopt;
     if (has_bias) {
-      if (!bf16(*bs[i]) || !bs[i]->is_contiguous() || bs[i]->numel() != ws[i].size(0)) return py::none();
+      if (!bf16(*bs[i]) || !bs[i]->is_contiguous() || bs[i]->numel() != ws[i].size(0)) return std::nullopt;
       biases.push_back(*bs[i]);
     }
   }
   Tensor x2 = as_2d(x);
-  if (!gemm_operand(x2)) return py::none();
+  if (!gemm_operand(x2)) return std::nullopt;
   std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
   shape.back() = N;
   Tensor out = at::empty(shape, x.options());
@@ -192,7 +205,7 @@ py::object linear_fwd(const Tensor& x, const std::vector<Tensor>& ws, const std:
       o += ws[i].size(0) * 2;
     }
   }
-  return py::make_tuple(out, x2);
+  return Tensor2(out, x2);
 }
 
 using LinearBwdFn = int (*)(const void*, const void*, const void*, void*, void*, void*, float*, int, int, int, int, int, int, int, int, int, int,
@@ -203,10 +216,10 @@ Entry<PartsFn> e_colsum_parts("csb_colsum_parts");
 
 // (dx or None, dW, db or None) of a linear layer whose operands the caller has looked over; w_main / b_main: the buffers that dW and
 // db are added to.
-py::object linear_bwd(const Tensor& dy2, const Tensor& x2, const Tensor& w, bool need_x, const OptTensor& w_main, bool has_bias, const OptTensor& b_main) {
-  if (!gemm_operand(dy2) || !gemm_operand(x2) || !gemm_operand(w)) return py::none();
+std::optional<Tensor3> linear_bwd(const Tensor& dy2, const Tensor& x2, const Tensor& w, bool need_x, const OptTensor& w_main, bool has_bias, const OptTensor& b_main) {
+  if (!gemm_operand(dy2) || !gemm_operand(x2) || !gemm_operand(w)) return std::nullopt;
   const int64_t T = dy2.size(0), N = w.size(0), K = w.size(1);
-  if (T == 0 || N % 8 || K % 8 || N == 0 || K == 0) return py::none();
+  if (T == 0 || N % 8 || K % 8 || N == 0 || K == 0) return std::nullopt;
   Tensor dW = w_main ? *w_main : at::empty({N, K}, dy2.options()), db, scratch, dx;
   if (has_bias) {
     scratch = at::empty({e_colsum_parts.get()((int)T) * N}, dy2.options().dtype(at::kFloat));
@@ -219,7 +232,7 @@ py::object linear_bwd(const Tensor& dy2, const Tensor& x2, const Tensor& w, bool
                            (int)K, (int)dy2.stride(0), (int)x2.stride(0), (int)w.stride(0), (int)dW.stride(0), is_fp32(dW), w_main.has_value(),
                            has_bias && is_fp32(db), b_main.has_value(), status_word(dy2), stream()),
         "csb_linear_bwd");
-  return py::make_tuple(need_x ? py::cast(dx) : py::none(), dW, has_bias ? py::cast(db) : py::none());
+  return Tensor3(dx, dW, db);
 }
 
 // --------------------------------------------------------------------------------------------------------------- norms
@@ -231,9 +244,9 @@ Entry<NormBwdFn> e_norm_bwd("csb_norm_bwd");
 Entry<PartsFn> e_norm_parts("csb_norm_bwd_parts");
 
 // (y, h or None, what the backward normalises, mean or None, rstd)
-py::object norm_fwd(const Tensor& x, const OptTensor& res, const Tensor& w, const OptTensor& b, double eps, bool is_ln, double w_offset) {
+std::optional<Tensor5> norm_fwd(const Tensor& x, const OptTensor& res, const Tensor& w, const OptTensor& b, double eps, bool is_ln, double w_offset) {
   const int64_t H = x.size(-1);
-  if (x.numel() == 0) return py::none();
+  if (x.numel() == 0) return std::nullopt;
   const Tensor x2 = dense(x.reshape({-1, H}));
   const int64_t rows = x2.size(0);
   Tensor r2, h, mean;
@@ -248,13 +261,13 @@ py::object norm_fwd(const Tensor& x, const OptTensor& res, const Tensor& w, cons
                          is_ln ? static_cast<float*>(mean.data_ptr()) : nullptr, static_cast<float*>(rstd.data_ptr()), (int)rows, (int)H, (float)eps,
                          (float)w_offset, stream()),
         "csb_norm_fwd");
-  return py::make_tuple(y.view(x.sizes()), res ? py::cast(h.view(x.sizes())) : py::none(), res ? h : x2, is_ln ? py::cast(mean) : py::none(), rstd);
+  return Tensor5(y.view(x.sizes()), res ? h.view(x.sizes()) : Tensor(), res ? h : x2, mean, rstd);
 }
 // (dx, dw, db or None); w_main / b_main: buffers to add to instead of new gradients
-py::object norm_bwd(const Tensor& dy, const OptTensor& dh, const Tensor& hs, const Tensor& w, const OptTensor& mean, const Tensor& rstd, bool is_ln,
+std::optional<Tensor3> norm_bwd(const Tensor& dy, const OptTensor& dh, const Tensor& hs, const Tensor& w, const OptTensor& mean, const Tensor& rstd, bool is_ln,
                     bool has_b, double w_offset, const OptTensor& w_main, const OptTensor& b_main) {
   const int64_t rows = hs.size(0), H = hs.size(1);
-  if (rows == 0) return py::none();
+  if (rows == 0) return std::nullopt;
   const Tensor dy2 = dense(dy.reshape({-1, H}));
   Tensor dres, dbp, dw, db;
   if (dh) dres = dense(dh->reshape({-1, H}));
@@ -272,7 +285,7 @@ py::object norm_bwd(const Tensor& dy, const OptTensor& dh, const Tensor& hs, con
                          bias ? static_cast<float*>(dbp.data_ptr()) : nullptr, dw.data_ptr(), db.defined() ? db.data_ptr() : nullptr, is_fp32(dw), main,
                          (int)rows, (int)H, (float)w_offset, stream()),
         "csb_norm_bwd");
-  return py::make_tuple(dx, dw, db.defined() ? py::cast(db) : py::none());
+  return Tensor3(dx, dw, db);
 }
 
 // ---------------------------------------------------------------------------------------------------------- activations
@@ -285,12 +298,12 @@ Entry<ActBwdFn> e_act_bwd("csb_act_bwd");
 Entry<GluFwdFn> e_glu_fwd("csb_glu_fwd");
 Entry<GluBwdFn> e_glu_bwd("csb_glu_bwd");
 
-py::object act_fwd(const Tensor& x, int kind) {
+Tensor2 act_fwd(const Tensor& x, int kind) {
   const Tensor xc = dense(x);
   Tensor y = at::empty_like(xc);
   ++g_launches;
   check(e_act_fwd.get()(xc.data_ptr(), y.data_ptr(), xc.numel(), kind, stream()), "csb_act_fwd");
-  return py::make_tuple(y, xc);
+  return {y, xc};
 }
 Tensor act_bwd(const Tensor& xc, const Tensor& dy, int kind) {
   const Tensor d = dense(dy);
@@ -299,7 +312,7 @@ Tensor act_bwd(const Tensor& xc, const Tensor& dy, int kind) {
   check(e_act_bwd.get()(xc.data_ptr(), d.data_ptr(), dx.data_ptr(), xc.numel(), kind, stream()), "csb_act_bwd");
   return dx;
 }
-py::object glu_fwd(const Tensor& gu, int act) {
+Tensor2 glu_fwd(const Tensor& gu, int act) {
   const int64_t I = gu.size(-1) / 2;
   const Tensor g2 = dense(gu.reshape({-1, 2 * I}));
   std::vector<int64_t> shape(gu.sizes().begin(), gu.sizes().end());
@@ -307,7 +320,7 @@ py::object glu_fwd(const Tensor& gu, int act) {
   Tensor y = at::empty(shape, gu.options());
   ++g_launches;
   check(e_glu_fwd.get()(g2.data_ptr(), y.data_ptr(), g2.size(0), (int)I, act, stream()), "csb_glu_fwd");
-  return py::make_tuple(y, g2);
+  return {y, g2};
 }
 Tensor glu_bwd(const Tensor& g2, const Tensor& dy, int act) {
   const int64_t I = g2.size(1) / 2;
@@ -333,24 +346,24 @@ bool attn_layout(const Tensor& t) {
   return t.dim() == 4 && t.stride(3) == 1 && t.stride(2) == t.size(3) && t.stride(1) % 8 == 0 && on_grid(t) && t.is_cuda() && bf16(t);
 }
 // (out, lse); the mask is a mode with optional per-token bits and positions ([B, S], dense) and its class map
-py::object attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, int mode, const OptTensor& qb, const OptTensor& kb,
+std::optional<Tensor2> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, int mode, const OptTensor& qb, const OptTensor& kb,
                     const OptTensor& qp, const OptTensor& kp, const OptTensor& cls) {
-  if (!attn_layout(q) || !attn_layout(k) || !attn_layout(v)) return py::none();
+  if (!attn_layout(q) || !attn_layout(k) || !attn_layout(v)) return std::nullopt;
   const int64_t B = q.size(0), Sq = q.size(1), Hq = q.size(2), D = q.size(3), Sk = k.size(1), Hk = k.size(2);
-  if (k.size(0) != B || k.size(3) != D || v.sizes() != k.sizes() || q.numel() == 0 || k.numel() == 0) return py::none();
+  if (k.size(0) != B || k.size(3) != D || v.sizes() != k.sizes() || q.numel() == 0 || k.numel() == 0) return std::nullopt;
   Tensor out = at::empty({B, Sq, Hq, D}, q.options()), lse = at::empty({B, Hq, Sq}, q.options().dtype(at::kFloat));
   ++g_launches;
   check(e_attn_fwd.get()(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), static_cast<float*>(lse.data_ptr()), (int)B, (int)Sq, (int)Sk,
                          (int)Hq, (int)Hk, (int)D, q.stride(1), q.stride(0), k.stride(1), k.stride(0), v.stride(1), v.stride(0), out.stride(1),
                          out.stride(0), (float)scale, mode, ptr(qb), ptr(kb), ptr(qp), ptr(kp), ptr(cls), status_word(q), stream()),
         "csb_attn_fwd");
-  return py::make_tuple(out, lse);
+  return Tensor2(out, lse);
 }
-py::object attn_bwd(const Tensor& do_, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse, const Tensor& acc, double scale,
+std::optional<Tensor3> attn_bwd(const Tensor& do_, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse, const Tensor& acc, double scale,
                     int mode, const OptTensor& qb, const OptTensor& kb, const OptTensor& qp, const OptTensor& kp, const OptTensor& cls, const OptTensor& dq_,
                     const OptTensor& dk_, const OptTensor& dv_) {
   const int64_t B = q.size(0), Sq = q.size(1), Hq = q.size(2), D = q.size(3), Sk = k.size(1), Hk = k.size(2);
-  if (q.numel() == 0 || k.numel() == 0) return py::none();
+  if (q.numel() == 0 || k.numel() == 0) return std::nullopt;
   const Tensor dout = do_.stride(3) != 1 || do_.stride(2) != D || do_.stride(1) % 8 ? do_.contiguous() : do_;
   const auto f32 = q.options().dtype(at::kFloat);
   Tensor dq = dq_ ? *dq_ : at::empty({B, Sq, Hq, D}, q.options()), dk = dk_ ? *dk_ : at::empty({B, Sk, Hk, D}, q.options()),
@@ -366,28 +379,32 @@ py::object attn_bwd(const Tensor& do_, const Tensor& q, const Tensor& k, const T
                          dk.stride(0), dv.stride(1), dv.stride(0), (float)scale, mode, ptr(qb), ptr(kb), ptr(qp), ptr(kp), ptr(cls), status_word(q),
                          stream(), splits > 1 ? static_cast<float*>(part.data_ptr()) : nullptr, splits),
         "csb_attn_bwd");
-  return py::make_tuple(dq, dk, dv);
+  return Tensor3(dq, dk, dv);
 }
 
 }  // namespace
 
 PYBIND11_MODULE(_host_ops, m) {
   m.def("bind", [](const std::unordered_map<std::string, uintptr_t>& entries, py::object status) {
-    for (const auto& e : entries) g_entry[e.first] = reinterpret_cast<void*>(e.second);
+    for (EntryPoint* e : EntryPoint::all()) {
+      const auto it = entries.find(e->name);
+      if (it != entries.end()) e->address.store(reinterpret_cast<void*>(it->second));
+    }
     g_status_word = new py::object(std::move(status));  // kept for the life of the process
   });
   m.def("launches", [] { return g_launches.load(); });
-  m.def("as_2d", &as_2d);
+  const auto no_gil = py::call_guard<py::gil_scoped_release>();
+  m.def("as_2d", &as_2d, no_gil);
   m.def("fuse_adjacent", [](const std::vector<Tensor>& ts) { return fuse_adjacent(ts, 2); });
-  m.def("gemm", &gemm);
-  m.def("linear_fwd", &linear_fwd);
-  m.def("linear_bwd", &linear_bwd);
-  m.def("norm_fwd", &norm_fwd);
-  m.def("norm_bwd", &norm_bwd);
-  m.def("act_fwd", &act_fwd);
-  m.def("act_bwd", &act_bwd);
-  m.def("glu_fwd", &glu_fwd);
-  m.def("glu_bwd", &glu_bwd);
-  m.def("attn_fwd", &attn_fwd);
-  m.def("attn_bwd", &attn_bwd);
+  m.def("gemm", &gemm, no_gil);
+  m.def("linear_fwd", &linear_fwd, no_gil);
+  m.def("linear_bwd", &linear_bwd, no_gil);
+  m.def("norm_fwd", &norm_fwd, no_gil);
+  m.def("norm_bwd", &norm_bwd, no_gil);
+  m.def("act_fwd", &act_fwd, no_gil);
+  m.def("act_bwd", &act_bwd, no_gil);
+  m.def("glu_fwd", &glu_fwd, no_gil);
+  m.def("glu_bwd", &glu_bwd, no_gil);
+  m.def("attn_fwd", &attn_fwd, no_gil);
+  m.def("attn_bwd", &attn_bwd, no_gil);
 }

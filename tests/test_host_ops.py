@@ -1,6 +1,11 @@
 """The native host path (``csrc/host_ops.cpp``) against the Python statement of the same operators: the same kernels with the same
 arguments, so the same bits, and every form that it does not take still goes where it went."""
 
+import subprocess
+import sys
+import threading
+import time
+
 import pytest
 import torch
 
@@ -184,3 +189,117 @@ def test_projections_of_separate_weights(widths, one, T, bias):
     assert nat.launch_count - before == (1 if one else len(widths))
     ref = torch.cat([x.double() @ w.double().t() + (b.double() if b is not None else 0) for w, b in zip(ws, bs)], -1)
     assert (y.double() - ref).norm() <= 2.0**-8 * ref.norm() and (y.double() - ref).abs().max() <= 2.0**-7 * ref.abs().max()
+
+
+# An entry point that takes its time (libc's usleep under the name of one that takes an int) with another Python thread beside it.  In a
+# process of its own: the entry points are bound once per process.  getpid stands in for the launch behind it, refused as code != 0.
+SLOW_ENTRY = """
+import ctypes, importlib.util, threading, time, torch
+from cornstarch_b200.csrc.build import HOST_OPS_PATH
+spec = importlib.util.spec_from_file_location("_host_ops", HOST_OPS_PATH)
+host = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(host)
+libc = ctypes.CDLL(None)
+at = lambda f: ctypes.cast(f, ctypes.c_void_p).value
+host.bind({"csb_norm_bwd_parts": at(libc.usleep), "csb_norm_bwd": at(libc.getpid)}, lambda index: 0)
+ticks, stop = [], threading.Event()
+def watch():
+    while not stop.is_set():
+        ticks.append(time.monotonic())
+        time.sleep(0.01)
+t = threading.Thread(target=watch)
+x, w = torch.zeros(500_000, 8, dtype=torch.bfloat16), torch.zeros(8, dtype=torch.bfloat16)
+t.start()
+t0 = time.monotonic()
+try:
+    host.norm_bwd(x, None, x, w, None, torch.zeros(500_000), False, False, 0.0, None, None)
+except RuntimeError:
+    pass
+t1 = time.monotonic()
+stop.set()
+t.join()
+assert t1 - t0 >= 0.5, "the entry point was not called"
+print(sum(t0 < k < t1 for k in ticks))
+"""
+
+
+def test_other_threads_run_during_a_native_call():
+    out = subprocess.run([sys.executable, "-c", SLOW_ENTRY], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    assert int(out.stdout.split()[-1]) >= 10  # of about 50; with the GIL held at most one
+
+
+@pytest.mark.gpu
+def test_other_threads_run_while_the_launch_queue_is_full():
+    """A launch behind a full queue waits for the device (here for one long kernel); a watchdog thread must not wait with it."""
+    x = _randn(64, 64)
+    E.activation(x, "silu")
+    torch.cuda.synchronize()
+    gaps, stop = [0.0], threading.Event()
+
+    def watch():
+        last = time.monotonic()
+        while not stop.is_set():
+            time.sleep(0.005)
+            now = time.monotonic()
+            gaps[0], last = max(gaps[0], now - last), now
+
+    t = threading.Thread(target=watch)
+    t.start()
+    torch.cuda._sleep(2_000_000_000)  # about a second
+    t0 = time.monotonic()
+    with torch.no_grad():
+        for _ in range(4000):  # more than a queue holds
+            E.activation(x, "silu")
+    blocked = time.monotonic() - t0
+    stop.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert blocked >= 0.5, "the queue was never full"
+    assert gaps[0] < 0.25
+
+
+def _layer(seed):
+    """A small layer forward and backward through every function of the native host path, on the current stream."""
+    x = _leaves([_randn(3, 70, 128, seed=seed)])[0]
+    ws = _leaves([_randn(n, 128, seed=seed + i) * 0.1 for i, n in enumerate((128, 64, 64))])
+    o, w = _leaves([_randn(128, 128, seed=seed + 5) * 0.1, _randn(128, seed=seed + 6)])
+    y, h = E.rms_norm(x, w, 1e-5, x)
+    q, k, v = (t.contiguous().view(3, 70, -1, 64) for t in torch.split(L.multi_linear(y, ws), (128, 64, 64), -1))
+    a = A.attention(q, k, v, A.AttnMask.causal()).reshape(3, 70, 128)
+    z = E.activation(L.linear(a, o), "gelu") + h
+    z = E.glu(torch.cat([z, h], -1), "silu")
+    z.backward(_randn(*z.shape, seed=seed + 7))
+    return [z.detach(), *(t.grad for t in (*ws, o, w))]  # (x.grad: dQ is summed in no fixed order)
+
+
+@pytest.mark.gpu
+def test_streams_and_threads_of_their_own():
+    """Four threads with a stream each, several passes, against the same work in one thread on the default stream."""
+    seeds = range(4)
+    want = [_layer(10 * s) for s in seeds]
+    torch.cuda.synchronize()
+    got, errors = [[] for _ in seeds], []
+
+    def work(s):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                for _ in range(5):
+                    got[s].append(_layer(10 * s))
+            stream.synchronize()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in seeds]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors
+    for s in seeds:
+        for g in got[s]:
+            for a, b in zip(g, want[s]):
+                # dQ's sums come in any order: fp32 sums of the same terms, rounded to bf16 and carried through the norm's gradient
+                assert (a.double() - b.double()).norm() <= 2.0**-7 * b.double().norm()
