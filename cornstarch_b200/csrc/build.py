@@ -115,12 +115,13 @@ def build(force: bool = False, verbose: bool = False, bounds_check: bool = False
     return lib_path
 
 
+HOST_OPS_SRC = CSRC / "host_ops.cpp"
 HOST_OPS_PATH = LIB_DIR / "_host_ops.so"
 
 
 def build_host_ops(force: bool = False) -> Path:
     """The Python module of ``host_ops.cpp`` (torch's C++ interface around the library's entry points; no device code)."""
-    src = CSRC / "host_ops.cpp"
+    src = HOST_OPS_SRC
     torch_dir = Path(importlib.util.find_spec("torch").submodule_search_locations[0])
     newest = max(src.stat().st_mtime, (torch_dir / "version.py").stat().st_mtime)
     if not force and HOST_OPS_PATH.exists() and HOST_OPS_PATH.stat().st_mtime >= newest:

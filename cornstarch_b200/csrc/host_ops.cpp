@@ -8,9 +8,9 @@
 // take all that Python sends them): the Python statement of the operator decides what happens then (another route, a copy, an
 // error).
 //
-// What allocates or launches runs without the GIL (60 ns a call), as calls through ctypes do: a launch waits while the stream's queue is full, an allocation
-// may wait for the device, and the threads that watch over a hanging step are Python threads.  What is Python (arguments, results, the
-// one look-up of a status word) is done before, after, or with the GIL taken back for it.
+// What allocates or launches runs without the GIL (60 ns a call), as calls through ctypes do: a launch waits while the stream's
+// queue is full, an allocation may wait for the device, and the threads that watch over a hanging step are Python threads.  What is
+// Python (arguments, results, the one look-up of a status word) is done before, after, or with the GIL taken back for it.
 //
 // The kernels' entry points are looked up once in the library that ctypes has loaded (bind), so there is one library per process
 // whichever file it came from.
