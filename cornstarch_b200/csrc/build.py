@@ -4,7 +4,7 @@ Every ``*.cu`` file in this directory is compiled with nvcc for ``sm_100a`` only
 ``cornstarch_b200/lib/libcornstarch_b200.so``.  The library exposes a plain C ABI (see the
 ``CSB_API`` functions) that :mod:`cornstarch_b200.ops._native` loads with ``ctypes``; no torch
 headers are involved there.  ``host_ops.cpp`` (the host side of the hot calls, torch's C++ interface) becomes the Python module
-``cornstarch_b200/lib/_host_ops.so``.  A full rebuild takes one to two minutes and works on a machine without a GPU (nvcc
+``cornstarch_b200/lib/_host_ops.torch-<version><Python's suffix>``.  A full rebuild takes one to two minutes and works on a machine without a GPU (nvcc
 cross-compiles).
 
 Run ``python -m cornstarch_b200.csrc.build`` (add ``--force`` to rebuild everything, ``-v`` for the
@@ -14,12 +14,15 @@ ptxas resource report, ``--bounds-check`` for the debug library with index check
 from __future__ import annotations
 
 import concurrent.futures as cf
+import functools
 import importlib.util
 import os
+import re
 import shutil
 import subprocess
 import sys
 import sysconfig
+import uuid
 from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent
@@ -116,26 +119,41 @@ def build(force: bool = False, verbose: bool = False, bounds_check: bool = False
 
 
 HOST_OPS_SRC = CSRC / "host_ops.cpp"
-HOST_OPS_PATH = LIB_DIR / "_host_ops.so"
+
+
+def _torch_dir() -> Path:
+    return Path(importlib.util.find_spec("torch").submodule_search_locations[0])
+
+
+@functools.cache
+def host_ops_path() -> Path:
+    """Where the module of ``host_ops.cpp`` for THIS torch and Python is (or would be): it is linked against torch's C++ interface, so a
+    module of another build of either is never looked at."""
+    version = re.search(r"__version__ = ['\"]([^'\"]+)", (_torch_dir() / "version.py").read_text()).group(1)
+    return LIB_DIR / f"_host_ops.torch-{version}{sysconfig.get_config_var('EXT_SUFFIX')}"
 
 
 def build_host_ops(force: bool = False) -> Path:
     """The Python module of ``host_ops.cpp`` (torch's C++ interface around the library's entry points; no device code)."""
-    src = HOST_OPS_SRC
-    torch_dir = Path(importlib.util.find_spec("torch").submodule_search_locations[0])
-    newest = max(src.stat().st_mtime, (torch_dir / "version.py").stat().st_mtime)
-    if not force and HOST_OPS_PATH.exists() and HOST_OPS_PATH.stat().st_mtime >= newest:
-        return HOST_OPS_PATH
+    path, torch_dir = host_ops_path(), _torch_dir()
+    if not force and path.exists() and path.stat().st_mtime >= HOST_OPS_SRC.stat().st_mtime:
+        return path
+    import torch  # for the ABI of its libraries; only where there is something to compile
+
     cuda = Path(_nvcc()).resolve().parent.parent
     inc = [torch_dir / "include", torch_dir / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
-    tmp = HOST_OPS_PATH.with_suffix(".tmp.so")
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", *[f"-I{i}" for i in inc], str(src), "-o",
-           str(tmp), f"-L{torch_dir / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{torch_dir / 'lib'}"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"{cmd[0]} failed for {src.name}:\n{res.stdout}\n{res.stderr}")
-    os.replace(tmp, HOST_OPS_PATH)
-    return HOST_OPS_PATH
+    tmp = path.with_name(f".{uuid.uuid4().hex}.so")  # a name of its own: builds may run side by side
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *[f"-I{i}" for i in inc], str(HOST_OPS_SRC), "-o", str(tmp),
+           f"-L{torch_dir / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{torch_dir / 'lib'}"]
+    try:
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"{cmd[0]} failed for {HOST_OPS_SRC.name}:\n{res.stdout}\n{res.stderr}")
+        os.replace(tmp, path)
+    finally:
+        tmp.unlink(missing_ok=True)
+    return path
 
 
 if __name__ == "__main__":

@@ -9,7 +9,9 @@ fall back silently to eager PyTorch.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
+import warnings
 from pathlib import Path
 
 import torch
@@ -149,26 +151,29 @@ _HOST_ENTRIES = ("csb_gemm_bf16", "csb_gemm_cols_bf16", "csb_linear_bwd", "csb_c
 
 def host_ops():
     """``csrc/host_ops.cpp``: checks, output allocation and launch of one operator on CUDA tensors in one native call (each answers
-    ``None`` for a form that it does not take).  ``None`` while every call is timed on its own (KERNEL_TIMES).  Like the library it
-    is mandatory on a machine with a GPU."""
+    ``None`` for a form that it does not take).  ``None`` while every call is timed on its own (KERNEL_TIMES), and, with a warning,
+    where there is no module for this torch and Python: the library itself knows neither, and its calls then go through ctypes."""
     global _HOST
     if _HOST is None:
-        if KERNEL_TIMES:
-            _HOST = False
-        else:
-            import importlib.util
-
-            path = _LIB_PATH.parent / "_host_ops.so"
-            if not path.exists():
-                raise RuntimeError(f"{path} not found: run `python -m cornstarch_b200.csrc.build`")
-            spec = importlib.util.spec_from_file_location("_host_ops", path)
-            mod = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(mod)
-            raw = lib()._raw
-            mod.bind({n: C.cast(getattr(raw, n), vp).value for n in _HOST_ENTRIES},
-                     lambda index: status_word(torch.device("cuda", index)).data_ptr())
-            _HOST = mod
+        _HOST = False if KERNEL_TIMES else _load_host_ops()
     return _HOST or None
+
+
+def _load_host_ops():
+    from ..csrc.build import host_ops_path
+
+    path = host_ops_path()
+    try:
+        spec = importlib.util.spec_from_file_location("_host_ops", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+    except ImportError as e:
+        warnings.warn(f"no native host path for torch {torch.__version__} ({e}); operators are issued through ctypes, up to 45 us a call "
+                      "slower: run `python -m cornstarch_b200.csrc.build`", RuntimeWarning, stacklevel=3)
+        return False
+    raw = lib()._raw
+    mod.bind({n: C.cast(getattr(raw, n), vp).value for n in _HOST_ENTRIES}, lambda index: status_word(torch.device("cuda", index)).data_ptr())
+    return mod
 
 
 def declare(name: str, argtypes: list) -> None:

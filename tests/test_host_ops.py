@@ -195,8 +195,8 @@ def test_projections_of_separate_weights(widths, one, T, bias):
 # process of its own: the entry points are bound once per process.  getpid stands in for the launch behind it, refused as code != 0.
 SLOW_ENTRY = """
 import ctypes, importlib.util, threading, time, torch
-from cornstarch_b200.csrc.build import HOST_OPS_PATH
-spec = importlib.util.spec_from_file_location("_host_ops", HOST_OPS_PATH)
+from cornstarch_b200.csrc.build import host_ops_path
+spec = importlib.util.spec_from_file_location("_host_ops", host_ops_path())
 host = importlib.util.module_from_spec(spec)
 spec.loader.exec_module(host)
 libc = ctypes.CDLL(None)
