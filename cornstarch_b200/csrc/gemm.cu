@@ -1062,21 +1062,25 @@ static TileChoice choose_tile(int M, int N, int K, int tile_n, int max_ctas, boo
 // (`tile_n`, `max_ctas` and CORNSTARCH_B200_GEMM_CG=1 ask for blocks that work alone.)
 constexpr float SPLIT_US = 6.f, SPLIT_K_US = 0.26f;
 constexpr int SPLIT_CLUSTERS[SK_MAX_SPLIT + 1] = {0, 0, 66, 40, 33, 0, 18, 0, 15};
-static int choose_split(int M, int N, int K, int tile_n, int max_ctas, TileChoice tc, bool a_mn_major, bool b_mn_major) {
+// `us`: the predicted time of the call.
+static int choose_split(int M, int N, int K, int tile_n, int max_ctas, TileChoice tc, bool a_mn_major, bool b_mn_major, float* us = nullptr) {
+  const int layout = a_mn_major ? 2 : (b_mn_major ? 1 : 0);
+  float whole = 0.f;
+  for (const TileCost& c : TILE_COSTS)
+    if (c.bn == tc.bn && c.cg == tc.cg) whole = tile_cost(c, layout, M, N, K);
+  if (us) *us = whole;
   if (tile_n == 128 || tile_n == 256 || max_ctas > 0 || gemm_cg_choice() == 1) return 1;
   const long tiles = (long)((M + BM - 1) / BM) * ((N + SK_BN - 1) / SK_BN);
   const int kb = (K + BK - 1) / BK;
   if (kb < 16 || tiles > SPLIT_CLUSTERS[2]) return 1;
-  const int layout = a_mn_major ? 2 : (b_mn_major ? 1 : 0);
-  float best = 0.f;
-  for (const TileCost& c : TILE_COSTS)
-    if (c.bn == tc.bn && c.cg == tc.cg) best = 0.93f * tile_cost(c, layout, M, N, K);
+  float best = 0.93f * whole;
   int split = 1;
   for (int n : {2, 3, 4, 6, 8}) {
     const float t = 6.f + SPLIT_US + SPLIT_K_US * ((kb + n - 1) / n);
     if (t < best && tiles <= SPLIT_CLUSTERS[n] && tiles <= splitk_clusters(n)) {
       best = t;
       split = n;
+      if (us) *us = t;
     }
   }
   return split;
@@ -1171,11 +1175,69 @@ CSB_API int csb_linear_bwd(const void* dy, const void* x, const void* w, void* d
   return r;
 }
 
+namespace csb {
+// Tile of `groups` projections of one input in one launch (csb_gemm_cols_bf16), or one of 0 columns: separate calls.  One launch has
+// the start and the last round of one, but needs a tile whose width divides all widths, where a call for each weight takes the tile that
+// suits it and may share its contraction.  So: never where the whole would share its contraction, and only where the predicted time is
+// no longer than that of the separate calls, of which each but the first counts COLS_LAUNCH_US of the six in tile_cost (the next
+// kernel starts while the last one ends).
+// Both ways replayed in turn, 20 groups of 2 or 3 weights x 16 to 8192 tokens, 375 pairs: 0.06 % more time than the better one of
+// each pair with COLS_LAUNCH_US = 4, 0.07 % with 3, 0.1 % with 6.  Joined wherever a tile divides is 0.5 % and up to 23 % slower (4096 x
+// (4096, 128, 128) of 8192 tokens 254 us joined, 207 apart; 5120 x (5120, 640, 640) of 4575 tokens 258 / 214), always apart 64 % (1531 x 4096
+// x (4096, 1024, 1024) 53 / 81; 729 x 1152 x 3 x 1152 12 / 28).  Left: six pairs joined at 1.01 to 1.08 (7300 x 1024 x (4096, 128)
+// 61.1 / 56.8), none apart above 1.02.
+constexpr float COLS_LAUNCH_US = 4.f;
+static TileChoice choose_cols_tile(int M, const int* widths, int groups, int K) {
+  int N = 0;
+  float apart = 6.f - COLS_LAUNCH_US;
+  for (int g = 0; g < groups; ++g) {
+    float t;
+    choose_split(M, widths[g], K, 0, 0, choose_tile(M, widths[g], K, 0, 0, false, false), false, false, &t);
+    apart += t - 6.f + COLS_LAUNCH_US;
+    N += widths[g];
+  }
+  auto divides = [&](int bn) {
+    for (int g = 0; g < groups; ++g)
+      if (widths[g] % bn) return false;
+    return true;
+  };
+  TileChoice tc = choose_tile(M, N, K, 0, 0, false, false);
+  float together;
+  if (choose_split(M, N, K, 0, 0, tc, false, false, &together) > 1) return {0, 1};
+  if (!divides(tc.bn)) {  // the cheapest one that does
+    tc.bn = 0;
+    for (const TileCost& c : TILE_COSTS) {
+      if (!divides(c.bn) || (c.cg == 2 && (gemm_cg_choice() != 2 || M <= BM))) continue;
+      const float t = tile_cost(c, 0, M, N, K);
+      if (tc.bn == 0 || t < together) {
+        together = t;
+        tc = {c.bn, c.cg};
+      }
+    }
+  }
+  if (tc.bn != 0 && together > apart) tc.bn = 0;
+  return tc;
+}
+}  // namespace csb
+
+// What csb_gemm_cols_bf16 takes: columns of a tile (0: it does not take them) and blocks that work on one tile.
+CSB_API int csb_gemm_cols_choice(const int* widths, int groups, int M, int K, int* bn, int* cg) {
+  using namespace csb;
+  if (groups < 2 || M <= 0 || K <= 0 || widths == nullptr) return CSB_ERR_BAD_ARG;
+  long total = 0;
+  for (int g = 0; g < groups; ++g) {
+    if (widths[g] <= 0) return CSB_ERR_BAD_ARG;
+    total += widths[g];
+  }
+  const TileChoice tc = groups > MAX_COL_GROUPS || total > 0x7fffffffL ? TileChoice{0, 1} : choose_cols_tile(M, widths, groups, K);
+  *bn = tc.bn;
+  *cg = tc.cg;
+  return 0;
+}
+
 // Projections of one input whose weights are matrices of their own, in ONE launch: C[:, o_g : o_g + N_g] = A * B_g^T + bias_g with
-// o_g the widths before.  A and all B are K-major (pitches lda, ldb); bias: one pointer per group (0 = none), or null.  Taken where a
-// tile width divides all N_g and the whole would not share its contractions (choose_split); CSB_ERR_NO_FIT otherwise, and the
-// caller makes one call per weight.  Each of those ends in a round of its own, mostly empty for narrow ones: 1531 x 4096 -> 4096, 1024
-// and 1024 40.4 + 20.3 + 20.3 us, together 53; 729 x 1152 -> 3 x 1152 with biases 3 x 9.5, together 12.
+// o_g the widths before.  A and all B are K-major (pitches lda, ldb); bias: one pointer per group (0 = none), or null.
+// CSB_ERR_NO_FIT where choose_cols_tile takes separate calls: the caller makes one per weight.
 CSB_API int csb_gemm_cols_bf16(const void* A, const void* const* B, const void* const* bias, const int* widths, int groups, void* C, int M, int K,
                                int lda, int ldb, int ldc, int* status, void* stream) {
   using namespace csb;
@@ -1188,26 +1250,8 @@ CSB_API int csb_gemm_cols_bf16(const void* A, const void* const* B, const void* 
   }
   if (total > 0x7fffffffL || ldc < total || (ldc & 7)) return CSB_ERR_BAD_ARG;
   const int N = (int)total;
-  auto divides = [&](int bn) {
-    for (int g = 0; g < groups; ++g)
-      if (widths[g] % bn) return false;
-    return true;
-  };
-  TileChoice tc = choose_tile(M, N, K, 0, 0, false, false);
-  if (choose_split(M, N, K, 0, 0, tc, false, false) > 1) return CSB_ERR_NO_FIT;
-  if (!divides(tc.bn)) {  // the cheapest one that does
-    float best = 0.f;
-    tc.bn = 0;
-    for (const TileCost& c : TILE_COSTS) {
-      if (!divides(c.bn) || (c.cg == 2 && (gemm_cg_choice() != 2 || M <= BM))) continue;
-      const float t = tile_cost(c, 0, M, N, K);
-      if (tc.bn == 0 || t < best) {
-        best = t;
-        tc = {c.bn, c.cg};
-      }
-    }
-    if (tc.bn == 0) return CSB_ERR_NO_FIT;
-  }
+  const TileChoice tc = choose_cols_tile(M, widths, groups, K);
+  if (tc.bn == 0) return CSB_ERR_NO_FIT;
   GemmParams p;
   p.C = C;
   p.bias = nullptr;

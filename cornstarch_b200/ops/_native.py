@@ -28,6 +28,7 @@ _PROTOS = {
     "csb_gemm_bf16": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp],
     "csb_gemm_grouped_bf16": [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp],
     "csb_gemm_choice": [i32] * 7 + [C.POINTER(i32)] * 3,
+    "csb_gemm_cols_choice": [C.POINTER(i32), i32, i32, i32, C.POINTER(i32), C.POINTER(i32)],
     "csb_linear_bwd": [vp] * 7 + [i32] * 11 + [vp, vp],
     "csb_norm_bwd_parts": [i32],
     "csb_norm_fwd": [i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, f32, f32, vp],
@@ -87,7 +88,8 @@ def lib():
 class _CountingLib:
     """Forwards attribute access to the CDLL and counts calls of kernel-launching entry points."""
 
-    _NO_LAUNCH = {"csb_norm_bwd_parts", "csb_colsum_parts", "csb_attn_bwd_splits", "csb_gemm_choice", "csb_lm_stats_parts"}
+    _NO_LAUNCH = {"csb_norm_bwd_parts", "csb_colsum_parts", "csb_attn_bwd_splits", "csb_gemm_choice", "csb_gemm_cols_choice",
+                  "csb_lm_stats_parts"}
 
     def __init__(self, raw):
         self._raw = raw

@@ -55,3 +55,18 @@ def test_split_counts():
     assert splits(CAUSAL, 1, 1500, 1500, 8, 1) > 8 and splits(FULL, 1, 8192, 8192, 32, 8) == 2
     assert splits(CAUSAL, 1, 4096, 4096, 32, 8) == splits(FULL, 1, 4096, 4096, 32, 8) == 1
     assert splits(FULL, 1, 65536, 65536, 32, 8) == splits(FULL, 4, 729, 729, 16, 16) == 1
+
+
+# weights that are not adjacent: one launch where a tile suits them all, separate calls where the widths leave only a narrow one
+@pytest.mark.parametrize("T,K,widths,one", [
+    (1531, 4096, (4096, 1024, 1024), True), (729, 1152, (1152, 1152, 1152), True), (77, 1152, (1152, 1152, 1152), True),
+    (4575, 5120, (5120, 640, 640), False), (7300, 5120, (5120, 640, 640), False), (8192, 4096, (4096, 128, 128), False),
+    (251, 4096, (11008, 11008), False), (8192, 1024, (4096, 128), False), (64, 264, (136, 256), False), (64, 264, (128,) * 5, False),
+])
+def test_separate_weights_are_joined_where_that_is_faster(T, K, widths, one):
+    if not LIB_PATH.exists():
+        pytest.skip("the native library is not built")
+    bn, cg = ctypes.c_int(-1), ctypes.c_int(-1)
+    rc = ctypes.CDLL(str(LIB_PATH)).csb_gemm_cols_choice((ctypes.c_int * len(widths))(*widths), len(widths), T, K, ctypes.byref(bn), ctypes.byref(cg))
+    assert rc == 0 and (bn.value > 0) == one
+    assert not one or all(w % bn.value == 0 for w in widths)
