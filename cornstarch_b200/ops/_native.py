@@ -28,6 +28,7 @@ _PROTOS = {
     "csb_gemm_bf16": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp],
     "csb_gemm_grouped_bf16": [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp],
     "csb_gemm_choice": [i32] * 7 + [C.POINTER(i32)] * 3,
+    "csb_gemm_cols_bf16": [vp, C.POINTER(vp), C.POINTER(vp), C.POINTER(i32), i32, vp] + [i32] * 5 + [vp, vp],
     "csb_gemm_cols_choice": [C.POINTER(i32), i32, i32, i32, C.POINTER(i32), C.POINTER(i32)],
     "csb_linear_bwd": [vp] * 7 + [i32] * 11 + [vp, vp],
     "csb_norm_bwd_parts": [i32],

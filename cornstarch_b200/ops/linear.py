@@ -28,6 +28,9 @@ from .gemm import gemm
 _GRAD_TYPES = (torch.bfloat16, torch.float32)  # what the GEMM and the column sum write (the native calls know only "fp32 or not")
 
 
+_MAX_COL_GROUPS = 4  # weights of one csb_gemm_cols_bf16
+
+
 def _use_native(x: torch.Tensor) -> bool:
     return x.is_cuda and x.dtype == torch.bfloat16 and not nat.LIBRARY_MODE
 
@@ -129,33 +132,40 @@ def _native_backward(ctx, dy2, x2, weights, fused_w):
     dW, ok = _fused_grads(weights, fuse_adjacent)
     if not ok or (dW is not None and (dW.dim() != 2 or dW.stride(1) != 1 or dW.shape != fused_w.shape)):
         return None
-    db, scratch = None, None
+    db = None
     if ctx.has_bias:
         if any(b is None for b in biases) or not all(ctx.needs_input_grad[4 + n_w :]) or not dy2.is_contiguous():
             return None
         db, ok = _fused_grads(biases, fuse_adjacent_1d)
         if not ok or (db is not None and (not db.is_contiguous() or db.numel() != N)):
             return None
-    acc_w, acc_b = int(dW is not None), int(db is not None)
+    acc_w, acc_b = dW is not None, db is not None
+    return _native_results(ctx, *_backward_gemms(dy2, x2, fused_w, ctx.needs_input_grad[0], dW, ctx.has_bias, db), weights, acc_w, acc_b)
+
+
+def _backward_gemms(dy2, x2, fused_w, need_x, dW, has_bias, db):
+    """``(dx or None, dW, db or None)``, the latter two added to the buffers that are given."""
     host = nat.host_ops() if dy2.is_cuda else None
-    got = host.linear_bwd(dy2, x2, fused_w, ctx.needs_input_grad[0], dW, ctx.has_bias, db) if host is not None else None
+    got = host.linear_bwd(dy2, x2, fused_w, need_x, dW, has_bias, db) if host is not None else None
     if got is not None:
-        return _native_results(ctx, *got, weights, acc_w, acc_b)
+        return got
+    T, (N, K) = dy2.shape[0], fused_w.shape
     dev, lib = dy2.device, nat.lib()
+    acc_w, acc_b, scratch = int(dW is not None), int(db is not None), None
     if dW is None:
         dW = torch.empty((N, K), dtype=dy2.dtype, device=dev)
-    if ctx.has_bias:
+    if has_bias:
         scratch = torch.empty(lib.csb_colsum_parts(T) * N, dtype=torch.float32, device=dev)
         if db is None:
             db = torch.empty(N, dtype=dy2.dtype, device=dev)
-    dx = torch.empty((T, K), dtype=dy2.dtype, device=dev) if ctx.needs_input_grad[0] else None
+    dx = torch.empty((T, K), dtype=dy2.dtype, device=dev) if need_x else None
     nat.check(
         lib.csb_linear_bwd(dy2.data_ptr(), x2.data_ptr(), fused_w.data_ptr(), nat.ptr(dx), dW.data_ptr(), nat.ptr(db), nat.ptr(scratch),
                            T, N, K, dy2.stride(0), x2.stride(0), fused_w.stride(0), dW.stride(0), int(dW.dtype == torch.float32),
                            acc_w, int(db is not None and db.dtype == torch.float32), acc_b, nat.status_word(dev).data_ptr(), nat.stream()),
         "csb_linear_bwd",
     )
-    return _native_results(ctx, dx, dW, db, weights, acc_w, acc_b)
+    return dx, dW, db
 
 
 def _native_results(ctx, dx, dW, db, weights, acc_w, acc_b):
@@ -177,6 +187,55 @@ def _native_results(ctx, dx, dW, db, weights, acc_w, acc_b):
     return (dx.view(ctx.x_shape) if dx is not None else None, None, None, None, *dws, *dbs)
 
 
+def _cols_gemm(x2, weights, biases, y) -> bool:
+    """Weights that are not adjacent as one launch, by the rule and in the forms of ``host_ops.cpp``; ``False``: separate calls."""
+    n, (T, K), N = len(weights), x2.shape, y.shape[1]
+    if n > _MAX_COL_GROUPS or N % 8 or T == 0 or K == 0 or any(w.dim() != 2 or w.shape[1] != K or w.shape[0] == 0 for w in weights):
+        return False
+    if any(t.stride(1) != 1 or t.stride(0) % 8 or t.data_ptr() % 16 or t.dtype != torch.bfloat16 for t in (x2, *weights)) or y.data_ptr() % 16:
+        return False
+    if any(w.stride(0) != weights[0].stride(0) for w in weights) or len({b is None for b in biases}) > 1:
+        return False
+    if any(b is not None and (b.dtype != torch.bfloat16 or not b.is_contiguous() or b.numel() != w.shape[0]) for w, b in zip(weights, biases)):
+        return False
+    widths, choice = (nat.i32 * n)(*[w.shape[0] for w in weights]), [nat.i32(), nat.i32()]
+    nat.check(nat.lib().csb_gemm_cols_choice(widths, n, T, K, *choice), "csb_gemm_cols_choice")
+    if choice[0].value == 0:
+        return False
+    has_bias = biases[0] is not None
+    nat.check(
+        nat.lib().csb_gemm_cols_bf16(x2.data_ptr(), (nat.vp * n)(*[w.data_ptr() for w in weights]),
+                                     (nat.vp * n)(*[b.data_ptr() for b in biases]) if has_bias else None, widths, n, y.data_ptr(), T, K,
+                                     x2.stride(0), weights[0].stride(0), N, nat.status_word(x2.device).data_ptr(), nat.stream()),
+        "csb_gemm_cols_bf16",
+    )
+    return True
+
+
+def _forward_gemms(x, weights, biases, tp):
+    """``(out, x as 2-D)``: the concatenated projections of ``x``."""
+    host = nat.host_ops() if tp is None and x.is_cuda else None
+    got = host.linear_fwd(x, weights, biases) if host is not None else None
+    if got is not None:
+        return got
+    x2 = _as_2d(x)
+    fused_w = fuse_adjacent(weights) if len(weights) > 1 else weights[0]
+    has_bias = biases[0] is not None
+    fused_b = (fuse_adjacent_1d(biases) if len(weights) > 1 else biases[0]) if has_bias else None
+    n_total = sum(w.shape[0] for w in weights)
+    # the returned tensor owns its storage (callers such as RoPE modify it in place)
+    out = torch.empty((*x.shape[:-1], n_total), dtype=x.dtype, device=x.device)
+    y = out.view(-1, n_total)
+    if fused_w is not None and (not has_bias or fused_b is not None):
+        gemm(x2, fused_w, bias=fused_b, out=y)
+    elif not (tp is None and _use_native(x2) and _cols_gemm(x2, weights, biases, y)):
+        o = 0
+        for w, b in zip(weights, biases):
+            gemm(x2, w, bias=b, out=y[:, o : o + w.shape[0]])
+            o += w.shape[0]
+    return out, x2
+
+
 class _LinearFn(torch.autograd.Function):
     """y = x W^T + b with native backward; several (weight, bias) pairs share one input."""
 
@@ -185,32 +244,15 @@ class _LinearFn(torch.autograd.Function):
         weights = params[:n_w]
         biases = params[n_w:]
         ctx.tp = tp
-        host = nat.host_ops() if tp is None and act is None and x.is_cuda else None
-        got = host.linear_fwd(x, weights, biases) if host is not None else None
-        if got is not None:
-            out, x2 = got
-            ctx.save_for_backward(x2, *weights)
-            ctx.n_w, ctx.has_bias, ctx.x_shape, ctx.biases = n_w, biases[0] is not None, x.shape, biases
-            return out
-        x2 = _as_2d(x)
-        fused_w = fuse_adjacent(weights) if n_w > 1 else weights[0]
         has_bias = biases[0] is not None
-        fused_b = (fuse_adjacent_1d(biases) if n_w > 1 else biases[0]) if has_bias else None
-        n_total = sum(w.shape[0] for w in weights)
-        # the returned tensor owns its storage (callers such as RoPE modify it in place)
-        out = torch.empty((*x.shape[:-1], n_total), dtype=x.dtype, device=x.device)
-        y = out.view(-1, n_total)
         assert not (tp is not None and tp[0] == "row" and (has_bias or n_w != 1)), "row-parallel: one weight, bias added after the reduce"
-        if tp is not None and tp[0] == "row" and fused_w is not None and not has_bias:
+        if tp is not None and tp[0] == "row":
             # row-parallel: partial products of all ranks are summed by the fused GEMM + all-reduce kernel
-            tp[1].gemm_allreduce(x2, fused_w, out=y)
-        elif fused_w is not None and (not has_bias or fused_b is not None):
-            gemm(x2, fused_w, bias=fused_b, act=act, out=y)
+            x2 = _as_2d(x)
+            out = torch.empty((*x.shape[:-1], weights[0].shape[0]), dtype=x.dtype, device=x.device)
+            tp[1].gemm_allreduce(x2, weights[0], out=out.view(-1, weights[0].shape[0]))
         else:
-            o = 0
-            for w, b in zip(weights, biases):
-                gemm(x2, w, bias=b, act=act, out=y[:, o : o + w.shape[0]])
-                o += w.shape[0]
+            out, x2 = _forward_gemms(x, weights, biases, tp)
         ctx.save_for_backward(x2, *weights)
         ctx.n_w = n_w
         ctx.has_bias = has_bias

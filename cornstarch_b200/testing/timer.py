@@ -19,8 +19,13 @@ import torch
 
 
 # Entry points that do a listed function's work, with or without calling it: the layers' attention on a fused q|k|v buffer
-# goes to an autograd function of its own when gradients are recorded.
-_ALSO = {"cornstarch_b200.ops.attention.attention": ["cornstarch_b200.ops.attention.attention_qkv"]}
+# goes to an autograd function of its own when gradients are recorded, and the GEMMs of a linear layer (a loss) are issued by one
+# native call.
+_ALSO = {
+    "cornstarch_b200.ops.attention.attention": ["cornstarch_b200.ops.attention.attention_qkv"],
+    "cornstarch_b200.ops.linear.gemm": ["cornstarch_b200.ops.linear._forward_gemms", "cornstarch_b200.ops.linear._backward_gemms"],
+    "cornstarch_b200.ops.cross_entropy.gemm": ["cornstarch_b200.ops.cross_entropy._logits_and_stats"],
+}
 
 
 def _resolve(path: str):

@@ -191,6 +191,45 @@ def test_projections_of_separate_weights(widths, one, T, bias):
     assert (y.double() - ref).norm() <= 2.0**-8 * ref.norm() and (y.double() - ref).abs().max() <= 2.0**-7 * ref.abs().max()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("widths", [(512, 256, 256), (136, 256)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_separate_weights_take_one_route(widths, bias, monkeypatch):
+    """What is timed call by call is what runs: as many launches with the native host path as without it, and the same bits."""
+    x, ws = _randn(700, 264), [_randn(n, 264, seed=i) for i, n in enumerate(widths)]
+    bs = [_randn(n, seed=9) if bias else None for n in widths]
+
+    def run():
+        with torch.no_grad():
+            return [L.multi_linear(x, ws, bs)]
+
+    _same(*_both(monkeypatch, run))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K,calls", [(64, 2), (60, 3)])  # forward and backward issued as one each; input and weight gradient apart
+def test_timer_sees_the_gemms_of_linear_layers(K, calls):
+    from cornstarch_b200.testing.timer import TimerContextManager
+
+    x, w = _leaves([_randn(24, K), _randn(32, K)])
+    path = "cornstarch_b200.ops.linear.gemm"
+    with TimerContextManager(path) as t:
+        L.linear(x, w).backward(_randn(24, 32))
+    assert len(t.get_elapsed_times()[path]) == calls
+
+
+@pytest.mark.gpu
+def test_timer_sees_the_gemms_of_the_loss():
+    from cornstarch_b200.ops.cross_entropy import linear_cross_entropy
+    from cornstarch_b200.testing.timer import TimerContextManager
+
+    h, w = _leaves([_randn(24, 64), _randn(32, 64)])
+    path = "cornstarch_b200.ops.cross_entropy.gemm"
+    with TimerContextManager(path) as t:
+        linear_cross_entropy(h, w, torch.zeros(24, dtype=torch.int64, device="cuda")).backward()
+    assert len(t.get_elapsed_times()[path]) == 3  # logits, input and weight gradient
+
+
 # An entry point that takes its time (libc's usleep under the name of one that takes an int) with another Python thread beside it.  In a
 # process of its own: the entry points are bound once per process.  getpid stands in for the launch behind it, refused as code != 0.
 SLOW_ENTRY = """
