@@ -4,7 +4,7 @@ Every ``*.cu`` file in this directory is compiled with nvcc for ``sm_100a`` only
 ``cornstarch_b200/lib/libcornstarch_b200.so``.  The library exposes a plain C ABI (see the
 ``CSB_API`` functions) that :mod:`cornstarch_b200.ops._native` loads with ``ctypes``; no torch
 headers are involved there.  ``host_ops.cpp`` (the host side of the hot calls, torch's C++ interface) becomes the Python module
-``cornstarch_b200/lib/_host_ops.torch-<version><Python's suffix>``.  A full rebuild takes one to two minutes and works on a machine without a GPU (nvcc
+``cornstarch_b200/lib/_host_ops.torch-<version><Python's suffix>``.  A full rebuild takes two minutes and works on a machine without a GPU (nvcc
 cross-compiles).
 
 Run ``python -m cornstarch_b200.csrc.build`` (add ``--force`` to rebuild everything, ``-v`` for the

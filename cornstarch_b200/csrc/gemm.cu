@@ -871,11 +871,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 template <int BN, bool A_MN, bool B_MN, int CG = 1, int EPI = EPI_PLAIN>
 static int launch_gemm(const void* A, const void* B, const GemmParams& p, int lda, int ldb, int max_ctas,
                        cudaStream_t stream, const void* const* group_b = nullptr, int groups = 0) {
-  // The bias form exists for the projections' layout; with an MN-major operand (no call of the framework has both) the direct stores
-  // of the epilogue add it.
+  // All operand orders have the form with a bias: through the direct stores, 4096 x 1024 -> 4096 with B MN-major takes 64 us, 29.5 here.
   bool any_bias = p.bias != nullptr;
   for (int g = 0; g < p.col_groups; ++g) any_bias = any_bias || p.col_bias[g] != nullptr;
-  if constexpr (EPI == EPI_PLAIN && !A_MN && !B_MN)
+  if constexpr (EPI == EPI_PLAIN)
     if (any_bias) return launch_gemm<BN, A_MN, B_MN, CG, EPI_BIAS>(A, B, p, lda, ldb, max_ctas, stream, group_b, groups);
   CUtensorMap ta, tb;
   int r;
@@ -910,7 +909,6 @@ static int launch_gemm(const void* A, const void* B, const GemmParams& p, int ld
   const int eb = q.out_fp32 ? 4 : 2;
   const int cps = 128 / eb;
   q.tma_epi = ((reinterpret_cast<uintptr_t>(q.C) & 15) == 0 && ((size_t)q.ldc * eb) % 16 == 0) ? 1 : 0;
-  if (EPI != EPI_BIAS && any_bias) q.tma_epi = 0;
   if (q.ar_world > 1 && !q.tma_epi) return CSB_ERR_BAD_ARG;
   if (q.group_rows > 0) {
     // grouped form: one B per group, same shape and row pitch (B above is group 0's and only serves the prefetch)
