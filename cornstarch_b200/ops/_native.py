@@ -201,6 +201,12 @@ def ptr(t: torch.Tensor | None):
     return None if t is None else t.data_ptr()
 
 
+def dense(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous and on the 16-byte grid of the kernels' vector loads; a copy where it is not."""
+    t = t if t.is_contiguous() else t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def stream() -> int:
     """Handle of the current stream of the current device (what ``torch.cuda.current_stream().cuda_stream`` is, without the
     stream object and the device look-ups around it: 0.3 against 3 us, once per launch)."""

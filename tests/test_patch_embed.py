@@ -3,6 +3,7 @@
 import pytest
 import torch
 import torch.nn as nn
+import torch.nn.functional as F
 
 from cornstarch_b200.ops import _native as nat
 from cornstarch_b200.ops.patch import patch_embed
@@ -65,6 +66,120 @@ def test_what_is_left_to_the_module():
     handle.remove()
     overlapping = nn.Conv2d(3, 16, 14, 7).to("cuda", BF16)
     assert torch.equal(patch_embed(overlapping, x), overlapping(x).flatten(2).transpose(1, 2))
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+def _own_forward(conv, x):
+    conv.forward = lambda t: nn.Conv2d.forward(conv, t) * 2
+    return patch_embed(conv, x), 2 * _module(conv, x)
+
+
+def _own_class_forward(conv, x):
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(nn.Conv2d, "forward", lambda self, t: self._conv_forward(t, self.weight, self.bias) * 2)
+        return patch_embed(conv, x), 2 * _module(conv, x)
+
+
+def _subclass_weight(conv, x):
+    conv.weight = nn.Parameter(conv.weight.detach().as_subclass(_Sub))
+    y = patch_embed(conv, x)
+    assert isinstance(y, _Sub)
+    return y.as_subclass(torch.Tensor), _module(conv, x).as_subclass(torch.Tensor)
+
+
+def _forward_mode(conv, x):
+    from torch.autograd import forward_ad
+
+    t = torch.ones_like(conv.weight)
+    weight = conv.weight.detach()
+    del conv.weight  # a dual tensor in its place
+    with torch.no_grad(), forward_ad.dual_level():
+        conv.weight = forward_ad.make_dual(weight, t)
+        y = forward_ad.unpack_dual(patch_embed(conv, x))
+        assert y.tangent is not None
+        return y.tangent, F.conv2d(x, t, None, conv.stride).flatten(2).transpose(1, 2)
+
+
+def _vmap(conv, x):
+    xs = torch.stack([x, x + 1])
+    return torch.vmap(lambda t: patch_embed(conv, t))(xs), torch.stack([_module(conv, t) for t in xs])
+
+
+def _timer(conv, x):
+    from cornstarch_b200.testing.timer import TimerContextManager
+
+    with TimerContextManager("torch.nn.functional.conv2d") as t:
+        y = patch_embed(conv, x)
+    assert len(t.get_elapsed_times()["torch.nn.functional.conv2d"]) == 1
+    return y, _module(conv, x)
+
+
+def _dispatch_mode(conv, x):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    seen = []
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    with Mode():
+        y = patch_embed(conv, x)
+    assert torch.ops.aten.convolution.default in seen
+    return y, _module(conv, x)
+
+
+def _module(conv, x):
+    with torch.no_grad():
+        return F.conv2d(x, conv.weight, conv.bias, conv.stride).flatten(2).transpose(1, 2)
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("case", [_own_forward, _own_class_forward, _subclass_weight, _forward_mode, _vmap, _timer, _dispatch_mode])
+def test_a_module_that_something_else_changes_or_watches(case, device):
+    conv, x = _conv(3, 16, 14, True, device), torch.randn(2, 3, 28, 42, generator=torch.Generator().manual_seed(0)).to(device, BF16)
+    got, want = case(conv, x)
+    assert torch.equal(got.detach(), want.detach())
+
+
+@pytest.mark.gpu
+def test_gradients_of_the_gradients():
+    conv, x = _conv(3, 16, 14, True), _pixels(2, 3, 28, 42, "plain")
+    v, u = torch.randn_like(conv.weight), torch.randn_like(conv.bias)
+    out = []
+    for embed in (lambda: patch_embed(conv, x), lambda: conv(x).flatten(2).transpose(1, 2)):
+        y = embed().float()
+        dw, db = torch.autograd.grad((y**3).sum(), [conv.weight, conv.bias], create_graph=True)
+        out.append([dw, db, *torch.autograd.grad([dw, db], [conv.weight, conv.bias], [v, u])])
+    for a, b in zip(*out):  # bf16 activations, cubed: two or three roundings on either side
+        assert (a.double() - b.double()).norm() <= 2.0**-5 * b.double().norm()
+
+
+@pytest.mark.gpu
+def test_a_gradient_off_the_16_byte_grid():
+    conv, x = _conv(3, 16, 14, True), _pixels(2, 3, 28, 42, "plain")
+    dy = torch.randn(12 * 16 + 1, device="cuda").to(BF16)[1:].view(2, 6, 16)
+    grads = []
+    for d in (dy, dy.clone()):
+        grads.append(torch.autograd.grad(patch_embed(conv, x), [conv.weight, conv.bias], d))
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("frozen", [False, True])
+def test_patches_are_kept_for_the_weight_only(frozen):
+    conv, x = _conv(3, 16, 14, True), _pixels(2, 3, 28, 42, "plain")
+    conv.weight.requires_grad_(not frozen)
+    kept = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.append(t.shape) or t, lambda t: t):
+        y = patch_embed(conv, x)
+    assert kept == ([] if frozen else [(12, 592)])
+    y.sum().backward()
+    assert torch.equal(conv.bias.grad, torch.full_like(conv.bias, 12)) and (conv.weight.grad is None) == frozen
 
 
 def test_cpu_path():
