@@ -84,7 +84,11 @@ bool bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16; }
 bool grad_type(const Tensor& t) { return bf16(t) || t.scalar_type() == at::kFloat; }
 bool is_fp32(const Tensor& t) { return t.scalar_type() == at::kFloat; }
 bool fits_int(int64_t v) { return v >= 0 && v <= 0x7fffffff; }
-Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+// Contiguous and on the 16-byte grid of the kernels' vector loads.
+Tensor dense(const Tensor& t) {
+  if (!t.is_contiguous()) return t.contiguous();
+  return on_grid(t) ? t : t.clone();
+}
 
 Tensor as_2d(const Tensor& x) {
   Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
@@ -256,8 +260,11 @@ std::optional<Tensor5> norm_fwd(const Tensor& x, const OptTensor& res, const Ten
   }
   Tensor y = at::empty_like(x2), rstd = at::empty({rows}, x.options().dtype(at::kFloat));
   if (is_ln) mean = at::empty({rows}, rstd.options());
+  const Tensor wd = dense(w);
+  OptTensor bd;
+  if (b) bd = dense(*b);
   ++g_launches;
-  check(e_norm_fwd.get()(is_ln, x2.data_ptr(), res ? r2.data_ptr() : nullptr, w.data_ptr(), ptr(b), y.data_ptr(), res ? h.data_ptr() : nullptr,
+  check(e_norm_fwd.get()(is_ln, x2.data_ptr(), res ? r2.data_ptr() : nullptr, wd.data_ptr(), ptr(bd), y.data_ptr(), res ? h.data_ptr() : nullptr,
                          is_ln ? static_cast<float*>(mean.data_ptr()) : nullptr, static_cast<float*>(rstd.data_ptr()), (int)rows, (int)H, (float)eps,
                          (float)w_offset, stream()),
         "csb_norm_fwd");
@@ -268,7 +275,7 @@ std::optional<Tensor3> norm_bwd(const Tensor& dy, const OptTensor& dh, const Ten
                     bool has_b, double w_offset, const OptTensor& w_main, const OptTensor& b_main) {
   const int64_t rows = hs.size(0), H = hs.size(1);
   if (rows == 0) return std::nullopt;
-  const Tensor dy2 = dense(dy.reshape({-1, H}));
+  const Tensor dy2 = dense(dy.reshape({-1, H})), wd = dense(w);
   Tensor dres, dbp, dw, db;
   if (dh) dres = dense(dh->reshape({-1, H}));
   Tensor dx = at::empty_like(hs);
@@ -280,7 +287,7 @@ std::optional<Tensor3> norm_bwd(const Tensor& dy, const OptTensor& dh, const Ten
   dw = main ? *w_main : at::empty({H}, hs.options());
   if (main ? b_main.has_value() : bias) db = main ? *b_main : at::empty({H}, hs.options());
   ++g_launches;
-  check(e_norm_bwd.get()(is_ln, dy2.data_ptr(), hs.data_ptr(), w.data_ptr(), mean ? static_cast<const float*>(mean->data_ptr()) : nullptr,
+  check(e_norm_bwd.get()(is_ln, dy2.data_ptr(), hs.data_ptr(), wd.data_ptr(), mean ? static_cast<const float*>(mean->data_ptr()) : nullptr,
                          static_cast<const float*>(rstd.data_ptr()), dh ? dres.data_ptr() : nullptr, dx.data_ptr(), static_cast<float*>(dwp.data_ptr()),
                          bias ? static_cast<float*>(dbp.data_ptr()) : nullptr, dw.data_ptr(), db.defined() ? db.data_ptr() : nullptr, is_fp32(dw), main,
                          (int)rows, (int)H, (float)w_offset, stream()),

@@ -59,19 +59,16 @@ class _NormFn(torch.autograd.Function):
             ctx.w_ref, ctx.b_ref = w, b
             return y, h
         H = x.shape[-1]
-        x2 = x.reshape(-1, H)
-        x2 = x2 if x2.is_contiguous() else x2.contiguous()
+        x2 = nat.dense(x.reshape(-1, H))
         rows = x2.shape[0]
-        r2 = None
-        if res is not None:
-            r2 = res.reshape(-1, H)
-            r2 = r2 if r2.is_contiguous() else r2.contiguous()
+        r2 = nat.dense(res.reshape(-1, H)) if res is not None else None
+        wd, bd = nat.dense(w), nat.dense(b) if b is not None else None
         y = torch.empty_like(x2)
         h = torch.empty_like(x2) if res is not None else None
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
         mean = torch.empty(rows, dtype=torch.float32, device=x.device) if is_ln else None
         nat.check(
-            nat.lib().csb_norm_fwd(int(is_ln), x2.data_ptr(), nat.ptr(r2), w.data_ptr(), nat.ptr(b), y.data_ptr(),
+            nat.lib().csb_norm_fwd(int(is_ln), x2.data_ptr(), nat.ptr(r2), wd.data_ptr(), nat.ptr(bd), y.data_ptr(),
                                    nat.ptr(h), nat.ptr(mean), rstd.data_ptr(), rows, H, eps, w_offset, nat.stream()),
             "csb_norm_fwd",
         )
@@ -95,12 +92,8 @@ class _NormFn(torch.autograd.Function):
         if got is not None:
             return _NormFn._results(ctx, *got, use_main)
         rows, H = hs.shape
-        dy2 = dy.reshape(-1, H)
-        dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
-        dres = None
-        if dh is not None:
-            dres = dh.reshape(-1, H)
-            dres = dres if dres.is_contiguous() else dres.contiguous()
+        dy2, wd = nat.dense(dy.reshape(-1, H)), nat.dense(w)
+        dres = nat.dense(dh.reshape(-1, H)) if dh is not None else None
         dx = torch.empty_like(hs)
         parts = nat.lib().csb_norm_bwd_parts(rows)
         dw_part = torch.empty(parts * H, dtype=torch.float32, device=hs.device)
@@ -112,7 +105,7 @@ class _NormFn(torch.autograd.Function):
             db_out = torch.empty(H, dtype=hs.dtype, device=hs.device) if db_part is not None else None
             acc = 0
         nat.check(
-            nat.lib().csb_norm_bwd(int(ctx.is_ln), dy2.data_ptr(), hs.data_ptr(), w.data_ptr(), nat.ptr(mean),
+            nat.lib().csb_norm_bwd(int(ctx.is_ln), dy2.data_ptr(), hs.data_ptr(), wd.data_ptr(), nat.ptr(mean),
                                    rstd.data_ptr(), nat.ptr(dres), dx.data_ptr(), dw_part.data_ptr(), nat.ptr(db_part),
                                    dw_out.data_ptr(), nat.ptr(db_out), int(dw_out.dtype == torch.float32), acc, rows, H,
                                    ctx.w_offset, nat.stream()),
@@ -209,7 +202,7 @@ class _RopeFn(torch.autograd.Function):
     def backward(ctx, g):
         cos, sin, p = ctx.saved_tensors
         n_heads, D, rot_dim = ctx.args
-        g = g.contiguous() if not (g.stride(2) == 1 and g.stride(0) == g.shape[1] * g.stride(1)) else g
+        g = nat.dense(g) if g.data_ptr() % 16 or not (g.stride(2) == 1 and g.stride(0) == g.shape[1] * g.stride(1)) else g
         B, S, W = g.shape
         nat.check(
             nat.lib().csb_rope(g.data_ptr(), cos.data_ptr(), sin.data_ptr(), nat.ptr(p), B * S, S, g.stride(1), n_heads,
@@ -223,7 +216,7 @@ def rope_(fused: torch.Tensor, cos, sin, pos, n_heads: int, head_dim: int, rot_d
     """Rotate the first ``n_heads`` heads of each token row of ``fused [B, S, W]`` (the q|k block of a fused
     q|k|v projection).  In place on CUDA/bf16 (the backward also rotates the incoming gradient in place)."""
     rot_dim = rot_dim or head_dim
-    if _native_ok(fused) and rot_dim % 16 == 0:
+    if _native_ok(fused) and rot_dim % 16 == 0 and fused.data_ptr() % 16 == 0:
         return _RopeFn.apply(fused, cos, sin, pos, n_heads, head_dim, rot_dim)
     B, S, W = fused.shape
     qk = fused[..., : n_heads * head_dim].reshape(B, S, n_heads, head_dim)
@@ -260,8 +253,7 @@ class _GluFn(torch.autograd.Function):
             ctx.act, ctx.shape = act, gu.shape
             return y
         I = gu.shape[-1] // 2
-        g2 = gu.reshape(-1, 2 * I)
-        g2 = g2 if g2.is_contiguous() else g2.contiguous()
+        g2 = nat.dense(gu.reshape(-1, 2 * I))
         y = torch.empty((g2.shape[0], I), dtype=gu.dtype, device=gu.device)
         nat.check(nat.lib().csb_glu_fwd(g2.data_ptr(), y.data_ptr(), g2.shape[0], I, act, nat.stream()), "csb_glu_fwd")
         ctx.save_for_backward(g2)
@@ -274,8 +266,7 @@ class _GluFn(torch.autograd.Function):
         if (host := nat.host_ops()) is not None:
             return host.glu_bwd(g2, dy, ctx.act).view(ctx.shape), None
         I = g2.shape[1] // 2
-        d2 = dy.reshape(-1, I)
-        d2 = d2 if d2.is_contiguous() else d2.contiguous()
+        d2 = nat.dense(dy.reshape(-1, I))
         dgu = torch.empty_like(g2)
         nat.check(nat.lib().csb_glu_bwd(g2.data_ptr(), d2.data_ptr(), dgu.data_ptr(), g2.shape[0], I, ctx.act, nat.stream()),
                   "csb_glu_bwd")
@@ -298,7 +289,7 @@ class _ActFn(torch.autograd.Function):
             ctx.save_for_backward(xc)
             ctx.kind = kind
             return y
-        xc = x if x.is_contiguous() else x.contiguous()
+        xc = nat.dense(x)
         y = torch.empty_like(xc)
         nat.check(nat.lib().csb_act_fwd(xc.data_ptr(), y.data_ptr(), xc.numel(), kind, nat.stream()), "csb_act_fwd")
         ctx.save_for_backward(xc)
@@ -310,7 +301,7 @@ class _ActFn(torch.autograd.Function):
         (xc,) = ctx.saved_tensors
         if (host := nat.host_ops()) is not None:
             return host.act_bwd(xc, dy, ctx.kind), None
-        d = dy if dy.is_contiguous() else dy.contiguous()
+        d = nat.dense(dy)
         dx = torch.empty_like(xc)
         nat.check(nat.lib().csb_act_bwd(xc.data_ptr(), d.data_ptr(), dx.data_ptr(), xc.numel(), ctx.kind, nat.stream()),
                   "csb_act_bwd")
@@ -330,8 +321,9 @@ class _EmbedMergeFn(torch.autograd.Function):
         T = src.numel()
         H = weight.shape[1]
         out = torch.empty((T, H), dtype=weight.dtype, device=weight.device)
-        f = feats if feats is not None else weight
-        nat.check(nat.lib().csb_gather_merge(weight.data_ptr(), f.data_ptr(), src.data_ptr(), out.data_ptr(), T, H,
+        wd = nat.dense(weight)
+        f = nat.dense(feats) if feats is not None else wd
+        nat.check(nat.lib().csb_gather_merge(wd.data_ptr(), f.data_ptr(), src.data_ptr(), out.data_ptr(), T, H,
                                              weight.shape[0], feats.shape[0] if feats is not None else 0, nat.stream()),
                   "csb_gather_merge")
         ctx.n_embed = weight.shape[0]
@@ -344,7 +336,7 @@ class _EmbedMergeFn(torch.autograd.Function):
     def backward(ctx, dout):
         (src,) = ctx.saved_tensors
         w = ctx.w_ref
-        d = dout if dout.is_contiguous() else dout.contiguous()
+        d = nat.dense(dout)
         T, H = d.shape
         dfe = torch.zeros((ctx.n_feats, H), dtype=d.dtype, device=d.device) if ctx.n_feats and ctx.needs_input_grad[1] else None
         dw_ret = None

@@ -135,6 +135,41 @@ def test_activations(form, monkeypatch):
     _same(*_both(monkeypatch, run))
 
 
+def _off(t):
+    """The same values in memory that begins two bytes behind a 16-byte boundary."""
+    return torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("op", ["rms", "ln", "act", "glu", "rope", "embed"])
+def test_operands_off_the_16_byte_grid(op, native, monkeypatch):
+    """The kernels load 16 bytes at a time: operands and gradients that begin elsewhere are copied, whichever of them it is."""
+    if not native:
+        monkeypatch.setattr(nat, "_HOST", False)
+    x, r, w, b, dy = _randn(6, 48), _randn(6, 48, seed=1), _randn(48, seed=2), _randn(48, seed=3), _randn(6, 48, seed=4)
+    cos, sin = E.rope_tables(16, 16, device="cuda")
+    src = torch.tensor([0, 3, -1, 5, -2, 1], device="cuda")
+    fns = {"rms": (lambda x, r, w, b: E.rms_norm(x, w, 1e-5, r)[0], dy), "ln": (lambda x, r, w, b: E.layer_norm(x, w, b, 1e-5, r)[0], dy),
+           "act": (lambda x, r, w, b: E.activation(x, "gelu"), dy), "glu": (lambda x, r, w, b: E.glu(x, "silu"), dy[:, :24].contiguous()),
+           "rope": (lambda x, r, w, b: E.rope_(x.view(1, 6, 48) * 1 if x.data_ptr() % 16 == 0 else _off(x.view(1, 6, 48)), cos, sin, None, 2, 16), dy.view(1, 6, 48)),
+           "embed": (lambda x, r, w, b: E.embed_merge(x, src, r), dy)}
+    fn, d = fns[op]
+    want = None
+    for which in range(6):  # none, x, r, w, b, the gradient
+        ts = _leaves([_off(t) if which == i + 1 else t for i, t in enumerate((x, r, w, b))])
+        y = fn(*ts)
+        y.backward(_off(d) if which == 5 else d.clone())
+        got = [y.detach(), *(t.grad for t in ts)]
+        want = want or got
+        for g, v in zip(got, want):
+            assert (g is None) == (v is None)
+            if op == "rope" and v is not None:  # off the grid: torch's fp32 arithmetic, rounded once as well
+                assert (g.double() - v.double()).norm() <= 2.0**-8 * v.double().norm()
+            elif v is not None:
+                assert torch.equal(g, v)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("mode", ["causal", "full", "bitfield", "shared bits", "positions", "dense"])
 @pytest.mark.parametrize("S", [60, 300])
