@@ -159,7 +159,9 @@ def linear_cross_entropy(hidden, weight, labels, ignore_index: int = -100, chunk
     n_valid = (lab != ignore_index).sum()
     if hidden.is_cuda and hidden.dtype == torch.bfloat16 and weight.shape[0] % 8 == 0 and not nat.LIBRARY_MODE:
         h2 = h2 if h2.is_contiguous() else h2.contiguous()
-        loss_sum = _LinearCEFn.apply(h2, weight, lab, ignore_index, chunk, tp_group, vocab_start, keep_logits)
+        # the kernels read one 64-bit label a row
+        assert lab.numel() == h2.shape[0] and lab.device == h2.device, f"{lab.numel()} labels on {lab.device} for {h2.shape[0]} rows on {h2.device}"
+        loss_sum = _LinearCEFn.apply(h2, weight, lab.long(), ignore_index, chunk, tp_group, vocab_start, keep_logits)
     else:
         loss_sum = _ce_torch(h2, weight, lab, ignore_index, tp_group, vocab_start)
     if reduction == "sum":
