@@ -135,6 +135,16 @@ def test_activations(form, monkeypatch):
     _same(*_both(monkeypatch, run))
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", ["weight", "bias", "residual"])
+def test_norms_of_mixed_types(which):
+    """Weights or a residual in fp32 beside bf16 activations: the torch statement (the kernels read bf16)."""
+    x, r, w, b = _randn(6, 48), _randn(6, 48, seed=1), _randn(48, seed=2), _randn(48, seed=3)
+    want = E.layer_norm(x, w, b, 1e-5, r)[0]
+    got = E.layer_norm(x, w.float() if which == "weight" else w, b.float() if which == "bias" else b, 1e-5, r.float() if which == "residual" else r)[0]
+    assert (got.double() - want.double()).norm() <= 2.0**-7 * want.double().norm()  # the sum is rounded to bf16 on one side
+
+
 def _off(t):
     """The same values in memory that begins two bytes behind a 16-byte boundary."""
     return torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)
