@@ -1176,44 +1176,40 @@ CSB_API int csb_linear_bwd(const void* dy, const void* x, const void* w, void* d
 namespace csb {
 // Tile of `groups` projections of one input in one launch (csb_gemm_cols_bf16), or one of 0 columns: separate calls.  One launch has
 // the start and the last round of one, but needs a tile whose width divides all widths, where a call for each weight takes the tile that
-// suits it and may share its contraction.  So: never where the whole would share its contraction, and only where the predicted time is
-// no longer than that of the separate calls, of which each but the first counts COLS_LAUNCH_US of the six in tile_cost (the next
-// kernel starts while the last one ends).
-// Both ways replayed in turn, 20 groups of 2 or 3 weights x 16 to 8192 tokens, 375 pairs: 0.06 % more time than the better one of
-// each pair with COLS_LAUNCH_US = 4, 0.07 % with 3, 0.1 % with 6.  Joined wherever a tile divides is 0.5 % and up to 23 % slower (4096 x
-// (4096, 128, 128) of 8192 tokens 254 us joined, 207 apart; 5120 x (5120, 640, 640) of 4575 tokens 258 / 214), always apart 64 % (1531 x 4096
-// x (4096, 1024, 1024) 53 / 81; 729 x 1152 x 3 x 1152 12 / 28).  Left: six pairs joined at 1.01 to 1.08 (7300 x 1024 x (4096, 128)
-// 61.1 / 56.8), none apart above 1.02.
-constexpr float COLS_LAUNCH_US = 4.f;
+// suits it and may share its contraction.  So: never where the whole would share its contraction; with the tile of the whole where that
+// divides; with the cheapest one that does where its predicted time is no longer than the sum of the separate calls'.
+// Both ways replayed in turn, 20 groups of 2 or 3 weights x 16 to 8192 tokens, 920 pairs: 0.09 % more time than the better one of each
+// pair in the geometric mean, none apart where one launch is more than 2 % faster, 16 joined where separate calls are (the worst 4096 x
+// (4096, 128, 128) of 4096 tokens, 123 / 111 us).  Joined wherever a tile divides is up to 28 % slower (7300 x 5120 -> 5120, 640, 640 445 us
+// joined, 348 apart; 8192 x 4096 -> 4096, 128, 128 241 / 199), always apart 60 % (1531 x 4096 -> 4096, 1024, 1024 53 / 81; 729 x 1152 -> 3
+// times 1152 12 / 28).
 static TileChoice choose_cols_tile(int M, const int* widths, int groups, int K) {
   int N = 0;
-  float apart = 6.f - COLS_LAUNCH_US;
-  for (int g = 0; g < groups; ++g) {
-    float t;
-    choose_split(M, widths[g], K, 0, 0, choose_tile(M, widths[g], K, 0, 0, false, false), false, false, &t);
-    apart += t - 6.f + COLS_LAUNCH_US;
-    N += widths[g];
-  }
+  for (int g = 0; g < groups; ++g) N += widths[g];
   auto divides = [&](int bn) {
     for (int g = 0; g < groups; ++g)
       if (widths[g] % bn) return false;
     return true;
   };
   TileChoice tc = choose_tile(M, N, K, 0, 0, false, false);
-  float together;
-  if (choose_split(M, N, K, 0, 0, tc, false, false, &together) > 1) return {0, 1};
-  if (!divides(tc.bn)) {  // the cheapest one that does
-    tc.bn = 0;
-    for (const TileCost& c : TILE_COSTS) {
-      if (!divides(c.bn) || (c.cg == 2 && (gemm_cg_choice() != 2 || M <= BM))) continue;
-      const float t = tile_cost(c, 0, M, N, K);
-      if (tc.bn == 0 || t < together) {
-        together = t;
-        tc = {c.bn, c.cg};
-      }
+  if (choose_split(M, N, K, 0, 0, tc, false, false) > 1) return {0, 1};
+  if (divides(tc.bn)) return tc;
+  float together = 0.f, apart = 0.f;
+  tc.bn = 0;
+  for (const TileCost& c : TILE_COSTS) {
+    if (!divides(c.bn) || (c.cg == 2 && (gemm_cg_choice() != 2 || M <= BM))) continue;
+    const float t = tile_cost(c, 0, M, N, K);
+    if (tc.bn == 0 || t < together) {
+      together = t;
+      tc = {c.bn, c.cg};
     }
   }
-  if (tc.bn != 0 && together > apart) tc.bn = 0;
+  for (int g = 0; tc.bn != 0 && g < groups; ++g) {
+    float t;
+    choose_split(M, widths[g], K, 0, 0, choose_tile(M, widths[g], K, 0, 0, false, false), false, false, &t);
+    apart += t;
+  }
+  if (together > apart) tc.bn = 0;
   return tc;
 }
 }  // namespace csb
