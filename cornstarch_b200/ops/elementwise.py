@@ -129,7 +129,8 @@ class _NormFn(torch.autograd.Function):
 
 def _norm(x, w, b, eps, residual, is_ln, w_offset):
     H = x.shape[-1]
-    same = w.dtype == x.dtype and (b is None or b.dtype == x.dtype) and (residual is None or residual.dtype == x.dtype)
+    dt = x.dtype
+    same = w.dtype is dt and (b is None or b.dtype is dt) and (residual is None or residual.dtype is dt)
     if _native_ok(x) and H % 8 == 0 and H <= 8192 and same:
         y, h = _NormFn.apply(x, residual, w, b, eps, is_ln, w_offset)
         return (y, h) if residual is not None else y

@@ -245,8 +245,8 @@ class _LinearFn(torch.autograd.Function):
         biases = params[n_w:]
         ctx.tp = tp
         has_bias = biases[0] is not None
-        assert not (tp is not None and tp[0] == "row" and (has_bias or n_w != 1)), "row-parallel: one weight, bias added after the reduce"
         if tp is not None and tp[0] == "row":
+            assert n_w == 1 and not has_bias, "row-parallel: one weight, bias added after the reduce"
             # row-parallel: partial products of all ranks are summed by the fused GEMM + all-reduce kernel
             x2 = _as_2d(x)
             out = torch.empty((*x.shape[:-1], weights[0].shape[0]), dtype=x.dtype, device=x.device)
