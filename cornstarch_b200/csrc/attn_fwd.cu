@@ -585,7 +585,7 @@ struct CsbAttnExtras {
 
 // Two query tiles per thread block (attn_fwd_pair_kernel) or one (attn_fwd_kernel); times are one tile against two.
 // A block of the paired kernel takes 1.3 times as long for a key tile and does twice the work, so it wins where the GPU is full:
-// 8192 tokens causal, 32 / 8 heads of 128: 776 / 455 us; 4 x 729 tokens, 16 heads of 72, full: 57 / 35 us.
+// 8192 tokens causal, 32 / 8 heads of 128: 776 / 460 us; 4 x 729 tokens, 16 heads of 72, full: 57 / 35 us.
 // - One query tile per head: its second stream idles.  Up to a chain of three key tiles the smaller set-up of the paired kernel
 //   wins on small and large grids (32 heads, 64 tokens: 8.3 / 6.6 us; 256 heads of 128, 100 queries, 256 keys: 16.7 / 16.6, 300:
 //   22.1 / 20.1, 384: 19.1 / 19.6; causal, where one key tile is in reach of 1024: 16.9 / 14.2), from four on it loses (512 keys:

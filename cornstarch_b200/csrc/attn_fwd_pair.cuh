@@ -17,8 +17,9 @@
 // power cap (990 W at 1.63 GHz).  Before, it was the MMA warp's own instructions: 90 cycles to issue an MMA that takes 64, 550 to
 // 1000 per tile for tile classes and waits.  Hence runs of MMAs (umma_f16_run_w), classes as bits in registers and one wait per
 // tile for K and V; P goes over in two halves so that P V starts beside the second half's exponentials.
-// Measured (B200, 32 / 8 heads of 128, before -> now): 8192 tokens causal 507 -> 455 us (1209 TFLOP/s), full 920 -> 830 us (1325
-// TFLOP/s); 1024 causal 23.4 -> 21.1 us; 4 x 729 tokens, 16 heads of 72: 35.7 -> 34.7 us.
+// Measured (B200, 32 / 8 heads of 128, before -> now): 8192 tokens causal 507 -> 460 us (1195 TFLOP/s), full 920 -> 837 to 866 us (1310 to
+// 1270 TFLOP/s, by the power cap); 1024 causal 23.4 -> 21.2 us; 4 x 729 tokens, 16 heads of 72: 35.7 -> 35.2 us.  1.2 % of it are two
+// waits for soundness: one verdict per warp (mbar_wait_abort_w), and tcgen05.wait::st between a P and its correction.
 //
 // Hand-overs per stream and tile: s_full (MMA -> softmax) and p_full, one per half of the keys (softmax -> MMA), strictly
 // alternating, so no parity wait can be two phases behind.  S(next) of a stream is issued after P V of its current tile, whose
