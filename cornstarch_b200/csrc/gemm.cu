@@ -275,6 +275,20 @@ __device__ __forceinline__ void arrive_tmem_empty(uint64_t* bar, bool remote_lea
   else mbar_arrive(bar);
 }
 
+// Whether all four epilogue warps say `ok` (barrier 2, which their slabs use as well).
+__device__ __forceinline__ bool epilogue_agrees(bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, 2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"(ok ? 1u : 0u)
+      : "memory");
+  return all != 0;
+}
+
 // What the epilogue does to a tile besides storing it.  Forms of the kernel, not branches: code for a bias in the plain one, untaken, costs
 // calls of few tokens 1.5 % (90 calls with 256 columns 3.3 %, weight gradients of 77 tokens up to 6 %).
 // EPI_CE: besides storing them (bf16), take each row's maximum over the tile's columns and the sum of exp(x - maximum) of the ROUNDED values
@@ -651,7 +665,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       m_blk = m_blk * CG + cta_rank;
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
-      if (!mbar_wait_abort_w(&tmem_full[acc], acc_ph, abort_flag)) {
+      // one verdict for the four warps: they meet in named barriers from here on, and a warp that gave up alone would be missing there
+      if (!epilogue_agrees(mbar_wait_abort_w(&tmem_full[acc], acc_ph, abort_flag))) {
         if (lane == 0) atomicExch(p.status, ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
         ok = false;
